@@ -137,6 +137,24 @@ def lib() -> C.CDLL:
     return L
 
 
+_front = None
+
+
+def front():
+    """The native front end of the operators (``csrc/front.cpp``), bound to the entries of the library :func:`lib` loaded."""
+    global _front
+    if _front is None:
+        L = lib()
+        try:
+            from . import _front as module
+        except ImportError as e:
+            raise ImportError("gcnasm_b200/_front.so is missing or does not load: build it with `python -m gcnasm_b200.build`. "
+                              "There is no fallback for these operators.") from e
+        module.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in EXPORTS})
+        _front = module
+    return _front
+
+
 def check(code: int, where: str) -> None:
     if code != 0:
         raise B200Error(code, where)

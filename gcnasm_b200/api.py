@@ -17,6 +17,13 @@ from . import _lib as L
 from ._lib import GemmArgs, check, lib
 
 _FP8 = (torch.uint8, torch.float8_e4m3fn)
+_bound = None              # the native front end, once the library is loaded
+
+
+def front():
+    global _bound
+    _bound = L.front()
+    return _bound
 
 
 def _stream() -> C.c_void_p:
@@ -52,97 +59,16 @@ def _as_u8(t: torch.Tensor, what: str) -> torch.Tensor:
     return t.view(torch.uint8)
 
 
-def _out_code(dtype) -> int:
-    if dtype == torch.bfloat16:
-        return L.OUT_BF16
-    if dtype == torch.float32:
-        return L.OUT_F32
-    raise TypeError("output dtype must be torch.bfloat16 or torch.float32")
-
-
 def _gemm(a, b, *, n=None, sfa=None, sfb=None, scale_a=None, scale_b=None, scale_mode=L.SCALE_NONE,
           b_layout=L.B_NK_ROWMAJOR, out=None, out_dtype=torch.bfloat16, tile=L.TILE_AUTO, simple=False, inputs_ready=False,
-          batch_ready=None, batch_epoch=0):
-    a = _as_u8(a, "A")
-    b = _as_u8(b, "B")
-    _same_device(a, b, sfa, sfb, scale_a, scale_b, out, batch_ready)
-    squeeze = a.dim() == 2
-    if squeeze:
-        a = a.unsqueeze(0)
-    batch, m, k = a.shape
-    if a.stride(2) != 1:
-        raise ValueError("A must be K-contiguous")
-    # a 2-D B (or scale tensor) given with a batched A is ONE operand shared by every batch (batch stride 0)
-    b_shared = batch > 1 and b_layout == L.B_NK_ROWMAJOR and b.dim() == 2
-    if b_layout == L.B_NK_ROWMAJOR:
-        if b.dim() == 2:
-            b = b.unsqueeze(0)
-        if (not b_shared and b.shape[0] != batch) or b.shape[2] != k or b.stride(2) != 1:
-            raise ValueError("B must be [batch, N, K] (or [N, K], shared by all batches), K-contiguous, matching A")
-        n = b.shape[1]
-        stride_b, stride_b_batch = b.stride(1), (0 if b_shared else b.stride(0))
-    else:
-        if n is None:
-            raise ValueError("flat B needs n=")
-        if not b.is_contiguous() or b.numel() != batch * n * k:
-            raise ValueError("flat B must be a contiguous image of batch*N*K bytes")
-        stride_b, stride_b_batch = n, n * k       # the reference sets stride_b = N (flatmm_a8w8_gfx950.cc:765)
-    if out is None:
-        out = torch.empty((batch, m, n), dtype=out_dtype, device=a.device)
-    else:
-        if out.dim() == 2:
-            out = out.unsqueeze(0)
-        if out.shape != (batch, m, n) or out.stride(2) != 1:
-            raise ValueError("out must be [batch, M, N], N-contiguous")
-    args = GemmArgs()
-    args.ptr_a, args.ptr_b, args.ptr_c = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.m, args.n, args.k, args.batch = m, n, k, batch
-    args.stride_a, args.stride_b, args.stride_c = a.stride(1), stride_b, out.stride(1)
-    args.stride_a_batch, args.stride_b_batch, args.stride_c_batch = a.stride(0), stride_b_batch, out.stride(0)
-    keep = [a, b, out]
-    if scale_mode == L.SCALE_BLOCK:
-        if sfa.dim() == 2:
-            sfa = sfa.unsqueeze(0)
-        if sfb.dim() == 2:
-            sfb = sfb.unsqueeze(0)
-        if sfa.dtype != torch.float32 or sfb.dtype != torch.float32:
-            raise TypeError("block scales are float32")
-        if sfa.shape != (batch, k // 128, m) or sfb.shape != (1 if b_shared else batch, n // 128, k // 128):
-            raise ValueError("SFA must be [batch, K/128, M] and SFB [batch, N/128, K/128] ([N/128, K/128] with a shared B)")
-        if sfa.stride(2) != 1 or sfb.stride(2) != 1:
-            raise ValueError("scale tensors must be contiguous in their last dimension")
-        args.ptr_sfa, args.ptr_sfb = sfa.data_ptr(), sfb.data_ptr()
-        args.stride_sfa, args.stride_sfb = sfa.stride(1), sfb.stride(1)
-        args.stride_sfa_batch, args.stride_sfb_batch = sfa.stride(0), (0 if b_shared else sfb.stride(0))
-        keep += [sfa, sfb]
-    elif scale_mode == L.SCALE_MX:
-        need_a, need_b = lib().b200_mx_sf_bytes(m, k), lib().b200_mx_sf_bytes(n, k)
-        sfa = sfa.view(torch.uint8).reshape(batch, -1)
-        sfb = sfb.view(torch.uint8).reshape(batch, -1)
-        if sfa.shape[1] != need_a or sfb.shape[1] != need_b or not sfa.is_contiguous() or not sfb.is_contiguous():
-            raise ValueError("MX scales must be the relayouted atom images (see mx_sf_relayout)")
-        args.ptr_sfa, args.ptr_sfb = sfa.data_ptr(), sfb.data_ptr()
-        args.stride_sfa_batch, args.stride_sfb_batch = need_a, need_b
-        keep += [sfa, sfb]
-    elif scale_mode == L.SCALE_TENSOR:
-        for name, s in (("ptr_scale_a", scale_a), ("ptr_scale_b", scale_b)):
-            if s is not None:
-                if s.dtype != torch.float32 or not s.is_cuda or s.numel() != 1:
-                    raise TypeError("per-tensor scales are 1-element float32 CUDA tensors")
-                setattr(args, name, s.data_ptr())
-                keep.append(s)
-    args.scale_mode, args.b_layout = scale_mode, b_layout
-    args.out_dtype, args.tile_hint = _out_code(out.dtype), tile
-    args.flags = L.GEMM_INPUTS_READY if inputs_ready else 0
-    if batch_ready is not None:
-        if batch_ready.dtype != torch.int32 or batch_ready.numel() < batch or not batch_ready.is_contiguous():
-            raise ValueError("batch_ready must be a contiguous int32 CUDA tensor with one word per batch")
-        args.flags |= L.GEMM_BATCH_READY
-        args.ptr_batch_ready, args.batch_epoch = batch_ready.data_ptr(), int(batch_epoch)
-        keep.append(batch_ready)
-    fn = lib().b200_gemm_a8w8_simple if simple else lib().b200_gemm_a8w8
-    check(fn(C.byref(args), _stream()), "b200_gemm_a8w8_simple" if simple else "b200_gemm_a8w8")
-    return out[0] if squeeze else out
+          batch_ready=None, batch_epoch=0, where="b200_gemm_a8w8"):
+    """Checks, output allocation, argument block and launch happen in the native front end (``csrc/front.cpp``): the same
+    work costs more in the interpreter than a small GEMM takes on the GPU."""
+    r = (_bound or front()).gemm(a, b, out, sfa, sfb, scale_a, scale_b, batch_ready, n, scale_mode, b_layout, out_dtype, tile,
+                                 L.GEMM_INPUTS_READY if inputs_ready else 0, batch_epoch, simple)
+    if type(r) is int:
+        check(r, where + "_simple" if simple else where)
+    return r
 
 
 # ---- operators ---------------------------------------------------------------------------------
@@ -286,34 +212,18 @@ def quantize_mx32(x):
 def quantize_act_bf16_1x128(x, q=None, sfa=None):
     """Fused activation quantiser: bf16 [M,K] (rows may be strided) -> (q [M,K] uint8, sfa [K/128, M] fp32) in one
     pass.  `q` / `sfa` may be preallocated views (e.g. slices of a broadcast buffer); q rows may be strided."""
-    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride(1) != 1:
-        raise ValueError("x must be a 2-D bf16 tensor with unit column stride")
-    _same_device(x, q, sfa)
-    m, k = x.shape
-    if q is None:
-        q = torch.empty((m, k), dtype=torch.uint8, device=x.device)
-    if sfa is None:
-        sfa = torch.empty((k // 128, m), dtype=torch.float32, device=x.device)
-    if q.shape != (m, k) or q.dtype != torch.uint8 or q.stride(1) != 1:
-        raise ValueError("q must be a [M,K] uint8 tensor with unit column stride")
-    if sfa.shape != (k // 128, m) or sfa.dtype != torch.float32 or sfa.stride(1) != 1:
-        raise ValueError("sfa must be a [K/128, M] fp32 tensor with unit column stride")
-    check(lib().b200_quantize_act_bf16_1x128(x.data_ptr(), x.stride(0), q.data_ptr(), q.stride(0), sfa.data_ptr(),
-                                             sfa.stride(0) if k > 128 else m, m, k, _stream()), "b200_quantize_act_bf16_1x128")
-    return q, sfa
+    r = (_bound or front()).act_quant_1x128(x, q, sfa)
+    if type(r) is int:
+        check(r, "b200_quantize_act_bf16_1x128")
+    return r
 
 
 def quantize_act_bf16_mx32(x):
     """Fused MX activation quantiser: bf16 [R,K] -> (q [R,K] uint8, scale atoms for the MX GEMM) in one pass."""
-    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.stride(1) != 1:
-        raise ValueError("x must be a 2-D bf16 tensor with unit column stride")
-    _same_device(x)
-    r, k = x.shape
-    q = torch.empty((r, k), dtype=torch.uint8, device=x.device)
-    atoms = torch.empty(lib().b200_mx_sf_bytes(r, k), dtype=torch.uint8, device=x.device)
-    check(lib().b200_quantize_act_bf16_mx32(x.data_ptr(), x.stride(0), q.data_ptr(), q.stride(0), atoms.data_ptr(), r, k,
-                                            _stream()), "b200_quantize_act_bf16_mx32")
-    return q, atoms
+    r = (_bound or front()).act_quant_mx32(x)
+    if type(r) is int:
+        check(r, "b200_quantize_act_bf16_mx32")
+    return r
 
 
 # ---- a16w16 siblings (bf16 operands) ----------------------------------------------------------------
@@ -324,52 +234,9 @@ def gemm_a16w16(a, b, scale_a=None, scale_b=None, *, n=None, flat=False, out=Non
     image made by :func:`shuffle_b_bf16` (then ``n=`` is required)."""
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
         raise TypeError("A and B must be torch.bfloat16")
-    _same_device(a, b, scale_a, scale_b, out)
-    squeeze = a.dim() == 2
-    if squeeze:
-        a = a.unsqueeze(0)
-    batch, m, k = a.shape
-    if a.stride(2) != 1:
-        raise ValueError("A must be K-contiguous")
-    if not flat:
-        if b.dim() == 2:
-            b = b.unsqueeze(0)
-        if b.shape[0] != batch or b.shape[2] != k or b.stride(2) != 1:
-            raise ValueError("B must be [batch, N, K], K-contiguous, matching A")
-        n = b.shape[1]
-        stride_b, stride_b_batch = b.stride(1), b.stride(0)
-    else:
-        if n is None:
-            raise ValueError("flat B needs n=")
-        if not b.is_contiguous() or b.numel() != batch * n * k:
-            raise ValueError("flat B must be a contiguous image of batch*N*K values")
-        stride_b, stride_b_batch = n, n * k
-    if out is None:
-        out = torch.empty((batch, m, n), dtype=out_dtype, device=a.device)
-    else:
-        if out.dim() == 2:
-            out = out.unsqueeze(0)
-        if out.shape != (batch, m, n) or out.stride(2) != 1:
-            raise ValueError("out must be [batch, M, N], N-contiguous")
-    args = GemmArgs()
-    args.ptr_a, args.ptr_b, args.ptr_c = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.m, args.n, args.k, args.batch = m, n, k, batch
-    args.stride_a, args.stride_b, args.stride_c = a.stride(1), stride_b, out.stride(1)
-    args.stride_a_batch, args.stride_b_batch, args.stride_c_batch = a.stride(0), stride_b_batch, out.stride(0)
-    keep = [a, b, out]
-    mode = L.SCALE_NONE
-    if scale_a is not None or scale_b is not None:
-        mode = L.SCALE_TENSOR
-        for name, sc in (("ptr_scale_a", scale_a), ("ptr_scale_b", scale_b)):
-            if sc is not None:
-                if sc.dtype != torch.float32 or not sc.is_cuda or sc.numel() != 1:
-                    raise TypeError("per-tensor scales are 1-element float32 CUDA tensors")
-                setattr(args, name, sc.data_ptr())
-                keep.append(sc)
-    args.scale_mode, args.b_layout = mode, (L.B_FLAT_16x16 if flat else L.B_NK_ROWMAJOR)
-    args.out_dtype, args.tile_hint = _out_code(out.dtype), tile
-    check(lib().b200_gemm_a16w16(C.byref(args), _stream()), "b200_gemm_a16w16")
-    return out[0] if squeeze else out
+    mode = L.SCALE_TENSOR if (scale_a is not None or scale_b is not None) else L.SCALE_NONE
+    return _gemm(a, b, n=n, scale_a=scale_a, scale_b=scale_b, scale_mode=mode, out=out, out_dtype=out_dtype, tile=tile,
+                 b_layout=L.B_FLAT_16x16 if flat else L.B_NK_ROWMAJOR, where="b200_gemm_a16w16")
 
 
 def shuffle_b_bf16(b: torch.Tensor, src: str = "kn") -> torch.Tensor:

@@ -14,6 +14,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 DRIVERS = os.path.join(PKG, "drivers")
 LIB = os.path.join(PKG, "libb200gemm.so")
+FRONT = os.path.join(PKG, "_front.so")
 BIN = os.path.join(PKG, "bin")
 
 NVCC_FLAGS = [
@@ -45,14 +46,35 @@ def _newer(target: str, sources) -> bool:
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    srcs = [os.path.join(CSRC, f) for f in sorted(os.listdir(CSRC))] + [os.path.join(ROOT, "include", "b200gemm.h")]
+    srcs = [os.path.join(CSRC, f) for f in sorted(os.listdir(CSRC)) if not f.endswith(".cpp")]
+    srcs.append(os.path.join(ROOT, "include", "b200gemm.h"))
     if force or _newer(LIB, srcs):
         cmd = [_nvcc(), *NVCC_FLAGS, "-ccbin", _host_cxx(), "-shared", "-o", LIB, os.path.join(CSRC, "b200gemm.cu")]
         if verbose:
             cmd.insert(1, "-Xptxas")
             cmd.insert(2, "-v")
         subprocess.check_call(cmd)
+    build_front(force)
     return LIB
+
+
+def build_front(force: bool = False) -> str:
+    """The Python front end of the per-call operators (a CPython extension on torch's C++ tensors)."""
+    src = os.path.join(CSRC, "front.cpp")
+    if force or _newer(FRONT, [src, os.path.join(ROOT, "include", "b200gemm.h")]):
+        import sysconfig
+
+        import torch
+
+        troot = os.path.dirname(torch.__file__)
+        nvcc_root = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+        subprocess.check_call([
+            _host_cxx(), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-isystem", os.path.join(troot, "include"), "-isystem", os.path.join(troot, "include", "torch", "csrc", "api", "include"),
+            "-isystem", os.path.join(nvcc_root, "include"), "-isystem", sysconfig.get_paths()["include"], src, "-o", FRONT,
+            "-L", os.path.join(troot, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+        ])
+    return FRONT
 
 
 def build_drivers(force: bool = False) -> list:

@@ -247,3 +247,22 @@ def test_operands_must_share_the_current_device(monkeypatch):
     cpu.is_cuda = False
     with pytest.raises(ValueError, match="CUDA tensors"):
         api._same_device(cpu)
+
+
+@pytest.mark.parametrize("a,b,error,match", [
+    ((16, 16, "uint8"), (16, 16, "uint8"), ValueError, "CUDA tensors"),
+    ((16, 16, "float32"), (16, 16, "uint8"), TypeError, "E4M3"),
+    ((16, 16, "bfloat16"), (16, 16, "uint8"), TypeError, "bfloat16"),
+    (None, (16, 16, "uint8"), TypeError, "A must be a tensor"),
+])
+def test_front_end_refuses_misuse(native, a, b, error, match):
+    """The native front end of the operators raises what the operators document, before anything is launched."""
+    import torch
+
+    from gcnasm_b200 import api
+
+    make = lambda spec: spec and torch.zeros(spec[:2], dtype=getattr(torch, spec[2]))
+    with pytest.raises(error, match=match):
+        api._gemm(make(a), make(b))
+    with pytest.raises(ValueError, match="2-D bf16"):
+        api.quantize_act_bf16_1x128(torch.zeros(2, 128))
