@@ -311,133 +311,212 @@ __global__ void __launch_bounds__(1024) membw_copy_kernel(const uint4* __restric
 
 // x / s, correctly rounded, for many x and one s.  With r = RN(1/s): q0 = RN(x*r), rem = x - q0*s (exact in an
 // FMA), q = RN(q0 + rem*r) is the correctly rounded quotient when nothing overflows or loses bits to underflow
-// (Markstein).  `fast` (uniform per group) says s is a normal number of moderate size; the callers guarantee
+// (Markstein).  The fast path is for an s that is a normal number of moderate size; the callers guarantee
 // |x| <= 448*s*(1+2^-23), and a quotient too small to be exact becomes a zero byte either way.  Everything else takes
 // the IEEE division.
-__device__ __forceinline__ float div_by_scale(float x, float s, float r, bool fast) {
-    if (fast) {
+__device__ __forceinline__ bool scale_is_moderate(float s) { return s >= 0x1p-100f && s <= 0x1p100f; }
+__device__ __forceinline__ float div_by_scale(float x, float s, float r) {
+    if (scale_is_moderate(s)) {
         const float q0 = __fmul_rn(x, r);
         return __fmaf_rn(__fmaf_rn(-q0, s, x), r, q0);
     }
     return __fdiv_rn(x, s);
 }
+// ... and its fast path for two values, with s already negated
+__device__ __forceinline__ unsigned long long div2_by_scale(unsigned long long x, unsigned long long neg_s, unsigned long long r) {
+    const unsigned long long q0 = fmul2(x, r);
+    return ffma2(ffma2(q0, neg_s, x), r, q0);
+}
+
+// |max| of two bf16 pairs; the result's sign bits are arbitrary.  A NaN gives way to the other operand.
+__device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+// largest magnitude of the eight bf16 values of a 16-byte piece, NaNs ignored (starts from 0, as the fp32 quantisers do)
+__device__ __forceinline__ uint32_t bf16x8_absmax(const uint4& w) {
+    return bf16x2_absmax(bf16x2_absmax(bf16x2_absmax(bf16x2_absmax(0u, w.x), w.y), w.z), w.w);
+}
+__device__ __forceinline__ float bf16x2_top(uint32_t m2) {
+    return fmaxf(__uint_as_float((m2 & 0x7FFFu) << 16), __uint_as_float(m2 & 0x7FFF0000u));
+}
+__device__ __forceinline__ unsigned long long bf16x2_widen(uint32_t w) {
+    return pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+__device__ __forceinline__ uint32_t f32x2x2_to_e4m3x4(unsigned long long p, unsigned long long q) {
+    float a, b, c, d;
+    unpack_f32x2(p, a, b);
+    unpack_f32x2(q, c, d);
+    return f32x4_to_e4m3x4(a, b, c, d);
+}
 
 // Fused activation quantiser: bf16 [M][K] (row pitch ldx) -> e4m3 [M][K] (row pitch ldq) + fp32 scales in the
-// GEMM's [K/128][M] layout (group pitch stride_sfa), one pass.  A block covers 32 rows x 16 K groups; warp w walks
-// the 32 rows of groups g0+2w and g0+2w+1 (512 contiguous bytes per row: lanes 0-15 the first group, 16-31 the
-// second, 16 bytes = 8 values per lane) and lane r keeps the two scales of row r, so that the scales leave as two
-// 128-byte lines per warp.  Same arithmetic as the fp32 quantiser: scale = amax/448 (1 for an all-zero group),
-// q = e4m3(x / scale), both divisions correctly rounded.
+// GEMM's [K/128][M] layout (group pitch stride_sfa), one pass.  Same arithmetic as the fp32 quantiser: scale = amax/448
+// (1 for an all-zero group), q = e4m3(x / scale), both divisions correctly rounded.
+//
+// HBM bounds the large sizes, the length of one warp's chain the small ones.  A warp takes R rows of two neighbouring K
+// groups (512 contiguous bytes per row, 16 per lane) and has the loads of all its rows in flight at once; lanes r and
+// 16+r then hold the amax of row r's two groups, so the two divisions and the reciprocal are done once per warp and not
+// once per row.  The launcher takes R = 4 when that still gives every SM eight warps, else R = 1 (16384 x 8192: R = 1
+// 104 us, 2 78, 4 68, 8 102; below 1000 x 4096 no difference between 1 and 4).  Back to back, against one warp walking 32
+// rows in eight dependent rounds: 64 x 7168 12.2 -> 1.6 us, 333 x 2048 12.3 -> 1.7, 4096 x 2048 15.2 -> 7.3,
+// 16384 x 8192 77 -> 68 (6.0 TB/s).
+template <int R>
 __global__ void __launch_bounds__(256) act_quant_bf16_1x128_kernel(const uint16_t* __restrict__ x, long long ldx,
                                                                    uint8_t* __restrict__ q, long long ldq,
                                                                    float* __restrict__ sfa, long long stride_sfa,
-                                                                   long long M, long long K) {
-    const long long KG = K >> 7;
+                                                                   long long M, int KG) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long gpair = (static_cast<long long>(blockIdx.x) * 8 + warp) * 2;     // first of the warp's two groups
-    const long long row0 = static_cast<long long>(blockIdx.y) * 32;
-    if (gpair >= KG) return;
-    const bool live = gpair + (lane >> 4) < KG;                  // the second group may not exist
-    const int nrows = (M - row0) < 32 ? static_cast<int>(M - row0) : 32;
-    float my_a = 1.0f, my_b = 1.0f;
-#pragma unroll 1
-    for (int r0 = 0; r0 < nrows; r0 += 4) {
-        uint4 raw[4];
+    const unsigned pairs = static_cast<unsigned>(KG + 1) >> 1;
+    const unsigned wid = blockIdx.x * 8 + warp;
+    const unsigned rb = wid / pairs;
+    const int g = static_cast<int>(wid - rb * pairs) * 2 + (lane >> 4);      // this half-warp's K group
+    const long long row0 = static_cast<long long>(rb) * R;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (row0 >= M) return;
+    const bool live = g < KG;                                    // the second group may not exist
+    const int nrows = (M - row0) < R ? static_cast<int>(M - row0) : R;
+    const uint16_t* src = x + row0 * ldx + static_cast<long long>(g) * 128 + (lane & 15) * 8;
+    uint4 raw[R];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            raw[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (live && r0 + i < nrows)
-                raw[i] = __ldg(reinterpret_cast<const uint4*>(x + (row0 + r0 + i) * ldx + gpair * 128) + lane);
+    for (int i = 0; i < R; ++i) {
+        raw[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (live && i < nrows) raw[i] = __ldcs(reinterpret_cast<const uint4*>(src + i * ldx));
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        uint32_t m2 = bf16x8_absmax(raw[i]);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) m2 = bf16x2_absmax(m2, __shfl_xor_sync(0xFFFFFFFFu, m2, o));
+        if ((lane & 15) == i) mine = m2;
+    }
+    const float m = bf16x2_top(mine);
+    const float sc = m > 0.0f ? __fdiv_rn(m, 448.0f) : 1.0f;
+    const float rc = __frcp_rn(sc);
+    if (live && (lane & 15) < nrows) sfa[g * stride_sfa + row0 + (lane & 15)] = sc;
+    uint8_t* dst = q + row0 * ldq + static_cast<long long>(g) * 128 + (lane & 15) * 8;
+    auto put = [&](int i, auto divide) {
+        const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+        const uint2 out = make_uint2(f32x2x2_to_e4m3x4(divide(w[0]), divide(w[1])), f32x2x2_to_e4m3x4(divide(w[2]), divide(w[3])));
+        if (live && i < nrows) *reinterpret_cast<uint2*>(dst + i * ldq) = out;
+    };
+    if (__all_sync(0xFFFFFFFFu, scale_is_moderate(sc))) {        // two values at a time
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float s = __shfl_sync(0xFFFFFFFFu, -sc, (lane & 16) + i), r = __shfl_sync(0xFFFFFFFFu, rc, (lane & 16) + i);
+            const unsigned long long s2 = pack_f32x2(s, s), r2 = pack_f32x2(r, r);
+            put(i, [&](uint32_t w) { return div2_by_scale(bf16x2_widen(w), s2, r2); });
         }
+    } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (r0 + i >= nrows) break;                                  // uniform across the warp
-            const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-            float v[8];
-            float m = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[2 * j] = __uint_as_float(w[j] << 16);
-                v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
-                m = fmaxf(m, fmaxf(fabsf(v[2 * j]), fabsf(v[2 * j + 1])));
-            }
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-            const float sc = m > 0.0f ? __fdiv_rn(m, 448.0f) : 1.0f;     // one per half-warp
-            const float rc = __frcp_rn(sc);
-            const bool fast = sc >= 0x1p-100f && sc <= 0x1p100f;
-            auto dv = [&](float val) { return div_by_scale(val, sc, rc, fast); };
-            uint2 out;
-            out.x = f32x4_to_e4m3x4(dv(v[0]), dv(v[1]), dv(v[2]), dv(v[3]));
-            out.y = f32x4_to_e4m3x4(dv(v[4]), dv(v[5]), dv(v[6]), dv(v[7]));
-            if (live) reinterpret_cast<uint2*>(q + (row0 + r0 + i) * ldq + gpair * 128)[lane] = out;
-            const float sa = __shfl_sync(0xFFFFFFFFu, sc, 0), sb = __shfl_sync(0xFFFFFFFFu, sc, 16);
-            if (lane == r0 + i) {
-                my_a = sa;
-                my_b = sb;
-            }
+        for (int i = 0; i < R; ++i) {
+            const float s = __shfl_sync(0xFFFFFFFFu, sc, (lane & 16) + i), r = __shfl_sync(0xFFFFFFFFu, rc, (lane & 16) + i);
+            put(i, [&](uint32_t w) {
+                const float a = __uint_as_float(w << 16), b = __uint_as_float(w & 0xFFFF0000u);
+                return pack_f32x2(div_by_scale(a, s, r), div_by_scale(b, s, r));
+            });
         }
     }
-    if (lane < nrows) {
-        sfa[gpair * stride_sfa + row0 + lane] = my_a;
-        if (gpair + 1 < KG) sfa[(gpair + 1) * stride_sfa + row0 + lane] = my_b;
-    }
+}
+
+// E8M0 byte of a 32-wide block from its amax (> 0): floor(log2(amax)) - 8 + 127, clamped to [0, 254].  The exponent field IS
+// floor(log2) + 127 for normal numbers, and everything smaller clamps to 0.  An infinite amax takes the largest byte.
+__device__ __forceinline__ int mx_scale_byte(float m) {
+    const int e = static_cast<int>(__float_as_uint(m) >> 23);
+    return e == 255 ? 254 : (e < 8 ? 0 : e - 8);
+}
+// 2^-(byte - 127): a normal number for every finite amax (byte <= 246)
+__device__ __forceinline__ float mx_inv_scale(int byte) {
+    return __uint_as_float(byte == 254 ? 0x00400000u : static_cast<uint32_t>(254 - byte) << 23);
 }
 
 // Fused MX activation quantiser: bf16 [rows][K] -> e4m3 [rows][K] + E8M0 scales written straight into the
 // tensor-core atom order [K/128][ceil(rows/128)][32][4][4] (what quant_mx32 followed by mx_sf_relayout produce).
-// Same block shape as above: warp w owns K group g0+w of the block's 32 rows; eight lanes share one 32-wide
-// scale block; lane r keeps the four scale bytes of row r as one word.  Rows of the last atom beyond `rows`
-// get 127 (scale 1.0).  grid.y covers ceil(rows/128)*4 row blocks.
+// Rows of the last atom beyond `rows` get 127 (scale 1.0).
+//
+// Bound and shape as above: a warp takes four rows of two neighbouring K groups, all loads in flight at once; four lanes
+// share a 32-wide block.  (One warp walking 32 rows, ilogbf / scalbnf per value: 8192 x 8192 took 75 us back to
+// back, now 37; 64 x 7168 14.0, now 1.7.)  kAligned: x is 16-byte and q 8-byte aligned, pitches
+// included; the entry also takes 8- and 4-byte aligned ones, which move in two halves.
+template <bool kAligned>
 __global__ void __launch_bounds__(256) act_quant_bf16_mx32_kernel(const uint16_t* __restrict__ x, long long ldx,
                                                                   uint8_t* __restrict__ q, long long ldq,
-                                                                  uint32_t* __restrict__ atoms, long long rows,
-                                                                  long long K) {
-    const long long KG = K >> 7;
+                                                                  uint32_t* __restrict__ atoms, long long rows, int KG) {
     const long long R128 = (rows + 127) >> 7;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long g = static_cast<long long>(blockIdx.x) * 8 + warp;
-    const long long row0 = static_cast<long long>(blockIdx.y) * 32;
-    if (g >= KG) return;
-    const int nrows = row0 >= rows ? 0 : ((rows - row0) < 32 ? static_cast<int>(rows - row0) : 32);
-    uint32_t my_word = 0x7F7F7F7Fu;
-#pragma unroll 1
-    for (int r0 = 0; r0 < nrows; r0 += 4) {
-        uint2 raw[4];
+    const unsigned pairs = static_cast<unsigned>(KG + 1) >> 1;
+    const unsigned wid = blockIdx.x * 8 + warp;
+    const unsigned rb = wid / pairs;                                         // rows 4 * rb .. 4 * rb + 3
+    const int g = static_cast<int>(wid - rb * pairs) * 2 + (lane >> 4);
+    const long long row0 = static_cast<long long>(rb) * 4;
+    pdl_launch_dependents();
+    pdl_wait();
+    if ((rb >> 5) >= R128) return;
+    const bool live = g < KG;
+    const long long col = static_cast<long long>(g) * 128 + (lane & 15) * 8;
+    uint4 raw[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            raw[i] = make_uint2(0u, 0u);
-            if (r0 + i < nrows) raw[i] = __ldg(reinterpret_cast<const uint2*>(x + (row0 + r0 + i) * ldx + g * 128) + lane);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (r0 + i >= nrows) break;                                  // uniform across the warp
-            const float a = __uint_as_float(raw[i].x << 16), b = __uint_as_float(raw[i].x & 0xFFFF0000u);
-            const float c = __uint_as_float(raw[i].y << 16), d = __uint_as_float(raw[i].y & 0xFFFF0000u);
-            float m = fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(d)));
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-            uint32_t packed;
-            int byte = 0;
-            if (!(m > 0.0f)) {
-                packed = ((__float_as_uint(a) >> 24) & 0x80u) | (((__float_as_uint(b) >> 24) & 0x80u) << 8) |
-                         (((__float_as_uint(c) >> 24) & 0x80u) << 16) | (((__float_as_uint(d) >> 24) & 0x80u) << 24);
+    for (int i = 0; i < 4; ++i) {
+        const long long row = row0 + i;
+        raw[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (live && row < rows) {
+            const uint16_t* src = x + row * ldx + col;
+            if (kAligned) {
+                raw[i] = __ldcs(reinterpret_cast<const uint4*>(src));
             } else {
-                byte = ilogbf(m) - 8 + 127;
-                byte = byte < 0 ? 0 : (byte > 254 ? 254 : byte);
-                const int e = byte - 127;
-                packed = f32x4_to_e4m3x4(scalbnf(a, -e), scalbnf(b, -e), scalbnf(c, -e), scalbnf(d, -e));
+                const uint2 lo = __ldcs(reinterpret_cast<const uint2*>(src)), hi = __ldcs(reinterpret_cast<const uint2*>(src) + 1);
+                raw[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
             }
-            reinterpret_cast<uint32_t*>(q + (row0 + r0 + i) * ldq + g * 128)[lane] = packed;
-            const uint32_t word = static_cast<uint32_t>(__shfl_sync(0xFFFFFFFFu, byte, 0)) |
-                                  (static_cast<uint32_t>(__shfl_sync(0xFFFFFFFFu, byte, 8)) << 8) |
-                                  (static_cast<uint32_t>(__shfl_sync(0xFFFFFFFFu, byte, 16)) << 16) |
-                                  (static_cast<uint32_t>(__shfl_sync(0xFFFFFFFFu, byte, 24)) << 24);
-            if (lane == r0 + i) my_word = word;
         }
     }
-    const long long row = row0 + lane;                                   // row0 is a multiple of 32
-    atoms[(g * R128 + (row >> 7)) * 128 + lane * 4 + ((row & 127) >> 5)] = my_word;
+    float m[4];
+    bool plain = true;                                                       // no block of zeros among these rows
+    uint32_t my_word = 0x7F7F7F7Fu;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t m2 = bf16x8_absmax(raw[i]);
+        m2 = bf16x2_absmax(m2, __shfl_xor_sync(0xFFFFFFFFu, m2, 2));
+        m2 = bf16x2_absmax(m2, __shfl_xor_sync(0xFFFFFFFFu, m2, 1));
+        m[i] = bf16x2_top(m2);
+        plain = plain && m[i] > 0.0f;
+        uint32_t word = static_cast<uint32_t>(mx_scale_byte(m[i])) << (8 * ((lane >> 2) & 3));
+        word |= __shfl_xor_sync(0xFFFFFFFFu, word, 4);
+        word |= __shfl_xor_sync(0xFFFFFFFFu, word, 8);
+        if ((lane & 15) == i && row0 + i < rows) my_word = word;
+    }
+    auto put = [&](int i, bool zeros) {
+        if (!live || row0 + i >= rows) return;
+        const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+        const float inv = mx_inv_scale(mx_scale_byte(m[i]));
+        const unsigned long long inv2 = pack_f32x2(inv, inv);
+        uint2 out;
+        out.x = f32x2x2_to_e4m3x4(fmul2(bf16x2_widen(w[0]), inv2), fmul2(bf16x2_widen(w[1]), inv2));
+        out.y = f32x2x2_to_e4m3x4(fmul2(bf16x2_widen(w[2]), inv2), fmul2(bf16x2_widen(w[3]), inv2));
+        if (zeros) {                                                         // nothing but zeros (or NaNs): sign bits only
+            out.x = __byte_perm(w[0], w[1], 0x7531) & 0x80808080u;
+            out.y = __byte_perm(w[2], w[3], 0x7531) & 0x80808080u;
+        }
+        uint8_t* dst = q + (row0 + i) * ldq + col;
+        if (kAligned) {
+            *reinterpret_cast<uint2*>(dst) = out;
+        } else {
+            reinterpret_cast<uint32_t*>(dst)[0] = out.x;
+            reinterpret_cast<uint32_t*>(dst)[1] = out.y;
+        }
+    };
+    if (__all_sync(0xFFFFFFFFu, plain)) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) put(i, false);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) put(i, !(m[i] > 0.0f));
+    }
+    // lane i holds row 4 * rb + i: word (row % 32) * 4 + (row % 128) / 32 of the atom
+    if (live && (lane & 15) < 4)
+        atoms[(g * R128 + (rb >> 5)) * 128 + ((rb & 7) * 4 + (lane & 15)) * 4 + ((rb & 31) >> 3)] = my_word;
 }
 
 // one 256-thread block per 128x128 block; the block stays in registers between amax and quantise
@@ -495,11 +574,9 @@ __global__ void quant_mx32_kernel(const float* __restrict__ x, uint8_t* __restri
         if (sub == 0) sf[blk] = 0;
         return;
     }
-    int byte = ilogbf(m) - 8 + 127;
-    byte = byte < 0 ? 0 : (byte > 254 ? 254 : byte);
-    const int e = byte - 127;
-    reinterpret_cast<uint32_t*>(q + blk * 32)[sub] =
-        f32x4_to_e4m3x4(scalbnf(v.x, -e), scalbnf(v.y, -e), scalbnf(v.z, -e), scalbnf(v.w, -e));
+    const int byte = mx_scale_byte(m);
+    const float inv = mx_inv_scale(byte);
+    reinterpret_cast<uint32_t*>(q + blk * 32)[sub] = f32x4_to_e4m3x4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
     if (sub == 0) sf[blk] = static_cast<uint8_t>(byte);
 }
 

@@ -359,6 +359,27 @@ int set_smem(Kernel kernel, int bytes) {
     return B200_OK;
 }
 
+// Launch with programmatic serialization: the kernel may be scheduled while its predecessor drains, and itself waits
+// (griddepcontrol.wait) before it touches anything the predecessor may still be writing or reading.
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    std::memset(&attr, 0, sizeof(attr));
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    CU_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+    g_launches.fetch_add(1);
+    return B200_OK;
+}
+
 template <int BN, int MODE, int BL>
 int launch_gemm(const GemmParams& p, int grid, cudaStream_t st) {
     using Cfg = GemmCfg<BN, MODE, BL>;
@@ -377,23 +398,7 @@ int launch_decode(const DecodeParams& p, int grid, cudaStream_t st) {
     auto kernel = decode_a8w8_sm100_kernel<Cfg>;
     int rc = set_smem(kernel, Cfg::SMEM_BYTES);
     if (rc) return rc;
-    // programmatic serialization: a following decode launch may begin (and request its first weight tiles)
-    // while this one drains; the kernel waits for its predecessor before it touches tokens, scales or C
-    cudaLaunchConfig_t cfg;
-    std::memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-    cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    std::memset(&attr, 0, sizeof(attr));
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    CU_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
-    g_launches.fetch_add(1);
-    return B200_OK;
+    return launch_pdl(kernel, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
 
 // number of CTA pairs that can be resident at once (GPCs with an odd SM count strand one SM)
@@ -1152,24 +1157,15 @@ int b200_quantize_act_bf16_1x128(const void* x_bf16, int64_t ldx, void* q, int64
     if (k % 128 != 0 || ldx % 8 != 0 || ldq % 8 != 0 || (reinterpret_cast<uintptr_t>(x_bf16) & 15) ||
         (reinterpret_cast<uintptr_t>(q) & 7))
         return B200_ERR_UNSUPPORTED;
-    const int64_t gx = (k / 128 + 15) / 16, gy = (m + 31) / 32;
-    if (gy > 65535) {
-        // rows beyond the grid's y range: run in slabs of 65535 x 32 rows
-        int rc = B200_OK;
-        const int64_t slab = 65535LL * 32;
-        for (int64_t r = 0; r < m && rc == B200_OK; r += slab) {
-            const int64_t mm = (m - r) < slab ? (m - r) : slab;
-            rc = b200_quantize_act_bf16_1x128(static_cast<const uint16_t*>(x_bf16) + r * ldx, ldx, static_cast<uint8_t*>(q) + r * ldq,
-                                              ldq, sfa + r, stride_sfa, mm, k, stream);
-        }
-        return rc;
-    }
-    dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-    act_quant_bf16_1x128_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint16_t*>(x_bf16), ldx, static_cast<uint8_t*>(q), ldq, sfa, stride_sfa, m, k);
-    CU_TRY(cudaGetLastError());
-    g_launches.fetch_add(1);
-    return B200_OK;
+    // four rows per warp (see the kernel) unless that leaves an SM with fewer than eight warps
+    const int64_t pairs = (k / 128 + 1) / 2;
+    const bool wide = (m + 3) / 4 * pairs >= 148 * 8;
+    const int64_t blocks = ((wide ? (m + 3) / 4 : m) * pairs + 7) / 8;
+    if (k > 0x7FFFFFFF || blocks > (1 << 28)) return B200_ERR_TOO_LARGE;
+    return launch_pdl(wide ? act_quant_bf16_1x128_kernel<4> : act_quant_bf16_1x128_kernel<1>, static_cast<unsigned>(blocks), 256, 0,
+                      static_cast<cudaStream_t>(stream), static_cast<const uint16_t*>(x_bf16), static_cast<long long>(ldx),
+                      static_cast<uint8_t*>(q), static_cast<long long>(ldq), sfa, static_cast<long long>(stride_sfa),
+                      static_cast<long long>(m), static_cast<int>(k / 128));
 }
 int b200_quantize_act_bf16_mx32(const void* x_bf16, int64_t ldx, void* q, int64_t ldq, void* sf_atoms, int64_t rows, int64_t k,
                                 void* stream) {
@@ -1178,14 +1174,14 @@ int b200_quantize_act_bf16_mx32(const void* x_bf16, int64_t ldx, void* q, int64_
     if (k % 128 != 0 || ldx % 4 != 0 || ldq % 4 != 0 || (reinterpret_cast<uintptr_t>(x_bf16) & 7) ||
         (reinterpret_cast<uintptr_t>(q) & 3) || (reinterpret_cast<uintptr_t>(sf_atoms) & 3))
         return B200_ERR_UNSUPPORTED;
-    const int64_t gx = (k / 128 + 7) / 8, gy = ((rows + 127) / 128) * 4;
-    if (gy > 65535) return B200_ERR_TOO_LARGE;          // more than 2,097,120 rows
-    dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-    act_quant_bf16_mx32_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint16_t*>(x_bf16), ldx, static_cast<uint8_t*>(q), ldq, static_cast<uint32_t*>(sf_atoms), rows, k);
-    CU_TRY(cudaGetLastError());
-    g_launches.fetch_add(1);
-    return B200_OK;
+    const int64_t blocks = ((rows + 127) / 128 * 32 * ((k / 128 + 1) / 2) + 7) / 8;
+    if (k > 0x7FFFFFFF || blocks > (1 << 28)) return B200_ERR_TOO_LARGE;
+    const bool aligned = ldx % 8 == 0 && ldq % 8 == 0 && aligned16(x_bf16) && (reinterpret_cast<uintptr_t>(q) & 7) == 0;
+    return launch_pdl(aligned ? act_quant_bf16_mx32_kernel<true> : act_quant_bf16_mx32_kernel<false>,
+                      static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
+                      static_cast<const uint16_t*>(x_bf16), static_cast<long long>(ldx), static_cast<uint8_t*>(q),
+                      static_cast<long long>(ldq), static_cast<uint32_t*>(sf_atoms), static_cast<long long>(rows),
+                      static_cast<int>(k / 128));
 }
 int b200_quantize_128x128(const float* x, void* q, float* sfb, int64_t n, int64_t k, void* stream) {
     if (!x || !q || !sfb || n <= 0 || k <= 0) return B200_ERR_BAD_ARG;

@@ -128,3 +128,24 @@ def test_sharded_forward_bf16_single_gpu(api, O):
     _, va, vs = op.activation_buffer(m, k, DEV)
     assert np.array_equal(va.cpu().numpy(), qa) and np.array_equal(vs.cpu().numpy(), sfa)
     assert_close(O, out.float().cpu().numpy(), O.gemm_ref_blockscale(qa, qb, sfa, sfb))
+
+
+@pytest.mark.parametrize("m,k", [(3, 384), (588, 1920), (592, 2048), (597, 2048)])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_act_quant_at_the_edges_of_the_dispatch(api, O, m, k, offset):
+    """Both sides of the one-row / four-rows-per-warp rule (four from 1184 warps on), a last row group of one row, an odd
+    number of K groups; and for MX an input that is only 8-byte aligned.  Magnitudes run over many binades, so that single
+    groups leave the fast division."""
+    wide = O.fill_normal((m, k + 8), 31, 0) * np.exp2(np.floor(O.fill_uniform((m, 1), 31, 1, -125.0, 120.0))).astype(np.float32)
+    wide[m // 2, :] = 0.0
+    bits = O.f32_to_bf16_bits(wide)
+    x = torch.from_numpy(bits.view(np.int16)).to(DEV).view(torch.bfloat16)[:, offset:offset + k]
+    xf = np.ascontiguousarray(O.bf16_bits_to_f32(bits)[:, offset:offset + k])
+    if offset % 8 == 0:
+        q, sfa = api.quantize_act_bf16_1x128(x)
+        qr, sr = O.quant_1x128(xf)
+        assert np.array_equal(q.cpu().numpy(), qr) and np.array_equal(sfa.cpu().numpy(), sr)
+    q, atoms = api.quantize_act_bf16_mx32(x)
+    qr, sr = O.quant_mx32(xf)
+    assert np.array_equal(q.cpu().numpy(), qr)
+    assert torch.equal(atoms, api.mx_sf_relayout(T(sr), m, k))
