@@ -17,6 +17,7 @@
 #include "decode_sm100.cuh"
 #include "gemm_pair_sm100.cuh"
 #include "gemm_sm100.cuh"
+#include "host_staging.h"
 #include "weight_file.h"
 
 namespace {
@@ -53,6 +54,8 @@ struct DeviceState {
                                  nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t copies_done = nullptr;
     cudaStream_t peek_stream = nullptr;   // b200_peek_status: reads the status word without waiting for other streams
+    Staging staging;                      // b200_gemm_a8w8_host: pinned ring for pageable operands (host_entry_mu)
+    int* status_host = nullptr;           // ... and the pinned word its final look at the status goes to
     std::mutex host_entry_mu;             // b200_gemm_a8w8_host: one caller at a time per device (shared staging buffers)
 };
 DeviceState g_dev[kMaxDevices];
@@ -904,10 +907,11 @@ int b200_gemm_a8w8_simple(const b200_gemm_args* a, void* cuda_stream) {
 // that gave up (an expired wait, a pair whose CTAs disagreed on their tensor-memory address) is an error HERE and
 // not a silently wrong C.  The word is left for b200_last_status() to report and clear.
 static int host_entry_finish(DeviceState* ds, cudaStream_t st) {
+    if (!ds->status_host) CU_TRY(cudaHostAlloc(&ds->status_host, sizeof(int), cudaHostAllocDefault));
+    CU_TRY(cudaMemcpyAsync(ds->status_host, ds->status_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CU_TRY(ds->staging.finish_downloads());
     CU_TRY(cudaStreamSynchronize(st));
-    int v = 0;
-    CU_TRY(cudaMemcpy(&v, ds->status_ptr, sizeof(int), cudaMemcpyDeviceToHost));
-    return v == 0 ? B200_OK : B200_ERR_DEVICE_TIMEOUT;
+    return *ds->status_host == 0 ? B200_OK : B200_ERR_DEVICE_TIMEOUT;
 }
 
 // a * b for non-negative operands, or -1 when the product does not fit in 2^46 bytes (64 TiB: far above any device)
@@ -968,10 +972,12 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
     d.ptr_c = ds->buf[2];
     rc = validate(&d, ds->sm_count, &pl);
     if (rc) return rc;
-    CU_TRY(cudaMemcpyAsync(ds->buf[1], h->ptr_b, b_bytes, cudaMemcpyHostToDevice, st));
+    Staging& io = ds->staging;
+    io.abandon();
+    CU_TRY(io.upload(ds->buf[1], h->ptr_b, b_bytes, st));
     if (sfa_bytes) {
-        CU_TRY(cudaMemcpyAsync(ds->buf[3], h->ptr_sfa, sfa_bytes, cudaMemcpyHostToDevice, st));
-        CU_TRY(cudaMemcpyAsync(ds->buf[4], h->ptr_sfb, sfb_bytes, cudaMemcpyHostToDevice, st));
+        CU_TRY(io.upload(ds->buf[3], h->ptr_sfa, sfa_bytes, st));
+        CU_TRY(io.upload(ds->buf[4], h->ptr_sfb, sfb_bytes, st));
         d.ptr_sfa = ds->buf[3];
         d.ptr_sfb = ds->buf[4];
     }
@@ -992,10 +998,10 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
     const int64_t slab_rows = ((h->m + 7) / 8 + 255) / 256 * 256;
     const bool slabs = h->batch == 1 && h->m >= 2048 && h->scale_mode != B200_SCALE_MX && (h->m + slab_rows - 1) / slab_rows <= 16;
     if (!slabs) {
-        CU_TRY(cudaMemcpyAsync(ds->buf[0], h->ptr_a, a_bytes, cudaMemcpyHostToDevice, st));
+        CU_TRY(io.upload(ds->buf[0], h->ptr_a, a_bytes, st));
         rc = b200_gemm_a8w8(&d, st);
         if (rc) return rc;
-        CU_TRY(cudaMemcpyAsync(h->ptr_c, ds->buf[2], c_bytes, cudaMemcpyDeviceToHost, st));
+        CU_TRY(io.download(h->ptr_c, ds->buf[2], c_bytes, st));
         return host_entry_finish(ds, st);
     }
     {
@@ -1014,14 +1020,14 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
         s.ptr_a = static_cast<const uint8_t*>(d.ptr_a) + r0 * h->stride_a;
         s.ptr_c = static_cast<uint8_t*>(d.ptr_c) + static_cast<size_t>(r0) * h->stride_c * esz;
         if (h->scale_mode == B200_SCALE_BLOCK) s.ptr_sfa = static_cast<const float*>(d.ptr_sfa) + r0;   // [K/128][M]: same pitch
-        CU_TRY(cudaMemcpyAsync(const_cast<void*>(s.ptr_a), static_cast<const uint8_t*>(h->ptr_a) + r0 * h->stride_a,
-                               static_cast<size_t>(rows * h->stride_a), cudaMemcpyHostToDevice, st));
+        CU_TRY(io.upload(const_cast<void*>(s.ptr_a), static_cast<const uint8_t*>(h->ptr_a) + r0 * h->stride_a,
+                         static_cast<size_t>(rows * h->stride_a), st));
         rc = b200_gemm_a8w8(&s, st);
         if (rc) return rc;
         CU_TRY(cudaEventRecord(ds->slab_done[slab], st));
         CU_TRY(cudaStreamWaitEvent(ds->copy_stream, ds->slab_done[slab], 0));
-        CU_TRY(cudaMemcpyAsync(static_cast<uint8_t*>(h->ptr_c) + static_cast<size_t>(r0) * h->stride_c * esz, s.ptr_c,
-                               static_cast<size_t>(rows * h->stride_c) * esz, cudaMemcpyDeviceToHost, ds->copy_stream));
+        CU_TRY(io.download(static_cast<uint8_t*>(h->ptr_c) + static_cast<size_t>(r0) * h->stride_c * esz, s.ptr_c,
+                           static_cast<size_t>(rows * h->stride_c) * esz, ds->copy_stream));
     }
     CU_TRY(cudaEventRecord(ds->copies_done, ds->copy_stream));
     CU_TRY(cudaStreamWaitEvent(st, ds->copies_done, 0));
@@ -1433,6 +1439,10 @@ int b200_release(void) {
         }
         g_scratch_count = kept;
     }
+    s.staging.release();
+    if (s.status_host) cudaFreeHost(s.status_host);
+    s.status_host = nullptr;
+    CopyPool::get().release();
     if (s.copy_stream) {
         cudaStreamDestroy(s.copy_stream);
         s.copy_stream = nullptr;

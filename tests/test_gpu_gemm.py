@@ -332,3 +332,19 @@ def test_chained_launches_with_inputs_ready(api, O):
     c0 = api.gemm_a8w8(sets[0][0], sets[0][1], out_dtype=torch.float32)
     c1 = api.gemm_a8w8(sets[0][0], sets[0][1], out_dtype=torch.float32, inputs_ready=True)
     assert torch.equal(c0, c1)
+
+
+@pytest.mark.parametrize("m", [40, 2500])
+@pytest.mark.parametrize("pinned", ["none", "operands", "result"])
+def test_host_entry_staging_ring(api, O, m, pinned):
+    """Pageable operands and results pass through a pinned ring in 2 MB chunks: five chunks of B (four upload slots), 20 of C
+    (eight result slots; row slabs of 320 rows end inside chunks), or one partial chunk.  Same bytes as on the device."""
+    n, k = 4096, 2304
+    a, b = e4m3(O, (m, k), 14, 0, 0.0, 1.0), e4m3(O, (n, k), 14, 1, -0.5, 0.5)
+    want = api.gemm_a8w8(T(a), T(b), out_dtype=torch.float32, tile=1).cpu().numpy()
+    pin = lambda x, on: torch.from_numpy(x).pin_memory().numpy() if on else x
+    ha, hb = pin(a, pinned == "operands"), pin(b, pinned == "operands")
+    for _ in range(2):
+        c = pin(np.full((m, n), np.nan, np.float32), pinned == "result")
+        api.gemm_a8w8_host(ha, hb, c, tile=1)
+        assert np.array_equal(c, want)
