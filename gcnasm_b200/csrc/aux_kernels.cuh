@@ -309,23 +309,25 @@ __global__ void __launch_bounds__(1024) membw_copy_kernel(const uint4* __restric
     for (; i < n16; i += stride) __stcs(dst + i, __ldcs(src + i));
 }
 
-// x / s, correctly rounded, for many x and one s.  With r = RN(1/s): q0 = RN(x*r), rem = x - q0*s (exact in an
-// FMA), q = RN(q0 + rem*r) is the correctly rounded quotient when nothing overflows or loses bits to underflow
-// (Markstein).  The fast path is for an s that is a normal number of moderate size; the callers guarantee
+// x / s, correctly rounded, for many x and one s.  With r = RN(1/s): q0 = RN(x*r), rem = q0*s - x (exact in an
+// FMA), q = RN(q0 - rem*r) is the correctly rounded quotient when nothing overflows or loses bits to underflow
+// (Markstein).  The remainder is taken with this sign because a zero keeps its own then: x = -0 gives rem = +0 and
+// q = -0 - 0 = -0, where x - q0*s would have made it +0.  The fast path is for an s that is a normal number of moderate size; the callers guarantee
 // |x| <= 448*s*(1+2^-23), and a quotient too small to be exact becomes a zero byte either way.  Everything else takes
 // the IEEE division.
 __device__ __forceinline__ bool scale_is_moderate(float s) { return s >= 0x1p-100f && s <= 0x1p100f; }
 __device__ __forceinline__ float div_by_scale(float x, float s, float r) {
     if (scale_is_moderate(s)) {
         const float q0 = __fmul_rn(x, r);
-        return __fmaf_rn(__fmaf_rn(-q0, s, x), r, q0);
+        return __fmaf_rn(__fmaf_rn(q0, s, -x), -r, q0);
     }
     return __fdiv_rn(x, s);
 }
-// ... and its fast path for two values, with s already negated
-__device__ __forceinline__ unsigned long long div2_by_scale(unsigned long long x, unsigned long long neg_s, unsigned long long r) {
+// ... and its fast path for two values, with r negated as well
+__device__ __forceinline__ unsigned long long div2_by_scale(unsigned long long x, unsigned long long s, unsigned long long r,
+                                                            unsigned long long neg_r) {
     const unsigned long long q0 = fmul2(x, r);
-    return ffma2(ffma2(q0, neg_s, x), r, q0);
+    return ffma2(ffma2(q0, s, x ^ 0x8000000080000000ull), neg_r, q0);
 }
 
 // |max| of two bf16 pairs; the result's sign bits are arbitrary.  A NaN gives way to the other operand.
@@ -406,9 +408,9 @@ __global__ void __launch_bounds__(256) act_quant_bf16_1x128_kernel(const uint16_
     if (__all_sync(0xFFFFFFFFu, scale_is_moderate(sc))) {        // two values at a time
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const float s = __shfl_sync(0xFFFFFFFFu, -sc, (lane & 16) + i), r = __shfl_sync(0xFFFFFFFFu, rc, (lane & 16) + i);
-            const unsigned long long s2 = pack_f32x2(s, s), r2 = pack_f32x2(r, r);
-            put(i, [&](uint32_t w) { return div2_by_scale(bf16x2_widen(w), s2, r2); });
+            const float s = __shfl_sync(0xFFFFFFFFu, sc, (lane & 16) + i), r = __shfl_sync(0xFFFFFFFFu, rc, (lane & 16) + i);
+            const unsigned long long s2 = pack_f32x2(s, s), r2 = pack_f32x2(r, r), nr2 = pack_f32x2(-r, -r);
+            put(i, [&](uint32_t w) { return div2_by_scale(bf16x2_widen(w), s2, r2, nr2); });
         }
     } else {
 #pragma unroll

@@ -81,6 +81,25 @@ def test_act_quant_1x128_wide_dynamic_range(api, O):
     assert np.array_equal(q.cpu().numpy(), qr)
 
 
+@pytest.mark.parametrize("m", [5, 1200])
+def test_act_quant_keeps_the_sign_of_zeros(api, O, m):
+    """Negative zeros among ordinary values, in groups of nothing but zeros and in groups whose scale is out of the
+    fast division's range keep their sign bit, as the division gives it."""
+    k = 512
+    x = O.fill_normal((m, k), 33, 0)
+    x[:, ::3] = -0.0
+    x[:, 128:256] = np.where(x[:, 128:256] > 0, 0.0, -0.0)
+    x[:, 256:384] *= np.float32(2.0 ** -115)
+    bits = O.f32_to_bf16_bits(x.astype(np.float32))
+    assert (bits == 0x8000).sum() > 100
+    xb, xf = torch.from_numpy(bits.view(np.int16)).to(DEV).view(torch.bfloat16), O.bf16_bits_to_f32(bits)
+    q, sfa = api.quantize_act_bf16_1x128(xb)
+    qr, sr = O.quant_1x128(xf)
+    assert np.array_equal(q.cpu().numpy(), qr) and np.array_equal(sfa.cpu().numpy(), sr)
+    q, _ = api.quantize_act_bf16_mx32(xb)
+    assert np.array_equal(q.cpu().numpy(), O.quant_mx32(xf)[0])
+
+
 @pytest.mark.parametrize("shape", [(256, 512), (200, 384), (1, 128), (129, 256), (2048, 1024)])
 def test_act_quant_mx32_bit_exact(api, O, shape):
     xb, xf = _bf16_input(O, shape, 24)
