@@ -1046,7 +1046,7 @@ static int shuffle_common(const void* src, void* dst, int64_t n, int64_t k, int3
         if (to_flat) shuffle_kn_kernel<true><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), n, k);
         else shuffle_kn_kernel<false><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), n, k);
     } else {
-        dim3 grid(static_cast<unsigned>((k / 16 + 15) / 16), static_cast<unsigned>(n / 16));
+        dim3 grid(static_cast<unsigned>((k / 16 + 63) / 64), static_cast<unsigned>(n / 16));
         if (grid.y > 65535) return B200_ERR_TOO_LARGE;
         if (to_flat) shuffle_nk_kernel<true><<<grid, 256, 0, st>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), n, k);
         else shuffle_nk_kernel<false><<<grid, 256, 0, st>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), n, k);

@@ -103,3 +103,38 @@ def test_mx_sf_relayout_atoms(api):
         for kb in range(k // 32):
             assert atoms[kb // 4, r // 128, r % 32, (r % 128) // 32, kb % 4] == sf[r, kb]
     assert atoms[0, 1, 8, 2, 0] == 127        # row 128 + 72 = 200 is padding -> scale 1.0
+
+
+def test_quant_128x128_over_the_whole_range(api, O):
+    """One block per binade of its largest value, most of them inside and some outside the range of the reciprocal division;
+    negative zeros, a block of zeros, and values next to the points between two e4m3 values."""
+    k = 128 * 252
+    x = O.fill_normal((128, k), 41, 0).reshape(128, 252, 128)
+    x[:, :, ::7] = -0.0
+    top = np.abs(x).max(axis=(0, 2), keepdims=True)
+    mid = (np.arange(128) % 16 + 16.5) / 16 * top / 448 * 16
+    x[5] = np.nextafter(mid[0], np.where(np.arange(128) % 3 == 0, 0, 1e9)).astype(np.float32)
+    x[:, 100] = 0.0
+    x = np.ldexp(x, (np.arange(252) - 128)[None, :, None]).astype(np.float32).reshape(128, k)
+    q, s = api.quantize_128x128(T(x))
+    qr, sr = O.quant_128x128(x)
+    assert np.array_equal(s.cpu().numpy(), sr) and np.array_equal(q.cpu().numpy(), qr)
+
+
+def test_quant_128x128_nan_and_infinity(api):
+    x = torch.ones(128, 256, device=DEV)
+    x[3, 5], x[7, 200], x[8, 201] = float("nan"), float("inf"), float("-inf")
+    q, s = api.quantize_128x128(x)
+    q = q.cpu().numpy()
+    assert s[0, 0].item() == np.float32(1 / 448) and s[0, 1].item() == float("inf")
+    assert q[3, 5] & 0x7F == 0x7F and (np.delete(q[:, :128].ravel(), 3 * 128 + 5) == 0x7E).all()
+    assert q[7, 200] & 0x7F == 0x7F and q[8, 201] & 0x7F == 0x7F and (q[9:, 128:] == 0).all()
+
+
+# a block takes 64 chunks of 16 bytes: one chunk, one short of a block, a whole one, one more
+@pytest.mark.parametrize("n,k", [(16, 16), (48, 1008), (16, 1024), (32, 1040), (272, 2192)])
+def test_shuffle_nk_at_the_edges_of_a_block(api, O, n, k):
+    b = np.random.default_rng(n + k).integers(0, 256, (n, k), dtype=np.uint8)
+    flat = api.shuffle_b(T(b), "nk")
+    assert np.array_equal(flat.cpu().numpy(), O.shuffle_b_nk(b))
+    assert np.array_equal(api.unshuffle_b(flat, n, k, "nk").cpu().numpy(), b)
