@@ -165,8 +165,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ------------------------------ UMMA issuer -------------------------------
+        {
+            // ------------------------------ UMMA issuer (the warp; an elected lane issues) ------------
+            const bool elected = elect_one() != 0;
             constexpr uint32_t idesc = make_idesc_f8(BNW, MT);
             uint32_t phase = 0;
             bool ok = true;
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                 const uint32_t set = phase % NBUF;
                 if constexpr (MODE == MODE_BLOCK) {
                     const uint32_t aph = (phase / NBUF) & 1;
-                    if (!mbar_wait_poll<false, 20>(bar_acce0 + set * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E)) {
+                    if (!role_all<true>(mbar_wait_poll<false, 20>(bar_acce0 + set * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
                         ok = false;
                         break;
                     }
@@ -188,11 +189,12 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                     const int i = i0 + j;
                     const uint32_t s = i % STAGES;
                     const uint32_t ph = (i / STAGES) & 1;
-                    if (!mbar_wait_poll<false, 20>(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL)) {
+                    if (!role_all<true>(mbar_wait_poll<false, 20>(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
+                    if (!elected) continue;
                     const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
                     const uint32_t sx = sw + Cfg::W_BYTES;
                     const uint32_t tacc = (MODE == MODE_BLOCK) ? tmem_base + (set * Cfg::GB + j) * MT : tmem_base;
@@ -213,9 +215,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                 }
                 if (!ok) break;
                 if constexpr (MODE == MODE_BLOCK) {
-                    umma_commit<1>(bar_accf0 + set * 8);
+                    if (elected) umma_commit<1>(bar_accf0 + set * 8);
                 } else {
-                    if (i0 + gb >= nkb) umma_commit<1>(bar_accf0);
+                    if (i0 + gb >= nkb && elected) umma_commit<1>(bar_accf0);
                 }
             }
         }

@@ -111,7 +111,7 @@ __device__ long long g_trace[2 * 8 * 128 * 8 + 128 * 8 + 128];
     } while (0)
 #define B200_TRACE_MMA(slot)                                                                     \
     do {                                                                                         \
-        if (pair_id == 0 && phase < 128) g_trace[2 * 8 * 128 * 8 + phase * 8 + (slot)] = clock64(); \
+        if (pair_id == 0 && elected && phase < 128) g_trace[2 * 8 * 128 * 8 + phase * 8 + (slot)] = clock64(); \
     } while (0)
 // the producers' stamps share the issuer rows: slots 6 and 7 of row it (leader CTA only)
 #define B200_TRACE_PROD(slot)                                                                    \
@@ -195,14 +195,18 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
     // With inputs_ready only the writes to C wait (in the epilogue, before the first tile is stored).
     if (!p.inputs_ready) pdl_wait();
 
+    // The producer too runs as a whole warp with an elected lane (see elect_one) where a stage takes four loads, for MX
+    // (8192^3 396 -> 381 us); with two loads it is better off as a single lane (8-bit 4096^3 53 against 58 us).
+    constexpr bool kWarpLoad = MODE == MODE_MX;
     if (!tmem_ok) {
         // fall through to the teardown
     } else if (warp < 4) {
         setmaxnreg_dec<Cfg::ROLE_REGS>();
-        if (warp == kProducerWarp && lane == 0) {
+        if (warp == kProducerWarp && (kWarpLoad || lane == 0)) {
             // ------------------------------ TMA producer (both CTAs) ------------------------------
             uint32_t it = 0;
             bool ok = true;
+            const bool elected = kWarpLoad ? elect_one() != 0 : true;
             int ready_b = -1;                         // last batch whose ready word has been seen
             const uint32_t leader_full0 = mapa_shared(bar_full0, 0);
             for (int u = pair_id; u < units_total && ok; u += num_pairs) {
@@ -212,7 +216,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                 tile_coords(p, t, b, mi, ni);
                 if (p.batch_ready && b != ready_b) {
                     // this batch's activation slab may still be on its way (a copy or collective on another stream)
-                    if (!wait_ready_word(p.batch_ready + b, p.batch_epoch, abort_flag, p.status)) break;
+                    if (!role_all<kWarpLoad>(!elected || wait_ready_word(p.batch_ready + b, p.batch_epoch, abort_flag, p.status))) break;
                     ready_b = b;
                 }
                 const int bq = p.b_shared ? 0 : b;    // batch coordinate of the weights
@@ -224,12 +228,13 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                 for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
                     const uint32_t s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
-                    if (!B200_PROD_WAIT(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY)) {
+                    if (!role_all<kWarpLoad>(B200_PROD_WAIT(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY))) {
                         ok = false;
                         break;
                     }
                     const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
                     const uint32_t sb = sa + Cfg::A_BYTES;
+                    if (!elected) continue;
                     B200_TRACE_PROD(0);
                     if (cta == 0)
                         mbar_arrive_expect_tx(bar_full0 + s * 8,
@@ -250,7 +255,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     }
                 }
             }
-        } else if (warp >= 1 && warp <= ((MODE == MODE_BLOCK) ? kBlockIssuers : 1) && lane == 0 && cta == 0) {
+        } else if (warp >= 1 && warp <= ((MODE == MODE_BLOCK) ? kBlockIssuers : 1) && cta == 0) {
             // ------------------------------ UMMA issuer (leader only) ------------------------------
             // Block-scale mode runs several issuer threads (warps 1..kBlockIssuers, one per scheduler) that take the
             // K groups round-robin.  An issuer is effectively tied up until its own MMAs and commits have gone
@@ -259,6 +264,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
             // barrier, order on a ring stage by its full barrier.
             constexpr uint32_t kIssuers = (MODE == MODE_BLOCK) ? kBlockIssuers : 1;
             const uint32_t my_slot = static_cast<uint32_t>(warp - 1);
+            const bool elected = elect_one() != 0;          // the whole warp walks the loop
             uint32_t it = 0, phase = 0;
             bool ok = true;
             constexpr uint32_t idesc = make_idesc_f8(2 * BM, BN);
@@ -284,13 +290,13 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                         const uint32_t ph = (it / STAGES) & 1;
                         // operands first (they were prefetched long ago), then the accumulator buffer: the
                         // second wait is the latency-critical one and the MMAs follow it immediately
-                        if (!B200_MMA_WAIT(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL)) {
+                        if (!role_all<true>(B200_MMA_WAIT(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
                             ok = false;
                             break;
                         }
                         if (kb == 0 && j == 0) {
                             B200_TRACE_MMA(0);
-                            if (!B200_MMA_WAIT(bar_acce0 + as * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E)) {
+                            if (!role_all<true>(B200_MMA_WAIT(bar_acce0 + as * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
                                 ok = false;
                                 break;
                             }
@@ -298,6 +304,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                         }
                         B200_TRACE_MMA(2);
                         tc_fence_after();
+                        if (elected) {
                         const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
                         const uint32_t sb = sa + Cfg::A_BYTES;
                         if constexpr (MODE == MODE_MX) {
@@ -330,9 +337,10 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                         B200_TRACE_MMA(4);
                         umma_commit_pair(bar_empty0 + s * 8);       // frees stage s in both CTAs
                         B200_TRACE_MMA(5);
+                        }
                     }
                     }
-                    if (ok) umma_commit_pair(bar_accf0 + as * 8);   // wakes the epilogues of both CTAs
+                    if (ok && elected) umma_commit_pair(bar_accf0 + as * 8);   // wakes the epilogues of both CTAs
                     B200_TRACE_MMA(3);
                 }
             }

@@ -278,8 +278,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     }
                 }
             }
-        } else if (warp == 1 && lane == 0) {
-            // ------------------------------ UMMA issuer -------------------------------
+        } else if (warp == 1) {
+            // ------------------------------ UMMA issuer (the warp; an elected lane issues) ------------
+            const bool elected = elect_one() != 0;
             uint32_t it = 0, phase = 0;
             bool ok = true;
             constexpr uint32_t idesc = make_idesc_f8(BM, BN);
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 for (int g = 0; g < groups && ok; ++g, ++phase) {
                     const uint32_t as = phase & 1;
                     const uint32_t aph = (phase >> 1) & 1;
-                    if (!mbar_wait(bar_acce0 + as * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E)) {
+                    if (!role_all<true>(mbar_wait(bar_acce0 + as * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
                         ok = false;
                         break;
                     }
@@ -296,11 +297,12 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     for (int kb = 0; kb < kb_per_group; ++kb, ++it) {
                         const uint32_t s = it % STAGES;
                         const uint32_t ph = (it / STAGES) & 1;
-                        if (!mbar_wait(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL)) {
+                        if (!role_all<true>(mbar_wait(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
                             ok = false;
                             break;
                         }
                         tc_fence_after();
+                        if (!elected) continue;
                         const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
                         const uint32_t sb = sa + Cfg::A_BYTES;
                         if constexpr (MODE == MODE_MX) {
@@ -332,7 +334,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         }
                         umma_commit<1>(bar_empty0 + s * 8);      // stage free once these MMAs retire
                     }
-                    if (ok) umma_commit<1>(bar_accf0 + as * 8);  // accumulator phase complete
+                    if (ok && elected) umma_commit<1>(bar_accf0 + as * 8);  // accumulator phase complete
                 }
             }
         }

@@ -38,6 +38,12 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
+// True in one lane of a converged warp.  The roles that issue tcgen05 instructions walk their loops as whole warps and guard
+// the instructions with this predicate.  Behind `if (lane == 0)` every MMA cost the issuing thread at least 61 clocks and
+// every ring stage 340 more, and the tensor pipe ran dry in between.  us before / after, same box:
+//   8-bit 4096^3 69 / 53, 4096 x 7168 x 2048 56 / 47; bf16 4096^3 103 / 94; MX 8192^3 456 / 396; block scales, where two
+//   issuers hid the cost, 4096 x 7168 x 2048 68.6 / 67.6; single-CTA 128 x 128 tiles with block scales, 2048 x 2048 x 4096
+//   45.4 / 35.5.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t pred;
     asm volatile(
@@ -46,6 +52,13 @@ __device__ __forceinline__ uint32_t elect_one() {
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(pred));
     return pred;
+}
+
+// The outcome of a role's wait: its own, or, in a role that runs as a whole warp, the same for all lanes.
+template <bool kWholeWarp>
+__device__ __forceinline__ bool role_all(bool ok) {
+    if constexpr (kWholeWarp) return __all_sync(0xFFFFFFFFu, ok);
+    else return ok;
 }
 
 // ---- mbarrier ----------------------------------------------------------------------------
