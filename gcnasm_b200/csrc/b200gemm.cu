@@ -365,22 +365,29 @@ int set_smem(Kernel kernel, int bytes) {
 // Launch with programmatic serialization: the kernel may be scheduled while its predecessor drains, and itself waits
 // (griddepcontrol.wait) before it touches anything the predecessor may still be writing or reading.
 template <class... P, class... A>
-int launch_pdl(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+int launch_pdl_cluster(int cluster, void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr;
-    std::memset(&attr, 0, sizeof(attr));
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    std::memset(attr, 0, sizeof(attr));
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     CU_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
     g_launches.fetch_add(1);
     return B200_OK;
+}
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+    return launch_pdl_cluster(1, kernel, grid, threads, smem, st, args...);
 }
 
 template <int BN, int MODE, int BL>
@@ -395,13 +402,63 @@ int launch_gemm(const GemmParams& p, int grid, cudaStream_t st) {
     return B200_OK;
 }
 
+// K splits of the decode kernel that work as one cluster (above 8 the size is not portable and asked for explicitly)
+constexpr int kMaxDecodeCluster = 16;
+
+template <int MT, int MODE, int BL>
+int decode_attrs() {
+    using Cfg = DecodeCfg<MT, MODE, BL>;
+    auto kernel = decode_a8w8_sm100_kernel<Cfg>;
+    static std::atomic<bool> done[kMaxDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return B200_ERR_NO_DEVICE;
+    if (done[dev].load()) return B200_OK;
+    CU_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    CU_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    done[dev].store(true);
+    return B200_OK;
+}
+
+// Clusters of `size` CTAs of this kernel that are resident at once (one CTA per SM; the SMs of a cluster belong to one
+// GPC, so 16 clusters of 9 do not fit where 9 of 16 do).  Asked once per device and size.
+template <int MT, int MODE, int BL>
+int decode_clusters(int size, int sm_count) {
+    using Cfg = DecodeCfg<MT, MODE, BL>;
+    static std::atomic<int> known[kMaxDevices][kMaxDecodeCluster + 1];     // capacity + 1; 0: not asked yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    int n = known[dev][size].load() - 1;
+    if (n < 0) {
+        if (decode_attrs<MT, MODE, BL>()) return 0;
+        cudaLaunchConfig_t cfg;
+        std::memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(static_cast<unsigned>(size), 1, 1);
+        cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
+        cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+        cudaLaunchAttribute attr;
+        std::memset(&attr, 0, sizeof(attr));
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = static_cast<unsigned>(size);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, decode_a8w8_sm100_kernel<Cfg>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        known[dev][size].store(n + 1);
+    }
+    return n < sm_count / size ? n : sm_count / size;
+}
+
+// splits == 1: plain launch; > 1 without a workspace: the splits of a panel form a cluster
 template <int MT, int MODE, int BL>
 int launch_decode(const DecodeParams& p, int grid, cudaStream_t st) {
     using Cfg = DecodeCfg<MT, MODE, BL>;
-    auto kernel = decode_a8w8_sm100_kernel<Cfg>;
-    int rc = set_smem(kernel, Cfg::SMEM_BYTES);
+    int rc = decode_attrs<MT, MODE, BL>();
     if (rc) return rc;
-    return launch_pdl(kernel, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
+    const int cluster = p.splits > 1 && !p.partial ? p.splits : 1;
+    return launch_pdl_cluster(cluster, decode_a8w8_sm100_kernel<Cfg>, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
 
 // number of CTA pairs that can be resident at once (GPCs with an odd SM count strand one SM)
@@ -524,6 +581,34 @@ int launch_decode_mt(int mt, const DecodeParams& p, int grid, cudaStream_t st) {
         default: return launch_decode<64, MODE, BL>(p, grid, st);
     }
 }
+template <int MODE, int BL>
+int decode_clusters_mt(int mt, int size, int sm_count) {
+    switch (mt) {
+        case 16: return decode_clusters<16, MODE, BL>(size, sm_count);
+        case 32: return decode_clusters<32, MODE, BL>(size, sm_count);
+        default: return decode_clusters<64, MODE, BL>(size, sm_count);
+    }
+}
+int decode_clusters_any(bool block, bool flat, int mt, int size, int sm_count) {
+    if (block) return flat ? decode_clusters_mt<MODE_BLOCK, BL_FLAT>(mt, size, sm_count) : decode_clusters_mt<MODE_BLOCK, BL_NK>(mt, size, sm_count);
+    return flat ? decode_clusters_mt<MODE_ACC, BL_FLAT>(mt, size, sm_count) : decode_clusters_mt<MODE_ACC, BL_NK>(mt, size, sm_count);
+}
+
+// K splits of a decode launch that reduces in its clusters: of the counts whose clusters are all resident at once, the
+// smallest one with the fewest K blocks per CTA, at least kMinSplitBlocks (1024 x 1024: 1 split 5.8 us, 2 5.3, 4 5.0, 8
+// 5.3; a count whose clusters are not all resident costs a second wave: 7168 x 2048 2 splits 8.6 us, 3 12.9).  Block scales
+// bound a CTA's K blocks by its staging area; when that takes more splits than fit a cluster the answer is 0 and the partials
+// go through a workspace.
+int cluster_splits(int64_t tiles, int64_t kblocks, bool block, bool flat, int mt, int sm_count) {
+    constexpr int kMinSplitBlocks = 2;
+    const int64_t most = block ? decode_sf_bytes(mt) / 4 / (mt + 1) : kblocks;      // K blocks one CTA can take
+    const int64_t need = (kblocks + most - 1) / most;
+    if (need > kMaxDecodeCluster || (need > 1 && decode_clusters_any(block, flat, mt, static_cast<int>(need), sm_count) < 1)) return 0;
+    int best = static_cast<int>(need);
+    for (int s = best + 1; s <= kMaxDecodeCluster && (kblocks + s - 1) / s >= kMinSplitBlocks; ++s)
+        if ((kblocks + s - 1) / s < (kblocks + best - 1) / best && decode_clusters_any(block, flat, mt, s, sm_count) >= tiles) best = s;
+    return best;
+}
 
 // Split-K workspaces of the skinny-M path.  One per (device, stream): launches on different streams never share
 // partials.  A workspace that has been handed to a launch is never freed or moved before b200_release() -- a
@@ -592,17 +677,25 @@ int static_scratch(size_t need_floats, float** out) {
 int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStream_t st, bool use_static = false) {
     DecodeParams p;
     std::memset(&p, 0, sizeof(p));
+    const bool block = a->scale_mode == B200_SCALE_BLOCK, flat = a->b_layout == B200_B_FLAT_16x16;
+    // (the limit of b200_gemm_a8w8_decode_static counts the splits a launch without clusters would make)
     const size_t need_floats = pl.splits > 1 ? static_cast<size_t>(pl.splits) * a->batch * a->m * a->n : 0;
+    float* scratch = nullptr;
     if (use_static) {
-        float* scratch = nullptr;
         int rc0 = static_scratch(need_floats, &scratch);
         if (rc0) return rc0;
-        p.partial = pl.splits > 1 ? scratch : nullptr;
-    } else if (pl.splits > 1) {
-        int dev = 0;
-        CU_TRY(cudaGetDevice(&dev));
-        int rc0 = scratch_for(dev, st, need_floats * sizeof(float), &p.partial);
-        if (rc0) return rc0;
+    }
+    int splits = cluster_splits((a->n + 127) / 128 * a->batch, (a->k + 127) / 128, block, flat, pl.mt, ds->sm_count);
+    if (splits == 0) {
+        splits = pl.splits;
+        if (use_static) {
+            p.partial = scratch;
+        } else if (splits > 1) {
+            int dev = 0;
+            CU_TRY(cudaGetDevice(&dev));
+            int rc0 = scratch_for(dev, st, need_floats * sizeof(float), &p.partial);
+            if (rc0) return rc0;
+        }
     }
     int rc;
     if (a->b_layout == B200_B_NK_ROWMAJOR)
@@ -629,23 +722,22 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
     p.batch = static_cast<int>(a->batch);
     p.tiles_n = static_cast<int>((a->n + 127) / 128);
     p.kblocks = static_cast<int>((a->k + 127) / 128);
-    p.splits = pl.splits;
-    p.kb_per_split = (p.kblocks + pl.splits - 1) / pl.splits;
+    p.splits = splits;
+    p.kb_per_split = (p.kblocks + splits - 1) / splits;
     p.out_dtype = a->out_dtype;
     p.inputs_ready = (a->flags & B200_GEMM_INPUTS_READY) ? 1 : 0;
     p.status = ds->status_ptr;
-    const int grid = p.tiles_n * p.batch * pl.splits;
-    const bool block = a->scale_mode == B200_SCALE_BLOCK;
+    const int grid = p.tiles_n * p.batch * splits;
     if (a->b_layout == B200_B_NK_ROWMAJOR)
         rc = block ? launch_decode_mt<MODE_BLOCK, BL_NK>(pl.mt, p, grid, st) : launch_decode_mt<MODE_ACC, BL_NK>(pl.mt, p, grid, st);
     else
         rc = block ? launch_decode_mt<MODE_BLOCK, BL_FLAT>(pl.mt, p, grid, st) : launch_decode_mt<MODE_ACC, BL_FLAT>(pl.mt, p, grid, st);
     if (rc) return rc;
-    if (pl.splits > 1) {
+    if (splits > 1 && p.partial) {
         const long long per_split = static_cast<long long>(a->batch) * a->m * a->n;
         const int threads = 256;
         const unsigned blocks = static_cast<unsigned>((per_split + threads - 1) / threads);
-        decode_splitk_reduce_kernel<<<blocks, threads, 0, st>>>(p.partial, a->ptr_c, pl.splits, per_split, p.m, p.n,
+        decode_splitk_reduce_kernel<<<blocks, threads, 0, st>>>(p.partial, a->ptr_c, splits, per_split, p.m, p.n,
                                                                p.ldc, p.c_batch, p.out_dtype);
         CU_TRY(cudaGetLastError());
         g_launches.fetch_add(1);

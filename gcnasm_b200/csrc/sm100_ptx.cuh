@@ -205,6 +205,16 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, uint
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
+// Requests a box into L2 only.  L2 is where every write on the device meets, so this is allowed at any time, also while
+// a kernel that writes the box is still running: what it later reads is what was last written.
+__device__ __forceinline__ void tma_prefetch_3d(const void* tmap, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                 ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_4d(const void* tmap, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
+                 ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
 // Pair variants: the data lands in this CTA's shared memory, the transaction bytes are
 // counted on the barrier at the same offset in the pair's leader CTA (`bar` is a
 // shared::cluster address).  No multicast: each CTA of the pair fetches its own half.

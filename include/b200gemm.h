@@ -108,10 +108,12 @@ enum b200_gemm_flags { B200_GEMM_INPUTS_READY = 1, B200_GEMM_BATCH_READY = 2 };
  * `cuda_stream` (a cudaStream_t, 0 = default stream); buffers are caller-owned device memory.           */
 int b200_gemm_a8w8(const b200_gemm_args* args, void* cuda_stream);
 /* Rules of the skinny-M path (M <= 64) of b200_gemm_a8w8.  When a problem has fewer 128-row weight panels than the
- * GPU has SMs the kernel splits K and needs an fp32 workspace.  The library keeps one workspace per (device,
+ * GPU has SMs the kernel splits K; the splits of a panel are one cluster and sum their partials through each other's shared
+ * memory.  Block scales with more K groups than 16 CTAs can stage (K above 192,512 at 64 tokens, above 1 M at 16) take more
+ * splits than a cluster has CTAs and need an fp32 workspace.  The library keeps one workspace per (device,
  * stream) -- launches on different streams never share one -- allocates it with cudaMalloc on first use or when a
  * larger one is needed, and never frees or moves a workspace that a launch has been given (b200_release frees them
- * all).  So: make the first split-K call of a stream, at the largest size it will see, before capturing that stream
+ * all).  So: make the first such call of a stream, at the largest size it will see, before capturing that stream
  * into a CUDA graph (an allocation cannot happen inside a capture, and a captured launch keeps the pointer it was
  * given); and do not call b200_release while captured graphs that contain these launches are still replayed.      */
 
@@ -149,11 +151,12 @@ int b200_gemm_a8w8_host(const b200_gemm_args* host_args, void* cuda_stream);
  * b200_gemm_a8w8, for callers that must not allocate device memory while they run: code inside a serving
  * loop whose memory was carved up ahead of time, a real-time or latency-critical thread where cudaMalloc's
  * device-wide synchronisation is unacceptable, or a host that hands this library a fixed memory budget and
- * forbids it to grow.  b200_gemm_a8w8 may cudaMalloc (and later cudaFree) a split-K workspace when a skinny
- * problem has fewer 128-row weight panels than the GPU has SMs; this entry point never calls cudaMalloc,
+ * forbids it to grow.  b200_gemm_a8w8 may cudaMalloc (and later cudaFree) a split-K workspace for a skinny
+ * problem with a very long K; this entry point never calls cudaMalloc,
  * cudaFree or any allocating routine.  Its split-K workspace is a fixed 1 MiB array inside the library image
  * (every GPU that loads the library holds it until the process exits).
- *   - Limit: splits * batch * M * N fp32 partials must fit in 1 MiB (262,144 floats); otherwise the call
+ *   - Limit: splits * batch * M * N fp32 partials must fit in 1 MiB (262,144 floats), whether or not the launch
+ *     goes through the workspace (splits: the power of two, at most 16, that fills the SMs with CTAs); otherwise the call
  *     returns B200_ERR_TOO_LARGE and launches nothing.  Shapes the launcher would not send to the skinny-M
  *     kernel (M > 64, MX scales) return B200_ERR_UNSUPPORTED.
  *   - The first call on each device looks up that device's address of the array (and the library's other

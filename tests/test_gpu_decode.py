@@ -75,3 +75,50 @@ def test_decode_batched_and_scaled(api, O):
     status_ok(api)
     for i in range(B):
         assert_close(O, c[i], O.gemm_ref_nt(a[i], b[i], 0.25, 3.0), f"batch {i}")
+
+
+# K splits of a panel form a cluster: two panels on as many splits as a cluster takes, an odd number of splits with a
+# short last one, panels x batches, more K groups than the staged scales of one CTA hold (K split for that reason alone),
+# and so many that not even a cluster holds them (partials in a workspace, summed by a second kernel)
+@pytest.mark.parametrize("m,n,k,batch", [(1, 256, 8192, 1), (16, 2688, 2432, 1), (40, 1280, 1664, 2), (64, 18432, 12288, 1),
+                                         (33, 128, 192640, 1)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_decode_splits(api, O, m, n, k, batch, out_dtype):
+    a = e4m3(O, (batch, m, k), 6, 0, 0.0, 1.0)
+    b = e4m3(O, (batch, n, k), 6, 1, -0.5, 0.5)
+    sfa = O.fill_uniform((batch, k // 128, m), 6, 2, 0.8, 1.2)
+    sfb = O.fill_uniform((batch, n // 128, k // 128), 6, 3, 0.8, 1.2)
+    wide = torch.full((batch, m, n + 3), -7.0, dtype=out_dtype, device=DEV)      # an odd row pitch
+    api.gemm_a8w8_blockscale(T(a), T(b), T(sfa), T(sfb), out=wide[:, :, :n])
+    c = api.gemm_a8w8_blockscale(T(a), T(b), T(sfa), T(sfb), out_dtype=out_dtype)
+    status_ok(api)
+    assert torch.equal(wide[:, :, :n], c) and torch.all(wide[:, :, n:] == -7.0)
+    for i in range(batch):
+        assert_close(O, c[i].float().cpu().numpy(), O.gemm_ref_blockscale(a[i], b[i], sfa[i], sfb[i]), f"batch {i}")
+
+
+# unscaled: one K block, two (one per accumulator), an odd number, ragged K and N, several splits
+@pytest.mark.parametrize("m,n,k", [(3, 272, 128), (17, 272, 256), (64, 400, 1136), (9, 512, 8192)])
+def test_decode_unscaled_splits(api, O, m, n, k):
+    a, b = e4m3(O, (m, k), 8, 0, 0.0, 1.0), e4m3(O, (n, k), 8, 1, -0.5, 0.5)
+    c = api.gemm_a8w8(T(a), T(b), out_dtype=torch.float32)
+    status_ok(api)
+    assert_close(O, c.cpu().numpy(), O.gemm_ref_nt(a, b), "decode unscaled")
+
+
+def test_decode_splits_under_capture(api, O):
+    """A launch that splits K needs no workspace: the first call of a stream may be inside a capture."""
+    m, n, k = 16, 1024, 4096
+    a, b = T(e4m3(O, (m, k), 7, 0, 0.0, 1.0)), T(e4m3(O, (n, k), 7, 1, -0.5, 0.5))
+    want = api.gemm_a8w8(a, b, out_dtype=torch.float32)
+    out = torch.zeros_like(want)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        api.gemm_a8w8(a, b, out=out)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    status_ok(api)
