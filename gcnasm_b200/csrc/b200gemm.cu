@@ -499,10 +499,11 @@ int pair_capacity(int sm_count) {
 }
 
 // The last round of a persistent schedule is rarely full: 448 tiles on 74 CTA pairs leave 4 tiles for a seventh round, and 70
-// pairs idle while those are computed.  Block-scale GEMMs on 256 x 256 tiles (row-major B) therefore compute the
+// pairs idle while those are computed.  GEMMs of 8-bit operands on 256 x 256 tiles (MX apart) therefore compute the
 // tiles of a partial last round as 4 (or 2) column parts each, one part per pair, when there are pairs enough: the
 // same K loop with 64- (128-) column MMAs, so every element is summed in exactly the order of a whole tile and
-// nothing meets in memory.  Sets p.tail_first / p.tail_split; B200GEMM_TAIL_SPLIT=0 in the environment (read once)
+// nothing meets in memory.  4096 x 7168 x 2048, block scales, pre-shuffled B, without and with: 67.7 / 64.2 us; bf16 4096^3
+// gains nothing (105.6 / 104.6, in a loop 119.9 both).  Sets p.tail_first / p.tail_split; B200GEMM_TAIL_SPLIT=0 in the environment (read once)
 // switches it off.
 thread_local int t_last_tail[2] = {0, 0};      // the calling thread's last pair launch (b200_last_tail_split)
 void plan_tail(GemmParams& p, int capacity) {
@@ -826,20 +827,24 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
         p.sfa_batch = a->stride_sfa_batch;
         p.sfb_batch = a->stride_sfb_batch;
     }
-    if (pair && BN == 256 && !ab16 && a->scale_mode == B200_SCALE_BLOCK && a->b_layout == B200_B_NK_ROWMAJOR) {
-        plan_tail(p, pair_capacity<256, MODE_BLOCK, BL_NK>(ds->sm_count));
+    const bool flat = a->b_layout == B200_B_FLAT_16x16;
+    if (pair && BN == 256 && !ab16 && a->scale_mode != B200_SCALE_MX) {
+        const int sms = ds->sm_count;
+        plan_tail(p, a->scale_mode == B200_SCALE_BLOCK
+                         ? (flat ? pair_capacity<256, MODE_BLOCK, BL_FLAT>(sms) : pair_capacity<256, MODE_BLOCK, BL_NK>(sms))
+                         : (flat ? pair_capacity<256, MODE_ACC, BL_FLAT>(sms) : pair_capacity<256, MODE_ACC, BL_NK>(sms)));
         if (p.tail_split) {
-            rc = make_rowmajor_tmap(&p.tmap_b_tail, a->ptr_b, a->n, a->k, a->stride_b, b_batches, a->stride_b_batch,
-                                    static_cast<uint32_t>(BROWS / p.tail_split));
+            const uint32_t rows = static_cast<uint32_t>(BROWS / p.tail_split);
+            rc = flat ? make_flat_tmap(&p.tmap_b_tail, a->ptr_b, a->n, a->k, b_batches, a->stride_b_batch, rows)
+                      : make_rowmajor_tmap(&p.tmap_b_tail, a->ptr_b, a->n, a->k, a->stride_b, b_batches, a->stride_b_batch, rows);
             if (rc) return rc;
         }
     }
     if (ab16) {
-        const bool flat16 = a->b_layout == B200_B_FLAT_16x16;
-        if (pair) return flat16 ? launch_pair<256, MODE_ACC16, BL_FLAT>(p, ds->sm_count, st) : launch_pair<256, MODE_ACC16, BL_NK>(p, ds->sm_count, st);
+        if (pair) return flat ? launch_pair<256, MODE_ACC16, BL_FLAT>(p, ds->sm_count, st) : launch_pair<256, MODE_ACC16, BL_NK>(p, ds->sm_count, st);
         const int grid16 = p.tiles_total < ds->sm_count ? p.tiles_total : ds->sm_count;
-        if (BN == 256) return flat16 ? launch_gemm<256, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<256, MODE_ACC16, BL_NK>(p, grid16, st);
-        return flat16 ? launch_gemm<128, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<128, MODE_ACC16, BL_NK>(p, grid16, st);
+        if (BN == 256) return flat ? launch_gemm<256, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<256, MODE_ACC16, BL_NK>(p, grid16, st);
+        return flat ? launch_gemm<128, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<128, MODE_ACC16, BL_NK>(p, grid16, st);
     }
     if (pair) {
         switch (BN) {
@@ -850,7 +855,6 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
         }
     }
     const int grid = p.tiles_total < ds->sm_count ? p.tiles_total : ds->sm_count;
-    const bool flat = a->b_layout == B200_B_FLAT_16x16;
     switch (a->scale_mode) {
         case B200_SCALE_BLOCK:
             if (BN == 256) return flat ? launch_gemm<256, MODE_BLOCK, BL_FLAT>(p, grid, st) : launch_gemm<256, MODE_BLOCK, BL_NK>(p, grid, st);

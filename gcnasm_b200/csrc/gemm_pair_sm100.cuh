@@ -56,7 +56,7 @@ struct PairCfg {
     static constexpr int THREADS = 128 + 32 * EPI_WARPS;
     // setmaxnreg only redistributes the registers the CTA got at launch (THREADS x the per-thread count the
     // launch bound allows, a multiple of 8); an increase beyond that pool blocks forever
-    static constexpr int ROLE_REGS = 40, EPI_REGS = 232;
+    static constexpr int ROLE_REGS = (MODE == MODE_BLOCK) ? 40 : 64, EPI_REGS = (MODE == MODE_BLOCK) ? 232 : 216;
     static constexpr int LAUNCH_REGS = (65536 / THREADS) / 8 * 8;
     static_assert(128 * ROLE_REGS + 32 * EPI_WARPS * EPI_REGS <= THREADS * LAUNCH_REGS, "setmaxnreg pool");
     static constexpr int LW = 32;                                   // columns per TMEM load in block-scale mode
@@ -187,8 +187,8 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
 
     const int groups = (MODE == MODE_BLOCK) ? p.kblocks : 1;
     const int kb_per_group = (MODE == MODE_BLOCK) ? 1 : p.kblocks;
-    // work units: whole tiles, then (block-scale, when the launcher set it up) the column parts of the tail tiles
-    constexpr bool kTail = (MODE == MODE_BLOCK) && BN == 256 && Cfg::BLAYOUT == BL_NK;
+    // work units: whole tiles, then (when the launcher set it up) the column parts of the tail tiles
+    constexpr bool kTail = (MODE == MODE_BLOCK || (MODE == MODE_ACC && !Cfg::AB16)) && BN == 256;
     const int units_total = (kTail && p.tail_split) ? p.tail_first + (p.tiles_total - p.tail_first) * p.tail_split
                                                     : p.tiles_total;
     // Unless the caller vouched for the operands, nothing is read or written before the previous kernel is complete.
@@ -244,7 +244,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     if constexpr (Cfg::BLAYOUT == BL_NK)
                         tma_load_3d_pair(sb, tmap_b_u, full, kb * BK, row_b, bq);
                     else
-                        tma_load_4d_pair(sb, &p.tmap_b, full, 0, row_b / 16, kb * (BK / 16), bq);
+                        tma_load_4d_pair(sb, tmap_b_u, full, 0, row_b / 16, kb * (BK / 16), bq);
                     B200_TRACE_PROD(1);
                     if constexpr (MODE == MODE_MX) {
                         // scale atoms [batch][K/128][rows/128][512 B], addressed as rows of 256 bytes
@@ -269,11 +269,12 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
             bool ok = true;
             constexpr uint32_t idesc = make_idesc_f8(2 * BM, BN);
             for (int u = pair_id; u < units_total && ok; u += num_pairs) {
-                // A column part of a tail tile: the same K loop with a narrower instruction, and tail_split K groups per
-                // accumulator hand-off -- their partial sums lie side by side in the 256-column buffer (4 x 64 or 2 x 128).
+                // A column part of a tail tile: the same K loop with a narrower instruction; block scales: tail_split K groups
+                // per accumulator hand-off -- their partial sums lie side by side in the 256-column buffer (4 x 64 or 2 x 128).
                 const bool tail_u = kTail && p.tail_split && u >= p.tail_first;
                 const uint32_t idesc_u = tail_u ? make_idesc_f8(2 * BM, BN / p.tail_split) : idesc;
-                const int gp = tail_u ? p.tail_split : 1;
+                const uint32_t lbo_u = tail_u ? static_cast<uint32_t>(BH / 16) * 256 / p.tail_split : (BH / 16) * 256;   // flat B
+                const int gp = (MODE == MODE_BLOCK && tail_u) ? p.tail_split : 1;
                 const uint32_t nsub = tail_u ? static_cast<uint32_t>(BN / p.tail_split) : 0u;
                 for (int g = 0; g < groups && ok; g += gp, ++phase) {
                     const int cnt = (groups - g) < gp ? (groups - g) : gp;
@@ -322,8 +323,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                             if constexpr (Cfg::BLAYOUT == BL_NK) {
                                 db = make_smem_desc(sb + k * 32, 16, 1024, kSwizzle128B);
                             } else {
-                                constexpr uint32_t LBO = (BH / 16) * 256;
-                                db = make_smem_desc(sb + k * 2 * LBO, LBO, 128, kSwizzleNone);
+                                db = make_smem_desc(sb + k * 2 * lbo_u, lbo_u, 128, kSwizzleNone);
                             }
                             const uint32_t accum = (kb > 0 || k > 0) ? 1u : 0u;
                             if constexpr (MODE == MODE_MX) {
@@ -692,7 +692,9 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                 }
             } else {
                 const int row0 = row - lane;                       // output row of this warp's lane 0
-                const int col_base = ni * BN + half * NCH;
+                // a column part is BN / tail_split columns wide, at the start of the accumulator buffer
+                const int my_cols = (kTail && part >= 0) ? NCH / p.tail_split : NCH;
+                const int col_base = ni * BN + ((kTail && part >= 0) ? part * 2 * my_cols : 0) + half * my_cols;
                 uint8_t* cbatch = reinterpret_cast<uint8_t*>(p.c) + static_cast<size_t>(b) * p.c_batch * esz;
                 uint8_t* out_stage = smem_gen + STAGES * Cfg::STAGE_BYTES + 1024 + ew * kOutStageBytesPerWarp;
                 const uint32_t as = phase % ACC_STAGES;
@@ -706,7 +708,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     pdl_wait();
                     c_ordered = true;
                 }
-                const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
+                const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * my_cols;
                 constexpr int CW = (NCH % 32 == 0) ? 32 : 16;      // columns per TMEM load
                 constexpr int NC = NCH / CW;
                 if constexpr (ACC_STAGES == 1) {
@@ -738,9 +740,11 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     tmem_ld<CW>(taddr, v[0]);
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
+                        if (kTail && c * CW >= my_cols) break;
+                        const bool last = kTail ? (c + 1) * CW >= my_cols : c + 1 == NC;
                         tmem_ld_wait();
-                        if (c + 1 < NC) tmem_ld<CW>(taddr + (c + 1) * CW, v[(c + 1) & 1]);
-                        if (c + 1 == NC) {
+                        if (c + 1 < NC && !last) tmem_ld<CW>(taddr + (c + 1) * CW, v[(c + 1) & 1]);
+                        if (last) {
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) mbar_arrive_cluster(leader_acce0 + as * 8);

@@ -46,7 +46,7 @@ struct GemmParams {
     int b_shared;                // pair kernels: every batch multiplies by the same B (B is read at batch coordinate 0)
     int batch_epoch;             // pair kernels: value a batch's ready word must have reached (with batch_ready)
     const int* batch_ready;      // pair kernels: one ready word per batch, or null
-    // pair kernels, block-scale, 256 x 256 tiles, row-major B: the tiles from tail_first on (the last, partly filled
+    // pair kernels, 256 x 256 tiles, 8-bit operands, not MX: the tiles from tail_first on (the last, partly filled
     // round of the persistent schedule) are each computed as tail_split (2 or 4) column parts of 256 / tail_split
     // columns by as many CTA pairs -- narrower MMAs over the full K, so every output element is summed exactly as in a
     // whole tile.  tmap_b_tail is B with a box of 128 / tail_split rows.  tail_split == 0: whole tiles only.

@@ -131,3 +131,33 @@ def test_overlapped_launches_with_tail(api, O):
             api.gemm_a8w8_blockscale(*s, out=shared, tile=4, inputs_ready=True)
     done(api)
     assert torch.equal(shared, want[2])
+
+
+# 80 tiles (6 in 4 parts), 98 tiles (24 in 2 parts), ragged edges in both directions
+@pytest.mark.parametrize("m,n,k", [(2560, 2048, 512), (1792, 3584, 640), (2500, 2000, 1152)])
+@pytest.mark.parametrize("kind", ["fp8", "fp8 flat", "block flat"])
+def test_split_in_every_kind(api, O, m, n, k, kind):
+    """Unscaled and pre-shuffled problems split their tail too: same sums as on tiles that are never split, in the same
+    order, and close to the oracle."""
+    flat = kind.endswith("flat")
+    if kind == "block flat":
+        n = n // 128 * 128
+        a, b, sfa, sfb = inputs(O, m, n, k, 61)
+        bb = api.shuffle_b(T(b), "nk")
+        run = lambda tile: api.gemm_a8w8_blockscale(T(a), bb, T(sfa), T(sfb), out_dtype=torch.float32, tile=tile, b_flat_n=n)
+        ref = O.gemm_ref_blockscale(a, b, sfa, sfb)
+    else:
+        a, b, _, _ = inputs(O, m, n, k, 62)
+        if flat:
+            fb = api.shuffle_b(T(b), "nk")
+            run = lambda tile: api.flatmm_a8w8(T(a), fb, n, out_dtype=torch.float32, tile=tile)
+        else:
+            run = lambda tile: api.gemm_a8w8(T(a), T(b), out_dtype=torch.float32, tile=tile)
+        ref = O.gemm_ref_nt(a, b)
+    c = run(4)
+    assert api.last_tail_split() == expected_plan(api, m, n)
+    done(api)
+    assert_close(O, c.cpu().numpy(), ref, f"{kind} tail {m}x{n}x{k}")
+    whole = run(6)
+    done(api)
+    assert torch.equal(c, whole), "a split tile differs from a whole one"
