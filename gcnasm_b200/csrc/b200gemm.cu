@@ -274,20 +274,31 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
         if (decode_ok) {
             hint = B200_TILE_DECODE;
         } else {
-            // cost of a persistent schedule: rounds x time per tile (proportional to the tile's N)
+            // cost of a persistent schedule: rounds (in tenths) x time per tile, proportional to the tile's N; with block
+            // scales the tail of 256 x 256 pair tiles counts with the share of a round that its column parts take (plan_tail)
             const int pairs = sm_count / 2;
             const int64_t tm2 = (a->m + 255) / 256, tm1 = (a->m + 127) / 128;
             int64_t best = -1;
             auto consider = [&](int tile, int bn, bool pair) {
                 const int64_t tiles = (pair ? tm2 : tm1) * ((a->n + bn - 1) / bn) * a->batch;
                 const int64_t units = pair ? pairs : sm_count;
-                const int64_t rounds = (tiles + units - 1) / units;
-                // weight = relative time per output column: pairs with wide tiles feed the tensor pipe best,
-                // narrow and single-CTA tiles re-read more of A/B per flop from L2
-                // (block-scale tiles that straddle the 128-column scale blocks pay for the second scale)
-                int64_t w = pair ? (bn >= 192 ? 10 : 13) : (bn >= 256 ? 14 : 18);
-                if (a->scale_mode == B200_SCALE_BLOCK && bn % 128 != 0) w += 2;
-                const int64_t cost = rounds * bn * w;
+                const bool block = a->scale_mode == B200_SCALE_BLOCK;
+                int64_t tenths = (tiles + units - 1) / units * 10;
+                const int64_t rem = tiles % units;
+                if (pair && bn == 256 && block && tiles > units && rem > 0 && kblocks >= 4 && rem * 2 <= units)
+                    tenths += (rem * 4 <= units ? 4 : 6) - 10;
+                // w = time per output column, measured on 4096 x 7168 x 2048 (us a round and 1000 columns, 8-bit / block scales:
+                // pair 256 27 / 40, 224 30 / 54, 192 30 / 56, 128 39 / 53; one CTA 256 33 / 49, 128 42 / 69): narrow and
+                // single-CTA tiles re-read more of A and B per flop, tiles that straddle the 128-column scale blocks
+                // pay for the second scale, and the 224-column epilogue works in half-width pieces, which a short K shows.
+                // Against the weights before (us): 4096^3 52.6 -> 47.9, 3794 x 3712 x 512 20.3 -> 16.7, 2750 x 7040 x 384 23.6 ->
+                // 18.5; with block scales 3794 x 3712 x 512 20.3 -> 16.7.
+                int64_t w;
+                if (!pair) w = bn >= 256 ? 125 : (block ? 170 : 155);
+                else if (bn == 256) w = 100;
+                else if (bn == 128) w = block ? 130 : 140;
+                else w = block ? 140 : (bn == 224 && kblocks < 8 ? 120 : 110);
+                const int64_t cost = tenths * bn * w;
                 if (best < 0 || cost < best) {
                     best = cost;
                     hint = tile;
@@ -503,8 +514,8 @@ int pair_capacity(int sm_count) {
 // tiles of a partial last round as 4 (or 2) column parts each, one part per pair, when there are pairs enough: the
 // same K loop with 64- (128-) column MMAs, so every element is summed in exactly the order of a whole tile and
 // nothing meets in memory.  4096 x 7168 x 2048, block scales, pre-shuffled B, without and with: 67.7 / 64.2 us; bf16 4096^3
-// gains nothing (105.6 / 104.6, in a loop 119.9 both).  Sets p.tail_first / p.tail_split; B200GEMM_TAIL_SPLIT=0 in the environment (read once)
-// switches it off.
+// gains nothing (105.6 / 104.6, in a loop 119.9 both).  Sets p.tail_first / p.tail_split; B200GEMM_TAIL_SPLIT=0 in the
+// environment (read once) switches it off.
 thread_local int t_last_tail[2] = {0, 0};      // the calling thread's last pair launch (b200_last_tail_split)
 void plan_tail(GemmParams& p, int capacity) {
     static const bool off = [] {

@@ -161,3 +161,17 @@ def test_split_in_every_kind(api, O, m, n, k, kind):
     whole = run(6)
     done(api)
     assert torch.equal(c, whole), "a split tile differs from a whole one"
+
+
+# the automatic choice on both sides of its rules: short K, a tail that splits or does not, block scales; ragged M and N
+@pytest.mark.parametrize("m,n,k", [(2570, 2048, 384), (2570, 2048, 512), (1900, 3712, 1024), (300, 7168, 256)])
+@pytest.mark.parametrize("block", [False, True])
+def test_automatic_tile_gives_the_same_bits(api, O, m, n, k, block):
+    a, b, sfa, sfb = (T(x) for x in inputs(O, m, n, k, 71))
+    if block:
+        run = lambda tile: api.gemm_a8w8_blockscale(a, b, sfa, sfb, out_dtype=torch.float32, tile=tile)
+    else:
+        run = lambda tile: api.gemm_a8w8(a, b, out_dtype=torch.float32, tile=tile)
+    c, whole = run(0), run(6)
+    done(api)
+    assert torch.equal(c, whole)
