@@ -97,7 +97,7 @@ def test_decode_splits(api, O, m, n, k, batch, out_dtype):
         assert_close(O, c[i].float().cpu().numpy(), O.gemm_ref_blockscale(a[i], b[i], sfa[i], sfb[i]), f"batch {i}")
 
 
-# unscaled: one K block, two (one per accumulator), an odd number, ragged K and N, several splits
+# unscaled: one K block, two, an odd number, ragged K and N, several splits
 @pytest.mark.parametrize("m,n,k", [(3, 272, 128), (17, 272, 256), (64, 400, 1136), (9, 512, 8192)])
 def test_decode_unscaled_splits(api, O, m, n, k):
     a, b = e4m3(O, (m, k), 8, 0, 0.0, 1.0), e4m3(O, (n, k), 8, 1, -0.5, 0.5)
