@@ -407,10 +407,7 @@ int launch_gemm(const GemmParams& p, int grid, cudaStream_t st) {
     auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
     int rc = set_smem(kernel, Cfg::SMEM_BYTES);
     if (rc) return rc;
-    kernel<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(p);
-    CU_TRY(cudaGetLastError());
-    g_launches.fetch_add(1);
-    return B200_OK;
+    return launch_pdl(kernel, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
 
 // K splits of the decode kernel that work as one cluster (above 8 the size is not portable and asked for explicitly)

@@ -348,3 +348,28 @@ def test_host_entry_staging_ring(api, O, m, pinned):
         c = pin(np.full((m, n), np.nan, np.float32), pinned == "result")
         api.gemm_a8w8_host(ha, hb, c, tile=1)
         assert np.array_equal(c, want)
+
+
+@pytest.mark.parametrize("m", [65, 100])
+def test_chained_layers_on_single_cta_tiles(api, O, m):
+    """Launches that begin while their predecessor drains: each layer quantises what the one before wrote into the same buffer,
+    on single-CTA tiles; the same numbers as with a synchronisation after every launch."""
+    k = 512
+    w = [api.quantize_128x128(T(O.fill_normal((k, k), 90 + j, 1))) for j in range(3)]
+    x0 = T(O.fill_normal((m, k), 89, 0)).bfloat16()
+
+    def layers(sync):
+        x = x0.clone()
+        for rep in range(4):
+            for b, sfb in w:
+                q, sfa = api.quantize_act_bf16_1x128(x)
+                if sync:
+                    torch.cuda.synchronize()
+                api.gemm_a8w8_blockscale(q, b, sfa, sfb, out=x, tile=1)
+                if sync:
+                    torch.cuda.synchronize()
+        return x
+
+    want, got = layers(True), layers(False)
+    status_ok(api)
+    assert torch.equal(got, want) and torch.isfinite(want.float()).all()
