@@ -8,6 +8,7 @@ import os
 import shutil
 import subprocess
 import sys
+from typing import Optional
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -58,13 +59,17 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
-def build_front(force: bool = False) -> str:
-    """The Python front end of the per-call operators (a CPython extension on torch's C++ tensors)."""
+def build_front(force: bool = False) -> Optional[str]:
+    """The Python front end of the per-call operators (a CPython extension on torch's C++ tensors).  Without torch there is
+    nothing for it to serve: the C ABI and the drivers are built and it is left out."""
+    try:
+        import torch
+    except ImportError as e:
+        print(f"_front.so, the front end of the Python operators, is not built: {e}")
+        return None
     src = os.path.join(CSRC, "front.cpp")
     if force or _newer(FRONT, [src, os.path.join(ROOT, "include", "b200gemm.h")]):
         import sysconfig
-
-        import torch
 
         troot = os.path.dirname(torch.__file__)
         nvcc_root = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))

@@ -266,3 +266,16 @@ def test_front_end_refuses_misuse(native, a, b, error, match):
         api._gemm(make(a), make(b))
     with pytest.raises(ValueError, match="2-D bf16"):
         api.quantize_act_bf16_1x128(torch.zeros(2, 128))
+
+
+def test_build_without_torch(native, monkeypatch, tmp_path, capsys):
+    """The C ABI and the drivers need no torch to be built; only the front end of the Python operators is left out."""
+    import sys
+
+    from gcnasm_b200 import build
+
+    monkeypatch.setitem(sys.modules, "torch", None)                  # import torch: ImportError
+    monkeypatch.setattr(build, "FRONT", str(tmp_path / "_front.so"))
+    lib, exes = build.build_all()
+    assert os.path.exists(lib) and len(exes) >= 4 and all(os.path.exists(e) for e in exes)
+    assert not os.path.exists(build.FRONT) and "not built" in capsys.readouterr().out
