@@ -68,7 +68,10 @@ def build_front(force: bool = False) -> Optional[str]:
         print(f"_front.so, the front end of the Python operators, is not built: {e}")
         return None
     src = os.path.join(CSRC, "front.cpp")
-    if force or _newer(FRONT, [src, os.path.join(ROOT, "include", "b200gemm.h")]):
+    # the binary fits one Python and one torch: those it was built for are noted beside it
+    made_for, tag = f"{sys.implementation.cache_tag} torch {torch.__version__}", FRONT + ".tag"
+    noted = open(tag).read() if os.path.exists(tag) else ""
+    if force or noted != made_for or _newer(FRONT, [src, os.path.join(ROOT, "include", "b200gemm.h")]):
         import sysconfig
 
         troot = os.path.dirname(torch.__file__)
@@ -79,6 +82,8 @@ def build_front(force: bool = False) -> Optional[str]:
             "-isystem", os.path.join(nvcc_root, "include"), "-isystem", sysconfig.get_paths()["include"], src, "-o", FRONT,
             "-L", os.path.join(troot, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
         ])
+        with open(tag, "w") as f:
+            f.write(made_for)
     return FRONT
 
 

@@ -279,3 +279,26 @@ def test_build_without_torch(native, monkeypatch, tmp_path, capsys):
     lib, exes = build.build_all()
     assert os.path.exists(lib) and len(exes) >= 4 and all(os.path.exists(e) for e in exes)
     assert not os.path.exists(build.FRONT) and "not built" in capsys.readouterr().out
+
+
+def test_front_end_is_rebuilt_for_another_torch(native, monkeypatch, tmp_path):
+    """_front.so fits one Python and one torch: the build makes it again when either has changed, and only then."""
+    import torch
+
+    from gcnasm_b200 import build
+
+    built = []
+
+    def compile_(cmd):
+        built.append(cmd)
+        open(build.FRONT, "w").close()
+
+    monkeypatch.setattr(build, "FRONT", str(tmp_path / "_front.so"))
+    monkeypatch.setattr(build.subprocess, "check_call", compile_)
+    for _ in range(2):
+        build.build_front()
+    assert len(built) == 1
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    for _ in range(2):
+        build.build_front()
+    assert len(built) == 2
