@@ -152,7 +152,10 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
     // Programmatic dependent launch: the next kernel on the stream may be scheduled as soon as every CTA of this
     // one has passed this point and an SM is free.  What THIS kernel may do before its own predecessor has
     // completed is decided by pdl_wait() below.
-    pdl_launch_dependents();
+    // Not while batches may still be on their way: blocks of a chained successor (an activation quantiser, another GEMM) would
+    // park in their own pdl_wait() on the SMs that a capped grid (B200GEMM_MAX_SMS) leaves free for the collective that
+    // delivers the batches, and the ready words could never be written.  The successor then starts at completion.
+    if (!p.batch_ready) pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(bar_full0 + s * 8, 1);          // leader's arrive.expect_tx; bytes from both CTAs

@@ -100,6 +100,75 @@ def test_batch_that_never_arrives_ends_as_a_status_code(api, O):
     assert_close(O, out.cpu().numpy().reshape(batch * m, n), O.gemm_ref_blockscale(a, b, sfa, sfb), "after the timeout")
 
 
+_SUCCESSOR_WORKER = """
+import sys, time
+sys.path[:0] = [{root!r}, {tests!r}]
+import torch
+from gcnasm_b200 import api
+from oracle import oracle as O
+from test_gpu_batch_ready import DEV, T, _slab_problem, _views, assert_close
+
+batch, m, n, k = 4, 512, 4096, 512                       # 128 tiles: every pair of the capped grid has one
+a, b, sfa, sfb, buf, slab_bytes = _slab_problem(O, batch, m, n, k, 45)
+a_v, sfa_v = _views(T(buf), batch, m, k, slab_bytes)
+b, sfb_d = T(b), T(sfb)
+ready = torch.zeros(batch, dtype=torch.int32, device=DEV)
+out = torch.zeros(batch, m, n, dtype=torch.float32, device=DEV)
+x = torch.ones(8192, 8192, dtype=torch.bfloat16, device=DEV)
+q, sc = torch.empty(8192, 8192, dtype=torch.uint8, device=DEV), torch.empty(64, 8192, dtype=torch.float32, device=DEV)
+data, word = torch.ones(1 << 22, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+main, side, writer = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream()
+
+def step(epoch, early):
+    with torch.cuda.stream(writer):
+        for s in range(batch if early else 1):
+            api.flag_write(ready, s, epoch)
+    writer.synchronize()
+    with torch.cuda.stream(main):
+        api.gemm_a8w8_blockscale(a_v, b, sfa_v, sfb_d, out=out, batch_ready=ready, batch_epoch=epoch)
+        api.quantize_act_bf16_1x128(x, q, sc)
+    time.sleep(0.05)
+    done = torch.cuda.Event()
+    with torch.cuda.stream(side):                        # blocks of 1024 threads: need an SM that nothing else fills
+        api.membw_read(data, word)
+        done.record()
+    end = time.time() + 0.7
+    while not done.query() and time.time() < end:
+        time.sleep(0.001)
+    ran = done.query()
+    with torch.cuda.stream(writer):                      # whatever happened, the words are written from here
+        for s in range(batch):
+            api.flag_write(ready, s, epoch)
+    torch.cuda.synchronize()
+    return ran
+
+torch.cuda.synchronize()
+step(1, True)                                            # everything is loaded and warm
+ran = step(2, False)
+assert api.last_status() == 0
+assert ran, "the kernel on the side stream found no SM while the GEMM waited for its batches"
+assert_close(O, out.cpu().numpy().reshape(batch * m, n), O.gemm_ref_blockscale(a, b.cpu().numpy(), sfa, sfb), "late batches")
+print("ok")
+"""
+
+
+def test_successor_leaves_the_free_sms_alone(native):
+    """A chained kernel behind a GEMM that waits for batches must not occupy the SMs which B200GEMM_MAX_SMS sets aside: a
+    kernel of another stream (where the collective would be) still runs there.  The words themselves are written by the
+    host in any case, 0.7 s later at most, and the GEMM's wait is bounded.  The cap is read once, hence the child process."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    tests = os.path.join(ROOT, "tests")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    r = subprocess.run([sys.executable, "-c", _SUCCESSOR_WORKER.format(root=ROOT, tests=tests)], cwd=tests, timeout=300,
+                       env=dict(os.environ, B200GEMM_MAX_SMS=str(sms - 16)), capture_output=True, text=True)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stdout[-1500:] + r.stderr[-3000:]
+
+
 def test_split_k_decode_on_two_streams(api, O):
     """Two skinny-M GEMMs that both split K run on two streams at once: each stream has its own workspace."""
     probs = []
