@@ -1010,11 +1010,9 @@ int b200_gemm_a8w8_simple(const b200_gemm_args* a, void* cuda_stream) {
 // End of the synchronous host-buffer entry: wait for the stream, then look at the status word, so that a launch
 // that gave up (an expired wait, a pair whose CTAs disagreed on their tensor-memory address) is an error HERE and
 // not a silently wrong C.  The word is left for b200_last_status() to report and clear.
-static int host_entry_finish(DeviceState* ds, cudaStream_t st) {
-    if (!ds->status_host) CU_TRY(cudaHostAlloc(&ds->status_host, sizeof(int), cudaHostAllocDefault));
+static int host_entry_finish(DeviceState* ds, HostCall& call, cudaStream_t st) {
     CU_TRY(cudaMemcpyAsync(ds->status_host, ds->status_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CU_TRY(ds->staging.finish_downloads());
-    CU_TRY(cudaStreamSynchronize(st));
+    CU_TRY(call.finish());
     return *ds->status_host == 0 ? B200_OK : B200_ERR_DEVICE_TIMEOUT;
 }
 
@@ -1076,8 +1074,22 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
     d.ptr_c = ds->buf[2];
     rc = validate(&d, ds->sm_count, &pl);
     if (rc) return rc;
+    // Large single-batch problems run as row slabs: the copy-back of slab i (the largest transfer of the call)
+    // proceeds on a second stream while slab i+1 is uploaded and computed, so the two PCIe directions overlap.
+    // (MX scale atoms are indexed by the full M, so MX problems take the single-shot path.)
+    const int64_t slab_rows = ((h->m + 7) / 8 + 255) / 256 * 256;
+    const bool slabs = h->batch == 1 && h->m >= 2048 && h->scale_mode != B200_SCALE_MX && (h->m + slab_rows - 1) / slab_rows <= 16;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (slabs && !ds->copy_stream) {
+            CU_TRY(cudaStreamCreateWithFlags(&ds->copy_stream, cudaStreamNonBlocking));
+            for (auto& e : ds->slab_done) CU_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            CU_TRY(cudaEventCreateWithFlags(&ds->copies_done, cudaEventDisableTiming));
+        }
+        if (!ds->status_host) CU_TRY(cudaHostAlloc(&ds->status_host, sizeof(int), cudaHostAllocDefault));
+    }
     Staging& io = ds->staging;
-    io.abandon();
+    HostCall call(io, st, ds->copy_stream);              // from here on every way out waits for what has been queued
     CU_TRY(io.upload(ds->buf[1], h->ptr_b, b_bytes, st));
     if (sfa_bytes) {
         CU_TRY(io.upload(ds->buf[3], h->ptr_sfa, sfa_bytes, st));
@@ -1096,25 +1108,12 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
             d.ptr_scale_b = sc + 1;
         }
     }
-    // Large single-batch problems run as row slabs: the copy-back of slab i (the largest transfer of the call)
-    // proceeds on a second stream while slab i+1 is uploaded and computed, so the two PCIe directions overlap.
-    // (MX scale atoms are indexed by the full M, so MX problems take the single-shot path.)
-    const int64_t slab_rows = ((h->m + 7) / 8 + 255) / 256 * 256;
-    const bool slabs = h->batch == 1 && h->m >= 2048 && h->scale_mode != B200_SCALE_MX && (h->m + slab_rows - 1) / slab_rows <= 16;
     if (!slabs) {
         CU_TRY(io.upload(ds->buf[0], h->ptr_a, a_bytes, st));
         rc = b200_gemm_a8w8(&d, st);
         if (rc) return rc;
         CU_TRY(io.download(h->ptr_c, ds->buf[2], c_bytes, st));
-        return host_entry_finish(ds, st);
-    }
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        if (!ds->copy_stream) {
-            CU_TRY(cudaStreamCreateWithFlags(&ds->copy_stream, cudaStreamNonBlocking));
-            for (auto& e : ds->slab_done) CU_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            CU_TRY(cudaEventCreateWithFlags(&ds->copies_done, cudaEventDisableTiming));
-        }
+        return host_entry_finish(ds, call, st);
     }
     int slab = 0;
     for (int64_t r0 = 0; r0 < h->m; r0 += slab_rows, ++slab) {
@@ -1135,7 +1134,7 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
     }
     CU_TRY(cudaEventRecord(ds->copies_done, ds->copy_stream));
     CU_TRY(cudaStreamWaitEvent(st, ds->copies_done, 0));
-    return host_entry_finish(ds, st);
+    return host_entry_finish(ds, call, st);
 }
 
 // ---- layout ----------------------------------------------------------------------------------------

@@ -219,7 +219,17 @@ public:
         for (auto& j : down_job_) CopyPool::get().wait(j);
         return e;
     }
-    void abandon() { posted_ = issued_ = 0; }            // a call that failed leaves nothing behind
+    // The end of a call that failed half way: waits for what its streams hold (copies into the ring and into pinned memory)
+    // and for the pieces that copy threads still move, so that nothing touches the caller's memory or the ring any
+    // more.  Results that only reached the ring are dropped.
+    void settle(cudaStream_t st, cudaStream_t copies) {
+        cudaStreamSynchronize(st);
+        if (copies) cudaStreamSynchronize(copies);
+        cudaGetLastError();
+        for (auto& j : up_job_) CopyPool::get().wait(j);
+        for (auto& j : down_job_) CopyPool::get().wait(j);
+        posted_ = issued_ = 0;
+    }
     void release() {
         if (!ring_) return;
         cudaFreeHost(ring_);
@@ -267,6 +277,29 @@ private:
     unsigned up_next_ = 0, issued_ = 0, posted_ = 0;     // chunks: of all uploads; results whose DMA is queued; ... handed to the pool
     uint8_t* down_to_[kDown] = {};
     size_t down_bytes_[kDown] = {};
+};
+
+// One call through the ring, on stream `st` and, for results, `copies` (or null).  Whichever way the call ends, nothing of it
+// is left running: finish() on the way that succeeds, the destructor on every other one.
+class HostCall {
+public:
+    HostCall(Staging& io, cudaStream_t st, cudaStream_t copies) : io_(io), st_(st), copies_(copies) {}
+    HostCall(const HostCall&) = delete;
+    ~HostCall() {
+        if (!finished_) io_.settle(st_, copies_);
+    }
+    // The results are in the caller's memory and `st`, which waits for `copies`, is idle.
+    cudaError_t finish() {
+        cudaError_t e = io_.finish_downloads();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+        finished_ = e == cudaSuccess;
+        return e;
+    }
+
+private:
+    Staging& io_;
+    cudaStream_t st_, copies_;
+    bool finished_ = false;
 };
 
 }  // namespace b200

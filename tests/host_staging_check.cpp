@@ -1,0 +1,86 @@
+// Scenarios for csrc/host_staging.h on the CPU, against the stand-in runtime of fake_cuda/cuda_runtime.h.
+#include "host_staging.h"
+
+#include <cstdio>
+#include <string>
+
+using namespace b200;
+using Bytes = std::vector<uint8_t>;
+
+#define CHECK(cond)                                                     \
+    do {                                                                \
+        if (!(cond)) {                                                  \
+            std::printf("line %d: %s\n", __LINE__, #cond);              \
+            return 1;                                                   \
+        }                                                               \
+    } while (0)
+
+static Bytes pattern(size_t n, unsigned seed) {
+    Bytes b(n);
+    for (size_t i = 0; i < n; ++i) b[i] = static_cast<uint8_t>((i * 2654435761u + seed * 40503u) >> 13);
+    return b;
+}
+
+// One call as the host entry makes it: up on `up`, "compute" by leaving the bytes as they are, down on `down` in slabs.
+static cudaError_t call(Staging& io, fake::Stream& up, fake::Stream& down, const Bytes& in, Bytes& dev, uint8_t* out, size_t slab) {
+    HostCall host(io, &up, &down);
+    cudaError_t e = io.upload(dev.data(), in.data(), in.size(), &up);
+    if (e != cudaSuccess) return e;
+    cudaStreamSynchronize(&up);
+    for (size_t at = 0; at < in.size(); at += slab) {
+        const size_t n = in.size() - at < slab ? in.size() - at : slab;
+        if ((e = io.download(out + at, dev.data() + at, n, &down)) != cudaSuccess) return e;
+    }
+    return host.finish();
+}
+
+static const size_t kSizes[] = {1, 4095, 65537, Staging::kChunk - 1, Staging::kChunk, 5 * Staging::kChunk + 13, 21 * Staging::kChunk + 1};
+
+static int round_trip() {
+    Staging io;
+    fake::Stream up, down;
+    for (size_t n : kSizes) {
+        const Bytes in = pattern(n, 1);
+        Bytes dev(n), out(n);
+        CHECK(call(io, up, down, in, dev, out.data(), 3 * Staging::kChunk + 77) == cudaSuccess);
+        CHECK(out == in);
+    }
+    io.release();
+    CHECK(fake::live_events == 0 && fake::live_host == 0);
+    return 0;
+}
+
+// A call that fails half way leaves nothing running: no copy is pending on a stream, the caller's memory changes no more,
+// and the next call, on other streams, is correct.
+static int failed_call() {
+    const size_t n = 20 * Staging::kChunk + 5;
+    const Bytes in = pattern(n, 2);
+    for (int good : {0, 3, 21, 24, 30, 38}) {            // copies that still go out: 21 up, 21 down
+        Staging io;
+        fake::Stream up, down;
+        Bytes dev(n), out(n);
+        fake::delay_us = 3000;
+        fake::fail_copy_in = good;
+        CHECK(call(io, up, down, in, dev, out.data(), n) == cudaErrorInvalidValue);
+        CHECK(fake::queued == 0);
+        const Bytes then = out;
+        std::this_thread::sleep_for(std::chrono::milliseconds(60));
+        CHECK(out == then);
+        fake::delay_us = 100;
+        const Bytes in2 = pattern(n, 3);
+        CHECK(call(io, down, up, in2, dev, out.data(), n) == cudaSuccess);
+        CHECK(out == in2);
+        io.release();
+    }
+    return 0;
+}
+
+int main(int, char** argv) {
+    const std::string what = argv[1];
+    int rc = 2;
+    if (what == "round_trip") rc = round_trip();
+    if (what == "failed_call") rc = failed_call();
+    CopyPool::get().release();
+    if (rc == 0) std::printf("ok\n");
+    return rc;
+}
