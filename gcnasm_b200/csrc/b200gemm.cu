@@ -1011,9 +1011,11 @@ int b200_gemm_a8w8_simple(const b200_gemm_args* a, void* cuda_stream) {
 // that gave up (an expired wait, a pair whose CTAs disagreed on their tensor-memory address) is an error HERE and
 // not a silently wrong C.  The word is left for b200_last_status() to report and clear.
 static int host_entry_finish(DeviceState* ds, HostCall& call, cudaStream_t st) {
-    CU_TRY(cudaMemcpyAsync(ds->status_host, ds->status_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    int unpinned = 0;                                    // (no pinned word to be had: the copy then waits for the stream)
+    int* v = ds->status_host ? ds->status_host : &unpinned;
+    CU_TRY(cudaMemcpyAsync(v, ds->status_ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(call.finish());
-    return *ds->status_host == 0 ? B200_OK : B200_ERR_DEVICE_TIMEOUT;
+    return *v == 0 ? B200_OK : B200_ERR_DEVICE_TIMEOUT;
 }
 
 // a * b for non-negative operands, or -1 when the product does not fit in 2^46 bytes (64 TiB: far above any device)
@@ -1086,7 +1088,10 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
             for (auto& e : ds->slab_done) CU_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             CU_TRY(cudaEventCreateWithFlags(&ds->copies_done, cudaEventDisableTiming));
         }
-        if (!ds->status_host) CU_TRY(cudaHostAlloc(&ds->status_host, sizeof(int), cudaHostAllocDefault));
+        if (!ds->status_host && cudaHostAlloc(&ds->status_host, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            ds->status_host = nullptr;
+        }
     }
     Staging& io = ds->staging;
     HostCall call(io, st, ds->copy_stream);              // from here on every way out waits for what has been queued

@@ -171,8 +171,8 @@ public:
     }
     // Queued on `st`; the caller's memory has been read when this returns, or (pinned memory) when the stream gets there.
     cudaError_t upload(void* dev, const void* host, size_t n, cudaStream_t st) {
-        if (!pageable(host)) return cudaMemcpyAsync(dev, host, n, cudaMemcpyHostToDevice, st);
-        cudaError_t e = prepare();
+        if (!pageable(host) || !prepare()) return cudaMemcpyAsync(dev, host, n, cudaMemcpyHostToDevice, st);
+        cudaError_t e = cudaSuccess;
         const size_t chunks = (n + kChunk - 1) / kChunk;
         const unsigned first = up_next_;
         auto bytes = [&](size_t i) { return n - i * kChunk < kChunk ? n - i * kChunk : kChunk; };
@@ -196,8 +196,8 @@ public:
     }
     // Queued on `st`; what goes through the ring is in the caller's memory after finish_downloads().
     cudaError_t download(void* host, const void* dev, size_t n, cudaStream_t st) {
-        if (!pageable(host)) return cudaMemcpyAsync(host, dev, n, cudaMemcpyDeviceToHost, st);
-        cudaError_t e = prepare();
+        if (!pageable(host) || !prepare()) return cudaMemcpyAsync(host, dev, n, cudaMemcpyDeviceToHost, st);
+        cudaError_t e = cudaSuccess;
         for (size_t at = 0; at < n && e == cudaSuccess; at += kChunk) {
             const size_t c = n - at < kChunk ? n - at : kChunk;
             const int slot = issued_ % kDown;
@@ -231,22 +231,30 @@ public:
         posted_ = issued_ = 0;
     }
     void release() {
-        if (!ring_) return;
-        cudaFreeHost(ring_);
-        for (auto& e : up_free_) cudaEventDestroy(e);
-        for (auto& e : down_done_) cudaEventDestroy(e);
+        auto destroy = [](cudaEvent_t& e) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        };
+        for (auto& e : up_free_) destroy(e);
+        for (auto& e : down_done_) destroy(e);
+        if (ring_) cudaFreeHost(ring_);
         ring_ = nullptr;
     }
 
 private:
-    cudaError_t prepare() {
-        if (ring_) return cudaSuccess;
+    // False where there is no pinned memory to be had (a process near its limit on locked memory): the driver then stages
+    // the copies, slower, and the next call asks again.
+    bool prepare() {
+        if (ring_) return true;
         void* p = nullptr;
         cudaError_t e = cudaHostAlloc(&p, (kUp + kDown) * kChunk, cudaHostAllocDefault);
+        if (e == cudaSuccess) ring_ = static_cast<uint8_t*>(p);
         for (int i = 0; i < kUp && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&up_free_[i], cudaEventDisableTiming);
         for (int i = 0; i < kDown && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&down_done_[i], cudaEventDisableTiming);
-        if (e == cudaSuccess) ring_ = static_cast<uint8_t*>(p);
-        return e;
+        if (e == cudaSuccess) return true;
+        cudaGetLastError();
+        release();
+        return false;
     }
     // result chunks that have arrived in the ring go to the pool
     cudaError_t post_arrived() {

@@ -22,6 +22,7 @@ namespace fake {
 inline std::atomic<int> fail_copy_in{-1}, fail_event_in{-1}, fail_host_alloc_in{-1};       // calls that still succeed; -1: all
 inline std::atomic<int> live_events{0}, live_host{0}, queued{0};
 inline std::atomic<int> delay_us{200};                                                       // of every copy
+inline std::atomic<bool> pageable_copies_wait{false};                                        // a copy is complete when its call returns
 inline bool fails(std::atomic<int>& left) { return left.load() >= 0 && left.fetch_sub(1) == 0; }
 
 struct Stream {
@@ -119,5 +120,6 @@ inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyK
         std::this_thread::sleep_for(std::chrono::microseconds(fake::delay_us.load()));
         std::memcpy(d, s, n);
     });
+    if (fake::pageable_copies_wait) st->drain();
     return cudaSuccess;
 }

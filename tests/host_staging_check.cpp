@@ -75,11 +75,42 @@ static int failed_call() {
     return 0;
 }
 
+// Where there is no pinned memory, or no event, the copies go the driver's way; nothing is lost, and a later call gets its ring.
+static int no_ring() {
+    const size_t n = 5 * Staging::kChunk + 13;
+    const Bytes in = pattern(n, 4);
+    for (int event : {-1, 0, 3, 4, 11}) {                // events that can still be made; -1: no pinned memory
+        Staging io;
+        fake::Stream up, down;
+        Bytes dev(n), out(n), again(n);
+        fake::pageable_copies_wait = true;
+        for (int i = 0; i < 2; ++i) {
+            (event < 0 ? fake::fail_host_alloc_in : fake::fail_event_in) = event < 0 ? 0 : event;
+            Bytes got(n);
+            HostCall host(io, &up, &down);
+            CHECK(io.upload(dev.data(), in.data(), n, &up) == cudaSuccess);
+            CHECK(fake::live_events == 0 && fake::live_host == 0);
+            (event < 0 ? fake::fail_host_alloc_in : fake::fail_event_in) = event < 0 ? 0 : event;
+            CHECK(io.download(got.data(), dev.data(), n, &down) == cudaSuccess);
+            CHECK(fake::live_events == 0 && fake::live_host == 0);
+            CHECK(host.finish() == cudaSuccess);
+            CHECK(got == in);
+        }
+        fake::pageable_copies_wait = false;
+        CHECK(call(io, up, down, in, dev, again.data(), n) == cudaSuccess);
+        CHECK(again == in && fake::live_host == 1 && fake::live_events == Staging::kUp + Staging::kDown);
+        io.release();
+        CHECK(fake::live_events == 0 && fake::live_host == 0);
+    }
+    return 0;
+}
+
 int main(int, char** argv) {
     const std::string what = argv[1];
     int rc = 2;
     if (what == "round_trip") rc = round_trip();
     if (what == "failed_call") rc = failed_call();
+    if (what == "no_ring") rc = no_ring();
     CopyPool::get().release();
     if (rc == 0) std::printf("ok\n");
     return rc;
