@@ -14,8 +14,8 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
-#include <deque>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -24,7 +24,8 @@ namespace b200 {
 struct CopyJob {
     uint8_t* dst = nullptr;
     const uint8_t* src = nullptr;
-    size_t n = 0, taken = 0;                             // taken: under the pool's lock
+    size_t n = 0, taken = 0;                             // taken and next: under the pool's lock
+    CopyJob* next = nullptr;
     std::atomic<size_t> left{0};
 };
 
@@ -34,7 +35,8 @@ struct CopyJob {
 class CopyPool {
 public:
     static CopyPool& get() {
-        static CopyPool* p = new CopyPool;               // never destroyed: threads may outlive static destructors
+        alignas(CopyPool) static unsigned char room[sizeof(CopyPool)];
+        static CopyPool* p = new (room) CopyPool;        // never destroyed: threads may outlive static destructors
         return *p;
     }
     void post(CopyJob& j, void* dst, const void* src, size_t n) {
@@ -42,10 +44,12 @@ public:
         j.src = static_cast<const uint8_t*>(src);
         j.n = n;
         j.taken = 0;
+        j.next = nullptr;
         j.left.store(n, std::memory_order_relaxed);
         if (n == 0) return;
         lock();
-        queue_.push_back(&j);
+        (first_ ? last_->next : first_) = &j;            // (linked through the jobs: nothing here can fail)
+        last_ = &j;
         queued_.fetch_add(1, std::memory_order_release);
         unlock();
         if (n < kWakeFrom) return;                       // the caller, waiting for it, does it alone
@@ -108,15 +112,15 @@ private:
     bool step() {
         if (queued_.load(std::memory_order_acquire) == 0) return false;
         lock();
-        if (queue_.empty()) {
+        CopyJob* j = first_;
+        if (!j) {
             unlock();
             return false;
         }
-        CopyJob* j = queue_.front();
         const size_t at = j->taken, c = j->n - at < kPiece ? j->n - at : kPiece;
         j->taken += c;
         if (j->taken == j->n) {
-            queue_.pop_front();
+            first_ = j->next;
             queued_.fetch_sub(1, std::memory_order_relaxed);
         }
         unlock();
@@ -145,8 +149,8 @@ private:
         std::memcpy(d, s, n);
     }
 
-    std::atomic_flag flag_ = ATOMIC_FLAG_INIT;           // guards queue_ and the jobs' `taken`
-    std::deque<CopyJob*> queue_;
+    std::atomic_flag flag_ = ATOMIC_FLAG_INIT;           // guards the queue and the jobs' `taken`
+    CopyJob *first_ = nullptr, *last_ = nullptr;         // the queue, oldest first
     std::atomic<unsigned> queued_{0}, generation_{0};
     std::mutex mu_;                                      // guards threads_ and asleep_
     std::condition_variable wake_;

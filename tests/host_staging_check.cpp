@@ -2,7 +2,18 @@
 #include "host_staging.h"
 
 #include <cstdio>
+#include <deque>
+#include <new>
 #include <string>
+
+static thread_local bool t_no_memory = false;
+void* operator new(size_t n) {
+    void* p = t_no_memory ? nullptr : std::malloc(n);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 using namespace b200;
 using Bytes = std::vector<uint8_t>;
@@ -105,12 +116,26 @@ static int no_ring() {
     return 0;
 }
 
+// Posting copies needs no memory: the host entry is called through a C ABI, which no exception may leave.
+static int no_memory() {
+    const Bytes in = pattern(200 * 1024, 5);
+    std::deque<CopyJob> jobs(2000);
+    Bytes out(in.size() + jobs.size());
+    t_no_memory = true;
+    for (size_t i = 0; i < jobs.size(); ++i) CopyPool::get().post(jobs[i], out.data() + i, in.data(), i == 0 ? in.size() : 1);
+    for (auto& j : jobs) CopyPool::get().wait(j);
+    t_no_memory = false;
+    CHECK(std::memcmp(out.data() + jobs.size(), in.data() + jobs.size(), in.size() - jobs.size()) == 0);
+    return 0;
+}
+
 int main(int, char** argv) {
     const std::string what = argv[1];
     int rc = 2;
     if (what == "round_trip") rc = round_trip();
     if (what == "failed_call") rc = failed_call();
     if (what == "no_ring") rc = no_ring();
+    if (what == "no_memory") rc = no_memory();
     CopyPool::get().release();
     if (rc == 0) std::printf("ok\n");
     return rc;

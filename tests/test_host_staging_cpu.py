@@ -19,7 +19,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["round_trip", "failed_call", "no_ring"])
+@pytest.mark.parametrize("scenario", ["round_trip", "failed_call", "no_ring", "no_memory"])
 def test_host_staging(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.endswith("ok\n"), r.stdout + r.stderr
