@@ -1046,6 +1046,11 @@ int b200_gemm_a8w8_host(const b200_gemm_args* h, void* cuda_stream) {
         if (h->b_layout == B200_B_NK_ROWMAJOR && h->stride_b < h->k) return B200_ERR_BAD_ARG;
     }
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
+    // A call that returns finished results cannot be captured.  Refused before the ring's events are recorded: an event that
+    // was last recorded inside a capture fails every later wait for it.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    CU_TRY(cudaStreamIsCapturing(st, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) CU_TRY(cudaErrorStreamCaptureUnsupported);
     const int64_t esz = h->out_dtype == B200_OUT_BF16 ? 2 : 4;
     const int64_t a_sz = h->batch > 1 ? mul_checked(h->stride_a_batch, h->batch) : mul_checked(h->stride_a, h->m);
     const int64_t b_sz = h->batch > 1 ? mul_checked(h->stride_b_batch, h->batch)

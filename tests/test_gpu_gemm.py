@@ -350,6 +350,31 @@ def test_host_entry_staging_ring(api, O, m, pinned):
         assert np.array_equal(c, want)
 
 
+def test_host_entry_inside_a_capture_is_refused(api, O):
+    """It returns finished results, so it cannot be captured; the refusal leaves the capture and the entry's ring usable."""
+    from gcnasm_b200 import B200Error
+
+    m, n, k = 40, 4096, 2304
+    a, b = e4m3(O, (m, k), 15, 0, 0.0, 1.0), e4m3(O, (n, k), 15, 1, -0.5, 0.5)
+    want = api.gemm_a8w8(T(a), T(b), out_dtype=torch.float32, tile=1).cpu().numpy()
+    c = np.zeros((m, n), np.float32)
+    api.gemm_a8w8_host(a, b, c, tile=1)
+    x = torch.zeros(4, device=DEV)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        x += 1
+        with pytest.raises(B200Error):
+            api.gemm_a8w8_host(a, b, c, tile=1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 4
+    for _ in range(2):
+        c[:] = np.nan
+        api.gemm_a8w8_host(a, b, c, tile=1)
+        assert np.array_equal(c, want)
+
+
 @pytest.mark.parametrize("m", [65, 100])
 def test_chained_layers_on_single_cta_tiles(api, O, m):
     """Launches that begin while their predecessor drains: each layer quantises what the one before wrote into the same buffer,
