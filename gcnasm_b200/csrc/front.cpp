@@ -231,7 +231,8 @@ PyObject* front_gemm(PyObject*, PyObject* const* v, Py_ssize_t nargs) {
         void* st = stream();
         const int rc = unlocked([&] { return fn(&g, st); });
         if (rc) return PyLong_FromLong(rc);
-        if (a.dim() == 2 && out.dim() == 3) out = out.select(0, 0);
+        if (a.dim() == 2 && out.dim() == 3) out = out.select(0, 0);       // the result has as many dimensions as A
+        else if (a.dim() == 3 && out.dim() == 2) out = out.unsqueeze(0);
         return THPVariable_Wrap(out);
     });
 }

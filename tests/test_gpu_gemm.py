@@ -375,6 +375,19 @@ def test_host_entry_inside_a_capture_is_refused(api, O):
         assert np.array_equal(c, want)
 
 
+@pytest.mark.parametrize("a_dims", [2, 3])
+@pytest.mark.parametrize("out_dims", [2, 3])
+def test_result_has_the_dimensions_of_a(api, O, a_dims, out_dims):
+    """One batch, with or without its dimension, in A and in a given ``out``: the result is a view of ``out`` like A."""
+    m, n, k = 100, 64, 128
+    a, b = T(e4m3(O, (m, k), 16, 0, 0.0, 1.0)), T(e4m3(O, (n, k), 16, 1, -0.5, 0.5))
+    want = api.gemm_a8w8(a, b)
+    out = torch.zeros(m, n, dtype=torch.bfloat16, device=DEV)
+    r = api.gemm_a8w8(a if a_dims == 2 else a[None], b, out=out if out_dims == 2 else out[None])
+    assert r.shape == ((m, n) if a_dims == 2 else (1, m, n)) and r.data_ptr() == out.data_ptr()
+    assert torch.equal(out, want) and torch.equal(r.reshape(m, n), want)
+
+
 @pytest.mark.parametrize("m", [65, 100])
 def test_chained_layers_on_single_cta_tiles(api, O, m):
     """Launches that begin while their predecessor drains: each layer quantises what the one before wrote into the same buffer,
