@@ -61,13 +61,14 @@ def _as_u8(t: torch.Tensor, what: str) -> torch.Tensor:
 
 def _gemm(a, b, *, n=None, sfa=None, sfb=None, scale_a=None, scale_b=None, scale_mode=L.SCALE_NONE,
           b_layout=L.B_NK_ROWMAJOR, out=None, out_dtype=torch.bfloat16, tile=L.TILE_AUTO, simple=False, inputs_ready=False,
-          batch_ready=None, batch_epoch=0, where="b200_gemm_a8w8"):
+          batch_ready=None, batch_epoch=0, bf16=False):
     """Checks, output allocation, argument block and launch happen in the native front end (``csrc/front.cpp``): the same
     work costs more in the interpreter than a small GEMM takes on the GPU."""
+    entry = 2 if bf16 else (1 if simple else 0)
     r = (_bound or front()).gemm(a, b, out, sfa, sfb, scale_a, scale_b, batch_ready, n, scale_mode, b_layout, out_dtype, tile,
-                                 L.GEMM_INPUTS_READY if inputs_ready else 0, batch_epoch, simple)
+                                 L.GEMM_INPUTS_READY if inputs_ready else 0, batch_epoch, entry)
     if type(r) is int:
-        check(r, where + "_simple" if simple else where)
+        check(r, ("b200_gemm_a8w8", "b200_gemm_a8w8_simple", "b200_gemm_a16w16")[entry])
     return r
 
 
@@ -236,7 +237,7 @@ def gemm_a16w16(a, b, scale_a=None, scale_b=None, *, n=None, flat=False, out=Non
         raise TypeError("A and B must be torch.bfloat16")
     mode = L.SCALE_TENSOR if (scale_a is not None or scale_b is not None) else L.SCALE_NONE
     return _gemm(a, b, n=n, scale_a=scale_a, scale_b=scale_b, scale_mode=mode, out=out, out_dtype=out_dtype, tile=tile,
-                 b_layout=L.B_FLAT_16x16 if flat else L.B_NK_ROWMAJOR, where="b200_gemm_a16w16")
+                 b_layout=L.B_FLAT_16x16 if flat else L.B_NK_ROWMAJOR, bf16=True)
 
 
 def shuffle_b_bf16(b: torch.Tensor, src: str = "kn") -> torch.Tensor:

@@ -126,15 +126,17 @@ void tensor_scale(const at::Tensor* t, const float** slot) {
     *slot = static_cast<const float*>(t->const_data_ptr());
 }
 
-// gemm(a, b, out, sfa, sfb, scale_a, scale_b, batch_ready, n, scale_mode, b_layout, out_dtype, tile, flags, epoch, simple)
-// bf16 operands (the a16w16 sibling) take the same path; A's type decides.
+// gemm(a, b, out, sfa, sfb, scale_a, scale_b, batch_ready, n, scale_mode, b_layout, out_dtype, tile, flags, epoch, entry)
+// entry: 0 b200_gemm_a8w8, 1 b200_gemm_a8w8_simple, 2 b200_gemm_a16w16 (bf16 operands).
 PyObject* front_gemm(PyObject*, PyObject* const* v, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         if (nargs != 16) type_error("gemm takes 16 arguments");
         const at::Tensor &a = tensor(v[0], "A must be a tensor"), &b = tensor(v[1], "B must be a tensor");
-        const bool ab16 = a.scalar_type() == at::kBFloat16;
-        if (ab16 ? b.scalar_type() != at::kBFloat16 : !(is_e4m3(a) && is_e4m3(b)))
-            type_error(ab16 ? "A and B must be torch.bfloat16" : "A and B must hold E4M3 bytes (uint8 or float8_e4m3fn)");
+        const int64_t entry = integer(v[15]);
+        const bool ab16 = entry == 2;
+        if (ab16 ? a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16 : !(is_e4m3(a) && is_e4m3(b)))
+            type_error(ab16 ? "A and B must be torch.bfloat16"
+                            : "A and B must hold E4M3 bytes: uint8 or float8_e4m3fn (torch.bfloat16 operands: gemm_a16w16)");
         const at::Tensor *out_in = opt_tensor(v[2], "out must be a tensor"), *sfa = opt_tensor(v[3], "SFA must be a tensor"),
                          *sfb = opt_tensor(v[4], "SFB must be a tensor"), *sca = opt_tensor(v[5], "scale_a must be a tensor"),
                          *scb = opt_tensor(v[6], "scale_b must be a tensor"), *ready = opt_tensor(v[7], "batch_ready must be a tensor");
@@ -227,7 +229,7 @@ PyObject* front_gemm(PyObject*, PyObject* const* v, Py_ssize_t nargs) {
             g.ptr_batch_ready = static_cast<const int32_t*>(ready->const_data_ptr());
             g.batch_epoch = static_cast<int32_t>(integer(v[14]));
         }
-        const GemmFn fn = ab16 ? g_gemm16 : (v[15] == Py_True ? g_gemm_simple : g_gemm);
+        const GemmFn fn = ab16 ? g_gemm16 : (entry == 1 ? g_gemm_simple : g_gemm);
         void* st = stream();
         const int rc = unlocked([&] { return fn(&g, st); });
         if (rc) return PyLong_FromLong(rc);

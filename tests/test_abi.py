@@ -302,3 +302,25 @@ def test_front_end_is_rebuilt_for_another_torch(native, monkeypatch, tmp_path):
     for _ in range(2):
         build.build_front()
     assert len(built) == 2
+
+
+@pytest.mark.parametrize("call", [
+    lambda api, a, b: api.gemm_a8w8(a, b),
+    lambda api, a, b: api.gemm_a8w8(a, b, simple=True),
+    lambda api, a, b: api.gemm_a8w8_blockscale(a, b, None, None),
+    lambda api, a, b: api.flatmm_a8w8(a, b, 128),
+    lambda api, a, b: api.gemm_a8w8_mx(a, b, None, None),
+])
+def test_8bit_operators_refuse_bf16_operands(native, call):
+    """Only gemm_a16w16 takes bf16 operands; the type is looked at before the device, so this needs no GPU."""
+    import torch
+
+    from gcnasm_b200 import api
+
+    x = torch.zeros(128, 128, dtype=torch.bfloat16)
+    with pytest.raises(TypeError, match="E4M3"):
+        call(api, x, x)
+    with pytest.raises(TypeError, match="bfloat16"):
+        api.gemm_a16w16(x, x.to(torch.uint8))
+    with pytest.raises(ValueError, match="CUDA"):
+        api.gemm_a16w16(x, x)
