@@ -66,7 +66,7 @@ def _gemm(a, b, *, n=None, sfa=None, sfb=None, scale_a=None, scale_b=None, scale
     work costs more in the interpreter than a small GEMM takes on the GPU."""
     entry = 2 if bf16 else (1 if simple else 0)
     r = (_bound or front()).gemm(a, b, out, sfa, sfb, scale_a, scale_b, batch_ready, n, scale_mode, b_layout, out_dtype, tile,
-                                 L.GEMM_INPUTS_READY if inputs_ready else 0, batch_epoch, entry)
+                                 L.GEMM_INPUTS_READY if inputs_ready else 0, int(batch_epoch) if batch_ready is not None else 0, entry)
     if type(r) is int:
         check(r, ("b200_gemm_a8w8", "b200_gemm_a8w8_simple", "b200_gemm_a16w16")[entry])
     return r

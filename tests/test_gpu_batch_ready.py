@@ -80,6 +80,17 @@ def test_batch_ready_words_set_beforehand_and_by_flag_write(api, O):
     assert_close(O, out.cpu().numpy().reshape(batch * m, n), ref, "ready words, epoch 5 <= 7")
 
 
+@pytest.mark.parametrize("epoch", [3.0, np.float32(3), np.int32(3), torch.tensor(3)])
+def test_batch_epoch_is_any_number(api, O, epoch):
+    batch, m, n, k = 2, 256, 256, 256
+    a, b, sfa, sfb, buf, slab_bytes = _slab_problem(O, batch, m, n, k, 46)
+    a_v, sfa_v = _views(T(buf), batch, m, k, slab_bytes)
+    ready = torch.full((batch,), 3, dtype=torch.int32, device=DEV)
+    out = api.gemm_a8w8_blockscale(a_v, T(b), sfa_v, T(sfb), out_dtype=torch.float32, batch_ready=ready, batch_epoch=epoch)
+    status_ok(api)
+    assert_close(O, out.cpu().numpy().reshape(batch * m, n), O.gemm_ref_blockscale(a, b, sfa, sfb), "epoch as a number")
+
+
 def test_batch_that_never_arrives_ends_as_a_status_code(api, O):
     """A ready word that nothing sets: the launch gives up after its bounded wait (about 2 s), the status word says
     which wait it was, and the context stays usable."""
