@@ -386,11 +386,13 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
             const size_t o = static_cast<size_t>(b) * p.c_batch + static_cast<size_t>(j) * p.ldc + ni * BNW + lane;
 #pragma unroll
             for (int c = 0; c < BNW / 32; ++c) {
-                if (ni * BNW + c * 32 + lane >= p.n) continue;
-                if (p.out_dtype == OUT_BF16) reinterpret_cast<__nv_bfloat16*>(p.c)[o + c * 32] = __float2bfloat16_rn(sum[c]);
-                else reinterpret_cast<float*>(p.c)[o + c * 32] = sum[c];
+                if (ni * BNW + c * 32 + lane < p.n) {
+                    if (p.out_dtype == OUT_BF16) reinterpret_cast<__nv_bfloat16*>(p.c)[o + c * 32] = __float2bfloat16_rn(sum[c]);
+                    else reinterpret_cast<float*>(p.c)[o + c * 32] = sum[c];
+                }
             }
         }
+        __syncwarp();              // (the lanes of a ragged panel part above; the barrier wants the warp together)
         cluster_arrive();          // no CTA leaves while another one reads its partials
         cluster_wait();
     }
