@@ -372,6 +372,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
         __syncwarp();
         cluster_arrive();
         cluster_wait();
+        // A split that gave up (an expired wait) has no sums to add: the panel is left unwritten then, as without a cluster.
+        // Asked for first and looked at after the first row's sums, whose loads cover it.
+        const uint32_t gave_up = lane < p.splits ? ld_shared_cluster_u32(mapa_shared(smem_u32(tmem_slot + 1), lane)) : 0u;
         for (int j = split + warp * p.splits; j < p.m; j += p.splits * (Cfg::THREADS / 32)) {
             const uint32_t row = smem_base + static_cast<uint32_t>(j * BNW + lane) * 4;
             float sum[BNW / 32];
@@ -383,6 +386,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
 #pragma unroll
                 for (int c = 0; c < BNW / 32; ++c) sum[c] += __uint_as_float(ld_shared_cluster_u32(src + c * 128));
             }
+            if (__any_sync(0xFFFFFFFFu, gave_up != 0u)) break;
             const size_t o = static_cast<size_t>(b) * p.c_batch + static_cast<size_t>(j) * p.ldc + ni * BNW + lane;
 #pragma unroll
             for (int c = 0; c < BNW / 32; ++c) {
