@@ -191,7 +191,8 @@ void orc_quant_128x128(const float *x, int N, int K, uint8_t *q, float *sfb) {
 
 /* MX 1x32: shared exponent e = floor(log2(amax)) - 8 (8 = emax of E4M3), stored as the
  * E8M0 byte clamp(e+127, 0, 254); elements are e4m3(x * 2^-e) with saturation.  An
- * all-zero block stores byte 0 and zero elements.  (The repository's only E8M0 code,
+ * all-zero block stores byte 0 and zero elements, one with an infinite value byte 254 (the
+ * clamp of a logarithm without bound).  (The repository's only E8M0 code,
  * mla_agentic_v0/flash_mla/quant.py:28-37, rounds the exponent UP and is not followed.)   */
 void orc_quant_mx32(const float *x, int R, int K, uint8_t *q, uint8_t *sf) {
     const int KB = K / 32;
@@ -207,8 +208,8 @@ void orc_quant_mx32(const float *x, int R, int K, uint8_t *q, uint8_t *sf) {
                 for (int p = 0; p < 32; ++p) dst[p] = (uint8_t)((f32_bits(src[p]) >> 24) & 0x80u);
                 continue;
             }
-            int ex;
-            (void)frexpf(amax, &ex);                 /* amax = f * 2^ex, f in [0.5,1) */
+            int ex = 1024;                           /* (frexpf leaves it open for an infinity) */
+            if (!isinf(amax)) (void)frexpf(amax, &ex);   /* amax = f * 2^ex, f in [0.5,1) */
             int e = (ex - 1) - 8;                    /* floor(log2(amax)) - emax */
             int byte = e + 127;
             if (byte < 0) byte = 0;

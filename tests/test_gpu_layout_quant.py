@@ -131,6 +131,25 @@ def test_quant_128x128_nan_and_infinity(api):
     assert q[7, 200] & 0x7F == 0x7F and q[8, 201] & 0x7F == 0x7F and (q[9:, 128:] == 0).all()
 
 
+def test_mx_quantisers_on_infinities_and_nan(api, O):
+    """A block with an infinite value takes the largest scale byte and keeps its infinities as the largest element; a NaN
+    does not count for the scale.  Same bytes from the fp32 and the bf16 quantiser, and as the oracle gives them."""
+    rows, k = 40, 256
+    x = O.bf16_bits_to_f32(O.f32_to_bf16_bits(O.fill_normal((rows, k), 43, 0)))
+    x[0, 3], x[1, 40], x[2, 64:96] = np.inf, -np.inf, np.inf
+    x[3, 100], x[3, 101], x[3, 102] = np.inf, 2.0 ** 120, -(2.0 ** 127)
+    x[4, 7], x[5, 200], x[5, 201] = np.nan, np.nan, -np.inf
+    q, sf, atoms = api.quantize_mx32(T(x))
+    q, sf = q.cpu().numpy(), sf.cpu().numpy()
+    qr, sr = O.quant_mx32(x)
+    assert np.array_equal(sf, sr) and np.array_equal(q, qr)
+    assert sf[0, 0] == sf[1, 1] == sf[2, 2] == sf[3, 3] == sf[5, 6] == 254 and (sf == 254).sum() == 5
+    assert q[0, 3] == 0x7E and q[1, 40] == 0xFE and (q[2, 64:96] == 0x7E).all() and q[3, 100] == 0x7E
+    assert q[3, 102] == 0xB8 and q[4, 7] & 0x7F == 0x7F and sf[4, 0] < 130         # -(2^127 / 2^127) = -1
+    qb, ab = api.quantize_act_bf16_mx32(T(x).bfloat16())
+    assert np.array_equal(qb.cpu().numpy() & 0x7F, q & 0x7F) and torch.equal(ab, atoms)
+
+
 # a block takes 64 chunks of 16 bytes: one chunk, one short of a block, a whole one, one more
 @pytest.mark.parametrize("n,k", [(16, 16), (48, 1008), (16, 1024), (32, 1040), (272, 2192)])
 def test_shuffle_nk_at_the_edges_of_a_block(api, O, n, k):
