@@ -121,6 +121,19 @@ int device_state(DeviceState** out) {
     return B200_OK;
 }
 
+// SMs of the current device, whatever B200GEMM_MAX_SMS says (148 where it cannot be asked; asked once per device)
+int physical_sms() {
+    static std::atomic<int> known[kMaxDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // u8 tensor map of rank `rank`; dims/strides innermost first, strides[i] = byte stride of dim i+1
 // Encoding a tensor map costs a driver call; serving loops present the same few buffers over and over, so
 // the most recent encodings are kept (keyed by every encode parameter; a map holds no device-specific state
@@ -275,7 +288,10 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
             hint = B200_TILE_DECODE;
         } else {
             // cost of a persistent schedule: rounds (in tenths) x time per tile, proportional to the tile's N; with block
-            // scales the tail of 256 x 256 pair tiles counts with the share of a round that its column parts take (plan_tail)
+            // scales the tail of 256 x 256 pair tiles counts with the share of a round that its column parts take (plan_tail).
+            // Not without: counted there too, 24 of 152 sizes (256...8192 in each dimension) go to 256 x 256 tiles, 10 of them up to
+            // 10 % faster (4486 x 1232 x 1104 16.1 -> 14.5 us) and 14 up to 15 % slower (705 x 6160 x 416 9.15 -> 10.5); 1 % slower
+            // in the mean.
             const int pairs = sm_count / 2;
             const int64_t tm2 = (a->m + 255) / 256, tm1 = (a->m + 127) / 128;
             int64_t best = -1;
@@ -1278,7 +1294,7 @@ int b200_quantize_act_bf16_1x128(const void* x_bf16, int64_t ldx, void* q, int64
         return B200_ERR_UNSUPPORTED;
     // four rows per warp (see the kernel) unless that leaves an SM with fewer than eight warps
     const int64_t pairs = (k / 128 + 1) / 2;
-    const bool wide = (m + 3) / 4 * pairs >= 148 * 8;
+    const bool wide = (m + 3) / 4 * pairs >= physical_sms() * 8;
     const int64_t blocks = ((wide ? (m + 3) / 4 : m) * pairs + 7) / 8;
     if (k > 0x7FFFFFFF || blocks > (1 << 28)) return B200_ERR_TOO_LARGE;
     return launch_pdl(wide ? act_quant_bf16_1x128_kernel<4> : act_quant_bf16_1x128_kernel<1>, static_cast<unsigned>(blocks), 256, 0,

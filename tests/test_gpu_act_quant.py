@@ -149,12 +149,15 @@ def test_sharded_forward_bf16_single_gpu(api, O):
     assert_close(O, out.float().cpu().numpy(), O.gemm_ref_blockscale(qa, qb, sfa, sfb))
 
 
-@pytest.mark.parametrize("m,k", [(3, 384), (588, 1920), (592, 2048), (597, 2048)])
+@pytest.mark.parametrize("m,k", [(3, 384), (-4, 1920), (0, 2048), (5, 2048)])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_act_quant_at_the_edges_of_the_dispatch(api, O, m, k, offset):
-    """Both sides of the one-row / four-rows-per-warp rule (four from 1184 warps on), a last row group of one row, an odd
-    number of K groups; and for MX an input that is only 8-byte aligned.  Magnitudes run over many binades, so that single
-    groups leave the fast division."""
+    """Both sides of the one-row / four-rows-per-warp rule (four rows from eight warps per SM on: with 8 pairs of K groups, from 4
+    rows per SM on; m counts from there for the larger k), a last row group of one row, an odd number of K groups; and for
+    MX an input that is only 8-byte aligned.  Magnitudes run over many binades, so that single groups leave the fast
+    division."""
+    if k >= 1920:
+        m += 4 * torch.cuda.get_device_properties(0).multi_processor_count
     wide = O.fill_normal((m, k + 8), 31, 0) * np.exp2(np.floor(O.fill_uniform((m, 1), 31, 1, -125.0, 120.0))).astype(np.float32)
     wide[m // 2, :] = 0.0
     bits = O.f32_to_bf16_bits(wide)
