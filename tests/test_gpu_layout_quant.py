@@ -111,9 +111,12 @@ def test_quant_128x128_over_the_whole_range(api, O):
     k = 128 * 252
     x = O.fill_normal((128, k), 41, 0).reshape(128, 252, 128)
     x[:, :, ::7] = -0.0
-    top = np.abs(x).max(axis=(0, 2), keepdims=True)
-    mid = (np.arange(128) % 16 + 16.5) / 16 * top / 448 * 16
-    x[5] = np.nextafter(mid[0], np.where(np.arange(128) % 3 == 0, 0, 1e9)).astype(np.float32)
+    x[5] = 0.0
+    scale = np.abs(x).max(axis=(0, 2)) / np.float32(448)
+    tie = scale[:, None] * (17 + 2 * (np.arange(128) % 8)).astype(np.float32)        # e4m3 steps by 2 between 16 and 32
+    side = np.arange(128) // 8 % 3
+    x[5] = np.where(side == 0, tie, np.nextafter(tie, np.where(side == 1, np.float32(0), np.float32(np.inf))))
+    assert x.dtype == np.float32
     x[:, 100] = 0.0
     x = np.ldexp(x, (np.arange(252) - 128)[None, :, None]).astype(np.float32).reshape(128, k)
     q, s = api.quantize_128x128(T(x))
