@@ -387,9 +387,9 @@ __device__ __forceinline__ uint32_t f32x2x2_to_e4m3x4(unsigned long long p, unsi
 // groups (512 contiguous bytes per row, 16 per lane) and has the loads of all its rows in flight at once; lanes r and
 // 16+r then hold the amax of row r's two groups, so the two divisions and the reciprocal are done once per warp and not
 // once per row.  The launcher takes R = 4 when that still gives every SM eight warps, else R = 1 (16384 x 8192: R = 1
-// 104 us, 2 78, 4 68, 8 102; below 1000 x 4096 no difference between 1 and 4).  Back to back, against one warp walking 32
-// rows in eight dependent rounds: 64 x 7168 12.2 -> 1.6 us, 333 x 2048 12.3 -> 1.7, 4096 x 2048 15.2 -> 7.3,
-// 16384 x 8192 77 -> 68 (6.0 TB/s).
+// 108 us, 2 78, 4 76, 8 97; 333 x 2048: 2.2, 2.0, 1.9, 3.0).  In a graph of 40 launches, against one warp walking 32 rows in
+// eight dependent rounds: 64 x 7168 12.1 -> 1.8 us, 333 x 2048 12.1 -> 2.2, 4096 x 2048 12.5 -> 5.3 (16.0 -> 6.8 with
+// inputs from HBM), 8192 x 8192 43 -> 37, 16384 x 8192 77 -> 72...76 (5.4...5.6 TB/s, by the box).
 template <int R>
 __global__ void __launch_bounds__(256) act_quant_bf16_1x128_kernel(const uint16_t* __restrict__ x, long long ldx,
                                                                    uint8_t* __restrict__ q, long long ldq,
@@ -467,7 +467,7 @@ __device__ __forceinline__ float mx_inv_scale(int byte) {
 //
 // Bound and shape as above: a warp takes four rows of two neighbouring K groups, all loads in flight at once; four lanes
 // share a 32-wide block.  (One warp walking 32 rows, ilogbf / scalbnf per value: 8192 x 8192 took 75 us back to
-// back, now 37; 64 x 7168 14.0, now 1.7.)  kAligned: x is 16-byte and q 8-byte aligned, pitches
+// back, now 37; 64 x 7168 14.0, now 2.0.)  kAligned: x is 16-byte and q 8-byte aligned, pitches
 // included; the entry also takes 8- and 4-byte aligned ones, which move in two halves.
 template <bool kAligned>
 __global__ void __launch_bounds__(256) act_quant_bf16_mx32_kernel(const uint16_t* __restrict__ x, long long ldx,

@@ -1,7 +1,7 @@
 // Python front end of the per-call operators: what api.py's GEMM and activation-quantiser functions do between the
 // user's tensors and the C ABI, in native code.  Checks, output allocation, argument block and launch of one call
 // cost about 20 us of interpreter and ctypes time in Python -- more than the small GEMMs and the decode layers take on the
-// GPU -- and 3-5 us here (256 x 512 x 1024 per-tensor GEMM: 22.7 us a call before, back to back; figures beside the callers).
+// GPU -- and 3-6 us here (256 x 512 x 1024 per-tensor GEMM, back to back: 22.7 us a call before, 6.4 now).
 //
 // The module holds no state but the addresses of the C ABI entries (bind()), which api.py takes from the library that
 // _lib.py has loaded, so that both sides use one copy of it.  Functions return the output tensor(s), or the C ABI's

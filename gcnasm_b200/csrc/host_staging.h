@@ -31,6 +31,8 @@ struct CopyJob {
 
 // Threads that work through posted copies in pieces of 64 KB.  At most eleven, started by the first large copy, asleep
 // between calls (after about 100 us of spinning: the chunks of one call follow each other closely), joined by release().
+// With the caller they take up three quarters of the CPUs that the process may run on: several processes of one machine
+// each get their share through their affinity masks.
 // Whoever waits for a job works on the queue meanwhile, so that jobs get done with no threads at all.
 class CopyPool {
 public:

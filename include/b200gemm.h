@@ -144,7 +144,12 @@ int b200_gemm_a8w8_simple(const b200_gemm_args* args, void* cuda_stream);
  * device buffers owned by the library, runs the GEMM and copies C back; returns after the copy-back.
  * Device buffers are cached per device and grown on demand; b200_release() frees them.  Single-batch problems
  * with M >= 2048 (not MX) run as row slabs whose copy-back overlaps the next slab's upload and GEMM on a second,
- * library-owned stream; the call still returns only when all of C is on the host.                        */
+ * library-owned stream; the call still returns only when all of C is on the host.
+ * Pageable operands and results pass through a pinned ring of 24 MB per device, which up to eleven threads of the library
+ * fill and empty (fewer where the process may use fewer CPUs); where there is no pinned memory the driver stages them.
+ * Whatever the call returns, nothing of it is still running then: no copy touches the caller's memory any more.  A
+ * stream that is being captured is refused (B200_ERR_CUDA); the capture stays valid, unless this is the library's first call
+ * on the device.  b200_release() also frees the ring and ends the threads.                                */
 int b200_gemm_a8w8_host(const b200_gemm_args* host_args, void* cuda_stream);
 
 /* No counterpart in the reference.  Skinny-M (M <= 64) GEMM with the same arguments and the same results as
@@ -156,9 +161,10 @@ int b200_gemm_a8w8_host(const b200_gemm_args* host_args, void* cuda_stream);
  * cudaFree or any allocating routine.  Its split-K workspace is a fixed 1 MiB array inside the library image
  * (every GPU that loads the library holds it until the process exits).
  *   - Limit: splits * batch * M * N fp32 partials must fit in 1 MiB (262,144 floats), whether or not the launch
- *     goes through the workspace (splits: the power of two, at most 16, that fills the SMs with CTAs); otherwise the call
- *     returns B200_ERR_TOO_LARGE and launches nothing.  Shapes the launcher would not send to the skinny-M
- *     kernel (M > 64, MX scales) return B200_ERR_UNSUPPORTED.
+ *     goes through the workspace (splits: the power of two, at most 16, that fills the SMs with CTAs; with block scales
+ *     doubled further until a CTA's scales fit its shared memory); otherwise the call returns B200_ERR_TOO_LARGE and
+ *     launches nothing.  Shapes the launcher would not send to the skinny-M kernel (M > 64, MX scales) return
+ *     B200_ERR_UNSUPPORTED.
  *   - The first call on each device looks up that device's address of the array (and the library's other
  *     per-device set-up); make that first call before starting any stream capture.
  *   - All calls on a device share the one array and it keeps the previous call's contents.  Nothing needs
