@@ -97,6 +97,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
     const int kb0 = split * p.kb_per_split;
     const int kb1 = (kb0 + p.kb_per_split < p.kblocks) ? kb0 + p.kb_per_split : p.kblocks;
     const int nkb = kb1 - kb0;
+    // C takes 16-byte stores (c_batch and ldc are in elements; the columns a store starts at are multiples of 4, of 32 without splits)
+    const bool c_vec = (reinterpret_cast<uintptr_t>(p.c) & 15) == 0 && (p.ldc * (p.out_dtype == OUT_BF16 ? 2 : 4)) % 16 == 0 &&
+                       (p.c_batch * (p.out_dtype == OUT_BF16 ? 2 : 4)) % 16 == 0;
 
     // Consecutive decode GEMMs of a serving step are launched with programmatic serialization: this kernel may
     // start while its predecessor is still draining.  When the caller has vouched for the weights
@@ -338,28 +341,43 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
             }
         }
 
+        // Every MMA of this CTA has completed, so the ring is free.  (A split that gave up leaves anything there: nobody adds it.)
         if (p.splits > 1 && !p.partial) {
-            // (every MMA of this CTA has completed, so the ring is free: partial sums [token][weight row] at its start)
-            float* mine = reinterpret_cast<float*>(smem_gen) + quad * 32 + lane;
+            float* mine = reinterpret_cast<float*>(smem_gen) + quad * 32 + lane;      // partial sums [token][weight row]
 #pragma unroll
-            for (int j = 0; j < MT; ++j)
-                if (j < p.m) mine[j * BNW] = acc[j];
-        } else if (ok && n_row < p.n) {
-            if (p.splits > 1) {
-                float* dst = p.partial + ((static_cast<size_t>(split) * p.batch + b) * p.m) * p.n + n_row;
+            for (int j = 0; j < MT; ++j) mine[j * BNW] = acc[j];
+        } else if (ok && p.splits == 1 && c_vec && ni * BNW + quad * 32 + 32 <= p.n) {
+            // a thread holds one column of the output: the warp turns its 32 columns round in shared memory and stores 16 bytes
+            // per lane, 64 (128) contiguous bytes per token.  One two-byte store per token and thread, written out token by token,
+            // was most of what a 64-token call took longer than one of 1 token whatever K (18432 x 7168, in a graph, 64 tokens:
+            // 24.9 -> 23.4 us, K = 3584 15.4 -> 13.7; 32 tokens 23.05 -> 22.35; 16 22.1 -> 21.8; one token the same).
+            uint8_t* mine = smem_gen + quad * (MT * 128);
+            const int pieces = p.out_dtype == OUT_BF16 ? 4 : 8;                       // 16-byte pieces per token
+            if (p.out_dtype == OUT_BF16) {
+                __nv_bfloat16* t = reinterpret_cast<__nv_bfloat16*>(mine) + lane;
 #pragma unroll
-                for (int j = 0; j < MT; ++j)
-                    if (j < p.m) dst[static_cast<size_t>(j) * p.n] = acc[j];
-            } else if (p.out_dtype == OUT_BF16) {
-                __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.c) + static_cast<size_t>(b) * p.c_batch + n_row;
-#pragma unroll
-                for (int j = 0; j < MT; ++j)
-                    if (j < p.m) dst[static_cast<size_t>(j) * p.ldc] = __float2bfloat16_rn(acc[j]);
+                for (int j = 0; j < MT; ++j) t[j * 32] = __float2bfloat16_rn(acc[j]);
             } else {
-                float* dst = reinterpret_cast<float*>(p.c) + static_cast<size_t>(b) * p.c_batch + n_row;
+                float* t = reinterpret_cast<float*>(mine) + lane;
 #pragma unroll
-                for (int j = 0; j < MT; ++j)
-                    if (j < p.m) dst[static_cast<size_t>(j) * p.ldc] = acc[j];
+                for (int j = 0; j < MT; ++j) t[j * 32] = acc[j];
+            }
+            __syncwarp();
+            const size_t esz = p.out_dtype == OUT_BF16 ? 2 : 4;
+            uint8_t* dst = reinterpret_cast<uint8_t*>(p.c) + (static_cast<size_t>(b) * p.c_batch + ni * BNW + quad * 32) * esz;
+#pragma unroll 4
+            for (int q = lane; q < p.m * pieces; q += 32)
+                *reinterpret_cast<uint4*>(dst + static_cast<size_t>(q / pieces) * p.ldc * esz + (q % pieces) * 16) =
+                    *reinterpret_cast<const uint4*>(mine + q * 16);
+        } else if (ok && n_row < p.n) {
+            float* part = p.partial ? p.partial + ((static_cast<size_t>(split) * p.batch + b) * p.m) * p.n + n_row : nullptr;
+            const size_t o = static_cast<size_t>(b) * p.c_batch + n_row;
+#pragma unroll
+            for (int j = 0; j < MT; ++j) {
+                if (j >= p.m) break;
+                if (p.splits > 1) part[static_cast<size_t>(j) * p.n] = acc[j];
+                else if (p.out_dtype == OUT_BF16) reinterpret_cast<__nv_bfloat16*>(p.c)[o + static_cast<size_t>(j) * p.ldc] = __float2bfloat16_rn(acc[j]);
+                else reinterpret_cast<float*>(p.c)[o + static_cast<size_t>(j) * p.ldc] = acc[j];
             }
         }
     }
@@ -375,24 +393,33 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
         // A split that gave up (an expired wait) has no sums to add: the panel is left unwritten then, as without a cluster.
         // Asked for first and looked at after the first row's sums, whose loads cover it.
         const uint32_t gave_up = lane < p.splits ? ld_shared_cluster_u32(mapa_shared(smem_u32(tmem_slot + 1), lane)) : 0u;
+        // a lane sums four neighbouring columns: a quarter of the remote loads
+        const int col = ni * BNW + lane * 4;
+        const bool whole = c_vec && col + 4 <= p.n;
         for (int j = split + warp * p.splits; j < p.m; j += p.splits * (Cfg::THREADS / 32)) {
-            const uint32_t row = smem_base + static_cast<uint32_t>(j * BNW + lane) * 4;
-            float sum[BNW / 32];
-#pragma unroll
-            for (int c = 0; c < BNW / 32; ++c) sum[c] = 0.0f;
-#pragma unroll 4
+            const uint32_t row = smem_base + static_cast<uint32_t>(j * BNW + lane * 4) * 4;
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 8
             for (int s = 0; s < p.splits; ++s) {
-                const uint32_t src = mapa_shared(row, s);
-#pragma unroll
-                for (int c = 0; c < BNW / 32; ++c) sum[c] += __uint_as_float(ld_shared_cluster_u32(src + c * 128));
+                const float4 v = ld_shared_cluster_f32x4(mapa_shared(row, s));
+                sum[0] += v.x;
+                sum[1] += v.y;
+                sum[2] += v.z;
+                sum[3] += v.w;
             }
             if (__any_sync(0xFFFFFFFFu, gave_up != 0u)) break;
-            const size_t o = static_cast<size_t>(b) * p.c_batch + static_cast<size_t>(j) * p.ldc + ni * BNW + lane;
+            const size_t o = static_cast<size_t>(b) * p.c_batch + static_cast<size_t>(j) * p.ldc + col;
+            if (whole && p.out_dtype == OUT_BF16) {
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.c) + o) = make_uint2(pack_bf16x2(sum[0], sum[1]), pack_bf16x2(sum[2], sum[3]));
+            } else if (whole) {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.c) + o) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+            } else {
 #pragma unroll
-            for (int c = 0; c < BNW / 32; ++c) {
-                if (ni * BNW + c * 32 + lane < p.n) {
-                    if (p.out_dtype == OUT_BF16) reinterpret_cast<__nv_bfloat16*>(p.c)[o + c * 32] = __float2bfloat16_rn(sum[c]);
-                    else reinterpret_cast<float*>(p.c)[o + c * 32] = sum[c];
+                for (int c = 0; c < 4; ++c) {
+                    if (col + c < p.n) {
+                        if (p.out_dtype == OUT_BF16) reinterpret_cast<__nv_bfloat16*>(p.c)[o + c] = __float2bfloat16_rn(sum[c]);
+                        else reinterpret_cast<float*>(p.c)[o + c] = sum[c];
+                    }
                 }
             }
         }

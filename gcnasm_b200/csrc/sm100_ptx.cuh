@@ -457,6 +457,11 @@ __device__ __forceinline__ uint32_t ld_shared_cluster_u32(uint32_t cluster_addr)
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
     return v;
 }
+__device__ __forceinline__ float4 ld_shared_cluster_f32x4(uint32_t cluster_addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+    return v;
+}
 // shared memory -> TMEM copy of one 32-row x 16-byte scale-factor atom, replicated into the
 // four 32-lane quadrants
 template <int kCtaGroup>
