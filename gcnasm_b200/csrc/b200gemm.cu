@@ -276,15 +276,18 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
 
     Plan pl{B200_TILE_128x128, 0, 1};
     const int64_t kblocks = (a->k + 127) / 128;
-    const bool decode_ok = !pair_only && !ab16 && a->m <= 64 && a->scale_mode != B200_SCALE_MX && (a->n % 16 == 0);
+    const bool decode_ok = !pair_only && !ab16 && a->m <= 64 && (a->n % 16 == 0);
     int hint = a->tile_hint;
-    if (hint == B200_TILE_DECODE && !decode_ok) return B200_ERR_UNSUPPORTED;
+    if (hint == B200_TILE_DECODE && (!decode_ok || a->scale_mode == B200_SCALE_MX)) return B200_ERR_UNSUPPORTED;
     if (hint == B200_TILE_128x64) return B200_ERR_UNSUPPORTED;
     const bool mx = a->scale_mode == B200_SCALE_MX;
     // MX pair kernels address the scale atoms through a tensor map: batch strides in whole atoms
     const bool mx_pair_ok = !mx || a->batch == 1 || (a->stride_sfa_batch % 512 == 0 && a->stride_sfb_batch % 512 == 0);
     if (hint == B200_TILE_AUTO) {
-        if (decode_ok) {
+        // MX: from twelve K blocks on.  Below that the 128 x 128 tiles' shorter fixed part wins; skinny kernel / tile, us: 64 x 512 x 512
+        // 5.0 / 3.8, 64 x 8192 x 512 5.7 / 4.1, 40 x 4096 x 1024 5.4 / 4.9; 64 x 2048 x 2048 6.0 / 7.4, 16 x 2048 x 2048 4.8 / 7.0,
+        // 1 x 512 x 8192 6.0 / 20.3, 1, 16, 64 x 8192 x 8192 13.8 / 28.6, 14.5 / 21.6, 16.6 / 22.0.
+        if (decode_ok && (!mx || kblocks >= 12)) {
             hint = B200_TILE_DECODE;
         } else {
             // cost of a persistent schedule: rounds (in tenths) x time per tile, proportional to the tile's N; with block
@@ -342,7 +345,7 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
     if (pair_only && !(hint == B200_TILE_PAIR_256x256 || hint == B200_TILE_PAIR_256x224 || hint == B200_TILE_PAIR_256x192 ||
                        hint == B200_TILE_PAIR_256x128))
         return B200_ERR_UNSUPPORTED;
-    if (mx && !(hint == B200_TILE_128x128 || (hint == B200_TILE_PAIR_256x256 && mx_pair_ok))) return B200_ERR_UNSUPPORTED;
+    if (mx && !(hint == B200_TILE_128x128 || hint == B200_TILE_DECODE || (hint == B200_TILE_PAIR_256x256 && mx_pair_ok))) return B200_ERR_UNSUPPORTED;
     // bf16 operands: pair 256x256 and the two single-CTA tiles are built
     if (ab16 && !(hint == B200_TILE_128x128 || hint == B200_TILE_128x256 || hint == B200_TILE_PAIR_256x256)) return B200_ERR_UNSUPPORTED;
     pl.tile = hint;
@@ -614,8 +617,9 @@ int decode_clusters_mt(int mt, int size, int sm_count) {
         default: return decode_clusters<64, MODE, BL>(size, sm_count);
     }
 }
-int decode_clusters_any(bool block, bool flat, int mt, int size, int sm_count) {
-    if (block) return flat ? decode_clusters_mt<MODE_BLOCK, BL_FLAT>(mt, size, sm_count) : decode_clusters_mt<MODE_BLOCK, BL_NK>(mt, size, sm_count);
+int decode_clusters_any(int scale_mode, bool flat, int mt, int size, int sm_count) {
+    if (scale_mode == B200_SCALE_MX) return flat ? decode_clusters_mt<MODE_MX, BL_FLAT>(mt, size, sm_count) : decode_clusters_mt<MODE_MX, BL_NK>(mt, size, sm_count);
+    if (scale_mode == B200_SCALE_BLOCK) return flat ? decode_clusters_mt<MODE_BLOCK, BL_FLAT>(mt, size, sm_count) : decode_clusters_mt<MODE_BLOCK, BL_NK>(mt, size, sm_count);
     return flat ? decode_clusters_mt<MODE_ACC, BL_FLAT>(mt, size, sm_count) : decode_clusters_mt<MODE_ACC, BL_NK>(mt, size, sm_count);
 }
 
@@ -624,14 +628,15 @@ int decode_clusters_any(bool block, bool flat, int mt, int size, int sm_count) {
 // 5.3; a count whose clusters are not all resident costs a second wave: 7168 x 2048 2 splits 8.6 us, 3 12.9).  Block scales
 // bound a CTA's K blocks by its staging area; when that takes more splits than fit a cluster the answer is 0 and the partials
 // go through a workspace.
-int cluster_splits(int64_t tiles, int64_t kblocks, bool block, bool flat, int mt, int sm_count) {
+int cluster_splits(int64_t tiles, int64_t kblocks, int scale_mode, bool flat, int mt, int sm_count) {
+    const bool block = scale_mode == B200_SCALE_BLOCK;
     constexpr int kMinSplitBlocks = 2;
     const int64_t most = block ? decode_sf_bytes(mt) / 4 / (mt + 1) : kblocks;      // K blocks one CTA can take
     const int64_t need = (kblocks + most - 1) / most;
-    if (need > kMaxDecodeCluster || (need > 1 && decode_clusters_any(block, flat, mt, static_cast<int>(need), sm_count) < 1)) return 0;
+    if (need > kMaxDecodeCluster || (need > 1 && decode_clusters_any(scale_mode, flat, mt, static_cast<int>(need), sm_count) < 1)) return 0;
     int best = static_cast<int>(need);
     for (int s = best + 1; s <= kMaxDecodeCluster && (kblocks + s - 1) / s >= kMinSplitBlocks; ++s)
-        if ((kblocks + s - 1) / s < (kblocks + best - 1) / best && decode_clusters_any(block, flat, mt, s, sm_count) >= tiles) best = s;
+        if ((kblocks + s - 1) / s < (kblocks + best - 1) / best && decode_clusters_any(scale_mode, flat, mt, s, sm_count) >= tiles) best = s;
     return best;
 }
 
@@ -710,7 +715,7 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
         int rc0 = static_scratch(need_floats, &scratch);
         if (rc0) return rc0;
     }
-    int splits = cluster_splits((a->n + 127) / 128 * a->batch, (a->k + 127) / 128, block, flat, pl.mt, ds->sm_count);
+    int splits = cluster_splits((a->n + 127) / 128 * a->batch, (a->k + 127) / 128, a->scale_mode, flat, pl.mt, ds->sm_count);
     if (splits == 0) {
         splits = pl.splits;
         if (use_static) {
@@ -737,8 +742,9 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
     p.scale_b = a->scale_mode == B200_SCALE_TENSOR ? a->ptr_scale_b : nullptr;
     p.ldc = a->stride_c;
     p.c_batch = a->stride_c_batch;
-    p.sfa_stride = a->stride_sfa;
-    p.sfb_stride = a->stride_sfb;
+    const bool mx = a->scale_mode == B200_SCALE_MX;
+    p.sfa_stride = mx ? (a->m + 127) / 128 : a->stride_sfa;       // MX: atoms per K block
+    p.sfb_stride = mx ? (a->n + 127) / 128 : a->stride_sfb;
     p.sfa_batch = a->stride_sfa_batch;
     p.sfb_batch = a->stride_sfb_batch;
     p.m = static_cast<int>(a->m);
@@ -753,10 +759,12 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
     p.inputs_ready = (a->flags & B200_GEMM_INPUTS_READY) ? 1 : 0;
     p.status = ds->status_ptr;
     const int grid = p.tiles_n * p.batch * splits;
-    if (a->b_layout == B200_B_NK_ROWMAJOR)
-        rc = block ? launch_decode_mt<MODE_BLOCK, BL_NK>(pl.mt, p, grid, st) : launch_decode_mt<MODE_ACC, BL_NK>(pl.mt, p, grid, st);
+    if (flat)
+        rc = mx ? launch_decode_mt<MODE_MX, BL_FLAT>(pl.mt, p, grid, st)
+                : (block ? launch_decode_mt<MODE_BLOCK, BL_FLAT>(pl.mt, p, grid, st) : launch_decode_mt<MODE_ACC, BL_FLAT>(pl.mt, p, grid, st));
     else
-        rc = block ? launch_decode_mt<MODE_BLOCK, BL_FLAT>(pl.mt, p, grid, st) : launch_decode_mt<MODE_ACC, BL_FLAT>(pl.mt, p, grid, st);
+        rc = mx ? launch_decode_mt<MODE_MX, BL_NK>(pl.mt, p, grid, st)
+                : (block ? launch_decode_mt<MODE_BLOCK, BL_NK>(pl.mt, p, grid, st) : launch_decode_mt<MODE_ACC, BL_NK>(pl.mt, p, grid, st));
     if (rc) return rc;
     if (splits > 1 && p.partial) {
         const long long per_split = static_cast<long long>(a->batch) * a->m * a->n;
@@ -987,7 +995,8 @@ int b200_gemm_a8w8_decode_static(const b200_gemm_args* args, void* cuda_stream) 
     if (rc) return rc;
     rc = validate(args, ds->sm_count, &pl);
     if (rc) return rc;
-    if (pl.tile != B200_TILE_DECODE) return B200_ERR_UNSUPPORTED;      // only the skinny-M kernel has this variant
+    // only the skinny-M kernel has this variant, and not with MX scales
+    if (pl.tile != B200_TILE_DECODE || args->scale_mode == B200_SCALE_MX) return B200_ERR_UNSUPPORTED;
     return run_decode(args, pl, ds, static_cast<cudaStream_t>(cuda_stream), true);
 }
 

@@ -16,6 +16,10 @@
 // Block scales (A: per token per 128 K, [K/128][M]; W: per 128x128 block, [N/128][K/128]) follow
 // gemm_a8w8_blockscale_host.cc:66-90: every K group gets a fresh TMEM buffer and is folded into
 // register accumulators as acc += partial * (sfa[g][token] * sfb[nblk][g]).
+//
+// MX scales: the tensor core applies them, so a CTA's whole K range accumulates in one TMEM buffer; the E8M0 atoms of the weight
+// panel and of the token block travel with their stage.  Such calls used to run on the 128 x 128 single-CTA tile, at most one
+// CTA per 128 weight rows; here a panel's K is split over a cluster.
 #pragma once
 
 #include "gemm_sm100.cuh"
@@ -27,7 +31,7 @@ struct DecodeParams {
     CUtensorMap tmap_x;          // tokens:  3-D [batch][M][K], box 128 x MT, 128-byte swizzle
     void* c;
     float* partial;              // split-K workspace [splits][batch][M][N] fp32, or null: the splits of a panel are a cluster
-    const float* sfa;
+    const float* sfa;            // MX: the atoms (bytes), as are sfb and, in atoms and bytes, the strides
     const float* sfb;
     const float* scale_a;
     const float* scale_b;
@@ -50,9 +54,11 @@ struct DecodeCfg {
     static constexpr int BNW = 128, BK = 128;
     static constexpr int W_BYTES = BNW * BK;
     static constexpr int X_BYTES = MT * BK;
-    static constexpr int STAGE_BYTES = ((W_BYTES + X_BYTES + 1023) / 1024) * 1024;
+    static constexpr int SF_BYTES = MODE == MODE_MX ? 1024 : 0;     // MX: the atom of the weight rows, then that of the tokens
+    static constexpr int LOAD_BYTES = W_BYTES + X_BYTES + SF_BYTES;
+    static constexpr int STAGE_BYTES = ((LOAD_BYTES + 1023) / 1024) * 1024;
     // combined scales [K groups of this CTA][MT]; problems whose groups do not fit are split along K by the launcher
-    static constexpr int SF_SMEM = decode_sf_bytes(MT_);
+    static constexpr int SF_SMEM = MODE == MODE_MX ? 0 : decode_sf_bytes(MT_);
     static constexpr int STAGES_RAW = (225 * 1024 - 1024 - SF_SMEM) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + SF_SMEM + 1024;
@@ -62,7 +68,8 @@ struct DecodeCfg {
     // group, so it is paid once per GB groups.  Two batch sets ping-pong: TMEM holds 2 x GB x MT columns.
     static constexpr int GB = 4;
     static constexpr int NBUF = 2;
-    static constexpr int TMEM_COLS = NBUF * GB * MT < 32 ? 32 : NBUF * GB * MT;
+    static constexpr int SF_COL = MT;                               // MX: scale columns behind the one accumulator
+    static constexpr int TMEM_COLS = MODE == MODE_MX ? (MT + 8 <= 32 ? 32 : (MT + 8 <= 64 ? 64 : 128)) : (NBUF * GB * MT < 32 ? 32 : NBUF * GB * MT);
     static constexpr int THREADS = 192;
     static constexpr int MAX_SF_FLOATS = SF_SMEM / 4;
     static_assert(MT == 16 || MT == 32 || MT == 64, "token block is 16, 32 or 64");
@@ -111,14 +118,20 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
     // long (18432 x 7168).
     pdl_launch_dependents();
     const int first = nkb < STAGES ? nkb : STAGES;
+    // MX: atom (kb, 128-row block) of an image [batch][K/128][rows/128][512 B]
+    auto mx_atom = [&](const float* image, long long batch_bytes, long long blocks, int kb, int blk) {
+        return reinterpret_cast<const uint8_t*>(image) + b * batch_bytes + (static_cast<long long>(kb) * blocks + blk) * 512;
+    };
     auto request_weights = [&](int i) {
         const uint32_t sw = smem_base + i * Cfg::STAGE_BYTES;
         const uint32_t full = bar_full0 + i * 8;
-        mbar_arrive_expect_tx(full, Cfg::W_BYTES + Cfg::X_BYTES);
+        mbar_arrive_expect_tx(full, Cfg::LOAD_BYTES);
         if constexpr (Cfg::BLAYOUT == BL_NK)
             tma_load_3d(sw, &p.tmap_w, full, (kb0 + i) * BK, ni * BNW, b);
         else
             tma_load_4d(sw, &p.tmap_w, full, 0, ni * (BNW / 16), (kb0 + i) * (BK / 16), b);
+        if constexpr (MODE == MODE_MX)
+            bulk_load(sw + Cfg::W_BYTES + Cfg::X_BYTES, mx_atom(p.sfb, p.sfb_batch, p.sfb_stride, kb0 + i, ni), 512, full);
     };
     if (threadIdx.x == 2 * 32 && !p.inputs_ready) {
         for (int i = 0; i < first; ++i) {
@@ -156,6 +169,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
         for (int i = 0; i < first; ++i) {
             if (!p.inputs_ready) request_weights(i);
             tma_load_3d(smem_base + i * Cfg::STAGE_BYTES + Cfg::W_BYTES, &p.tmap_x, bar_full0 + i * 8, (kb0 + i) * BK, 0, b);
+            if constexpr (MODE == MODE_MX)
+                bulk_load(smem_base + i * Cfg::STAGE_BYTES + Cfg::W_BYTES + Cfg::X_BYTES + 512, mx_atom(p.sfa, p.sfa_batch, p.sfa_stride, kb0 + i, 0),
+                          512, bar_full0 + i * 8);
         }
     }
 
@@ -170,12 +186,16 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                 const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
                 const uint32_t sx = sw + Cfg::W_BYTES;
                 const uint32_t full = bar_full0 + s * 8;
-                mbar_arrive_expect_tx(full, Cfg::W_BYTES + Cfg::X_BYTES);
+                mbar_arrive_expect_tx(full, Cfg::LOAD_BYTES);
                 if constexpr (Cfg::BLAYOUT == BL_NK)
                     tma_load_3d(sw, &p.tmap_w, full, kb * BK, ni * BNW, b);
                 else
                     tma_load_4d(sw, &p.tmap_w, full, 0, ni * (BNW / 16), kb * (BK / 16), b);
                 tma_load_3d(sx, &p.tmap_x, full, kb * BK, 0, b);
+                if constexpr (MODE == MODE_MX) {
+                    bulk_load(sx + Cfg::X_BYTES, mx_atom(p.sfb, p.sfb_batch, p.sfb_stride, kb, ni), 512, full);
+                    bulk_load(sx + Cfg::X_BYTES + 512, mx_atom(p.sfa, p.sfa_batch, p.sfa_stride, kb, 0), 512, full);
+                }
             }
         }
     } else if (warp == 1) {
@@ -212,6 +232,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                     const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
                     const uint32_t sx = sw + Cfg::W_BYTES;
                     const uint32_t tacc = (MODE == MODE_BLOCK) ? tmem_base + (set * Cfg::GB + j) * MT : tmem_base;
+                    const uint32_t tsf = tmem_base + Cfg::SF_COL;
+                    if constexpr (MODE == MODE_MX) {
+                        tmem_cp_sf<1>(tsf, make_smem_desc(sx + Cfg::X_BYTES, 0, 128, kSwizzleNone));
+                        tmem_cp_sf<1>(tsf + 4, make_smem_desc(sx + Cfg::X_BYTES + 512, 0, 128, kSwizzleNone));
+                    }
 #pragma unroll
                     for (int k = 0; k < BK / 32; ++k) {
                         uint64_t dw;
@@ -223,7 +248,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                         }
                         const uint64_t dx = make_smem_desc(sx + k * 32, 16, 1024, kSwizzle128B);
                         const uint32_t accum = (MODE == MODE_BLOCK) ? (k > 0 ? 1u : 0u) : ((i > 0 || k > 0) ? 1u : 0u);
-                        umma_f8<1>(tacc, dw, dx, idesc, accum);
+                        if constexpr (MODE == MODE_MX) umma_mxf8<1>(tacc, dw, dx, make_idesc_mxf8(BNW, MT, k, k), accum, tsf, tsf + 4);
+                        else umma_f8<1>(tacc, dw, dx, idesc, accum);
                     }
                     umma_commit<1>(bar_empty0 + s * 8);
                 }
@@ -393,7 +419,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
         // A split that gave up (an expired wait) has no sums to add: the panel is left unwritten then, as without a cluster.
         // Asked for first and looked at after the first row's sums, whose loads cover it.
         const uint32_t gave_up = lane < p.splits ? ld_shared_cluster_u32(mapa_shared(smem_u32(tmem_slot + 1), lane)) : 0u;
-        // a lane sums four neighbouring columns: a quarter of the remote loads
+        // a lane sums four neighbouring columns: a quarter of the remote loads (MX, 64 x 2048 x 2048 with eight splits 6.35 -> 6.04 us)
         const int col = ni * BNW + lane * 4;
         const bool whole = c_vec && col + 4 <= p.n;
         for (int j = split + warp * p.splits; j < p.m; j += p.splits * (Cfg::THREADS / 32)) {
