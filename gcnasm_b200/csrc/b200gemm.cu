@@ -307,13 +307,13 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 if (pair && bn == 256 && block && tiles > units && rem > 0 && kblocks >= 4 && rem * 2 <= units)
                     tenths += (rem * 4 <= units ? 4 : 6) - 10;
                 // w = time per output column, measured on 4096 x 7168 x 2048 (us a round and 1000 columns, 8-bit / block scales:
-                // pair 256 27 / 40, 224 30 / 54, 192 30 / 56, 128 39 / 53; one CTA 256 33 / 49, 128 42 / 69): narrow and
+                // pair 256 27 / 40, 224 30 / 54, 192 30 / 56, 128 39 / 53; one CTA 256 33 / 49, 128 42 / 59): narrow and
                 // single-CTA tiles re-read more of A and B per flop, tiles that straddle the 128-column scale blocks
                 // pay for the second scale, and the 224-column epilogue works in half-width pieces, which a short K shows.
                 // Against the weights before (us): 4096^3 52.6 -> 47.9, 3794 x 3712 x 512 20.3 -> 16.7, 2750 x 7040 x 384 23.6 ->
                 // 18.5; with block scales 3794 x 3712 x 512 20.3 -> 16.7.
                 int64_t w;
-                if (!pair) w = bn >= 256 ? 125 : (block ? 170 : 155);
+                if (!pair) w = bn >= 256 ? 125 : 155;
                 else if (bn == 256) w = 100;
                 else if (bn == 128) w = block ? 130 : 140;
                 else w = block ? 140 : (bn == 224 && kblocks < 8 ? 120 : 110);

@@ -81,7 +81,9 @@ struct GemmCfg {
     static constexpr int STAGES_RAW = (SMEM_BUDGET - 1024) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*barriers*/ + 1024 /*alignment slack*/;
-    static constexpr int ACC_COLS = 2 * BN;
+    // accumulator buffers; 128 columns with block scales, a hand-off per K block: as many as tensor memory holds
+    static constexpr int BUFS = (MODE == MODE_BLOCK && BN == 128) ? 4 : 2;
+    static constexpr int ACC_COLS = BUFS * BN;
     static constexpr int SF_COLS = (MODE == MODE_MX) ? 4 + 4 * SFB_ATOMS : 0;
     static constexpr int TMEM_COLS = (ACC_COLS + SF_COLS) <= 32 ? 32 : (ACC_COLS + SF_COLS) <= 64 ? 64
                                    : (ACC_COLS + SF_COLS) <= 128 ? 128 : (ACC_COLS + SF_COLS) <= 256 ? 256 : 512;
@@ -206,8 +208,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     const uint32_t bar_full0 = smem_base + STAGES * Cfg::STAGE_BYTES;
     const uint32_t bar_empty0 = bar_full0 + STAGES * 8;
     const uint32_t bar_accf0 = bar_empty0 + STAGES * 8;
-    const uint32_t bar_acce0 = bar_accf0 + 2 * 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+    constexpr int BUFS = Cfg::BUFS;
+    const uint32_t bar_acce0 = bar_accf0 + BUFS * 8;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * BUFS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             mbar_init(bar_full0 + s * 8, 1);
             mbar_init(bar_empty0 + s * 8, 1);
         }
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < BUFS; ++s) {
             mbar_init(bar_accf0 + s * 8, 1);
             mbar_init(bar_acce0 + s * 8, 8);     // one arrival per epilogue warp
         }
@@ -292,8 +295,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             constexpr uint32_t idesc = make_idesc_f8(BM, BN);
             for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {
                 for (int g = 0; g < groups && ok; ++g, ++phase) {
-                    const uint32_t as = phase & 1;
-                    const uint32_t aph = (phase >> 1) & 1;
+                    const uint32_t as = phase % BUFS;
+                    const uint32_t aph = (phase / BUFS) & 1;
                     if (!role_all<true>(mbar_wait(bar_acce0 + as * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
                         ok = false;
                         break;
@@ -370,7 +373,64 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             uint8_t* crow = reinterpret_cast<uint8_t*>(p.c) +
                             (static_cast<size_t>(b) * p.c_batch + static_cast<size_t>(row) * p.ldc) * esz;
 
-            if constexpr (MODE == MODE_BLOCK) {
+            if constexpr (MODE == MODE_BLOCK && NCH == 64) {
+                // 64 columns per thread leave room to have both loads of a group in flight, and the buffer goes back before the FMAs;
+                // four buffers keep the tensor core busy meanwhile.  Two buffers, handed back after the FMAs, and scalar FMAs, us: 100 x
+                // 7168 x 2048 9.85 -> 8.85, 200 x 7168 x 2048 10.7 -> 9.6, 512 x 4096 x 4096 16.5 -> 14.2, 2500 x 5120 x 3072 75 -> 65.  (The
+                // same loop for 128 columns per thread, two buffers, was slower: 700 x 2048 x 7168 28.9 -> 30.7.)
+                // Scales are requested two groups ahead, into two register sets that take turns (a copy from one to the
+                // other would wait for the load): a load queues behind the operand tiles in flight.
+                unsigned long long acc2[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc2[j] = 0ull;
+                const float* sfa_p = p.sfa + b * p.sfa_batch + (row < p.m ? row : 0);
+                const float* sfb_p = p.sfb + b * p.sfb_batch + static_cast<long long>(col_base / 128) * p.sfb_stride;
+                const bool col_ok = col_base < p.n;
+                float sa[2], sb[2];
+                auto request = [&](const int g, const int set) {
+                    sa[set] = __ldg(sfa_p + static_cast<long long>(g) * p.sfa_stride);
+                    sb[set] = col_ok ? __ldg(sfb_p + g) : 0.0f;
+                };
+                request(0, 0);
+                request(groups > 1 ? 1 : 0, 1);
+                for (int g0 = 0; g0 < groups && ok; g0 += 2) {
+#pragma unroll
+                    for (int set = 0; set < 2; ++set) {
+                        const int g = g0 + set;
+                        if (g >= groups) break;
+                        const uint32_t as = phase % BUFS;
+                        const uint32_t aph = (phase / BUFS) & 1;
+                        if (!mbar_wait(bar_accf0 + as * 8, aph, abort_flag, p.status, KSTAT_TIMEOUT_ACC_F)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
+                        float v[64];
+                        tmem_ld32(taddr, v);
+                        tmem_ld32(taddr + 32, v + 32);
+                        const float sc = sa[set] * sb[set];
+                        const unsigned long long sc2 = pack_f32x2(sc, sc);
+                        tmem_ld_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
+                        if (g + 2 < groups) request(g + 2, set);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) acc2[j] = ffma2(pack_f32x2(v[2 * j], v[2 * j + 1]), sc2, acc2[j]);
+                        ++phase;
+                    }
+                }
+                if (ok && row < p.m) {
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        float o[32];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) unpack_f32x2(acc2[c * 16 + j], o[2 * j], o[2 * j + 1]);
+                        store_row_chunk<32>(p, crow, col_base + c * 32, o, vec_ok);
+                    }
+                }
+            } else if constexpr (MODE == MODE_BLOCK) {
                 float acc[NCH];
 #pragma unroll
                 for (int j = 0; j < NCH; ++j) acc[j] = 0.0f;

@@ -1,0 +1,59 @@
+"""Block-scale tile kernels: every K group's partial sums meet the scales of their own group, row and 128-column block, whatever
+the number of groups and of accumulator buffers they go through.
+
+The values make the results exact: operands are whole numbers of at most 2, scales are powers of two from 2^-5 to 2^5 in
+the product, K is at most 11 groups.  A partial sum is a whole number of at most 512, so every sum is a multiple of 2^-5 below
+11 * 512 * 2^5 < 2^18: 23 bits, nothing is ever rounded, and the outputs have to be the reference's to the last bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+E4M3 = {0: 0x00, 1: 0x38, 2: 0x40, -1: 0xB8, -2: 0xC0}
+
+
+def problem(m, n, k, seed, pad=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    groups = k // 128
+    table = torch.zeros(5, dtype=torch.uint8, device=DEV)
+    for v, byte in E4M3.items():
+        table[v + 2] = byte
+    xa = torch.randint(-2, 3, (m, k), generator=g, device=DEV)
+    xb = torch.randint(-2, 3, (n, k), generator=g, device=DEV)
+    ea = torch.randint(-3, 4, (groups, m + pad), generator=g, device=DEV)[:, :m]
+    eb = torch.randint(-2, 3, (n // 128, groups), generator=g, device=DEV)
+    sfa, sfb = torch.empty((groups, m + pad), device=DEV)[:, :m], torch.exp2(eb.float())
+    sfa.copy_(torch.exp2(ea.float()))
+    ref = torch.zeros(m, n, dtype=torch.float64, device=DEV)
+    for i in range(groups):
+        part = xa[:, i * 128:(i + 1) * 128].double() @ xb[:, i * 128:(i + 1) * 128].double().t()
+        ref += part * sfa[i].double()[:, None] * sfb[:, i].double().repeat_interleave(128)[None, :]
+    return table[xa + 2], table[xb + 2], sfa, sfb, ref
+
+
+def check(api, m, n, k, tile, flat=False, pad=0):
+    a, b, sfa, sfb, ref = problem(m, n, k, m + 7 * n + k, pad)
+    c = api.gemm_a8w8_blockscale(a, api.shuffle_b(b, "nk") if flat else b, sfa, sfb, out_dtype=torch.float32, tile=tile,
+                                 b_flat_n=n if flat else None)
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+    assert torch.equal(c.double(), ref)
+
+
+# pair 256x256 / 256x128 / 256x224 / 256x192, one CTA 128x256 / 128x128; one group to eleven: fewer, as many and more than buffers
+@pytest.mark.parametrize("tile", [4, 6, 7, 8, 2, 1])
+@pytest.mark.parametrize("groups", [1, 2, 3, 4, 5, 6, 7, 11])
+def test_groups_meet_their_scales(api, tile, groups):
+    check(api, 333, 896, 128 * groups, tile, flat=groups % 2 == 0)
+
+
+# several tiles per CTA: the buffers' phases run on from one tile to the next, ragged rows, and (4) into the column parts of tail tiles
+@pytest.mark.parametrize("tile,m,n", [(4, 2309, 2048), (6, 2309, 1152), (7, 2309, 2048), (8, 2309, 1664), (2, 1601, 3328), (1, 1601, 1664)])
+@pytest.mark.parametrize("groups", [4, 5])
+def test_groups_across_tiles(api, tile, m, n, groups):
+    check(api, m, n, 128 * groups, tile)
+
+
+@pytest.mark.parametrize("tile", [4, 1])
+def test_scale_rows_of_any_pitch(api, tile):
+    check(api, 201, 256, 640, tile, pad=3)
