@@ -16,6 +16,8 @@
 // acc += partial * (sfa[g][row] * sfb[nblk][g]) -- the analogue of scale_c_tile.
 #pragma once
 
+#include <type_traits>
+
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -150,6 +152,9 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, void* crow,
 // to a warp-private shared-memory buffer (row pitch 80 B: 16-byte accesses stay conflict-free) and read back
 // transposed, so that one store instruction covers whole 32- or 64-byte row segments.
 // `row0` is the output row of lane 0; `stage` is this warp's 2560-byte buffer; CNT * element size is 32 or 64.
+// The way out of the last tile is in nobody's shadow.  With the pieces per row known at compile time and every read issued
+// ahead of the stores (a loop with run-time divisions, one read and one store at a time, before), us: four batches of 700 x 2064 x 1152,
+// fp32, 256 x 192 tiles 13.7 -> 12.7, 256 x 256 tiles 14.9 -> 13.2; 256 x 512 x 1024, bf16, 256 x 256 tiles 8.0 -> 7.3.
 static constexpr int kOutStagePitch = 80;
 static constexpr int kOutStageBytesPerWarp = 32 * kOutStagePitch;
 template <int CNT>
@@ -164,9 +169,30 @@ __device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8
         return;
     }
     uint8_t* mine = stage + lane * kOutStagePitch;
-    int row_bytes;
+    // kPieces 16-byte pieces per row, a compile-time power of two on either branch; with all rows in range the reads go out
+    // together, then the stores
+    auto put = [&](auto pieces, const size_t pitch_c) {
+        constexpr int kPieces = decltype(pieces)::value, kRows = 32 / kPieces;
+        __syncwarp();
+        const int c = lane % kPieces, r = lane / kPieces;
+        const uint8_t* src = stage + r * kOutStagePitch + c * 16;
+        uint8_t* dst = cbatch + (row0 + r) * pitch_c + static_cast<size_t>(col0) * esz + c * 16;
+        if (row0 + 32 <= p.m) {
+            uint4 w[kPieces];
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i) w[i] = *reinterpret_cast<const uint4*>(src + i * kRows * kOutStagePitch);
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i) *reinterpret_cast<uint4*>(dst + i * kRows * pitch_c) = w[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i)
+                if (row0 + r + i * kRows < p.m)
+                    *reinterpret_cast<uint4*>(dst + i * kRows * pitch_c) = *reinterpret_cast<const uint4*>(src + i * kRows * kOutStagePitch);
+        }
+        __syncwarp();
+    };
+    const size_t pitch_c = static_cast<size_t>(p.ldc) * esz;
     if (bf16) {
-        row_bytes = CNT * 2;
 #pragma unroll
         for (int j = 0; j < CNT; j += 8) {
             uint4 w;
@@ -176,23 +202,13 @@ __device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8
             w.w = pack_bf16x2(v[j + 6], v[j + 7]);
             *reinterpret_cast<uint4*>(mine + j * 2) = w;
         }
-    } else {
-        row_bytes = CNT * 4;
+        put(std::integral_constant<int, CNT / 8>{}, pitch_c);
+    } else if constexpr (CNT <= 16) {             // (fp32 chunks are at most 16 columns: 64 bytes, a row of the staging buffer)
 #pragma unroll
         for (int j = 0; j < CNT; j += 4)
             *reinterpret_cast<float4*>(mine + j * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        put(std::integral_constant<int, CNT / 4>{}, pitch_c);
     }
-    __syncwarp();
-    const int chunks = row_bytes >> 4;                  // 16-byte pieces per row: 2, 4 or 8
-    const int rows_per_pass = 32 / chunks;
-    const int c = lane % chunks, r_in = lane / chunks;
-    for (int r = r_in; r < 32; r += rows_per_pass) {
-        const uint4 w = *reinterpret_cast<const uint4*>(stage + r * kOutStagePitch + c * 16);
-        const int row = row0 + r;
-        if (row < p.m)
-            *reinterpret_cast<uint4*>(cbatch + (static_cast<size_t>(row) * p.ldc + col0) * esz + c * 16) = w;
-    }
-    __syncwarp();
 }
 
 template <class Cfg>
