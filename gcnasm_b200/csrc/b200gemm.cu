@@ -313,7 +313,13 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 // Against the weights before (us): 4096^3 52.6 -> 47.9, 3794 x 3712 x 512 20.3 -> 16.7, 2750 x 7040 x 384 23.6 ->
                 // 18.5; with block scales 3794 x 3712 x 512 20.3 -> 16.7.
                 int64_t w;
-                if (!pair) w = bn >= 256 ? 125 : 155;
+                // A grid of one round is another matter: nothing hides a tile's way in and out, and both are shorter without a
+                // partner CTA; with most SMs idle the feed is no limit either.  8-bit, one round, pair / one CTA of the same columns, us:
+                // 128 columns 256 x 512 x 1024 5.5 / 5.2, 1024 x 2048 x 512 5.5 / 4.8, 4096 x 512 x 8192 19.4 / 18.5 (256 x 8192 x 8192, which
+                // streams B, 20.5 / 20.9); 256 columns 1024 x 4096 x 512 7.2 / 6.4, 2048 x 2048 x 2048 10.95 / 10.3; block scales, 128 columns
+                // 512 x 4096 x 4096 15.0 / 14.2, 700 x 2048 x 7168 21.3 / 21.6.
+                if (!pair && tiles <= units && !ab16) w = bn >= 256 ? (block ? 125 : 95) : (block ? 125 : 130);
+                else if (!pair) w = bn >= 256 ? 125 : 155;
                 else if (bn == 256) w = 100;
                 else if (bn == 128) w = block ? 130 : 140;
                 else w = block ? 140 : (bn == 224 && kblocks < 8 ? 120 : 110);

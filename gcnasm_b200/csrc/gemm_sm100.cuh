@@ -9,7 +9,7 @@
 //   warp 1      UMMA issuer    (one elected lane)  tcgen05.mma kind::f8f6f4 / kind::mxf8f6f4, TMEM alloc
 //   warps 2-3   idle (they exist so that register re-allocation can work on whole warpgroups)
 //   warps 4-11  epilogue: TMEM -> registers -> scale -> global
-// TMEM holds two accumulator buffers of BN columns.  Per-tensor / unscaled / MX modes accumulate a
+// TMEM holds two accumulator buffers of BN columns (four with block scales and BN = 128).  Per-tensor / unscaled / MX modes accumulate a
 // whole tile in one buffer while the epilogue drains the other.  Block-scale mode gives every
 // 128-wide K group a FRESH buffer (the reference does the same with a fresh MFMA accumulator,
 // kernel_template.hpp:317,334) and the epilogue warps fold it into register accumulators with
@@ -69,6 +69,10 @@ __device__ __forceinline__ void unit_coords(const GemmParams& p, int u, int& t, 
     }
 }
 
+// store staging of one epilogue warp (see store_chunk_coalesced)
+static constexpr int kOutStagePitch = 80;
+static constexpr int kOutStageBytesPerWarp = 32 * kOutStagePitch;
+
 template <int BN_, int MODE_, int BLAYOUT_>
 struct GemmCfg {
     static constexpr bool AB16 = MODE_ == MODE_ACC16;               // bf16 operands: same bytes, kind::f16 MMAs
@@ -79,10 +83,10 @@ struct GemmCfg {
     static constexpr int SFB_ATOMS = (BN + 127) / 128;
     static constexpr int SFB_BYTES = (MODE == MODE_MX) ? SFB_ATOMS * 512 : 0;
     static constexpr int STAGE_BYTES = ((A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES + 1023) / 1024) * 1024;
-    static constexpr int SMEM_BUDGET = 225 * 1024;
-    static constexpr int STAGES_RAW = (SMEM_BUDGET - 1024) / STAGE_BYTES;
+    static constexpr int OUT_STAGE_BYTES = 8 * kOutStageBytesPerWarp;        // store staging of the eight epilogue warps
+    static constexpr int STAGES_RAW = (227 * 1024 - 2048 - OUT_STAGE_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*barriers*/ + 1024 /*alignment slack*/;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*barriers*/ + OUT_STAGE_BYTES + 1024 /*alignment slack*/;
     // accumulator buffers; 128 columns with block scales, a hand-off per K block: as many as tensor memory holds
     static constexpr int BUFS = (MODE == MODE_BLOCK && BN == 128) ? 4 : 2;
     static constexpr int ACC_COLS = BUFS * BN;
@@ -155,8 +159,6 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, void* crow,
 // The way out of the last tile is in nobody's shadow.  With the pieces per row known at compile time and every read issued
 // ahead of the stores (a loop with run-time divisions, one read and one store at a time, before), us: four batches of 700 x 2064 x 1152,
 // fp32, 256 x 192 tiles 13.7 -> 12.7, 256 x 256 tiles 14.9 -> 13.2; 256 x 512 x 1024, bf16, 256 x 256 tiles 8.0 -> 7.3.
-static constexpr int kOutStagePitch = 80;
-static constexpr int kOutStageBytesPerWarp = 32 * kOutStagePitch;
 template <int CNT>
 __device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8_t* cbatch, uint8_t* stage, int row0,
                                                       int col0, const float* v, int lane, bool vec_ok) {
@@ -379,6 +381,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             if (p.scale_a) tscale *= __ldg(p.scale_a);
             if (p.scale_b) tscale *= __ldg(p.scale_b);
         }
+        uint8_t* out_stage = smem_gen + STAGES * Cfg::STAGE_BYTES + 1024 + ew * kOutStageBytesPerWarp;
         uint32_t phase = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {
@@ -386,8 +389,16 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             tile_coords(p, t, b, mi, ni);
             const int row = mi * BM + row_in_tile;
             const int col_base = ni * BN + half * NCH;
-            uint8_t* crow = reinterpret_cast<uint8_t*>(p.c) +
-                            (static_cast<size_t>(b) * p.c_batch + static_cast<size_t>(row) * p.ldc) * esz;
+            uint8_t* cbatch = reinterpret_cast<uint8_t*>(p.c) + static_cast<size_t>(b) * p.c_batch * esz;
+            auto put32 = [&](const int c, const float* o) {              // this warp's 32 rows x columns [32 c, 32 c + 32) of its part
+                const int row0 = mi * BM + quad * 32, col0 = col_base + c * 32;
+                if (p.out_dtype == OUT_BF16) {
+                    store_chunk_coalesced<32>(p, cbatch, out_stage, row0, col0, o, lane, vec_ok);
+                } else {
+                    store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col0, o, lane, vec_ok);
+                    store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col0 + 16, o + 16, lane, vec_ok);
+                }
+            };
 
             if constexpr (MODE == MODE_BLOCK && NCH == 64) {
                 // 64 columns per thread leave room to have both loads of a group in flight, and the buffer goes back before the FMAs;
@@ -437,13 +448,13 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         ++phase;
                     }
                 }
-                if (ok && row < p.m) {
+                if (ok) {
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
                         float o[32];
 #pragma unroll
                         for (int j = 0; j < 16; ++j) unpack_f32x2(acc2[c * 16 + j], o[2 * j], o[2 * j + 1]);
-                        store_row_chunk<32>(p, crow, col_base + c * 32, o, vec_ok);
+                        put32(c, o);
                     }
                 }
             } else if constexpr (MODE == MODE_BLOCK) {
@@ -482,9 +493,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
                 }
-                if (ok && row < p.m) {
+                if (ok) {
 #pragma unroll
-                    for (int c = 0; c < NCH / 32; ++c) store_row_chunk<32>(p, crow, col_base + c * 32, &acc[c * 32], vec_ok);
+                    for (int c = 0; c < NCH / 32; ++c) put32(c, &acc[c * 32]);
                 }
             } else {
                 const uint32_t as = phase & 1;
@@ -511,7 +522,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[c & 1][j] *= tscale;
                     }
-                    if (row < p.m) store_row_chunk<32>(p, crow, col_base + c * 32, v[c & 1], vec_ok);
+                    put32(c, v[c & 1]);
                 }
                 ++phase;
             }
