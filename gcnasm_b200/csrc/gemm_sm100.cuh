@@ -16,8 +16,6 @@
 // acc += partial * (sfa[g][row] * sfb[nblk][g]) -- the analogue of scale_c_tile.
 #pragma once
 
-#include <type_traits>
-
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -155,46 +153,17 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, void* crow,
 // (the TMEM load layout), so a direct store would touch 32 different rows per instruction.  The chunk is written
 // to a warp-private shared-memory buffer (row pitch 80 B: 16-byte accesses stay conflict-free) and read back
 // transposed, so that one store instruction covers whole 32- or 64-byte row segments.
-// `row0` is the output row of lane 0; `stage` is this warp's 2560-byte buffer; CNT * element size is 32 or 64.
+// `row0` is the output row of lane 0; `stage` is this warp's 2560-byte buffer.
 // The way out of the last tile is in nobody's shadow.  With the pieces per row known at compile time and every read issued
 // ahead of the stores (a loop with run-time divisions, one read and one store at a time, before), us: four batches of 700 x 2064 x 1152,
 // fp32, 256 x 192 tiles 13.7 -> 12.7, 256 x 256 tiles 14.9 -> 13.2; 256 x 512 x 1024, bf16, 256 x 256 tiles 8.0 -> 7.3.
-template <int CNT>
-__device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8_t* cbatch, uint8_t* stage, int row0,
-                                                      int col0, const float* v, int lane, bool vec_ok) {
-    const bool bf16 = p.out_dtype == OUT_BF16;
-    const int esz = bf16 ? 2 : 4;
-    if (!(vec_ok && col0 + CNT <= p.n)) {
-        // ragged edge or unaligned output: per-lane path
-        const int row = row0 + lane;
-        if (row < p.m) store_row_chunk<CNT>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, v, false);
-        return;
-    }
+// store_chunk_staged: all columns in range, 16-byte stores allowed.  bf16: 16 or 32 columns; fp32: 16, a row of the buffer.
+template <int CNT, bool BF16>
+__device__ __forceinline__ void store_chunk_staged(const GemmParams& p, uint8_t* cbatch, uint8_t* stage, int row0, int col0, const float* v, int lane) {
+    static_assert(CNT * (BF16 ? 2 : 4) <= 64, "a row of the staging buffer holds 64 bytes");
+    constexpr int ESZ = BF16 ? 2 : 4, PIECES = CNT * ESZ / 16, ROWS = 32 / PIECES;       // 16-byte pieces per row, rows per instruction
     uint8_t* mine = stage + lane * kOutStagePitch;
-    // kPieces 16-byte pieces per row, a compile-time power of two on either branch; with all rows in range the reads go out
-    // together, then the stores
-    auto put = [&](auto pieces, const size_t pitch_c) {
-        constexpr int kPieces = decltype(pieces)::value, kRows = 32 / kPieces;
-        __syncwarp();
-        const int c = lane % kPieces, r = lane / kPieces;
-        const uint8_t* src = stage + r * kOutStagePitch + c * 16;
-        uint8_t* dst = cbatch + (row0 + r) * pitch_c + static_cast<size_t>(col0) * esz + c * 16;
-        if (row0 + 32 <= p.m) {
-            uint4 w[kPieces];
-#pragma unroll
-            for (int i = 0; i < kPieces; ++i) w[i] = *reinterpret_cast<const uint4*>(src + i * kRows * kOutStagePitch);
-#pragma unroll
-            for (int i = 0; i < kPieces; ++i) *reinterpret_cast<uint4*>(dst + i * kRows * pitch_c) = w[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < kPieces; ++i)
-                if (row0 + r + i * kRows < p.m)
-                    *reinterpret_cast<uint4*>(dst + i * kRows * pitch_c) = *reinterpret_cast<const uint4*>(src + i * kRows * kOutStagePitch);
-        }
-        __syncwarp();
-    };
-    const size_t pitch_c = static_cast<size_t>(p.ldc) * esz;
-    if (bf16) {
+    if constexpr (BF16) {
 #pragma unroll
         for (int j = 0; j < CNT; j += 8) {
             uint4 w;
@@ -204,13 +173,43 @@ __device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8
             w.w = pack_bf16x2(v[j + 6], v[j + 7]);
             *reinterpret_cast<uint4*>(mine + j * 2) = w;
         }
-        put(std::integral_constant<int, CNT / 8>{}, pitch_c);
-    } else if constexpr (CNT <= 16) {             // (fp32 chunks are at most 16 columns: 64 bytes, a row of the staging buffer)
+    } else {
 #pragma unroll
-        for (int j = 0; j < CNT; j += 4)
-            *reinterpret_cast<float4*>(mine + j * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        put(std::integral_constant<int, CNT / 4>{}, pitch_c);
+        for (int j = 0; j < CNT; j += 4) *reinterpret_cast<float4*>(mine + j * 4) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     }
+    __syncwarp();
+    const int c = lane % PIECES, r = lane / PIECES;
+    const size_t pitch_c = static_cast<size_t>(p.ldc) * ESZ;
+    const uint8_t* src = stage + r * kOutStagePitch + c * 16;
+    uint8_t* dst = cbatch + (row0 + r) * pitch_c + static_cast<size_t>(col0) * ESZ + c * 16;
+    // with all rows in range the reads go out together, then the stores
+    if (row0 + 32 <= p.m) {
+        uint4 w[PIECES];
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) w[i] = *reinterpret_cast<const uint4*>(src + i * ROWS * kOutStagePitch);
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) *reinterpret_cast<uint4*>(dst + i * ROWS * pitch_c) = w[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i)
+            if (row0 + r + i * ROWS < p.m)
+                *reinterpret_cast<uint4*>(dst + i * ROWS * pitch_c) = *reinterpret_cast<const uint4*>(src + i * ROWS * kOutStagePitch);
+    }
+    __syncwarp();
+}
+// a chunk of 16 columns, or of 32 when the output is bf16 (any other goes out lane by lane, as the ragged and unaligned ones do)
+template <int CNT>
+__device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8_t* cbatch, uint8_t* stage, int row0,
+                                                      int col0, const float* v, int lane, bool vec_ok) {
+    const bool bf16 = p.out_dtype == OUT_BF16;
+    const int esz = bf16 ? 2 : 4;
+    if (!(vec_ok && col0 + CNT <= p.n) || CNT * esz > 64) {
+        const int row = row0 + lane;
+        if (row < p.m) store_row_chunk<CNT>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, v, false);
+        return;
+    }
+    if (bf16) store_chunk_staged<CNT, true>(p, cbatch, stage, row0, col0, v, lane);
+    else if constexpr (CNT <= 16) store_chunk_staged<CNT, false>(p, cbatch, stage, row0, col0, v, lane);
 }
 
 template <class Cfg>
