@@ -389,13 +389,22 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             const int row = mi * BM + row_in_tile;
             const int col_base = ni * BN + half * NCH;
             uint8_t* cbatch = reinterpret_cast<uint8_t*>(p.c) + static_cast<size_t>(b) * p.c_batch * esz;
+            // A warp whose 32 rows are not all there, and every warp of a tile of at most 32 rows, stores from its registers: with few
+            // rows an instruction touches few lines, and there is nothing to wait for.  From registers / staged, us, 8-bit 128 x 128 tiles,
+            // fp32 result: 1, 16, 32 x 2048 x 1024 4.77 / 5.26, 4.78 / 5.24, 4.99 / 5.25; bf16 result 1 x 2048 x 1024 4.77 / 4.87.  From 33
+            // rows on staged, which wins where many CTAs store: 48, 64 x 12288 x 512 5.73 / 5.21, 6.19 / 5.25 (on few CTAs
+            // 48 x 2048 x 1024 5.28 / 5.32).  (Block scales have no such tiles but the last of many rows.)
+            const int rows = p.m - mi * BM;
+            const bool direct = MODE != MODE_BLOCK && (rows <= 32 || rows - quad * 32 < 32);
             auto put32 = [&](const int c, const float* o) {              // this warp's 32 rows x columns [32 c, 32 c + 32) of its part
                 const int row0 = mi * BM + quad * 32, col0 = col_base + c * 32;
-                if (p.out_dtype == OUT_BF16) {
-                    store_chunk_coalesced<32>(p, cbatch, out_stage, row0, col0, o, lane, vec_ok);
+                if (direct || !vec_ok || col0 + 32 > p.n) {
+                    if (row < p.m) store_row_chunk<32>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, o, vec_ok);
+                } else if (p.out_dtype == OUT_BF16) {
+                    store_chunk_staged<32, true>(p, cbatch, out_stage, row0, col0, o, lane);
                 } else {
-                    store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col0, o, lane, vec_ok);
-                    store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col0 + 16, o + 16, lane, vec_ok);
+                    store_chunk_staged<16, false>(p, cbatch, out_stage, row0, col0, o, lane);
+                    store_chunk_staged<16, false>(p, cbatch, out_stage, row0, col0 + 16, o + 16, lane);
                 }
             };
 

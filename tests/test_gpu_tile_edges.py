@@ -1,0 +1,68 @@
+"""Single-CTA tile kernels at the edges of what their ways out and their rings depend on: the rows of a tile that are there (stores from
+registers or through shared memory), one tile per CTA or several (staging in the ring or beside it, its depth), the K blocks against that
+depth, and with block scales the K groups against the number of scales requested ahead.
+
+Operands are whole numbers of at most 2 and scales powers of two, K is at most 2432: a sum is a multiple of 2^-4 below 4 * 2432 * 2^4 <
+2^18, 22 bits, so nothing is ever rounded.  The fp32 output has to equal the reference, the bf16 output its rounding."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+BYTES = torch.tensor([0xC0, 0xB8, 0x00, 0x38, 0x40], dtype=torch.uint8)       # e4m3 of -2 ... 2
+KINDS = [("none", 1), ("none", 2), ("mx", 1), ("bf16", 1), ("bf16", 2), ("block", 1), ("block", 2)]      # tile 1: 128 x 128, 2: 128 x 256
+
+
+def whole(rows, k, seed):
+    return torch.randint(-2, 3, (rows, k), generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+
+
+def product(xa, xb):
+    return (xa.double() @ xb.double().t()).float()
+
+
+def call(api, mode, xa, xb, tile):
+    """(function that multiplies into an output, reference)"""
+    m, k = xa.shape
+    n = xb.shape[0]
+    if mode == "bf16":
+        a, b = xa.bfloat16(), xb.bfloat16()
+        return lambda out: api.gemm_a16w16(a, b, out=out, tile=tile), product(xa, xb)
+    table = BYTES.to(DEV)
+    a, b = table[xa + 2], table[xb + 2]
+    if mode == "mx":
+        ea, eb = (127 + whole(m, k // 32, 3)).to(torch.uint8), (127 + whole(n, k // 32, 4)).to(torch.uint8)
+        sa, sb = api.mx_sf_relayout(ea, m, k), api.mx_sf_relayout(eb, n, k)
+        wa, wb = (x * torch.exp2(e.float() - 127).repeat_interleave(32, dim=1) for x, e in ((xa, ea), (xb, eb)))
+        return lambda out: api.gemm_a8w8_mx(a, b, sa, sb, out=out, tile=tile), product(wa, wb)
+    if mode == "block":
+        groups = k // 128
+        sfa, sfb = torch.exp2(whole(groups, m, 5).float()).contiguous(), torch.exp2(whole(n // 128, groups, 6).float()).contiguous()
+        wa = xa * sfa.t().repeat_interleave(128, dim=1)
+        wb = xb * sfb.repeat_interleave(128, dim=0).repeat_interleave(128, dim=1)
+        return lambda out: api.gemm_a8w8_blockscale(a, b, sfa, sfb, out=out, tile=tile), product(wa, wb)
+    return lambda out: api.gemm_a8w8(a, b, out=out, tile=tile), product(xa, xb)
+
+
+def check(api, mode, m, n, k, tile, around=False):
+    run, ref = call(api, mode, whole(m, k, 1), whole(n, k, 2), tile)
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.full((m, n), 7.0, dtype=dt, device=DEV)
+        run(out)
+        assert torch.equal(out, ref.to(dt)), (mode, m, n, k, tile, dt)
+        if around:
+            # pitches that 16-byte stores fit and do not fit; what lies around C stays as it is
+            for left, extra in ((8, 16), (3, 5)):
+                wide = torch.full((m + 2, n + extra), 7.0, dtype=dt, device=DEV)
+                run(wide[1:m + 1, left:n + left])
+                assert torch.equal(wide[1:m + 1, left:n + left], ref.to(dt))
+                wide[1:m + 1, left:n + left] = 7.0
+                assert torch.all(wide == 7.0)
+    assert api.last_status() == 0
+
+
+# rows of the last tile: one, the last and first of a warp, one to four warps; one tile and a second one below the first
+@pytest.mark.parametrize("mode,tile", KINDS)
+@pytest.mark.parametrize("m", [1, 31, 32, 33, 63, 64, 65, 96, 127, 128, 129, 160, 161])
+def test_rows_of_a_tile(api, mode, tile, m):
+    check(api, mode, m, 384 if mode == "block" else 360, 256, tile, around=True)
