@@ -82,9 +82,16 @@ struct GemmCfg {
     static constexpr int SFB_BYTES = (MODE == MODE_MX) ? SFB_ATOMS * 512 : 0;
     static constexpr int STAGE_BYTES = ((A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES + 1023) / 1024) * 1024;
     static constexpr int OUT_STAGE_BYTES = 8 * kOutStageBytesPerWarp;        // store staging of the eight epilogue warps
-    static constexpr int STAGES_RAW = (227 * 1024 - 2048 - OUT_STAGE_BYTES) / STAGE_BYTES;
-    static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*barriers*/ + OUT_STAGE_BYTES + 1024 /*alignment slack*/;
+    static constexpr int ROOM = 227 * 1024 - 1024 /*barriers*/ - 1024 /*alignment slack*/;
+    static constexpr int STAGES = (ROOM - OUT_STAGE_BYTES) / STAGE_BYTES;           // ring with the staging behind it
+    // Ring of a CTA with one tile, whose staging lies in the ring: 128 columns without MX scales seven stages instead of six.  Behind six
+    // of them a long K waits for its operands, us, six / seven: 8-bit 128 x 8192 x 8192 19.8 / 18.4, 512 x 4096 x 4096 11.6 / 11.0, bf16
+    // 128 x 8192 x 8192 35.1 / 33.0.  CTAs with several tiles keep the staging of its own: the next tile's loads are under way while
+    // a result leaves, and stores from registers instead cost more than the stage gives (2500 x 5120 x 3072 45.0 / 41.5).
+    static constexpr int STAGES_ONE = ROOM / STAGE_BYTES;
+    static constexpr int STAGING_END = STAGES * STAGE_BYTES + OUT_STAGE_BYTES;
+    static constexpr int RING_BYTES = STAGES_ONE * STAGE_BYTES > STAGING_END ? STAGES_ONE * STAGE_BYTES : STAGING_END;
+    static constexpr int SMEM_BYTES = RING_BYTES + 1024 /*barriers*/ + 1024 /*alignment slack*/;
     // accumulator buffers; 128 columns with block scales, a hand-off per K block: as many as tensor memory holds
     static constexpr int BUFS = (MODE == MODE_BLOCK && BN == 128) ? 4 : 2;
     static constexpr int ACC_COLS = BUFS * BN;
@@ -95,7 +102,8 @@ struct GemmCfg {
     static constexpr int THREADS = 384;
     static_assert(ACC_COLS + SF_COLS <= 512, "TMEM overflow");
     static_assert(BN % 32 == 0 && BN <= 256, "BN must be a multiple of 32, at most 256");
-    static_assert(STAGES >= 3, "ring too shallow");
+    static_assert(STAGES >= 3 && STAGES_ONE <= 8, "ring depth");
+    static_assert(OUT_STAGE_BYTES <= STAGES * STAGE_BYTES, "the staging fits the ring");
 };
 
 // tile index -> (batch, m tile, n tile): groups of 8 M tiles walk N, so that the tiles resident at
@@ -214,20 +222,23 @@ __device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8
 
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const __grid_constant__ GemmParams p) {
-    constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES, MODE = Cfg::MODE;
+    constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, MODE = Cfg::MODE;
     constexpr int NCH = Cfg::NCH;
 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    // A CTA that computes one tile stages its result in the ring: every load and MMA has completed when the last accumulator has.
+    const bool one_tile = p.tiles_total <= static_cast<int>(gridDim.x);
+    const uint32_t stages = one_tile ? Cfg::STAGES_ONE : Cfg::STAGES;
     // barrier block sits after the ring
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_gen + STAGES * Cfg::STAGE_BYTES);
-    const uint32_t bar_full0 = smem_base + STAGES * Cfg::STAGE_BYTES;
-    const uint32_t bar_empty0 = bar_full0 + STAGES * 8;
-    const uint32_t bar_accf0 = bar_empty0 + STAGES * 8;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_gen + Cfg::RING_BYTES);
+    const uint32_t bar_full0 = smem_base + Cfg::RING_BYTES;
+    const uint32_t bar_empty0 = bar_full0 + Cfg::STAGES_ONE * 8;
+    const uint32_t bar_accf0 = bar_empty0 + Cfg::STAGES_ONE * 8;
     constexpr int BUFS = Cfg::BUFS;
     const uint32_t bar_acce0 = bar_accf0 + BUFS * 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * BUFS);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * Cfg::STAGES_ONE + 2 * BUFS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -239,7 +250,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     // 10.0 / 8.8, bf16 1 x 4096 x 4096 16.6 / 16.0.
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < Cfg::STAGES_ONE; ++s) {
             mbar_init(bar_full0 + s * 8, 1);
             mbar_init(bar_empty0 + s * 8, 1);
         }
@@ -268,18 +279,23 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     const int groups = (MODE == MODE_BLOCK) ? p.kblocks : 1;          // accumulator phases per tile
     const int kb_per_group = (MODE == MODE_BLOCK) ? 1 : p.kblocks;
 
+    auto next_stage = [stages](uint32_t& s, uint32_t& ph) {           // ring stage and its phase
+        if (++s == stages) {
+            s = 0;
+            ph ^= 1;
+        }
+    };
+
     if (warp < 4) {
         setmaxnreg_dec<40>();
         if (warp == 0 && lane == 0) {
             // ------------------------------ TMA producer ------------------------------
-            uint32_t it = 0;
+            uint32_t s = 0, ph = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {
                 int b, mi, ni;
                 tile_coords(p, t, b, mi, ni);
-                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
-                    const uint32_t s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
+                for (int kb = 0; kb < p.kblocks; ++kb, next_stage(s, ph)) {
                     if (!mbar_wait(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY)) {
                         ok = false;
                         break;
@@ -307,7 +323,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
         } else if (warp == 1) {
             // ------------------------------ UMMA issuer (the warp; an elected lane issues) ------------
             const bool elected = elect_one() != 0;
-            uint32_t it = 0, phase = 0;
+            uint32_t s = 0, ph = 0, phase = 0;
             bool ok = true;
             constexpr uint32_t idesc = make_idesc_f8(BM, BN);
             for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {
@@ -320,9 +336,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     }
                     tc_fence_after();
                     const uint32_t tacc = tmem_base + as * BN;
-                    for (int kb = 0; kb < kb_per_group; ++kb, ++it) {
-                        const uint32_t s = it % STAGES;
-                        const uint32_t ph = (it / STAGES) & 1;
+                    for (int kb = 0; kb < kb_per_group; ++kb, next_stage(s, ph)) {
                         if (!role_all<true>(mbar_wait(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
                             ok = false;
                             break;
@@ -380,7 +394,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             if (p.scale_a) tscale *= __ldg(p.scale_a);
             if (p.scale_b) tscale *= __ldg(p.scale_b);
         }
-        uint8_t* out_stage = smem_gen + STAGES * Cfg::STAGE_BYTES + 1024 + ew * kOutStageBytesPerWarp;
+        uint8_t* out_stage = smem_gen + (one_tile ? 0 : Cfg::STAGES * Cfg::STAGE_BYTES) + ew * kOutStageBytesPerWarp;
         uint32_t phase = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {

@@ -66,3 +66,20 @@ def check(api, mode, m, n, k, tile, around=False):
 @pytest.mark.parametrize("m", [1, 31, 32, 33, 63, 64, 65, 96, 127, 128, 129, 160, 161])
 def test_rows_of_a_tile(api, mode, tile, m):
     check(api, mode, m, 384 if mode == "block" else 360, 256, tile, around=True)
+
+
+# several tiles per CTA and ragged rows and columns
+@pytest.mark.parametrize("mode,tile", KINDS)
+@pytest.mark.parametrize("k", [128, 896])
+def test_several_tiles_per_cta(api, mode, tile, k):
+    check(api, mode, 1313, 4096 if mode == "block" else 4072, k, tile, around=True)
+
+
+# K blocks (K groups with block scales): fewer, as many and more than the ring's stages (4, 6 or 7) and the scales ahead
+@pytest.mark.parametrize("mode,tile", KINDS)
+@pytest.mark.parametrize("kblocks", [1, 2, 3, 4, 5, 6, 7, 8, 11, 12, 13, 14, 15, 18, 19])
+def test_k_blocks_against_the_ring(api, mode, tile, kblocks):
+    k = kblocks * (64 if mode == "bf16" else 128)
+    check(api, mode, 200, 512, k, tile)
+    if kblocks in (1, 5, 6, 7, 8, 13):
+        check(api, mode, 1400, 3840, k, tile)              # 330 tiles of 128 x 128, 165 of 128 x 256
