@@ -427,24 +427,28 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 // four buffers keep the tensor core busy meanwhile.  Two buffers, handed back after the FMAs, and scalar FMAs, us: 100 x
                 // 7168 x 2048 9.85 -> 8.85, 200 x 7168 x 2048 10.7 -> 9.6, 512 x 4096 x 4096 16.5 -> 14.2, 2500 x 5120 x 3072 75 -> 65.  (The
                 // same loop for 128 columns per thread, two buffers, was slower: 700 x 2048 x 7168 28.9 -> 30.7.)
-                // Scales are requested two groups ahead, into two register sets that take turns (a copy from one to the
-                // other would wait for the load): a load queues behind the operand tiles in flight.
+                // Scales are requested six groups ahead, into six register sets that take turns (a copy from one to the
+                // other would wait for the load): a load queues behind the operand tiles in flight, and with the tensor core four buffers
+                // ahead there are more of those than with two.  Two / four / six / eight ahead, us: 128 x 8192 x 8192 32.8 / 27.8 / 25.6 /
+                // 25.1 (scalar FMAs, two buffers, one ahead: 31.4), 256 x 512 x 8192 27.2 / 24.5 / 23.6 / 23.6, 1024 x 1024 x 512 4.80 /
+                // 4.85 / 4.89 / 4.90; the loop's code grows with the sets.
                 unsigned long long acc2[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc2[j] = 0ull;
                 const float* sfa_p = p.sfa + b * p.sfa_batch + (row < p.m ? row : 0);
                 const float* sfb_p = p.sfb + b * p.sfb_batch + static_cast<long long>(col_base / 128) * p.sfb_stride;
                 const bool col_ok = col_base < p.n;
-                float sa[2], sb[2];
+                constexpr int SETS = 6;
+                float sa[SETS], sb[SETS];
                 auto request = [&](const int g, const int set) {
                     sa[set] = __ldg(sfa_p + static_cast<long long>(g) * p.sfa_stride);
                     sb[set] = col_ok ? __ldg(sfb_p + g) : 0.0f;
                 };
-                request(0, 0);
-                request(groups > 1 ? 1 : 0, 1);
-                for (int g0 = 0; g0 < groups && ok; g0 += 2) {
 #pragma unroll
-                    for (int set = 0; set < 2; ++set) {
+                for (int set = 0; set < SETS; ++set) request(set < groups ? set : 0, set);
+                for (int g0 = 0; g0 < groups && ok; g0 += SETS) {
+#pragma unroll
+                    for (int set = 0; set < SETS; ++set) {
                         const int g = g0 + set;
                         if (g >= groups) break;
                         const uint32_t as = phase % BUFS;
@@ -464,7 +468,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
-                        if (g + 2 < groups) request(g + 2, set);
+                        if (g + SETS < groups) request(g + SETS, set);
 #pragma unroll
                         for (int j = 0; j < 32; ++j) acc2[j] = ffma2(pack_f32x2(v[2 * j], v[2 * j + 1]), sc2, acc2[j]);
                         ++phase;
