@@ -314,11 +314,21 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 // 18.5; with block scales 3794 x 3712 x 512 20.3 -> 16.7.
                 int64_t w;
                 // A grid of one round is another matter: nothing hides a tile's way in and out, and both are shorter without a
-                // partner CTA; with most SMs idle the feed is no limit either.  8-bit, one round, pair / one CTA of the same columns, us:
-                // 128 columns 256 x 512 x 1024 5.5 / 5.2, 1024 x 2048 x 512 5.5 / 4.8, 4096 x 512 x 8192 19.4 / 18.5 (256 x 8192 x 8192, which
-                // streams B, 20.5 / 20.9); 256 columns 1024 x 4096 x 512 7.2 / 6.4, 2048 x 2048 x 2048 10.95 / 10.3; block scales, 128 columns
-                // 512 x 4096 x 4096 15.0 / 14.2, 700 x 2048 x 7168 21.3 / 21.6.
-                if (!pair && tiles <= units && !ab16) w = bn >= 256 ? (block ? 125 : 95) : (block ? 125 : 130);
+                // partner CTA.  Against that stands what a K block takes, so for some kinds K decides; pair / one CTA, us back to back at
+                // K = 512, 2048, 4096, 8192:
+                //   8-bit, 128 columns       256 x 512 (8 tiles)   4.5 / 3.9   7.1 / 6.2   10.6 / 9.3    17.7 / 15.5
+                //                            256 x 8192 (128)      5.3 / 4.0   8.3 / 7.0   12.2 / 10.5   21.5 / 20.0     one CTA
+                //   block scales, 128        256 x 512 (8)         5.1 / 4.5   8.6 / 8.1   13.2 / 13.1   22.5 / 23.0
+                //                            700 x 2048 (96)       5.6 / 4.5   9.4 / 9.0   14.7 / 14.7   24.6 / 25.6
+                //                            2048 x 1024 (128)     6.0 / 4.5   9.8 / 9.0   15.1 / 14.9   35.0 / 25.9
+                // With block scales a pair hands its accumulator over once for twice the rows, which wins from K = 4096 on until the
+                // single tiles, one per SM, have more SMs than the pairs can use.  8-bit, 256 columns against the pair's best:
+                // 769 x 4608 x 512 6.9 / 5.4, 1110 x 3968 x 3072 16.2 / 12.1, 1398 x 2688 x 4096 14.9 / 14.5, but 1096 x 2816 x 7168 21.5 /
+                // 23.4 and, two rows of tiles and B streaming from HBM, 190 x 16640 x 4096 18.7 / 20.0: a single tile fetches 48 KB per K
+                // block through four stages, a CTA of a pair 32 through six.
+                const bool one_round = !pair && tiles <= units && !ab16;
+                if (one_round && block && (bn >= 256 || kblocks <= 32 || tiles * 2 > units)) w = 125;
+                else if (one_round && !block && (bn < 256 || kblocks <= (tm1 > 2 ? 32 : 24))) w = bn >= 256 ? 95 : 130;
                 else if (!pair) w = bn >= 256 ? 125 : 155;
                 else if (bn == 256) w = 100;
                 else if (bn == 128) w = block ? 130 : 140;

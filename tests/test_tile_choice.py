@@ -1,0 +1,43 @@
+"""CPU: which kernel the launcher picks, at the lines where measured times cross (148 SMs)."""
+import ctypes as C
+
+import pytest
+
+from gcnasm_b200 import _lib as L
+
+
+def args(m, n, k, mode=L.SCALE_NONE, hint=L.TILE_AUTO, flags=0, layout=L.B_NK_ROWMAJOR, batch=1):
+    a = L.GemmArgs()
+    a.ptr_a, a.ptr_b, a.ptr_c = 0x10000, 0x20000, 0x30000
+    a.m, a.n, a.k, a.batch = m, n, k, batch
+    a.stride_a = a.stride_b = k
+    a.stride_c = n
+    a.stride_a_batch, a.stride_b_batch, a.stride_c_batch = m * k, n * k, m * n
+    a.scale_mode, a.tile_hint, a.flags, a.b_layout, a.out_dtype = mode, hint, flags, layout, L.OUT_BF16
+    if mode in (L.SCALE_BLOCK, L.SCALE_MX):
+        a.ptr_sfa, a.ptr_sfb = 0x40000, 0x50000
+    if mode == L.SCALE_BLOCK:
+        a.stride_sfa, a.stride_sfb = m, k // 128
+    if mode == L.SCALE_MX:
+        a.stride_sfa_batch, a.stride_sfb_batch = (m + 127) // 128 * (k // 128) * 512, (n + 127) // 128 * (k // 128) * 512
+    return a
+
+
+def choice(native, *problem, **more):
+    tile = C.c_int32(-1)
+    rc = native.b200_gemm_check(C.byref(args(*problem, **more)), C.byref(tile))
+    return tile.value if rc == L.OK else rc
+
+
+ONE, ONE256, PAIR256, PAIR128, PAIR224 = L.TILE_128x128, L.TILE_128x256, L.TILE_PAIR_256x256, L.TILE_PAIR_256x128, L.TILE_PAIR_256x224
+
+
+# a grid of one round: with block scales and few tiles a long K is the pair's, without scales never; 256 columns are for a short K
+@pytest.mark.parametrize("mode,m,n,k,tile", [
+    (L.SCALE_BLOCK, 256, 512, 512, ONE), (L.SCALE_BLOCK, 256, 512, 4096, ONE), (L.SCALE_BLOCK, 256, 512, 4224, PAIR128),
+    (L.SCALE_BLOCK, 256, 512, 8192, PAIR128), (L.SCALE_BLOCK, 1024, 1024, 8192, PAIR128), (L.SCALE_BLOCK, 2048, 1024, 8192, ONE),
+    (L.SCALE_NONE, 256, 512, 1024, ONE), (L.SCALE_NONE, 256, 512, 8192, ONE), (L.SCALE_NONE, 256, 8192, 8192, ONE),
+    (L.SCALE_NONE, 769, 4608, 512, ONE256), (L.SCALE_NONE, 1398, 2688, 4096, ONE256), (L.SCALE_NONE, 1096, 2816, 7168, PAIR224),
+    (L.SCALE_NONE, 190, 16640, 3072, ONE256), (L.SCALE_NONE, 190, 16640, 4096, PAIR256)])
+def test_one_round(native, mode, m, n, k, tile):
+    assert choice(native, m, n, k, mode) == tile
