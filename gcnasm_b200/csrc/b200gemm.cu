@@ -326,7 +326,8 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 // 769 x 4608 x 512 6.9 / 5.4, 1110 x 3968 x 3072 16.2 / 12.1, 1398 x 2688 x 4096 14.9 / 14.5, but 1096 x 2816 x 7168 21.5 /
                 // 23.4 and, two rows of tiles and B streaming from HBM, 190 x 16640 x 4096 18.7 / 20.0: a single tile fetches 48 KB per K
                 // block through four stages, a CTA of a pair 32 through six.
-                const bool one_round = !pair && tiles <= units && !ab16;
+                // (Calls whose inputs are ready keep the pair's tiles: those start under the predecessor's last tiles, a single CTA waits.)
+                const bool one_round = !pair && tiles <= units && !ab16 && !(a->flags & B200_GEMM_INPUTS_READY);
                 if (one_round && block && (bn >= 256 || kblocks <= 32 || tiles * 2 > units)) w = 125;
                 else if (one_round && !block && (bn < 256 || kblocks <= (tm1 > 2 ? 32 : 24))) w = bn >= 256 ? 95 : 130;
                 else if (!pair) w = bn >= 256 ? 125 : 155;

@@ -41,3 +41,11 @@ ONE, ONE256, PAIR256, PAIR128, PAIR224 = L.TILE_128x128, L.TILE_128x256, L.TILE_
     (L.SCALE_NONE, 190, 16640, 3072, ONE256), (L.SCALE_NONE, 190, 16640, 4096, PAIR256)])
 def test_one_round(native, mode, m, n, k, tile):
     assert choice(native, m, n, k, mode) == tile
+
+
+# inputs that are ready: the pair kernels start before the predecessor has finished, so what they would take is not given to single CTAs
+@pytest.mark.parametrize("mode", [L.SCALE_NONE, L.SCALE_TENSOR, L.SCALE_BLOCK])
+@pytest.mark.parametrize("m,n,k,tile", [(1024, 1792, 1024, PAIR128), (256, 512, 1024, PAIR128), (512, 4096, 4096, PAIR128)])
+def test_ready_inputs_keep_the_pair_kernels(native, mode, m, n, k, tile):
+    assert choice(native, m, n, k, mode) == ONE
+    assert choice(native, m, n, k, mode, flags=L.GEMM_INPUTS_READY) == tile
