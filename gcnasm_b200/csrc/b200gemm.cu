@@ -230,6 +230,24 @@ struct Plan {
     int splits;      // decode K splits
 };
 
+// MX with few tokens: the K blocks from which the skinny-M kernel beats the 128 x 128 tiles, which have the shorter fixed part.  Its own
+// is the sum over the splits of a panel: tokens / splits rows of remote loads, on every warp of the panel's CTAs; what the splits save
+// grows with K.  So one split (more panels than half the SMs) and few tokens cross over early, 64 tokens in two splits late.  Time with
+// the skinny kernel over time with the tiles, at 768, 1024, 1536, 2048, 2560 (N = 128 panels):
+//   panels 75, 144 (one split)   m = 1  0.65 0.66 0.73 0.72 0.69   64  0.81 0.83 0.95 0.98 0.94     144:  1  0.77 .. 0.67  64  0.93 .. 0.97
+//   panels 16                    m = 16 0.89 0.80 0.76 0.68 0.59   64  1.20 1.05 0.95 0.84 0.79
+//   panels 64 (two splits)       m = 16 0.97 0.94 0.90 0.86 0.84   32  1.08 1.04 0.98 0.93 0.91   48  1.14 1.09 1.03 0.98 0.91
+//                                m = 64 1.26 1.19 1.12 1.05 0.97
+//   panels 74                    m = 32 1.04 1.01 1.00 0.98 0.92   48  1.15 1.13 1.10 1.07 0.97   64  1.28 1.22 1.18 1.14 1.03
+// Below six K blocks nothing was measured but four (5.0 / 3.8 us, 64 x 512).
+constexpr int kMxSkinnyLeast = 6;
+int64_t mx_skinny_kblocks(int64_t m, int64_t panels, int sm_count) {
+    if (m <= 16 || panels * 2 > sm_count) return kMxSkinnyLeast;
+    if (m <= 32 || panels * 4 <= sm_count) return 12;
+    const int64_t line = (m + 2 * panels * 148 / sm_count - 88 + 5) / 6;       // a plane through the crossings of 33-64 tokens, 38-74 panels
+    return line > 12 ? line : 12;
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ab16: `a` is the byte view of a bf16 problem (K and the A/B strides counted in bytes)
@@ -284,10 +302,7 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
     // MX pair kernels address the scale atoms through a tensor map: batch strides in whole atoms
     const bool mx_pair_ok = !mx || a->batch == 1 || (a->stride_sfa_batch % 512 == 0 && a->stride_sfb_batch % 512 == 0);
     if (hint == B200_TILE_AUTO) {
-        // MX: from twelve K blocks on.  Below that the 128 x 128 tiles' shorter fixed part wins; skinny kernel / tile, us: 64 x 512 x 512
-        // 5.0 / 3.8, 64 x 8192 x 512 5.7 / 4.1, 40 x 4096 x 1024 5.4 / 4.9; 64 x 2048 x 2048 6.0 / 7.4, 16 x 2048 x 2048 4.8 / 7.0,
-        // 1 x 512 x 8192 6.0 / 20.3, 1, 16, 64 x 8192 x 8192 13.8 / 28.6, 14.5 / 21.6, 16.6 / 22.0.
-        if (decode_ok && (!mx || kblocks >= 12)) {
+        if (decode_ok && (!mx || kblocks >= mx_skinny_kblocks(a->m, (a->n + 127) / 128 * a->batch, sm_count))) {
             hint = B200_TILE_DECODE;
         } else {
             // cost of a persistent schedule: rounds (in tenths) x time per tile, proportional to the tile's N; with block

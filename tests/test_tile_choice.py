@@ -49,3 +49,16 @@ def test_one_round(native, mode, m, n, k, tile):
 def test_ready_inputs_keep_the_pair_kernels(native, mode, m, n, k, tile):
     assert choice(native, m, n, k, mode) == ONE
     assert choice(native, m, n, k, mode, flags=L.GEMM_INPUTS_READY) == tile
+
+
+# MX with few tokens: the skinny-M kernel from 6 K blocks on (few tokens, or one split a panel), 12, or later with many tokens in two splits
+@pytest.mark.parametrize("m,n,k,skinny", [
+    (1, 512, 640, False), (1, 512, 768, True), (16, 9472, 768, True), (17, 512, 768, False), (17, 512, 1408, False), (17, 512, 1536, True),
+    (64, 512, 1408, False), (64, 512, 1536, True), (64, 9600, 640, False), (64, 9600, 768, True), (32, 9472, 1536, True),
+    (48, 7168, 1536, True), (64, 7168, 1536, False), (64, 7168, 2048, True), (48, 8192, 1536, False), (64, 8192, 2048, False),
+    (64, 8192, 2304, True), (64, 9472, 2560, False), (64, 9472, 2688, True)])
+def test_mx_few_tokens(native, m, n, k, skinny):
+    assert (choice(native, m, n, k, L.SCALE_MX) == L.TILE_DECODE) == skinny
+    # the same panels as batches of one quarter of the columns
+    if n % 512 == 0:
+        assert (choice(native, m, n // 4, k, L.SCALE_MX, batch=4) == L.TILE_DECODE) == skinny
