@@ -296,7 +296,7 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
     const int64_t kblocks = (a->k + 127) / 128;
     const bool decode_ok = !pair_only && !ab16 && a->m <= 64 && (a->n % 16 == 0);
     int hint = a->tile_hint;
-    if (hint == B200_TILE_DECODE && (!decode_ok || a->scale_mode == B200_SCALE_MX)) return B200_ERR_UNSUPPORTED;
+    if (hint == B200_TILE_DECODE && (!decode_ok || (a->scale_mode == B200_SCALE_MX && kblocks < kMxSkinnyLeast))) return B200_ERR_UNSUPPORTED;
     if (hint == B200_TILE_128x64) return B200_ERR_UNSUPPORTED;
     const bool mx = a->scale_mode == B200_SCALE_MX;
     // MX pair kernels address the scale atoms through a tensor map: batch strides in whole atoms

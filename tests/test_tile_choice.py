@@ -62,3 +62,14 @@ def test_mx_few_tokens(native, m, n, k, skinny):
     # the same panels as batches of one quarter of the columns
     if n % 512 == 0:
         assert (choice(native, m, n // 4, k, L.SCALE_MX, batch=4) == L.TILE_DECODE) == skinny
+
+
+# what b200_gemm_check reports is accepted as a hint
+@pytest.mark.parametrize("mode", [L.SCALE_NONE, L.SCALE_BLOCK, L.SCALE_MX])
+@pytest.mark.parametrize("layout", [L.B_NK_ROWMAJOR, L.B_FLAT_16x16])
+def test_the_reported_tile_is_a_valid_hint(native, mode, layout):
+    for m in (1, 16, 40, 64, 65, 200, 4096):
+        for n in (512, 8192, 18432):
+            for k in (256, 768, 2048, 8192):
+                tile = choice(native, m, n, k, mode, layout=layout)
+                assert tile > 0 and choice(native, m, n, k, mode, layout=layout, hint=tile) == tile
