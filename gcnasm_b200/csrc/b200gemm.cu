@@ -239,7 +239,8 @@ struct Plan {
 //   panels 64 (two splits)       m = 16 0.97 0.94 0.90 0.86 0.84   32  1.08 1.04 0.98 0.93 0.91   48  1.14 1.09 1.03 0.98 0.91
 //                                m = 64 1.26 1.19 1.12 1.05 0.97
 //   panels 74                    m = 32 1.04 1.01 1.00 0.98 0.92   48  1.15 1.13 1.10 1.07 0.97   64  1.28 1.22 1.18 1.14 1.03
-// Below six K blocks nothing was measured but four (5.0 / 3.8 us, 64 x 512).
+// For instance, us, skinny kernel / tiles: 64 x 8192 x 1536 7.6 / 6.8, 64 x 9472 x 1664 8.5 / 7.2, 16 x 8192 x 1024 5.1 / 5.4, 64 x 9600 x 1024
+// 4.7 / 5.7, 1 x 12288 x 1024 4.6 / 7.3.  Below six K blocks only four were measured (64 x 512 x 512 5.0 / 3.8).
 constexpr int kMxSkinnyLeast = 6;
 int64_t mx_skinny_kblocks(int64_t m, int64_t panels, int sm_count) {
     if (m <= 16 || panels * 2 > sm_count) return kMxSkinnyLeast;

@@ -18,8 +18,8 @@
 // register accumulators as acc += partial * (sfa[g][token] * sfb[nblk][g]).
 //
 // MX scales: the tensor core applies them, so a CTA's whole K range accumulates in one TMEM buffer; the E8M0 atoms of the weight
-// panel and of the token block travel with their stage.  Such calls used to run on the 128 x 128 single-CTA tile, at most one
-// CTA per 128 weight rows; here a panel's K is split over a cluster.
+// panel and of the token block travel with their stage.  The 128 x 128 single-CTA tile has at most one CTA per 128 weight rows; here a
+// panel's K is split over a cluster (mx_skinny_kblocks() says from which K on that pays).
 #pragma once
 
 #include "gemm_sm100.cuh"
@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
             // a thread holds one column of the output: the warp turns its 32 columns round in shared memory and stores 16 bytes
             // per lane, 64 (128) contiguous bytes per token.  One two-byte store per token and thread, written out token by token,
             // was most of what a 64-token call took longer than one of 1 token whatever K (18432 x 7168, in a graph, 64 tokens:
-            // 24.9 -> 23.4 us, K = 3584 15.4 -> 13.7; 32 tokens 23.05 -> 22.35; 16 22.1 -> 21.8; one token the same).
+            // 24.9 -> 23.4 us, K = 3584 15.4 -> 13.7; 32 tokens 23.05 -> 22.35; 16 22.1 -> 21.8; one token the same; on another GPU of the
+            // kind 64 tokens 25.6 -> 24.15).
             uint8_t* mine = smem_gen + quad * (MT * 128);
             const int pieces = p.out_dtype == OUT_BF16 ? 4 : 8;                       // 16-byte pieces per token
             if (p.out_dtype == OUT_BF16) {

@@ -424,9 +424,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
 
             if constexpr (MODE == MODE_BLOCK && NCH == 64) {
                 // 64 columns per thread leave room to have both loads of a group in flight, and the buffer goes back before the FMAs;
-                // four buffers keep the tensor core busy meanwhile.  Two buffers, handed back after the FMAs, and scalar FMAs, us: 100 x
-                // 7168 x 2048 9.85 -> 8.85, 200 x 7168 x 2048 10.7 -> 9.6, 512 x 4096 x 4096 16.5 -> 14.2, 2500 x 5120 x 3072 75 -> 65.  (The
-                // same loop for 128 columns per thread, two buffers, was slower: 700 x 2048 x 7168 28.9 -> 30.7.)
+                // four buffers keep the tensor core busy meanwhile.  Two buffers, handed back after the FMAs, scalar FMAs and stores
+                // from registers / this loop and staged stores, us: 100 x 7168 x 2048 10.6 / 9.2, 200 x 7168 x 2048 11.3 / 9.6, 512 x 4096 x
+                // 4096 16.8 / 15.0, 2500 x 5120 x 3072 77 / 59.  (The same loop for 128 columns per thread, two buffers, was slower:
+                // 700 x 2048 x 7168 28.9 -> 30.7.)
                 // Scales are requested six groups ahead, into six register sets that take turns (a copy from one to the
                 // other would wait for the load): a load queues behind the operand tiles in flight, and with the tensor core four buffers
                 // ahead there are more of those than with two.  Two / four / six / eight ahead, us: 128 x 8192 x 8192 32.8 / 27.8 / 25.6 /

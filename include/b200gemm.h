@@ -84,9 +84,10 @@ typedef struct b200_gemm_args {
  * still in flight on the stream (for instance consecutive GEMMs of independent requests, or weights and
  * activations prepared earlier).  The 2-CTA tile kernels then start loading and multiplying at once -- on the SMs
  * the previous launch no longer uses, e.g. during its last, partly filled wave of tiles -- and only their writes to
- * C wait for the previous kernel.  The skinny-M kernel requests its first ring of WEIGHT tiles before it waits for
- * the previous kernel only when this flag is set (without it a weight written by the previous kernel -- a shuffle,
- * a quantiser, a copy -- is read only after that kernel has completed).  The single-CTA tile kernels ignore it.
+ * C wait for the previous kernel.  The skinny-M kernel requests its first ring of WEIGHT tiles, with MX their scale
+ * atoms too, before it waits for the previous kernel only when this flag is set (without it a weight written by the
+ * previous kernel -- a shuffle, a quantiser, a copy -- is read only after that kernel has completed).  The single-CTA
+ * tile kernels ignore it, so fewer problems are given to them when it is set.
  * B200_GEMM_BATCH_READY turns `batch` into a sequence of activation slabs that may still be arriving while the
  * kernel runs: before anything of batch b's A or SFA is read, the kernel waits until ptr_batch_ready[b] >=
  * batch_epoch (a bounded wait: after about 2 s the launch gives up and b200_last_status() reports 8).  Whoever delivers
@@ -163,8 +164,8 @@ int b200_gemm_a8w8_host(const b200_gemm_args* host_args, void* cuda_stream);
  *   - Limit: splits * batch * M * N fp32 partials must fit in 1 MiB (262,144 floats), whether or not the launch
  *     goes through the workspace (splits: the power of two, at most 16, that fills the SMs with CTAs; with block scales
  *     doubled further until a CTA's scales fit its shared memory); otherwise the call returns B200_ERR_TOO_LARGE and
- *     launches nothing.  Shapes the launcher would not send to the skinny-M kernel (M > 64, MX scales) return
- *     B200_ERR_UNSUPPORTED.
+ *     launches nothing.  Shapes the launcher would not send to the skinny-M kernel (M > 64) and MX scales, with which
+ *     b200_gemm_a8w8 does use that kernel, return B200_ERR_UNSUPPORTED.
  *   - The first call on each device looks up that device's address of the array (and the library's other
  *     per-device set-up); make that first call before starting any stream capture.
  *   - All calls on a device share the one array and it keeps the previous call's contents.  Nothing needs

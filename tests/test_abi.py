@@ -86,7 +86,7 @@ def test_validation_codes(native):
     # flat B: whole 16x16 blocks (asserts at flatmm_a8w8_gfx950.cc:650-651)
     assert chk(_args(b_layout=L.B_FLAT_16x16)) == L.OK
     assert chk(_args(b_layout=L.B_FLAT_16x16, n=500, stride_c=500)) == L.ERR_UNSUPPORTED
-    # tile selection: skinny M goes to the decode kernel, MX to 128x128
+    # tile selection: skinny M goes to the decode kernel, MX of more rows to 128x128 or pair tiles
     assert chk(_args(m=16)) == L.OK and tile.value == L.TILE_DECODE
     assert chk(_args(**{**bs, "m": 64, "stride_sfa": 64})) == L.OK and tile.value == L.TILE_DECODE
     assert chk(_args(m=65)) == L.OK and tile.value != L.TILE_DECODE
