@@ -17,8 +17,8 @@ def T(x):
     return torch.from_numpy(np.ascontiguousarray(x)).to(DEV)
 
 
-# token blocks of 16, 32 and 64 at their edges; N of one slab, one panel, ragged panels, many panels; the fewest K blocks that go
-# this way (twelve), one fewer (the tile kernel), more than the ring holds
+# token blocks of 16, 32 and 64 at their edges; N of one slab, one panel, ragged panels, many panels; twelve K blocks, the fewest that
+# more than 16 tokens in K splits go this way with, one fewer (the tile kernel), more than the ring holds
 @pytest.mark.parametrize("m,n,k", [(1, 16, 1536), (16, 128, 1536), (17, 208, 1664), (32, 1040, 2048), (33, 256, 4096), (63, 4096, 1536),
                                    (64, 2064, 1664), (1, 8192, 2048), (64, 128, 4096), (64, 128, 1408)])
 def test_skinny_mx(api, O, m, n, k):
