@@ -95,7 +95,7 @@ static constexpr int kProducerWarp = 3;
 // 7 loop top, 6 accumulator-full barrier passed, 0 first loads issued, 3 first wait::ld done, 4 last load landed,
 // 1 buffer handed back, 5 / 2 the FMAs of the hand-back chunk / of the last chunk have completed (these two read the
 // clock behind a data dependency on the accumulator; a plain clock read does not order against arithmetic)
-// then [phase < 128]: when a polling observer (warp 0 of the leader) saw the group's accumulator-full barrier flip
+// then [phase < 128]: when a polling observer (warp 2 of the other CTA) saw the group's accumulator-full barrier flip
 __device__ long long g_trace[2 * 8 * 128 * 8 + 128 * 8 + 128];
 #define B200_TRACE_EPI(slot)                                                                     \
     do {                                                                                         \
@@ -141,6 +141,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
     const uint32_t bar_acce0 = bar_accf0 + 2 * 8;                       // used in the leader only
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* requested = reinterpret_cast<volatile int*>(tmem_slot + 2);    // block scales: the K block the TMA producer is at
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -166,6 +167,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
             mbar_init(bar_acce0 + s * 8, 2 * Cfg::EPI_WARPS);   // every epilogue warp of the two CTAs
         }
         *abort_flag = 0;
+        *requested = 0;
         fence_barrier_init();
         fence_proxy_async_smem();
     }
@@ -238,6 +240,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
                     const uint32_t sb = sa + Cfg::A_BYTES;
                     if (!elected) continue;
+                    if constexpr (MODE == MODE_BLOCK) *requested = static_cast<int>(it);
                     B200_TRACE_PROD(0);
                     if (cta == 0)
                         mbar_arrive_expect_tx(bar_full0 + s * 8,
@@ -348,8 +351,62 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                 }
             }
         }
+        else if (MODE == MODE_BLOCK && warp == 0) {
+            // ------------------------------ scales into L1 (both CTAs) ------------------------------
+            // An epilogue warp that runs behind has some 300 clocks between asking for a group's scales and using them; a load
+            // that L1 misses takes 350 of a quiet L2 and 700 behind the operand tiles in flight, an L1 hit 110.  So this warp reads
+            // every scale of the tile once, some groups before the producer asks for the operands (a hint: nothing waits for it).
+            // Touched / not, us: 16384 x 7168 x 8192 958 / 1087, 8192^3 532 / 581, 4096 x 7168 x 2048 70.1 / 75.7, 512 x 9472 x 8192
+            // 39.3 / 45.2.  prefetch.global.L1 comes as far as L2 (a later load takes 280 clocks): 1001 / 1048 on the first of these.
+            // The same ring in shared memory, filled by cp.async or by this warp, had at most five groups of room beside the
+            // tiles: 4-8 % on 256 columns, a loss on 128 and on short K.
+            constexpr int kBatch = 4, kAhead = 3;            // groups per request; groups ahead of the producer
+            float x[kBatch + 1], sum = 0.0f;
+#pragma unroll
+            for (int i = 0; i <= kBatch; ++i) x[i] = 0.0f;
+            int q = 0, ready_b = -1;                         // K groups behind this one; last batch whose ready word has been seen
+            bool go = true;
+            for (int u = pair_id; u < units_total && go; u += num_pairs) {
+                int t = u, part = -1;
+                if constexpr (kTail) unit_coords(p, u, t, part);
+                int b, mi, ni;
+                tile_coords(p, t, b, mi, ni);
+                if (p.batch_ready && b != ready_b) {
+                    // (L1 would keep what a scale was before its slab came)
+                    int seen = 1;
+                    if (lane == 0) seen = wait_ready_word(p.batch_ready + b, p.batch_epoch, abort_flag, p.status) ? 1 : 0;
+                    if (!__shfl_sync(0xFFFFFFFFu, seen, 0)) break;
+                    ready_b = b;
+                }
+                // a lane per 16 bytes of A's 128 rows, and per 128-column block of B that the tile may touch
+                const int row = mi * (2 * BM) + static_cast<int>(cta) * BM + lane * 4, blk = ((ni * BN) >> 7) + lane;
+                const float* pa = p.sfa + b * p.sfa_batch + (row < p.m ? row : p.m - 1);
+                const bool col_ok = lane <= (BN + 127) / 128 && (blk << 7) < p.n;
+                const float* pb = p.sfb + b * p.sfb_batch + (col_ok ? static_cast<long long>(blk) * p.sfb_stride : 0);
+                for (int g = 0; g < groups && go; g += kBatch) {
+                    const int cnt = groups - g < kBatch ? groups - g : kBatch;
+                    int polls = 0;
+                    while (q > *requested + kAhead && go) {
+                        go = !*abort_flag && ++polls < (1 << 20);
+                        __nanosleep(200);
+                    }
+                    go = __all_sync(0xFFFFFFFFu, go);
+                    // (added up only here, so that the loads of the batch before have had its time to arrive)
+#pragma unroll
+                    for (int i = 0; i <= kBatch; ++i) sum += x[i];
+#pragma unroll
+                    for (int i = 0; i < kBatch; ++i)
+                        if (i < cnt) x[i] = ld_nc_f32(pa + static_cast<long long>(g + i) * p.sfa_stride);
+                    if (col_ok) x[kBatch] = ld_nc_f32(pb + g);
+                    q += cnt;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i <= kBatch; ++i) sum += x[i];
+            if (__float_as_uint(sum) == 0xFFFFFFFFu) *requested = -1;      // (keeps the loads; no sum has these bits)
+        }
 #ifdef B200_TRACE
-        else if (MODE == MODE_BLOCK && warp == 0 && lane == 0 && cta == 0 && pair_id == 0) {
+        else if (MODE == MODE_BLOCK && warp == 2 && lane == 0 && cta == 1 && pair_id == 0) {
             uint32_t phase = 0;
             bool ok = true;
             for (int u = pair_id; u < units_total && ok && phase < 128; u += num_pairs)
@@ -592,9 +649,13 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                             if (lane == 0) mbar_arrive_cluster(leader_acce0 + as * 8);
                             B200_TRACE_EPI(1);
                             if (g + 1 < groups) {
-                                sa_cur = __ldg(sfa_p + static_cast<long long>(g + 1) * p.sfa_stride);
-                                sb0_cur = col_ok ? __ldg(sfb_p + g + 1) : 0.0f;
-                                if (kStraddle) sb1_cur = has1 ? __ldg(sfb_p + p.sfb_stride + g + 1) : 0.0f;
+                                // (running pointers: with the address multiplied out per group, 16384 x 7168 x 8192 909 -> 958 us,
+                                // 4096 x 7168 x 4096 on 256 x 192 tiles 149 -> 171)
+                                sfa_p += p.sfa_stride;
+                                ++sfb_p;
+                                sa_cur = __ldg(sfa_p);
+                                sb0_cur = col_ok ? __ldg(sfb_p) : 0.0f;
+                                if (kStraddle) sb1_cur = has1 ? __ldg(sfb_p + p.sfb_stride) : 0.0f;
                             }
                         }
                         fma_chunk(c);

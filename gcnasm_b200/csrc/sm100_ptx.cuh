@@ -257,6 +257,13 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
         : "memory");
 }
 
+// load through L1 that stays where it is written
+__device__ __forceinline__ float ld_nc_f32(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 // ---- programmatic dependent launch -----------------------------------------------------------------
 // launch_dependents: the next kernel in the stream (if it was launched with programmatic serialization) may
 // start being scheduled.  wait: block until the previous kernel has completed and its writes are visible;

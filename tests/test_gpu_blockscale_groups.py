@@ -57,3 +57,28 @@ def test_groups_across_tiles(api, tile, m, n, groups):
 @pytest.mark.parametrize("tile", [4, 1])
 def test_scale_rows_of_any_pitch(api, tile):
     check(api, 201, 256, 640, tile, pad=3)
+
+
+# Layers back to back, scales rewritten in the same memory each time: a pair kernel reads them into L1 ahead of their use, and must not
+# find there what they were in the layer before.  Against the same layers run one at a time.
+@pytest.mark.parametrize("m,n,k", [(600, 768, 640), (2309, 2048, 1152)])
+def test_scales_rewritten_between_layers(api, m, n, k):
+    g = torch.Generator(device=DEV).manual_seed(m)
+    w, sfb = api.quantize_128x128(torch.randn(n, k, generator=g, device=DEV))
+    xs = [torch.randn(m, k, generator=g, device=DEV, dtype=torch.bfloat16) * 4.0 ** i for i in range(6)]
+    alone = []
+    for x in xs:
+        q, sfa = api.quantize_act_bf16_1x128(x)
+        alone.append(api.gemm_a8w8_blockscale(q, w, sfa, sfb, tile=4))
+        torch.cuda.synchronize()
+    q, sfa = api.quantize_act_bf16_1x128(xs[0])
+    buf, where, chained = q.clone(), sfa.clone(), []
+    torch.cuda.synchronize()
+    for x in xs:
+        q, sfa = api.quantize_act_bf16_1x128(x)
+        buf.copy_(q)
+        where.copy_(sfa)
+        chained.append(api.gemm_a8w8_blockscale(buf, w, where, sfb, tile=4))
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(alone, chained))
