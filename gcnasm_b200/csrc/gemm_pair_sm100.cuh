@@ -66,12 +66,14 @@ struct PairCfg {
     static_assert(ACC_COLS + SF_COLS <= 512, "TMEM overflow");
 };
 
-// Waits.  The single-thread roles poll (mbarrier.test_wait plus a short sleep), the epilogue warps use the
-// suspending try_wait.  Every wait uses the default CTA-scope acquire even when the arrivals come from the
+// Waits.  The TMA producer polls (mbarrier.test_wait plus a short sleep); the issuer, a whole warp, and the epilogue warps
+// use the suspending try_wait: an issuer that polled took issue slots from the epilogue warps of its scheduler (block
+// scales, 16384 x 7168 x 8192 965 -> 919 us, 4096 x 7168 x 2048 70.7 -> 68.2 when it stopped; nothing in the other modes; nothing for
+// the producer).  Every wait uses the default CTA-scope acquire even when the arrivals come from the
 // partner CTA: a cluster-scope acquire was measured at ~430 clocks per wait, and each hand-off here is ordered
 // through the async proxy (TMA complete_tx, tcgen05.commit) or tcgen05.fence, not through generic memory.
 #define B200_PROD_WAIT mbar_wait_poll<false, 64>
-#define B200_MMA_WAIT mbar_wait_poll<false, 20>
+#define B200_MMA_WAIT mbar_wait<false, 0>
 // One non-suspending look at the barrier before the suspending wait: an epilogue warp that runs behind finds the phase
 // already complete (measured: 0.7 % on 256 x 256 tiles, 4 % on the 224- and 192-column tiles).
 __device__ __forceinline__ bool mbar_probe(uint32_t bar, uint32_t parity) {
@@ -81,9 +83,6 @@ __device__ __forceinline__ bool mbar_probe(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 #define B200_EPI_WAIT(bar, ph, af, st, code) (mbar_probe(bar, ph) || mbar_wait<false, 0>(bar, ph, af, st, code))
-// UMMA issuer threads in block-scale mode (warps 1..kBlockIssuers of the leader CTA); at most the number of
-// TMEM buffers, because an issuer has to observe every phase of the barriers it waits on.
-static constexpr int kBlockIssuers = 2;
 // The TMA producer thread sits on the scheduler that hosts no issuer (warps 1..2 issue, warp w runs on scheduler w % 4):
 // measured against warp 0, 1.5-2 % on the 4096 x 7168 x 2048 and 16384 x 7168 x 8192 problems, nothing on 8192^3.
 static constexpr int kProducerWarp = 3;
@@ -261,15 +260,10 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     }
                 }
             }
-        } else if (warp >= 1 && warp <= ((MODE == MODE_BLOCK) ? kBlockIssuers : 1) && cta == 0) {
+        } else if (warp == 1 && cta == 0) {
             // ------------------------------ UMMA issuer (leader only) ------------------------------
-            // Block-scale mode runs several issuer threads (warps 1..kBlockIssuers, one per scheduler) that take the
-            // K groups round-robin.  An issuer is effectively tied up until its own MMAs and commits have gone
-            // through the tensor queue, so a single issuer cannot start group g+1 while group g executes; with
-            // several, the next group is already queued.  Order on a TMEM buffer is kept by its drained-buffer
-            // barrier, order on a ring stage by its full barrier.
-            constexpr uint32_t kIssuers = (MODE == MODE_BLOCK) ? kBlockIssuers : 1;
-            const uint32_t my_slot = static_cast<uint32_t>(warp - 1);
+            // (One, block scales too.  Two, taking K groups in turn, were worth 15-20 % while an MMA cost its thread 61 clocks; as
+            // whole warps that do not poll: 16384 x 7168 x 8192 946 with two, 938 with one, 4096 x 7168 x 2048 68.7 / 67.3.)
             const bool elected = elect_one() != 0;          // the whole warp walks the loop
             uint32_t it = 0, phase = 0;
             bool ok = true;
@@ -284,10 +278,6 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                 const uint32_t nsub = tail_u ? static_cast<uint32_t>(BN / p.tail_split) : 0u;
                 for (int g = 0; g < groups && ok; g += gp, ++phase) {
                     const int cnt = (groups - g) < gp ? (groups - g) : gp;
-                    if (kIssuers > 1 && (phase % kIssuers) != my_slot) {
-                        it += cnt * kb_per_group;     // another issuer's hand-off
-                        continue;
-                    }
                     const uint32_t as = phase % ACC_STAGES;
                     const uint32_t aph = (phase / ACC_STAGES) & 1;
                     for (int j = 0; j < cnt && ok; ++j) {
