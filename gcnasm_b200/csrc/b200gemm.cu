@@ -227,7 +227,7 @@ int make_flat_tmap(CUtensorMap* tm, const void* base, int64_t n, int64_t k, int6
 struct Plan {
     int tile;        // b200_tile_hint value actually used
     int mt;          // decode token block
-    int splits;      // decode K splits
+    int splits;      // decode K splits; CTAs that share a 128 x 128 tile
 };
 
 // MX with few tokens: the K blocks from which the skinny-M kernel beats the 128 x 128 tiles, which have the shorter fixed part.  Its own
@@ -247,6 +247,32 @@ int64_t mx_skinny_kblocks(int64_t m, int64_t panels, int sm_count) {
     if (m <= 32 || panels * 4 <= sm_count) return 12;
     const int64_t line = (m + 2 * panels * 148 / sm_count - 88 + 5) / 6;       // a plane through the crossings of 33-64 tokens, 38-74 panels
     return line > 12 ? line : 12;
+}
+
+// CTAs that share a 128 x 128 tile, each with a part of K: as many as bring the K blocks of a CTA down furthest, if the clusters are all
+// resident and what is saved is worth more than the exchange of the partial sums.  In K blocks, that takes 9 (block and MX scales, 0.31
+// us a block) or 13 (0.21 us; 15 on tiles of few rows, whose blocks are shorter) on few tiles, more on many, and a cluster of more than
+// four two more.  Whole / split, us, weights from HBM, K = 2048, 4096, 8192:
+//   8-bit         100 x 512 (4 tiles)    6.5 / 6.2    9.9 / 6.6   16.7 / 7.5     256 x 4608 (72)   7.2 / 8.3   10.8 / 10.4   17.6 / 14.4
+//                 256 x 2048 (32)        6.9 / 7.6   10.4 / 8.8   17.3 / 10.9
+//   block scales  100 x 512              8.2 / 6.8   13.2 / 7.3   23.3 / 8.5     256 x 4608        9.1 / 9.2   14.2 / 12.0   24.3 / 17.1
+//                 256 x 2048             8.7 / 8.2   13.8 / 9.6   23.9 / 12.4
+// (At 1024 8-bit operands lose 1 us, block scales 0.5; MX 1705 x 256 x 1536 6.4 / 6.9, 8-bit 12 x 4232 x 3328 8.1 / 8.7.)
+constexpr int kMaxTileSplits = 8;
+constexpr int kSplitClusters[kMaxTileSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};     // resident at once on 148 SMs
+// *equal: the K blocks that a CTA would take as long for
+int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, int sm_count, int64_t* equal = nullptr) {
+    const int64_t exchange = slow ? 9 + tiles / 32 : (m <= 32 ? 15 : 13) + tiles / 12;
+    int best = 1;
+    int64_t best_cost = kblocks;
+    for (int s = 2; s <= kMaxTileSplits; ++s) {
+        const int64_t per = (kblocks + s - 1) / s, cost = per + exchange + (s > 4 ? 2 : 0);
+        if (per * (s - 1) >= kblocks || tiles > static_cast<int64_t>(kSplitClusters[s]) * sm_count / 148 || cost >= best_cost) continue;
+        best = s;
+        best_cost = cost;
+    }
+    if (equal) *equal = best_cost;
+    return best;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -299,7 +325,7 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
     int hint = a->tile_hint;
     if (hint == B200_TILE_DECODE && (!decode_ok || (a->scale_mode == B200_SCALE_MX && kblocks < kMxSkinnyLeast))) return B200_ERR_UNSUPPORTED;
     if (hint == B200_TILE_128x64) return B200_ERR_UNSUPPORTED;
-    const bool mx = a->scale_mode == B200_SCALE_MX;
+    const bool mx = a->scale_mode == B200_SCALE_MX, slow = mx || a->scale_mode == B200_SCALE_BLOCK;
     // MX pair kernels address the scale atoms through a tensor map: batch strides in whole atoms
     const bool mx_pair_ok = !mx || a->batch == 1 || (a->stride_sfa_batch % 512 == 0 && a->stride_sfb_batch % 512 == 0);
     if (hint == B200_TILE_AUTO) {
@@ -350,7 +376,11 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 else if (bn == 256) w = 100;
                 else if (bn == 128) w = block ? 130 : 140;
                 else w = block ? 140 : (bn == 224 && kblocks < 8 ? 120 : 110);
-                const int64_t cost = tenths * bn * w;
+                int64_t cost = tenths * bn * w * kblocks;
+                if (tile == B200_TILE_128x128 && !(a->flags & B200_GEMM_INPUTS_READY)) {
+                    int64_t equal;
+                    if (tile_splits(a->m, tiles, kblocks, slow, sm_count, &equal) > 1) cost = 10 * bn * (ab16 ? 155 : block ? 125 : 130) * equal;
+                }
                 if (best < 0 || cost < best) {
                     best = cost;
                     hint = tile;
@@ -397,6 +427,8 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
             }
         }
         pl.splits = splits;
+    } else if (hint == B200_TILE_128x128) {
+        pl.splits = tile_splits(a->m, (a->m + 127) / 128 * ((a->n + 127) / 128) * a->batch, kblocks, slow, sm_count);
     }
     if (plan) *plan = pl;
     return B200_OK;
@@ -453,6 +485,29 @@ int launch_pdl(void (*kernel)(P...), unsigned grid, unsigned threads, size_t sme
     return launch_pdl_cluster(1, kernel, grid, threads, smem, st, args...);
 }
 
+// Clusters of `size` CTAs of a kernel that are resident at once (0: it cannot be told)
+template <class Kernel>
+int resident_clusters(Kernel kernel, int size, int threads, int smem) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(static_cast<unsigned>(size), 1, 1);
+    cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+    cudaLaunchAttribute attr;
+    std::memset(&attr, 0, sizeof(attr));
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(size);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return n;
+}
+
 template <int BN, int MODE, int BL>
 int launch_gemm(const GemmParams& p, int grid, cudaStream_t st) {
     using Cfg = GemmCfg<BN, MODE, BL>;
@@ -460,6 +515,37 @@ int launch_gemm(const GemmParams& p, int grid, cudaStream_t st) {
     int rc = set_smem(kernel, Cfg::SMEM_BYTES);
     if (rc) return rc;
     return launch_pdl(kernel, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
+}
+
+template <int MODE, int BL>
+int split_clusters(int size, int sm_count) {
+    using Cfg = GemmCfg<128, MODE, BL, true>;
+    auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
+    static std::atomic<int> known[kMaxDevices][kMaxTileSplits + 1];        // clusters resident at once + 1; 0: not asked yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    int n = known[dev][size].load() - 1;
+    if (n < 0) {
+        if (set_smem(kernel, Cfg::SMEM_BYTES)) return 0;
+        n = resident_clusters(kernel, size, Cfg::THREADS, Cfg::SMEM_BYTES);
+        known[dev][size].store(n + 1);
+    }
+    return n < sm_count / size ? n : sm_count / size;
+}
+
+// 128 x 128 tiles on one CTA each or, with p.splits > 1, on a cluster each
+template <int MODE, int BL>
+int launch_gemm128(GemmParams& p, int grid, int sm_count, cudaStream_t st) {
+    while (p.splits > 1 && split_clusters<MODE, BL>(p.splits, sm_count) < p.tiles_total) {
+        p.kb_per_split = (p.kblocks + p.splits - 2) / (p.splits - 1);
+        p.splits = (p.kblocks + p.kb_per_split - 1) / p.kb_per_split;
+    }
+    if (p.splits <= 1) return launch_gemm<128, MODE, BL>(p, grid, st);
+    using Cfg = GemmCfg<128, MODE, BL, true>;
+    auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
+    int rc = set_smem(kernel, Cfg::SMEM_BYTES);
+    if (rc) return rc;
+    return launch_pdl_cluster(p.splits, kernel, static_cast<unsigned>(p.tiles_total * p.splits), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
 
 // K splits of the decode kernel that work as one cluster (above 8 the size is not portable and asked for explicitly)
@@ -490,22 +576,7 @@ int decode_clusters(int size, int sm_count) {
     int n = known[dev][size].load() - 1;
     if (n < 0) {
         if (decode_attrs<MT, MODE, BL>()) return 0;
-        cudaLaunchConfig_t cfg;
-        std::memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3(static_cast<unsigned>(size), 1, 1);
-        cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
-        cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-        cudaLaunchAttribute attr;
-        std::memset(&attr, 0, sizeof(attr));
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = static_cast<unsigned>(size);
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&n, decode_a8w8_sm100_kernel<Cfg>, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            n = 0;
-        }
+        n = resident_clusters(decode_a8w8_sm100_kernel<Cfg>, size, Cfg::THREADS, Cfg::SMEM_BYTES);
         known[dev][size].store(n + 1);
     }
     return n < sm_count / size ? n : sm_count / size;
@@ -872,6 +943,8 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     if (total > 0x7FFFFFFF) return B200_ERR_TOO_LARGE;
     p.tiles_total = static_cast<int>(total);
     p.kblocks = static_cast<int>((a->k + 127) / 128);
+    p.kb_per_split = (p.kblocks + pl.splits - 1) / pl.splits;
+    p.splits = !pair && BN == 128 ? (p.kblocks + p.kb_per_split - 1) / p.kb_per_split : 1;
     p.out_dtype = a->out_dtype;
     p.inputs_ready = (a->flags & (B200_GEMM_INPUTS_READY | B200_GEMM_BATCH_READY)) ? 1 : 0;
     p.b_shared = b_shared ? 1 : 0;
@@ -909,7 +982,7 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
         if (pair) return flat ? launch_pair<256, MODE_ACC16, BL_FLAT>(p, ds->sm_count, st) : launch_pair<256, MODE_ACC16, BL_NK>(p, ds->sm_count, st);
         const int grid16 = p.tiles_total < ds->sm_count ? p.tiles_total : ds->sm_count;
         if (BN == 256) return flat ? launch_gemm<256, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<256, MODE_ACC16, BL_NK>(p, grid16, st);
-        return flat ? launch_gemm<128, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<128, MODE_ACC16, BL_NK>(p, grid16, st);
+        return flat ? launch_gemm128<MODE_ACC16, BL_FLAT>(p, grid16, ds->sm_count, st) : launch_gemm128<MODE_ACC16, BL_NK>(p, grid16, ds->sm_count, st);
     }
     if (pair) {
         switch (BN) {
@@ -923,12 +996,12 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     switch (a->scale_mode) {
         case B200_SCALE_BLOCK:
             if (BN == 256) return flat ? launch_gemm<256, MODE_BLOCK, BL_FLAT>(p, grid, st) : launch_gemm<256, MODE_BLOCK, BL_NK>(p, grid, st);
-            return flat ? launch_gemm<128, MODE_BLOCK, BL_FLAT>(p, grid, st) : launch_gemm<128, MODE_BLOCK, BL_NK>(p, grid, st);
+            return flat ? launch_gemm128<MODE_BLOCK, BL_FLAT>(p, grid, ds->sm_count, st) : launch_gemm128<MODE_BLOCK, BL_NK>(p, grid, ds->sm_count, st);
         case B200_SCALE_MX:
-            return flat ? launch_gemm<128, MODE_MX, BL_FLAT>(p, grid, st) : launch_gemm<128, MODE_MX, BL_NK>(p, grid, st);
+            return flat ? launch_gemm128<MODE_MX, BL_FLAT>(p, grid, ds->sm_count, st) : launch_gemm128<MODE_MX, BL_NK>(p, grid, ds->sm_count, st);
         default:
             if (BN == 256) return flat ? launch_gemm<256, MODE_ACC, BL_FLAT>(p, grid, st) : launch_gemm<256, MODE_ACC, BL_NK>(p, grid, st);
-            return flat ? launch_gemm<128, MODE_ACC, BL_FLAT>(p, grid, st) : launch_gemm<128, MODE_ACC, BL_NK>(p, grid, st);
+            return flat ? launch_gemm128<MODE_ACC, BL_FLAT>(p, grid, ds->sm_count, st) : launch_gemm128<MODE_ACC, BL_NK>(p, grid, ds->sm_count, st);
     }
 }
 

@@ -52,6 +52,8 @@ struct GemmParams {
     // whole tile.  tmap_b_tail is B with a box of 128 / tail_split rows.  tail_split == 0: whole tiles only.
     CUtensorMap tmap_b_tail;
     int tail_first, tail_split;
+    // single-CTA 128 x 128 tiles: the CTAs of a cluster take kb_per_split K blocks each of one tile (splits == 1: whole tiles)
+    int splits, kb_per_split;
     int* status;
 };
 
@@ -71,8 +73,9 @@ __device__ __forceinline__ void unit_coords(const GemmParams& p, int u, int& t, 
 static constexpr int kOutStagePitch = 80;
 static constexpr int kOutStageBytesPerWarp = 32 * kOutStagePitch;
 
-template <int BN_, int MODE_, int BLAYOUT_>
+template <int BN_, int MODE_, int BLAYOUT_, bool SPLIT_ = false>
 struct GemmCfg {
+    static constexpr bool SPLIT = SPLIT_;                           // a tile's K is split over a cluster
     static constexpr bool AB16 = MODE_ == MODE_ACC16;               // bf16 operands: same bytes, kind::f16 MMAs
     static constexpr int BM = 128, BN = BN_, BK = 128, MODE = AB16 ? MODE_ACC : MODE_, BLAYOUT = BLAYOUT_;
     static constexpr int A_BYTES = BM * BK;
@@ -104,6 +107,7 @@ struct GemmCfg {
     static_assert(BN % 32 == 0 && BN <= 256, "BN must be a multiple of 32, at most 256");
     static_assert(STAGES >= 3 && STAGES_ONE <= 8, "ring depth");
     static_assert(OUT_STAGE_BYTES <= STAGES * STAGE_BYTES, "the staging fits the ring");
+    static_assert(!SPLIT || (BN == 128 && BM * BN * 4 <= RING_BYTES), "the partial sums fit the ring");
 };
 
 // tile index -> (batch, m tile, n tile): groups of 8 M tiles walk N, so that the tiles resident at
@@ -220,6 +224,55 @@ __device__ __forceinline__ void store_chunk_coalesced(const GemmParams& p, uint8
     else if constexpr (CNT <= 16) store_chunk_staged<CNT, false>(p, cbatch, stage, row0, col0, v, lane);
 }
 
+// One epilogue warp's part of a split tile: rows split + ew * S, ... in steps of 8 S, each summed over the S CTAs of the cluster in
+// the order of K, a lane four columns.  All the loads of a step are issued before the first is waited for (one row at a time, a
+// remote load's latency per row, the sum of a 2-CTA cluster was most of what a split tile took longer).
+template <int S>
+__device__ __forceinline__ void sum_splits(const GemmParams& p, uint32_t smem_base, int t, int split, int ew, int lane, float scale, bool vec_ok) {
+    constexpr int ROWS = (16 + S - 1) / S;                          // rows per step: a whole tile's in one
+    int b, mi, ni;
+    tile_coords(p, t, b, mi, ni);
+    const int rows = p.m - mi * 128 < 128 ? p.m - mi * 128 : 128, col = ni * 128 + lane * 4;
+    const size_t esz = (p.out_dtype == OUT_BF16) ? 2 : 4;
+    float4 v[ROWS][S];
+    const int r0 = split + ew * S;
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int r = r0 + i * 8 * S;
+        const uint32_t at = smem_base + r * 512 + ((lane ^ (r & 7)) << 4);
+        if (r < rows) {
+#pragma unroll
+            for (int q = 0; q < S; ++q) v[i][q] = ld_shared_cluster_f32x4(mapa_shared(at, q));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int r = r0 + i * 8 * S;
+        if (r >= rows) break;
+        float4 sum = v[i][0];
+#pragma unroll
+        for (int q = 1; q < S; ++q) {
+            sum.x += v[i][q].x;
+            sum.y += v[i][q].y;
+            sum.z += v[i][q].z;
+            sum.w += v[i][q].w;
+        }
+        const float o[4] = {sum.x * scale, sum.y * scale, sum.z * scale, sum.w * scale};
+        uint8_t* dst = reinterpret_cast<uint8_t*>(p.c) + (static_cast<size_t>(b) * p.c_batch + static_cast<size_t>(mi * 128 + r) * p.ldc + col) * esz;
+        if (vec_ok && col + 4 <= p.n) {
+            if (p.out_dtype == OUT_BF16) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+            else *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (col + j >= p.n) continue;
+                if (p.out_dtype == OUT_BF16) reinterpret_cast<__nv_bfloat16*>(dst)[j] = __float2bfloat16_rn(o[j]);
+                else reinterpret_cast<float*>(dst)[j] = o[j];
+            }
+        }
+    }
+}
+
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const __grid_constant__ GemmParams p) {
     constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, MODE = Cfg::MODE;
@@ -229,7 +282,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
     // A CTA that computes one tile stages its result in the ring: every load and MMA has completed when the last accumulator has.
-    const bool one_tile = p.tiles_total <= static_cast<int>(gridDim.x);
+    const bool one_tile = Cfg::SPLIT || p.tiles_total <= static_cast<int>(gridDim.x);
     const uint32_t stages = one_tile ? Cfg::STAGES_ONE : Cfg::STAGES;
     // barrier block sits after the ring
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_gen + Cfg::RING_BYTES);
@@ -276,8 +329,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();
 
-    const int groups = (MODE == MODE_BLOCK) ? p.kblocks : 1;          // accumulator phases per tile
-    const int kb_per_group = (MODE == MODE_BLOCK) ? 1 : p.kblocks;
+    // A CTA of a split tile has that tile only, and K blocks [kb0, kb0 + kblocks) of it.  (Whole tiles walk blockIdx.x and gridDim.x
+    // themselves: through variables of their own, MX 436 x 2432 x 2432 8.9 -> 9.6 us, bf16 1216 x 1416 x 7040 26.8 -> 28.1.)
+    const int split = Cfg::SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+    const int split_tile = Cfg::SPLIT ? static_cast<int>(blockIdx.x) / p.splits : 0;
+    const int kb0 = split * p.kb_per_split;
+    const int kblocks = Cfg::SPLIT ? (p.kb_per_split < p.kblocks - kb0 ? p.kb_per_split : p.kblocks - kb0) : p.kblocks;
+    const int groups = (MODE == MODE_BLOCK) ? kblocks : 1;            // accumulator phases per tile
+    const int kb_per_group = (MODE == MODE_BLOCK) ? 1 : kblocks;
 
     auto next_stage = [stages](uint32_t& s, uint32_t& ph) {           // ring stage and its phase
         if (++s == stages) {
@@ -292,10 +351,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             // ------------------------------ TMA producer ------------------------------
             uint32_t s = 0, ph = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {
+            for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
                 int b, mi, ni;
                 tile_coords(p, t, b, mi, ni);
-                for (int kb = 0; kb < p.kblocks; ++kb, next_stage(s, ph)) {
+                for (int kb = kb0; kb < kb0 + kblocks; ++kb, next_stage(s, ph)) {
                     if (!mbar_wait(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY)) {
                         ok = false;
                         break;
@@ -326,7 +385,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             uint32_t s = 0, ph = 0, phase = 0;
             bool ok = true;
             constexpr uint32_t idesc = make_idesc_f8(BM, BN);
-            for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {
+            for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
                 for (int g = 0; g < groups && ok; ++g, ++phase) {
                     const uint32_t as = phase % BUFS;
                     const uint32_t aph = (phase / BUFS) & 1;
@@ -378,6 +437,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 }
             }
         }
+        if constexpr (Cfg::SPLIT) {
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+        }
     } else {
         // ---------------------------------- epilogue ----------------------------------
         setmaxnreg_inc<232>();
@@ -397,7 +461,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
         uint8_t* out_stage = smem_gen + (one_tile ? 0 : Cfg::STAGES * Cfg::STAGE_BYTES) + ew * kOutStageBytesPerWarp;
         uint32_t phase = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < p.tiles_total && ok; t += gridDim.x) {
+        for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
             int b, mi, ni;
             tile_coords(p, t, b, mi, ni);
             const int row = mi * BM + row_in_tile;
@@ -411,6 +475,15 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             const int rows = p.m - mi * BM;
             const bool direct = MODE != MODE_BLOCK && (rows <= 32 || rows - quad * 32 < 32);
             auto put32 = [&](const int c, const float* o) {              // this warp's 32 rows x columns [32 c, 32 c + 32) of its part
+                if constexpr (Cfg::SPLIT) {
+                    // partial sums, row by row; the 16-byte pieces of eight neighbouring rows lie in different banks
+                    uint8_t* mine = smem_gen + row_in_tile * (BN * 4);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        *reinterpret_cast<float4*>(mine + (((half * (NCH / 4) + c * 8 + j) ^ (lane & 7)) << 4)) =
+                            make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+                    return;
+                }
                 const int row0 = mi * BM + quad * 32, col0 = col_base + c * 32;
                 if (direct || !vec_ok || col0 + 32 > p.n) {
                     if (row < p.m) store_row_chunk<32>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, o, vec_ok);
@@ -436,17 +509,20 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 unsigned long long acc2[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc2[j] = 0ull;
-                const float* sfa_p = p.sfa + b * p.sfa_batch + (row < p.m ? row : 0);
-                const float* sfb_p = p.sfb + b * p.sfb_batch + static_cast<long long>(col_base / 128) * p.sfb_stride;
+                const float* sfa_p = p.sfa + b * p.sfa_batch + static_cast<long long>(kb0) * p.sfa_stride + (row < p.m ? row : 0);
+                const float* sfb_p = p.sfb + b * p.sfb_batch + static_cast<long long>(col_base / 128) * p.sfb_stride + kb0;
                 const bool col_ok = col_base < p.n;
                 constexpr int SETS = 6;
                 float sa[SETS], sb[SETS];
-                auto request = [&](const int g, const int set) {
-                    sa[set] = __ldg(sfa_p + static_cast<long long>(g) * p.sfa_stride);
-                    sb[set] = col_ok ? __ldg(sfb_p + g) : 0.0f;
+                auto request = [&](const int set) {
+                    sa[set] = __ldg(sfa_p);
+                    sb[set] = col_ok ? __ldg(sfb_p) : 0.0f;
+                    sfa_p += p.sfa_stride;
+                    ++sfb_p;
                 };
 #pragma unroll
-                for (int set = 0; set < SETS; ++set) request(set < groups ? set : 0, set);
+                for (int set = 0; set < SETS; ++set)
+                    if (set < groups) request(set);
                 for (int g0 = 0; g0 < groups && ok; g0 += SETS) {
 #pragma unroll
                     for (int set = 0; set < SETS; ++set) {
@@ -469,7 +545,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
-                        if (g + SETS < groups) request(g + SETS, set);
+                        if (g + SETS < groups) request(set);
 #pragma unroll
                         for (int j = 0; j < 32; ++j) acc2[j] = ffma2(pack_f32x2(v[2 * j], v[2 * j + 1]), sc2, acc2[j]);
                         ++phase;
@@ -545,7 +621,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
                     }
-                    if (MODE == MODE_ACC) {
+                    if (MODE == MODE_ACC && !Cfg::SPLIT) {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[c & 1][j] *= tscale;
                     }
@@ -554,8 +630,32 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 ++phase;
             }
         }
+        if constexpr (Cfg::SPLIT) {
+            // CTA r of the cluster sums rows r, r + splits, ... over all of them, in the order of K, a lane four columns
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+            // A split that gave up (an expired wait) has no sums to add: the tile is left unwritten then.
+            const uint32_t gave_up = lane < p.splits ? ld_shared_cluster_u32(mapa_shared(smem_u32(tmem_slot + 1), lane)) : 0u;
+            if (!__any_sync(0xFFFFFFFFu, gave_up != 0u)) {
+                switch (p.splits) {
+                    case 2: sum_splits<2>(p, smem_base, split_tile, split, ew, lane, tscale, vec_ok); break;
+                    case 3: sum_splits<3>(p, smem_base, split_tile, split, ew, lane, tscale, vec_ok); break;
+                    case 4: sum_splits<4>(p, smem_base, split_tile, split, ew, lane, tscale, vec_ok); break;
+                    case 5: sum_splits<5>(p, smem_base, split_tile, split, ew, lane, tscale, vec_ok); break;
+                    case 6: sum_splits<6>(p, smem_base, split_tile, split, ew, lane, tscale, vec_ok); break;
+                    case 7: sum_splits<7>(p, smem_base, split_tile, split, ew, lane, tscale, vec_ok); break;
+                    default: sum_splits<8>(p, smem_base, split_tile, split, ew, lane, tscale, vec_ok); break;
+                }
+            }
+        }
     }
-
+    if constexpr (Cfg::SPLIT) {
+        // no CTA leaves while another one reads its partial sums
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
     // ---------------------------------- teardown ----------------------------------
     tc_fence_before();
     __syncthreads();

@@ -1,0 +1,78 @@
+"""128 x 128 tiles whose K is split over a cluster: few tiles and a long K.
+
+Without scales, with block scales and with bf16 operands the values are whole numbers (of at most 2, block scales 2^-5 to 2^5 in the
+product): an fp32 sum of at most 8192 products, or of 32 groups' 512 * 2^5 in steps of 2^-5, takes 24 bits, nothing is rounded, and the result
+has to be the exact one.  MX: a sum of K products in any order and grouping is off by at most K * 2^-23 of the sum of their magnitudes."""
+import pytest
+import torch
+
+from test_gpu_blockscale_groups import problem
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+# four tiles (eight CTAs each), ragged rows and columns, an odd number of K blocks (a shorter last part), 32 tiles, 72 tiles (two CTAs each)
+SHAPES = [(100, 512, 4096), (129, 264, 4224), (1, 136, 8192), (256, 2048, 3968), (384, 768, 4096), (256, 4608, 4096)]
+
+
+def ints(g, *shape):
+    return torch.randint(-2, 3, shape, generator=g, device=DEV)
+
+
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", SHAPES)
+@pytest.mark.parametrize("kind", ["fp8", "tensor", "bf16"])
+def test_sums_are_exact(api, kind, m, n, k, out):
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    batch = 2 if m * n < 200000 else 1
+    a, b = ints(g, batch, m, k), ints(g, batch, n, k)
+    ref = torch.bmm(a.double(), b.double().transpose(1, 2))
+    if kind == "bf16":
+        c = torch.stack([api.gemm_a16w16(a[i].bfloat16(), b[i].bfloat16(), out_dtype=out) for i in range(batch)])
+    else:
+        qa, qb = (torch.stack([api.cast_e4m3(t[i].float()) for i in range(batch)]) for t in (a, b))
+        s = torch.tensor([0.5], device=DEV) if kind == "tensor" else None
+        ref = ref * 0.25 if kind == "tensor" else ref
+        c = api.gemm_a8w8(qa, qb, s, s, out_dtype=out, tile=1).reshape(batch, m, n)
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+    assert torch.equal(c, ref.float().to(out))
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("m,n,groups", [(100, 512, 32), (333, 384, 31), (129, 128, 23), (256, 4608, 32)])
+def test_groups_meet_their_scales(api, m, n, groups, flat):
+    a, b, sfa, sfb, ref = problem(m, n, 128 * groups, m + groups)
+    c = api.gemm_a8w8_blockscale(a, api.shuffle_b(b, "nk") if flat else b, sfa, sfb, out_dtype=torch.float32, tile=1, b_flat_n=n if flat else None)
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+    assert torch.equal(c.double(), ref)
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_mx(api, m, n, k):
+    g = torch.Generator(device=DEV).manual_seed(m)
+    sides = []
+    for rows in (m, n):
+        q, logical, atoms = api.quantize_mx32(torch.randn(rows, k, generator=g, device=DEV))
+        value = q.view(torch.float8_e4m3fn).double() * torch.exp2(logical.reshape(rows, -1).double() - 127).repeat_interleave(32, 1)
+        sides.append((q, atoms, value))
+    (a, sfa, va), (b, sfb, vb) = sides
+    c = api.gemm_a8w8_mx(a, b, sfa, sfb, out_dtype=torch.float32, tile=1)
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+    assert ((c.double() - va @ vb.t()).abs() <= k * 2.0 ** -23 * (va.abs() @ vb.abs().t())).all()
+
+
+def test_strided_result_in_a_chain(api):
+    """Rows of C further apart than N and not 16-byte aligned, behind the kernel that writes A."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    m, n, k = 200, 272, 4096
+    b = ints(g, n, k)
+    qb = api.cast_e4m3(b.float())
+    for i in range(3):
+        a = ints(g, m, k)
+        big = torch.full((m, n + 3), 7.0, device=DEV)
+        api.gemm_a8w8(api.cast_e4m3(a.float()), qb, out=big[:, 1:n + 1], tile=1)
+        torch.cuda.synchronize()
+        assert torch.equal(big[:, 1:n + 1].double(), a.double() @ b.double().t())
+        assert (big[:, 0] == 7).all() and (big[:, n + 1:] == 7).all()
