@@ -227,7 +227,7 @@ int make_flat_tmap(CUtensorMap* tm, const void* base, int64_t n, int64_t k, int6
 struct Plan {
     int tile;        // b200_tile_hint value actually used
     int mt;          // decode token block
-    int splits;      // decode K splits; CTAs that share a 128 x 128 tile
+    int splits;      // decode K splits; otherwise, above 1: 128 x 128 tiles, each shared by so many CTAs, whatever `tile` says
 };
 
 // MX with few tokens: the K blocks from which the skinny-M kernel beats the 128 x 128 tiles, which have the shorter fixed part.  Its own
@@ -376,11 +376,7 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 else if (bn == 256) w = 100;
                 else if (bn == 128) w = block ? 130 : 140;
                 else w = block ? 140 : (bn == 224 && kblocks < 8 ? 120 : 110);
-                int64_t cost = tenths * bn * w * kblocks;
-                if (tile == B200_TILE_128x128 && !(a->flags & B200_GEMM_INPUTS_READY)) {
-                    int64_t equal;
-                    if (tile_splits(a->m, tiles, kblocks, slow, sm_count, &equal) > 1) cost = 10 * bn * (ab16 ? 155 : block ? 125 : 130) * equal;
-                }
+                const int64_t cost = tenths * bn * w;
                 if (best < 0 || cost < best) {
                     best = cost;
                     hint = tile;
@@ -402,6 +398,12 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                     consider(B200_TILE_128x256, 256, false);
                     consider(B200_TILE_128x128, 128, false);
                 }
+            }
+            // Few tiles with a long K: 128 x 128 tiles whose K is split may be the better ones (w as for a grid of one round).
+            if (!pair_only && !(a->flags & B200_GEMM_INPUTS_READY)) {
+                int64_t equal;
+                const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, sm_count, &equal);
+                if (s > 1 && 10 * 128 * (ab16 ? 155 : a->scale_mode == B200_SCALE_BLOCK ? 125 : 130) * equal < best * kblocks) pl.splits = s;
             }
         }
     }
@@ -427,7 +429,7 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
             }
         }
         pl.splits = splits;
-    } else if (hint == B200_TILE_128x128) {
+    } else if (hint == B200_TILE_128x128 && a->tile_hint == hint) {
         pl.splits = tile_splits(a->m, (a->m + 127) / 128 * ((a->n + 127) / 128) * a->batch, kblocks, slow, sm_count);
     }
     if (plan) *plan = pl;
@@ -885,7 +887,7 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
 int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStream_t st, bool ab16 = false) {
     int BN = 128;
     bool pair = false;
-    switch (pl.tile) {
+    switch (pl.splits > 1 ? B200_TILE_128x128 : pl.tile) {
         case B200_TILE_128x256: BN = 256; break;
         case B200_TILE_PAIR_256x256: BN = 256; pair = true; break;
         case B200_TILE_PAIR_256x224: BN = 224; pair = true; break;

@@ -128,7 +128,10 @@ int b200_gemm_a8w8(const b200_gemm_args* args, void* cuda_stream);
 int b200_last_tail_split(int32_t* first_tile, int32_t* parts);
 
 /* Validates `args` exactly as b200_gemm_a8w8 would, without touching the GPU. Also reports the tile
- * configuration the launcher would pick (a b200_tile_hint value) when `chosen_tile` is not null.        */
+ * configuration the launcher would pick (a b200_tile_hint value) when `chosen_tile` is not null.  That is the tile of a
+ * launch in which a tile's K stays together: with TILE_AUTO (inputs not ready) a grid of few tiles with a long K may be
+ * computed on 128x128 tiles instead, each shared by the CTAs of a cluster that take a part of K; with the tile as a
+ * hint it is computed as reported, except that a hint of 128x128 is split by the same rule.                          */
 int b200_gemm_check(const b200_gemm_args* args, int32_t* chosen_tile);
 
 /* Same contract as b200_gemm_a8w8 but computed by a one-thread-per-output CUDA kernel that mirrors the
