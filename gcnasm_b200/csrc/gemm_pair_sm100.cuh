@@ -285,8 +285,15 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     for (int kb = 0; kb < kb_per_group; ++kb, ++it) {
                         const uint32_t s = it % STAGES;
                         const uint32_t ph = (it / STAGES) & 1;
-                        // operands first (they were prefetched long ago), then the accumulator buffer: the
-                        // second wait is the latency-critical one and the MMAs follow it immediately
+                        // The descriptors are formed before either wait is over: the accumulator's is the latency-critical one, and the MMAs
+                        // follow it at once.  Behind it / before it, us: block scales 4096 x 7168 x 2048 65.9 / 64.7, 16384 x 7168 x 8192 938 /
+                        // 926, MX 4096 x 7168 x 2048 55.4 / 54.3, 8192^3 449 / 436.
+                        uint64_t da0 = make_smem_desc(smem_base + s * Cfg::STAGE_BYTES, 16, 1024, kSwizzle128B);
+                        uint64_t db0 = Cfg::BLAYOUT == BL_NK ? make_smem_desc(smem_base + s * Cfg::STAGE_BYTES + Cfg::A_BYTES, 16, 1024, kSwizzle128B)
+                                                             : make_smem_desc(smem_base + s * Cfg::STAGE_BYTES + Cfg::A_BYTES, lbo_u, 128, kSwizzleNone);
+                        uint64_t dsf0 = make_smem_desc(smem_base + s * Cfg::STAGE_BYTES + Cfg::A_BYTES + Cfg::B_BYTES, 0, 128, kSwizzleNone);   // MX
+                        asm volatile("" : "+l"(da0), "+l"(db0), "+l"(dsf0));
+                        // operands first (they were prefetched long ago), then the accumulator buffer
                         if (!role_all<true>(B200_MMA_WAIT(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
                             ok = false;
                             break;
@@ -302,25 +309,15 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                         B200_TRACE_MMA(2);
                         tc_fence_after();
                         if (elected) {
-                        const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
-                        const uint32_t sb = sa + Cfg::A_BYTES;
                         if constexpr (MODE == MODE_MX) {
                             const uint32_t tsf = tmem_base + Cfg::ACC_COLS;
-                            tmem_cp_sf<2>(tsf, make_smem_desc(sb + Cfg::B_BYTES, 0, 128, kSwizzleNone));
+                            tmem_cp_sf<2>(tsf, dsf0);
 #pragma unroll
-                            for (int a = 0; a < Cfg::SFB_ATOMS; ++a)
-                                tmem_cp_sf<2>(tsf + 4 + 4 * a,
-                                              make_smem_desc(sb + Cfg::B_BYTES + 512 + 512 * a, 0, 128, kSwizzleNone));
+                            for (int a = 0; a < Cfg::SFB_ATOMS; ++a) tmem_cp_sf<2>(tsf + 4 + 4 * a, dsf0 + 32 + 32 * a);
                         }
 #pragma unroll
                         for (int k = 0; k < BK / 32; ++k) {
-                            const uint64_t da = make_smem_desc(sa + k * 32, 16, 1024, kSwizzle128B);
-                            uint64_t db;
-                            if constexpr (Cfg::BLAYOUT == BL_NK) {
-                                db = make_smem_desc(sb + k * 32, 16, 1024, kSwizzle128B);
-                            } else {
-                                db = make_smem_desc(sb + k * 2 * lbo_u, lbo_u, 128, kSwizzleNone);
-                            }
+                            const uint64_t da = da0 + k * 2, db = db0 + (Cfg::BLAYOUT == BL_NK ? k * 2u : (k * 2 * lbo_u) >> 4);
                             const uint32_t accum = (kb > 0 || k > 0) ? 1u : 0u;
                             if constexpr (MODE == MODE_MX) {
                                 const uint32_t tsf = tmem_base + Cfg::ACC_COLS;
