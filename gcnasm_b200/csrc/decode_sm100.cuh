@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                 const uint32_t set = phase % NBUF;
                 if constexpr (MODE == MODE_BLOCK) {
                     const uint32_t aph = (phase / NBUF) & 1;
-                    if (!role_all<true>(mbar_wait_poll<false, 20>(bar_acce0 + set * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
+                    if (!role_all<true>(mbar_wait<false, 0>(bar_acce0 + set * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
                         ok = false;
                         break;
                     }
@@ -223,30 +223,31 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                     const int i = i0 + j;
                     const uint32_t s = i % STAGES;
                     const uint32_t ph = (i / STAGES) & 1;
-                    if (!role_all<true>(mbar_wait_poll<false, 20>(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
+                    const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
+                    const uint32_t sx = sw + Cfg::W_BYTES;
+                    constexpr uint32_t LBO = (BNW / 16) * 256;
+                    // The descriptors are formed before the wait, and the wait suspends the warp.  Formed behind it, polling with 20 ns of
+                    // sleep / so, us: block scales, 16 tokens, 7168 x 2048 6.4 / 6.2, 2560 x 7168 8.0 / 7.75, 18432 x 7168 22.1 / 21.9; unscaled,
+                    // 64 tokens, 2048 x 7168 8.4 / 8.1; MX, 64 tokens, 7168 x 2048 8.0 / 7.75.
+                    uint64_t dw0 = Cfg::BLAYOUT == BL_NK ? make_smem_desc(sw, 16, 1024, kSwizzle128B) : make_smem_desc(sw, LBO, 128, kSwizzleNone);
+                    uint64_t dx0 = make_smem_desc(sx, 16, 1024, kSwizzle128B);
+                    uint64_t dsf0 = make_smem_desc(sx + Cfg::X_BYTES, 0, 128, kSwizzleNone);                 // MX
+                    asm volatile("" : "+l"(dw0), "+l"(dx0), "+l"(dsf0));
+                    if (!role_all<true>(mbar_wait<false, 0>(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     if (!elected) continue;
-                    const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
-                    const uint32_t sx = sw + Cfg::W_BYTES;
                     const uint32_t tacc = (MODE == MODE_BLOCK) ? tmem_base + (set * Cfg::GB + j) * MT : tmem_base;
                     const uint32_t tsf = tmem_base + Cfg::SF_COL;
                     if constexpr (MODE == MODE_MX) {
-                        tmem_cp_sf<1>(tsf, make_smem_desc(sx + Cfg::X_BYTES, 0, 128, kSwizzleNone));
-                        tmem_cp_sf<1>(tsf + 4, make_smem_desc(sx + Cfg::X_BYTES + 512, 0, 128, kSwizzleNone));
+                        tmem_cp_sf<1>(tsf, dsf0);
+                        tmem_cp_sf<1>(tsf + 4, dsf0 + 32);
                     }
 #pragma unroll
                     for (int k = 0; k < BK / 32; ++k) {
-                        uint64_t dw;
-                        if constexpr (Cfg::BLAYOUT == BL_NK) {
-                            dw = make_smem_desc(sw + k * 32, 16, 1024, kSwizzle128B);
-                        } else {
-                            constexpr uint32_t LBO = (BNW / 16) * 256;
-                            dw = make_smem_desc(sw + k * 2 * LBO, LBO, 128, kSwizzleNone);
-                        }
-                        const uint64_t dx = make_smem_desc(sx + k * 32, 16, 1024, kSwizzle128B);
+                        const uint64_t dw = dw0 + (Cfg::BLAYOUT == BL_NK ? k * 2u : (k * 2 * LBO) >> 4), dx = dx0 + k * 2;
                         const uint32_t accum = (MODE == MODE_BLOCK) ? (k > 0 ? 1u : 0u) : ((i > 0 || k > 0) ? 1u : 0u);
                         if constexpr (MODE == MODE_MX) umma_mxf8<1>(tacc, dw, dx, make_idesc_mxf8(BNW, MT, k, k), accum, tsf, tsf + 4);
                         else umma_f8<1>(tacc, dw, dx, idesc, accum);
