@@ -263,6 +263,8 @@ constexpr int kSplitClusters[kMaxTileSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 
 // *equal: the K blocks that a CTA would take as long for
 int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, int sm_count, int64_t* equal = nullptr) {
     const int64_t exchange = slow ? 9 + tiles / 32 : (m <= 32 ? 15 : 13) + tiles / 12;
+    if (equal) *equal = kblocks;
+    if (kblocks <= exchange) return 1;
     int best = 1;
     int64_t best_cost = kblocks;
     for (int s = 2; s <= kMaxTileSplits; ++s) {
@@ -349,8 +351,8 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 if (pair && bn == 256 && block && tiles > units && rem > 0 && kblocks >= 4 && rem * 2 <= units)
                     tenths += (rem * 4 <= units ? 4 : 6) - 10;
                 // w = time per output column, measured on 4096 x 7168 x 2048 (us a round and 1000 columns, 8-bit / block scales:
-                // pair 256 27 / 40, 224 30 / 54, 192 30 / 56, 128 39 / 53; one CTA 256 33 / 49, 128 42 / 59): narrow and
-                // single-CTA tiles re-read more of A and B per flop, tiles that straddle the 128-column scale blocks
+                // pair 256 27 / 40, 224 30 / 54, 192 30 / 56, 128 39 / 53; one CTA 256 33 / 49, 128 42 / 59; block scales, their scales
+                // read ahead into L1, 37, 48, 49, 55; 41, 57): narrow and single-CTA tiles re-read more of A and B per flop, tiles that straddle the 128-column scale blocks
                 // pay for the second scale, and the 224-column epilogue works in half-width pieces, which a short K shows.
                 // Against the weights before (us): 4096^3 52.6 -> 47.9, 3794 x 3712 x 512 20.3 -> 16.7, 2750 x 7040 x 384 23.6 ->
                 // 18.5; with block scales 3794 x 3712 x 512 20.3 -> 16.7.
@@ -369,12 +371,19 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 // 23.4 and, two rows of tiles and B streaming from HBM, 190 x 16640 x 4096 18.7 / 20.0: a single tile fetches 48 KB per K
                 // block through four stages, a CTA of a pair 32 through six.
                 // (Calls whose inputs are ready keep the pair's tiles: those start under the predecessor's last tiles, a single CTA waits.)
-                const bool one_round = !pair && tiles <= units && !ab16 && !(a->flags & B200_GEMM_INPUTS_READY);
-                if (one_round && block && (bn >= 256 || kblocks <= 32 || tiles * 2 > units)) w = 125;
+                // Block scales on 256 columns: as fast per column as the pair in one round, as long as K is not long (pair / one CTA 333 x 7168 x
+                // 2048 12.2 / 11.8, 769 x 4608 x 512 7.6 / 6.4, 1024 x 4608 x 2048 13.4 / 12.3, 512 x 9472 x 8192 37.8 / 39.0); in several rounds
+                // 1.02-1.18 times the pair's (the weights are the best of a sweep over 5783 sizes, all tiles timed; with fewer than four
+                // K blocks the ones before it stand: 1332 x 7296 x 256, four batches, 27.0 / 29.5 on this tile).
+                const bool ready = (a->flags & B200_GEMM_INPUTS_READY) != 0;
+                const bool one_round = !pair && tiles <= units && !ab16 && !ready;
+                if (one_round && block && bn >= 256) w = kblocks <= 40 ? 93 : 102;
+                else if (block && !pair && bn >= 256 && !ready && kblocks >= 4) w = 110;
+                else if (one_round && block && (kblocks <= 32 || tiles * 2 > units)) w = 125;
                 else if (one_round && !block && (bn < 256 || kblocks <= (tm1 > 2 ? 32 : 24))) w = bn >= 256 ? 95 : 130;
                 else if (!pair) w = bn >= 256 ? 125 : 155;
                 else if (bn == 256) w = 100;
-                else if (bn == 128) w = block ? 130 : 140;
+                else if (bn == 128) w = block && kblocks < 4 ? 130 : 140;
                 else w = block ? 140 : (bn == 224 && kblocks < 8 ? 120 : 110);
                 const int64_t cost = tenths * bn * w;
                 if (best < 0 || cost < best) {

@@ -7,9 +7,9 @@
 // from the two CTAs' shared memories.  Per CTA that is 16 + 16 KB per block instead of 48 KB.  No load is
 // ever shared between CTAs by multicast; each CTA issues plain TMA loads for its own bytes.
 //
-// Roles per CTA (12 warps, same split as the single-CTA kernel): warp 0 TMA producer, warp 1 UMMA issuer
-// (only the pair's leader, cluster rank 0, issues MMAs; it also frees ring stages in BOTH CTAs), warps
-// 4-11 epilogue.  Block-scale mode keeps the reference's structure (a fresh accumulator per 128-wide K
+// Roles per CTA (12 warps): warp 3 TMA producer, warp 1 UMMA issuer (only the pair's leader, cluster rank 0,
+// issues MMAs; it also frees ring stages in BOTH CTAs), with block scales warp 0 reads the scales into L1 ahead of their
+// use, warps 4-11 epilogue.  Block-scale mode keeps the reference's structure (a fresh accumulator per 128-wide K
 // group, gemm_a8w8_blockscale_kernel_template.hpp:317,334; scale_c_tile :24-39): partials ping-pong
 // between two TMEM buffers and are folded into register accumulators with packed fp32 FMAs.
 #pragma once
@@ -83,7 +83,7 @@ __device__ __forceinline__ bool mbar_probe(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 #define B200_EPI_WAIT(bar, ph, af, st, code) (mbar_probe(bar, ph) || mbar_wait<false, 0>(bar, ph, af, st, code))
-// The TMA producer thread sits on the scheduler that hosts no issuer (warps 1..2 issue, warp w runs on scheduler w % 4):
+// The TMA producer thread sits on the scheduler that hosts no issuer (warp 1 issues, 1 and 2 did when this was measured; warp w runs on scheduler w % 4):
 // measured against warp 0, 1.5-2 % on the 4096 x 7168 x 2048 and 16384 x 7168 x 8192 problems, nothing on 8192^3.
 static constexpr int kProducerWarp = 3;
 
@@ -340,18 +340,11 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
         }
         else if (MODE == MODE_BLOCK && warp == 0) {
             // ------------------------------ scales into L1 (both CTAs) ------------------------------
-            // An epilogue warp that runs behind has some 300 clocks between asking for a group's scales and using them; a load
-            // that L1 misses takes 350 of a quiet L2 and 700 behind the operand tiles in flight, an L1 hit 110.  So this warp reads
-            // every scale of the tile once, some groups before the producer asks for the operands (a hint: nothing waits for it).
-            // Touched / not, us: 16384 x 7168 x 8192 958 / 1087, 8192^3 532 / 581, 4096 x 7168 x 2048 70.1 / 75.7, 512 x 9472 x 8192
-            // 39.3 / 45.2.  prefetch.global.L1 comes as far as L2 (a later load takes 280 clocks): 1001 / 1048 on the first of these.
-            // The same ring in shared memory, filled by cp.async or by this warp, had at most five groups of room beside the
-            // tiles: 4-8 % on 256 columns, a loss on 128 and on short K.
-            constexpr int kBatch = 4, kAhead = 3;            // groups per request; groups ahead of the producer
-            float x[kBatch + 1], sum = 0.0f;
-#pragma unroll
-            for (int i = 0; i <= kBatch; ++i) x[i] = 0.0f;
-            int q = 0, ready_b = -1;                         // K groups behind this one; last batch whose ready word has been seen
+            // (see ScaleToucher.  Touched / not, us: 16384 x 7168 x 8192 958 / 1087, 8192^3 532 / 581, 4096 x 7168 x 2048 70.1 / 75.7, 512 x
+            // 9472 x 8192 39.3 / 45.2.  The same scales in a ring in shared memory, filled by cp.async or by this warp, had at most five
+            // groups of room beside the tiles: 4-8 % on 256 columns, a loss on 128 and on short K.)
+            ScaleToucher touch;
+            int ready_b = -1;                                // last batch whose ready word has been seen
             bool go = true;
             for (int u = pair_id; u < units_total && go; u += num_pairs) {
                 int t = u, part = -1;
@@ -365,32 +358,9 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                     if (!__shfl_sync(0xFFFFFFFFu, seen, 0)) break;
                     ready_b = b;
                 }
-                // a lane per 16 bytes of A's 128 rows, and per 128-column block of B that the tile may touch
-                const int row = mi * (2 * BM) + static_cast<int>(cta) * BM + lane * 4, blk = ((ni * BN) >> 7) + lane;
-                const float* pa = p.sfa + b * p.sfa_batch + (row < p.m ? row : p.m - 1);
-                const bool col_ok = lane <= (BN + 127) / 128 && (blk << 7) < p.n;
-                const float* pb = p.sfb + b * p.sfb_batch + (col_ok ? static_cast<long long>(blk) * p.sfb_stride : 0);
-                for (int g = 0; g < groups && go; g += kBatch) {
-                    const int cnt = groups - g < kBatch ? groups - g : kBatch;
-                    int polls = 0;
-                    while (q > *requested + kAhead && go) {
-                        go = !*abort_flag && ++polls < (1 << 20);
-                        __nanosleep(200);
-                    }
-                    go = __all_sync(0xFFFFFFFFu, go);
-                    // (added up only here, so that the loads of the batch before have had its time to arrive)
-#pragma unroll
-                    for (int i = 0; i <= kBatch; ++i) sum += x[i];
-#pragma unroll
-                    for (int i = 0; i < kBatch; ++i)
-                        if (i < cnt) x[i] = ld_nc_f32(pa + static_cast<long long>(g + i) * p.sfa_stride);
-                    if (col_ok) x[kBatch] = ld_nc_f32(pb + g);
-                    q += cnt;
-                }
+                go = touch.tile(p, b, mi * (2 * BM) + static_cast<int>(cta) * BM, ni * BN, BN, groups, lane, requested, abort_flag);
             }
-#pragma unroll
-            for (int i = 0; i <= kBatch; ++i) sum += x[i];
-            if (__float_as_uint(sum) == 0xFFFFFFFFu) *requested = -1;      // (keeps the loads; no sum has these bits)
+            touch.finish(requested);
         }
 #ifdef B200_TRACE
         else if (MODE == MODE_BLOCK && warp == 2 && lane == 0 && cta == 1 && pair_id == 0) {

@@ -7,13 +7,16 @@
 // One persistent CTA per SM, 12 warps:
 //   warp 0      TMA producer   (one elected lane)  global -> shared ring, mbarrier complete_tx
 //   warp 1      UMMA issuer    (one elected lane)  tcgen05.mma kind::f8f6f4 / kind::mxf8f6f4, TMEM alloc
-//   warps 2-3   idle (they exist so that register re-allocation can work on whole warpgroups)
+//   warp 2      block scales, 256 columns: reads the scales into L1 ahead of their use (ScaleToucher)
+//   warp 3      idle, as warp 2 otherwise (register re-allocation works on whole warpgroups)
 //   warps 4-11  epilogue: TMEM -> registers -> scale -> global
 // TMEM holds two accumulator buffers of BN columns (four with block scales and BN = 128).  Per-tensor / unscaled / MX modes accumulate a
 // whole tile in one buffer while the epilogue drains the other.  Block-scale mode gives every
 // 128-wide K group a FRESH buffer (the reference does the same with a fresh MFMA accumulator,
 // kernel_template.hpp:317,334) and the epilogue warps fold it into register accumulators with
 // acc += partial * (sfa[g][row] * sfb[nblk][g]) -- the analogue of scale_c_tile.
+// Few tiles with a long K: the CTAs of a cluster take a part of a 128 x 128 tile's K each (SPLIT) and sum their results in
+// distributed shared memory; tile_splits() of the launcher says when.
 #pragma once
 
 #include "sm100_ptx.cuh"
@@ -76,6 +79,7 @@ static constexpr int kOutStageBytesPerWarp = 32 * kOutStagePitch;
 template <int BN_, int MODE_, int BLAYOUT_, bool SPLIT_ = false>
 struct GemmCfg {
     static constexpr bool SPLIT = SPLIT_;                           // a tile's K is split over a cluster
+    static constexpr bool TOUCH = MODE_ == MODE_BLOCK && BN_ == 256;   // a warp reads the scales ahead of their use
     static constexpr bool AB16 = MODE_ == MODE_ACC16;               // bf16 operands: same bytes, kind::f16 MMAs
     static constexpr int BM = 128, BN = BN_, BK = 128, MODE = AB16 ? MODE_ACC : MODE_, BLAYOUT = BLAYOUT_;
     static constexpr int A_BYTES = BM * BK;
@@ -108,6 +112,50 @@ struct GemmCfg {
     static_assert(STAGES >= 3 && STAGES_ONE <= 8, "ring depth");
     static_assert(OUT_STAGE_BYTES <= STAGES * STAGE_BYTES, "the staging fits the ring");
     static_assert(!SPLIT || (BN == 128 && BM * BN * 4 <= RING_BYTES), "the partial sums fit the ring");
+};
+
+// Block scales: a warp that reads every scale of a tile once, a few K groups before the TMA producer asks for the operands, so that the
+// epilogue finds it in L1.  An epilogue warp that runs behind has some 300 clocks between asking for a group's scales and using
+// them; a load that L1 misses takes 350 of a quiet L2 and 700 behind the operand tiles in flight, an L1 hit 110.  A hint: nothing waits
+// for it.  (prefetch.global.L1 comes as far as L2, a later load takes 280 clocks: a third of the gain.)
+struct ScaleToucher {
+    static constexpr int kBatch = 4, kAhead = 3;             // groups per request; groups ahead of the producer
+    float x[kBatch + 1] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, sum = 0.0f;
+    int q = 0;                                               // K groups behind this one
+    // One tile: A's rows [row0, row0 + 128), B's columns from col0 on.  *requested: the K block the producer is at.  False: give up.
+    __device__ __forceinline__ bool tile(const GemmParams& p, int b, int row0, int col0, int bn, int groups, int lane, volatile int* requested,
+                                         volatile int* abort_flag, int kb0 = 0) {
+        // a lane per 16 bytes of A's 128 rows, and per 128-column block of B that the tile may touch
+        const int row = row0 + lane * 4, blk = (col0 >> 7) + lane;
+        const float* pa = p.sfa + b * p.sfa_batch + static_cast<long long>(kb0) * p.sfa_stride + (row < p.m ? row : p.m - 1);
+        const bool col_ok = lane <= (bn + 127) / 128 && (blk << 7) < p.n;
+        const float* pb = p.sfb + b * p.sfb_batch + (col_ok ? static_cast<long long>(blk) * p.sfb_stride : 0) + kb0;
+        bool go = true;
+        for (int g = 0; g < groups && go; g += kBatch) {
+            const int cnt = groups - g < kBatch ? groups - g : kBatch;
+            int polls = 0;
+            while (q > *requested + kAhead && go) {
+                go = !*abort_flag && ++polls < (1 << 20);
+                __nanosleep(200);
+            }
+            go = __all_sync(0xFFFFFFFFu, go);
+            // (added up only here, so that the loads of the batch before have had its time to arrive)
+#pragma unroll
+            for (int i = 0; i <= kBatch; ++i) sum += x[i];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i)
+                if (i < cnt) x[i] = ld_nc_f32(pa + static_cast<long long>(g + i) * p.sfa_stride);
+            if (col_ok) x[kBatch] = ld_nc_f32(pb + g);
+            q += cnt;
+        }
+        return go;
+    }
+    // keeps the loads (no sum has these bits)
+    __device__ __forceinline__ void finish(volatile int* requested) {
+#pragma unroll
+        for (int i = 0; i <= kBatch; ++i) sum += x[i];
+        if (__float_as_uint(sum) == 0xFFFFFFFFu) *requested = -1;
+    }
 };
 
 // tile index -> (batch, m tile, n tile): groups of 8 M tiles walk N, so that the tiles resident at
@@ -293,6 +341,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     const uint32_t bar_acce0 = bar_accf0 + BUFS * 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * Cfg::STAGES_ONE + 2 * BUFS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* requested = reinterpret_cast<volatile int*>(tmem_slot + 2);    // TOUCH: the K block the TMA producer is at
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -312,6 +361,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             mbar_init(bar_acce0 + s * 8, 8);     // one arrival per epilogue warp
         }
         *abort_flag = 0;
+        *requested = 0;
         fence_barrier_init();
         fence_proxy_async_smem();
     }
@@ -351,6 +401,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             // ------------------------------ TMA producer ------------------------------
             uint32_t s = 0, ph = 0;
             bool ok = true;
+            int asked = 0;
             for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
                 int b, mi, ni;
                 tile_coords(p, t, b, mi, ni);
@@ -362,6 +413,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     const uint32_t sa = smem_base + s * Cfg::STAGE_BYTES;
                     const uint32_t sb = sa + Cfg::A_BYTES;
                     const uint32_t full = bar_full0 + s * 8;
+                    if constexpr (Cfg::TOUCH) *requested = asked++;
                     mbar_arrive_expect_tx(full, Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES + Cfg::SFB_BYTES);
                     tma_load_3d(sa, &p.tmap_a, full, kb * BK, mi * BM, b);
                     if constexpr (Cfg::BLAYOUT == BL_NK)
@@ -436,6 +488,18 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 }
             }
         }
+        if constexpr (Cfg::TOUCH) {
+            if (warp == 2) {
+                ScaleToucher touch;
+                bool go = true;
+                for (int t = blockIdx.x; t < p.tiles_total && go; t += gridDim.x) {
+                    int b, mi, ni;
+                    tile_coords(p, t, b, mi, ni);
+                    go = touch.tile(p, b, mi * BM, ni * BN, BN, groups, lane, requested, abort_flag);
+                }
+                touch.finish(requested);
+            }
+        }
         if constexpr (Cfg::SPLIT) {
             __syncwarp();
             cluster_arrive();
@@ -498,8 +562,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 // 64 columns per thread leave room to have both loads of a group in flight, and the buffer goes back before the FMAs;
                 // four buffers keep the tensor core busy meanwhile.  Two buffers, handed back after the FMAs, scalar FMAs and stores
                 // from registers / this loop and staged stores, us: 100 x 7168 x 2048 10.6 / 9.2, 200 x 7168 x 2048 11.3 / 9.6, 512 x 4096 x
-                // 4096 16.8 / 15.0, 2500 x 5120 x 3072 77 / 59.  (The same loop for 128 columns per thread, two buffers, was slower:
-                // 700 x 2048 x 7168 28.9 -> 30.7.)
+                // 4096 16.8 / 15.0, 2500 x 5120 x 3072 77 / 59.
                 // Scales are requested six groups ahead, into six register sets that take turns (a copy from one to the
                 // other would wait for the load): a load queues behind the operand tiles in flight, and with the tensor core four buffers
                 // ahead there are more of those than with two.  Two / four / six / eight ahead, us: 128 x 8192 x 8192 32.8 / 27.8 / 25.6 /
@@ -560,20 +623,19 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     }
                 }
             } else if constexpr (MODE == MODE_BLOCK) {
-                float acc[NCH];
+                // 128 columns per thread: two 32-column loads in flight beside the accumulators, the buffer handed back when the last of
+                // four has landed, scales of the next group (in L1, see ScaleToucher) asked for after that.  One load at a time, scalar FMAs,
+                // the buffer handed back last and scales from L2 / so, us: 333 x 7168 x 2048 12.6 / 11.8, 4096 x 7168 x 2048 80.7 / 70.5, 8192^3
+                // 661 / 585, 700 x 2048 x 7168 44.8 / 39.5.
+                unsigned long long acc2[NCH / 2];
 #pragma unroll
-                for (int j = 0; j < NCH; ++j) acc[j] = 0.0f;
+                for (int j = 0; j < NCH / 2; ++j) acc2[j] = 0ull;
                 const float* sfa_p = p.sfa + b * p.sfa_batch + (row < p.m ? row : 0);
                 const float* sfb_p = p.sfb + b * p.sfb_batch + static_cast<long long>(col_base / 128) * p.sfb_stride;
                 const bool col_ok = col_base < p.n;
-                float sa_next = __ldg(sfa_p);
-                float sb_next = col_ok ? __ldg(sfb_p) : 0.0f;
+                float sa_cur = __ldg(sfa_p);
+                float sb_cur = col_ok ? __ldg(sfb_p) : 0.0f;
                 for (int g = 0; g < groups; ++g, ++phase) {
-                    const float sc = sa_next * sb_next;
-                    if (g + 1 < groups) {
-                        sa_next = __ldg(sfa_p + static_cast<long long>(g + 1) * p.sfa_stride);
-                        sb_next = col_ok ? __ldg(sfb_p + g + 1) : 0.0f;
-                    }
                     const uint32_t as = phase & 1;
                     const uint32_t aph = (phase >> 1) & 1;
                     if (!mbar_wait(bar_accf0 + as * 8, aph, abort_flag, p.status, KSTAT_TIMEOUT_ACC_F)) {
@@ -584,20 +646,36 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
                     float v[2][32];
                     tmem_ld32(taddr, v[0]);
+                    tmem_ld32(taddr + 32, v[1]);
+                    const float sc = sa_cur * sb_cur;
+                    const unsigned long long sc2 = pack_f32x2(sc, sc);
 #pragma unroll
                     for (int c = 0; c < NCH / 32; ++c) {
-                        tmem_ld_wait();
-                        if (c + 1 < NCH / 32) tmem_ld32(taddr + (c + 1) * 32, v[(c + 1) & 1]);
+                        if (c % 2 == 0) tmem_ld_wait();
+                        if (c == NCH / 32 - 2) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
+                            if (g + 1 < groups) {
+                                sfa_p += p.sfa_stride;
+                                ++sfb_p;
+                                sa_cur = __ldg(sfa_p);
+                                sb_cur = col_ok ? __ldg(sfb_p) : 0.0f;
+                            }
+                        }
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(v[c & 1][j], sc, acc[c * 32 + j]);
+                        for (int j = 0; j < 16; ++j) acc2[c * 16 + j] = ffma2(pack_f32x2(v[c & 1][2 * j], v[c & 1][2 * j + 1]), sc2, acc2[c * 16 + j]);
+                        if (c + 2 < NCH / 32) tmem_ld32(taddr + (c + 2) * 32, v[c & 1]);
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
                 }
                 if (ok) {
 #pragma unroll
-                    for (int c = 0; c < NCH / 32; ++c) put32(c, &acc[c * 32]);
+                    for (int c = 0; c < NCH / 32; ++c) {
+                        float o[32];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) unpack_f32x2(acc2[c * 16 + j], o[2 * j], o[2 * j + 1]);
+                        put32(c, o);
+                    }
                 }
             } else {
                 const uint32_t as = phase & 1;
