@@ -349,3 +349,8 @@ def last_tail_split():
     v = (C.c_int32 * 2)()
     hit = lib().b200_last_tail_split(C.byref(v, 0), C.byref(v, 4))
     return (v[0], v[1]) if hit else None
+
+
+def last_k_split():
+    """CTAs per tile of this thread's last tile-kernel launch when the K of a tile was split over a cluster, otherwise None."""
+    return lib().b200_last_k_split() or None

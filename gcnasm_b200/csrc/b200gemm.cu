@@ -544,6 +544,7 @@ int split_clusters(int size, int sm_count) {
     return n < sm_count / size ? n : sm_count / size;
 }
 
+thread_local int t_last_k_split = 0;           // the calling thread's last tile-kernel launch (b200_last_k_split)
 // 128 x 128 tiles on one CTA each or, with p.splits > 1, on a cluster each
 template <int MODE, int BL>
 int launch_gemm128(GemmParams& p, int grid, int sm_count, cudaStream_t st) {
@@ -556,6 +557,7 @@ int launch_gemm128(GemmParams& p, int grid, int sm_count, cudaStream_t st) {
     auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
     int rc = set_smem(kernel, Cfg::SMEM_BYTES);
     if (rc) return rc;
+    t_last_k_split = p.splits;
     return launch_pdl_cluster(p.splits, kernel, static_cast<unsigned>(p.tiles_total * p.splits), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
 
@@ -976,6 +978,7 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
         p.sfa_batch = a->stride_sfa_batch;
         p.sfb_batch = a->stride_sfb_batch;
     }
+    t_last_k_split = 0;
     const bool flat = a->b_layout == B200_B_FLAT_16x16;
     if (pair && BN == 256 && !ab16 && a->scale_mode != B200_SCALE_MX) {
         const int sms = ds->sm_count;
@@ -1051,6 +1054,12 @@ int b200_gemm_check(const b200_gemm_args* args, int32_t* chosen_tile) {
     if (rc == B200_OK && chosen_tile) *chosen_tile = pl.tile;
     return rc;
 }
+int b200_gemm_check_split(const b200_gemm_args* args, int32_t* parts) {
+    Plan pl;
+    int rc = validate(args, 148, &pl);
+    if (rc == B200_OK && parts) *parts = pl.tile == B200_TILE_DECODE ? 1 : pl.splits;
+    return rc;
+}
 
 int b200_gemm_a8w8(const b200_gemm_args* args, void* cuda_stream) {
     Plan pl;
@@ -1086,6 +1095,15 @@ int b200_gemm_a16w16_check(const b200_gemm_args* args, int32_t* chosen_tile) {
     Plan pl;
     rc = validate(&v, 148, &pl, true);
     if (rc == B200_OK && chosen_tile) *chosen_tile = pl.tile;
+    return rc;
+}
+int b200_gemm_a16w16_check_split(const b200_gemm_args* args, int32_t* parts) {
+    b200_gemm_args v;
+    int rc = byte_view16(args, &v);
+    if (rc) return rc;
+    Plan pl;
+    rc = validate(&v, 148, &pl, true);
+    if (rc == B200_OK && parts) *parts = pl.splits;
     return rc;
 }
 int b200_gemm_a16w16(const b200_gemm_args* args, void* cuda_stream) {
@@ -1724,5 +1742,6 @@ int b200_last_tail_split(int32_t* first_tile, int32_t* parts) {
     if (parts) *parts = t_last_tail[1];
     return t_last_tail[1] > 0 ? 1 : 0;
 }
+int b200_last_k_split(void) { return t_last_k_split; }
 
 }  // extern "C"

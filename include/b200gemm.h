@@ -133,6 +133,11 @@ int b200_last_tail_split(int32_t* first_tile, int32_t* parts);
  * computed on 128x128 tiles instead, each shared by the CTAs of a cluster that take a part of K; with the tile as a
  * hint it is computed as reported, except that a hint of 128x128 is split by the same rule.                          */
 int b200_gemm_check(const b200_gemm_args* args, int32_t* chosen_tile);
+/* The other half of that answer: how many CTAs share the K of a tile in this launch.  1: whole tiles of the kind that
+ * b200_gemm_check reports (or the skinny-M kernel, which splits K by rules of its own).  2 to 8: 128x128 tiles, so many CTAs each.   */
+int b200_gemm_check_split(const b200_gemm_args* args, int32_t* parts);
+/* What the calling thread's last launch of a tile kernel did: the CTAs per tile when K was split, otherwise 0.        */
+int b200_last_k_split(void);
 
 /* Same contract as b200_gemm_a8w8 but computed by a one-thread-per-output CUDA kernel that mirrors the
  * host gemm_ref loops (gemm_a8w8_8wave.cc:601-612, gemm_a8w8_blockscale_host.cc:66-90): the device-side
@@ -184,6 +189,7 @@ int b200_gemm_a8w8_decode_static(const b200_gemm_args* args, void* cuda_stream);
  * stride_a, stride_b multiples of 8, 16-byte aligned bases.  Tiles: AUTO, 128x128, 128x256, PAIR_256x256.       */
 int b200_gemm_a16w16(const b200_gemm_args* args, void* cuda_stream);
 int b200_gemm_a16w16_check(const b200_gemm_args* args, int32_t* chosen_tile);
+int b200_gemm_a16w16_check_split(const b200_gemm_args* args, int32_t* parts);    /* see b200_gemm_check_split */
 /* shuffle_b<bf16> of opus_fmm/flatmm_a16w16_gfx950.cc:623-666 (ItemsPerAccess 8): [K][N] (src_is_kn != 0) or
  * [N][K] row-major bf16 -> flat [N/16][K/8][16 n][8 k]; N % 16 == 0, K % 8 == 0.  Byte-exact.                     */
 int b200_shuffle_b_bf16(const void* src, void* dst, int64_t n, int64_t k, int32_t src_is_kn, void* cuda_stream);

@@ -3,10 +3,17 @@
 Without scales, with block scales and with bf16 operands the values are whole numbers (of at most 2, block scales 2^-5 to 2^5 in the
 product): an fp32 sum of at most 8192 products, or of 32 groups' 512 * 2^5 in steps of 2^-5, takes 24 bits, nothing is rounded, and the result
 has to be the exact one.  MX: a sum of K products in any order and grouping is off by at most K * 2^-23 of the sum of their magnitudes."""
+import ctypes as C
+import os
+import subprocess
+
 import pytest
 import torch
 
+from gcnasm_b200 import _lib as L
+
 from test_gpu_blockscale_groups import problem
+from test_tile_choice import args
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -61,6 +68,33 @@ def test_mx(api, m, n, k):
     torch.cuda.synchronize()
     assert api.last_status() == 0
     assert ((c.double() - va @ vb.t()).abs() <= k * 2.0 ** -23 * (va.abs() @ vb.abs().t())).all()
+
+
+@pytest.mark.parametrize("mode", [L.SCALE_NONE, L.SCALE_BLOCK, L.SCALE_MX])
+@pytest.mark.parametrize("m,n,k", [(256, 4608, 8192), (100, 5120, 8192), (256, 2048, 4096), (200, 1536, 8192), (100, 512, 512), (256, 512, 8192)])
+def test_the_launch_is_the_reported_one(api, native, mode, m, n, k):
+    a, b = (torch.zeros(rows, k, dtype=torch.uint8, device=DEV) for rows in (m, n))
+    run = {L.SCALE_NONE: lambda: api.gemm_a8w8(a, b),
+           L.SCALE_BLOCK: lambda: api.gemm_a8w8_blockscale(a, b, torch.ones(k // 128, m, device=DEV), torch.ones(n // 128, k // 128, device=DEV)),
+           L.SCALE_MX: lambda: api.gemm_a8w8_mx(a, b, *(torch.full((native.b200_mx_sf_bytes(rows, k),), 127, dtype=torch.uint8, device=DEV)
+                                                        for rows in (m, n)))}[mode]
+    run()
+    parts = C.c_int32(-1)
+    assert native.b200_gemm_check_split(C.byref(args(m, n, k, mode)), C.byref(parts)) == 0
+    assert (api.last_k_split() or 1) == parts.value
+    api.gemm_a8w8(a[:, :128].contiguous(), b[:, :128].contiguous())             # a launch of whole tiles
+    assert api.last_k_split() is None
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+
+
+def test_driver_names_the_tile_it_launches(native):
+    from gcnasm_b200 import build
+
+    build.build_drivers()
+    out = subprocess.run([os.path.join(build.BIN, "gemm_a8w8_blockscale"), "-m", "256", "-n", "512", "-k", "8192", "-b", "1", "--warmup", "1", "--iters", "1"],
+                         capture_output=True, text=True, timeout=300).stdout
+    assert "tile_config=1, k_split=8" in out
 
 
 def test_strided_result_in_a_chain(api):

@@ -1,4 +1,5 @@
-"""CPU: which kernel the launcher picks, at the lines where measured times cross (148 SMs)."""
+"""CPU: which kernel the launcher picks, at the lines where measured times cross (148 SMs): the kind of whole tile, and how many CTAs share
+a 128 x 128 tile's K where the launch takes such tiles instead."""
 import ctypes as C
 
 import pytest
@@ -29,6 +30,13 @@ def choice(native, *problem, **more):
     return tile.value if rc == L.OK else rc
 
 
+def k_split(native, *problem, bf16=False, **more):
+    parts = C.c_int32(-1)
+    entry = native.b200_gemm_a16w16_check_split if bf16 else native.b200_gemm_check_split
+    rc = entry(C.byref(args(*problem, **more)), C.byref(parts))
+    return parts.value if rc == L.OK else rc
+
+
 ONE, ONE256, PAIR256, PAIR128, PAIR224 = L.TILE_128x128, L.TILE_128x256, L.TILE_PAIR_256x256, L.TILE_PAIR_256x128, L.TILE_PAIR_256x224
 
 
@@ -41,6 +49,21 @@ ONE, ONE256, PAIR256, PAIR128, PAIR224 = L.TILE_128x128, L.TILE_128x256, L.TILE_
     (L.SCALE_NONE, 190, 16640, 3072, ONE256), (L.SCALE_NONE, 190, 16640, 4096, PAIR256)])
 def test_one_round(native, mode, m, n, k, tile):
     assert choice(native, m, n, k, mode) == tile
+
+
+# few tiles with a long K: the launch splits K, whatever kind of whole tile it would take; calls whose inputs are ready, slabs on their way, one
+# B for all batches and the skinny-M kernel do not
+@pytest.mark.parametrize("mode,m,n,k,parts", [
+    (L.SCALE_BLOCK, 256, 512, 4224, 7), (L.SCALE_BLOCK, 256, 512, 8192, 8), (L.SCALE_BLOCK, 1024, 1024, 8192, 2), (L.SCALE_BLOCK, 256, 512, 512, 1),
+    (L.SCALE_NONE, 256, 512, 8192, 8), (L.SCALE_NONE, 256, 8192, 8192, 1), (L.SCALE_NONE, 256, 4608, 4096, 1), (L.SCALE_NONE, 256, 4608, 8192, 2),
+    (L.SCALE_BLOCK, 256, 4608, 4096, 2), (L.SCALE_MX, 256, 4608, 4096, 2), (L.SCALE_NONE, 16, 512, 8192, 1), (L.SCALE_NONE, 16, 520, 8192, 8)])
+def test_split_of_few_tiles(native, mode, m, n, k, parts):
+    assert k_split(native, m, n, k, mode) == parts
+    assert k_split(native, m, n, k, mode, flags=L.GEMM_INPUTS_READY) == 1
+
+
+def test_split_of_few_tiles_bf16(native):
+    assert [k_split(native, *p, bf16=True) for p in ((100, 512, 4096), (256, 4608, 2048), (256, 4608, 4096), (4096, 4096, 4096))] == [8, 1, 2, 1]
 
 
 # inputs that are ready: the pair kernels start before the predecessor has finished, so what they would take is not given to single CTAs
