@@ -408,7 +408,8 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                     consider(B200_TILE_128x128, 128, false);
                 }
             }
-            // Few tiles with a long K: 128 x 128 tiles whose K is split may be the better ones (w as for a grid of one round).
+            // Few tiles with a long K: 128 x 128 tiles whose K is split may be the better ones (w as for a grid of one round).  A hint is
+            // another matter: who names a tile gets it whole, with the bits that every kind of whole tile gives.
             if (!pair_only && !(a->flags & B200_GEMM_INPUTS_READY)) {
                 int64_t equal;
                 const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, sm_count, &equal);
@@ -438,8 +439,6 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
             }
         }
         pl.splits = splits;
-    } else if (hint == B200_TILE_128x128 && a->tile_hint == hint) {
-        pl.splits = tile_splits(a->m, (a->m + 127) / 128 * ((a->n + 127) / 128) * a->batch, kblocks, slow, sm_count);
     }
     if (plan) *plan = pl;
     return B200_OK;

@@ -39,7 +39,7 @@ def test_sums_are_exact(api, kind, m, n, k, out):
         qa, qb = (torch.stack([api.cast_e4m3(t[i].float()) for i in range(batch)]) for t in (a, b))
         s = torch.tensor([0.5], device=DEV) if kind == "tensor" else None
         ref = ref * 0.25 if kind == "tensor" else ref
-        c = api.gemm_a8w8(qa, qb, s, s, out_dtype=out, tile=1).reshape(batch, m, n)
+        c = api.gemm_a8w8(qa, qb, s, s, out_dtype=out).reshape(batch, m, n)
     torch.cuda.synchronize()
     assert api.last_status() == 0
     assert torch.equal(c, ref.float().to(out))
@@ -49,7 +49,7 @@ def test_sums_are_exact(api, kind, m, n, k, out):
 @pytest.mark.parametrize("m,n,groups", [(100, 512, 32), (333, 384, 31), (129, 128, 23), (256, 4608, 32)])
 def test_groups_meet_their_scales(api, m, n, groups, flat):
     a, b, sfa, sfb, ref = problem(m, n, 128 * groups, m + groups)
-    c = api.gemm_a8w8_blockscale(a, api.shuffle_b(b, "nk") if flat else b, sfa, sfb, out_dtype=torch.float32, tile=1, b_flat_n=n if flat else None)
+    c = api.gemm_a8w8_blockscale(a, api.shuffle_b(b, "nk") if flat else b, sfa, sfb, out_dtype=torch.float32, b_flat_n=n if flat else None)
     torch.cuda.synchronize()
     assert api.last_status() == 0
     assert torch.equal(c.double(), ref)
@@ -64,7 +64,7 @@ def test_mx(api, m, n, k):
         value = q.view(torch.float8_e4m3fn).double() * torch.exp2(logical.reshape(rows, -1).double() - 127).repeat_interleave(32, 1)
         sides.append((q, atoms, value))
     (a, sfa, va), (b, sfb, vb) = sides
-    c = api.gemm_a8w8_mx(a, b, sfa, sfb, out_dtype=torch.float32, tile=1)
+    c = api.gemm_a8w8_mx(a, b, sfa, sfb, out_dtype=torch.float32)
     torch.cuda.synchronize()
     assert api.last_status() == 0
     assert ((c.double() - va @ vb.t()).abs() <= k * 2.0 ** -23 * (va.abs() @ vb.abs().t())).all()
@@ -97,6 +97,22 @@ def test_driver_names_the_tile_it_launches(native):
     assert "tile_config=1, k_split=8" in out
 
 
+# who names a 128 x 128 tile gets it whole: the bits of every other kind of whole tile
+@pytest.mark.parametrize("m,n,k", [(200, 512, 4096), (333, 384, 8192)])
+def test_a_tile_that_is_asked_for_stays_whole(api, m, n, k):
+    g = torch.Generator(device=DEV).manual_seed(k)
+    (a, sfa), (b, sfb) = (q(torch.randn(rows, k, generator=g, device=DEV)) for q, rows in ((api.quantize_1x128, m), (api.quantize_128x128, n)))
+    for run in (lambda t: api.gemm_a8w8(a, b, out_dtype=torch.float32, tile=t),
+                lambda t: api.gemm_a8w8_blockscale(a, b, sfa, sfb, out_dtype=torch.float32, tile=t)):
+        pair, one = run(6), run(1)
+        assert api.last_k_split() is None
+        assert torch.equal(pair, one)
+    x, y = (torch.randn(rows, k // 2, generator=g, device=DEV).bfloat16() for rows in (m, n))
+    assert torch.equal(api.gemm_a16w16(x, y, out_dtype=torch.float32, tile=4), api.gemm_a16w16(x, y, out_dtype=torch.float32, tile=1))
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+
+
 def test_strided_result_in_a_chain(api):
     """Rows of C further apart than N and not 16-byte aligned, behind the kernel that writes A."""
     g = torch.Generator(device=DEV).manual_seed(3)
@@ -106,7 +122,8 @@ def test_strided_result_in_a_chain(api):
     for i in range(3):
         a = ints(g, m, k)
         big = torch.full((m, n + 3), 7.0, device=DEV)
-        api.gemm_a8w8(api.cast_e4m3(a.float()), qb, out=big[:, 1:n + 1], tile=1)
+        api.gemm_a8w8(api.cast_e4m3(a.float()), qb, out=big[:, 1:n + 1])
+        assert api.last_k_split() == 8
         torch.cuda.synchronize()
         assert torch.equal(big[:, 1:n + 1].double(), a.double() @ b.double().t())
         assert (big[:, 0] == 7).all() and (big[:, n + 1:] == 7).all()

@@ -60,6 +60,7 @@ def test_one_round(native, mode, m, n, k, tile):
 def test_split_of_few_tiles(native, mode, m, n, k, parts):
     assert k_split(native, m, n, k, mode) == parts
     assert k_split(native, m, n, k, mode, flags=L.GEMM_INPUTS_READY) == 1
+    assert k_split(native, m, n, k, mode, hint=ONE) == 1                # a tile that is asked for stays whole
 
 
 def test_split_of_few_tiles_bf16(native):
