@@ -538,19 +538,24 @@ int split_clusters(int size, int sm_count) {
     if (n < 0) {
         if (set_smem(kernel, Cfg::SMEM_BYTES)) return 0;
         n = resident_clusters(kernel, size, Cfg::THREADS, Cfg::SMEM_BYTES);
-        known[dev][size].store(n + 1);
+        if (n > 0) known[dev][size].store(n + 1);                           // (a question that failed is asked again)
     }
     return n < sm_count / size ? n : sm_count / size;
+}
+template <int BL>
+int split_clusters(const b200_gemm_args* a, bool ab16, int size, int sm_count) {
+    if (ab16) return split_clusters<MODE_ACC16, BL>(size, sm_count);
+    switch (a->scale_mode) {
+        case B200_SCALE_BLOCK: return split_clusters<MODE_BLOCK, BL>(size, sm_count);
+        case B200_SCALE_MX: return split_clusters<MODE_MX, BL>(size, sm_count);
+        default: return split_clusters<MODE_ACC, BL>(size, sm_count);
+    }
 }
 
 thread_local int t_last_k_split = 0;           // the calling thread's last tile-kernel launch (b200_last_k_split)
 // 128 x 128 tiles on one CTA each or, with p.splits > 1, on a cluster each
 template <int MODE, int BL>
-int launch_gemm128(GemmParams& p, int grid, int sm_count, cudaStream_t st) {
-    while (p.splits > 1 && split_clusters<MODE, BL>(p.splits, sm_count) < p.tiles_total) {
-        p.kb_per_split = (p.kblocks + p.splits - 2) / (p.splits - 1);
-        p.splits = (p.kblocks + p.kb_per_split - 1) / p.kb_per_split;
-    }
+int launch_gemm128(const GemmParams& p, int grid, cudaStream_t st) {
     if (p.splits <= 1) return launch_gemm<128, MODE, BL>(p, grid, st);
     using Cfg = GemmCfg<128, MODE, BL, true>;
     auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
@@ -589,7 +594,7 @@ int decode_clusters(int size, int sm_count) {
     if (n < 0) {
         if (decode_attrs<MT, MODE, BL>()) return 0;
         n = resident_clusters(decode_a8w8_sm100_kernel<Cfg>, size, Cfg::THREADS, Cfg::SMEM_BYTES);
-        known[dev][size].store(n + 1);
+        if (n > 0) known[dev][size].store(n + 1);
     }
     return n < sm_count / size ? n : sm_count / size;
 }
@@ -897,7 +902,16 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
 int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStream_t st, bool ab16 = false) {
     int BN = 128;
     bool pair = false;
-    switch (pl.splits > 1 ? B200_TILE_128x128 : pl.tile) {
+    // The plan took the clusters that are resident at once from a table; where this device holds fewer, the tile that the split was
+    // compared with is the better one.
+    int splits = pl.splits;
+    if (splits > 1) {
+        const int64_t tiles = (a->m + 127) / 128 * ((a->n + 127) / 128) * a->batch;
+        const int room = a->b_layout == B200_B_FLAT_16x16 ? split_clusters<BL_FLAT>(a, ab16, splits, ds->sm_count)
+                                                          : split_clusters<BL_NK>(a, ab16, splits, ds->sm_count);
+        if (room < tiles) splits = 1;
+    }
+    switch (splits > 1 ? B200_TILE_128x128 : pl.tile) {
         case B200_TILE_128x256: BN = 256; break;
         case B200_TILE_PAIR_256x256: BN = 256; pair = true; break;
         case B200_TILE_PAIR_256x224: BN = 224; pair = true; break;
@@ -955,8 +969,8 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     if (total > 0x7FFFFFFF) return B200_ERR_TOO_LARGE;
     p.tiles_total = static_cast<int>(total);
     p.kblocks = static_cast<int>((a->k + 127) / 128);
-    p.kb_per_split = (p.kblocks + pl.splits - 1) / pl.splits;
-    p.splits = !pair && BN == 128 ? (p.kblocks + p.kb_per_split - 1) / p.kb_per_split : 1;
+    p.kb_per_split = (p.kblocks + splits - 1) / splits;
+    p.splits = splits;
     p.out_dtype = a->out_dtype;
     p.inputs_ready = (a->flags & (B200_GEMM_INPUTS_READY | B200_GEMM_BATCH_READY)) ? 1 : 0;
     p.b_shared = b_shared ? 1 : 0;
@@ -995,7 +1009,7 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
         if (pair) return flat ? launch_pair<256, MODE_ACC16, BL_FLAT>(p, ds->sm_count, st) : launch_pair<256, MODE_ACC16, BL_NK>(p, ds->sm_count, st);
         const int grid16 = p.tiles_total < ds->sm_count ? p.tiles_total : ds->sm_count;
         if (BN == 256) return flat ? launch_gemm<256, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<256, MODE_ACC16, BL_NK>(p, grid16, st);
-        return flat ? launch_gemm128<MODE_ACC16, BL_FLAT>(p, grid16, ds->sm_count, st) : launch_gemm128<MODE_ACC16, BL_NK>(p, grid16, ds->sm_count, st);
+        return flat ? launch_gemm128<MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm128<MODE_ACC16, BL_NK>(p, grid16, st);
     }
     if (pair) {
         switch (BN) {
@@ -1009,12 +1023,12 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     switch (a->scale_mode) {
         case B200_SCALE_BLOCK:
             if (BN == 256) return flat ? launch_gemm<256, MODE_BLOCK, BL_FLAT>(p, grid, st) : launch_gemm<256, MODE_BLOCK, BL_NK>(p, grid, st);
-            return flat ? launch_gemm128<MODE_BLOCK, BL_FLAT>(p, grid, ds->sm_count, st) : launch_gemm128<MODE_BLOCK, BL_NK>(p, grid, ds->sm_count, st);
+            return flat ? launch_gemm128<MODE_BLOCK, BL_FLAT>(p, grid, st) : launch_gemm128<MODE_BLOCK, BL_NK>(p, grid, st);
         case B200_SCALE_MX:
-            return flat ? launch_gemm128<MODE_MX, BL_FLAT>(p, grid, ds->sm_count, st) : launch_gemm128<MODE_MX, BL_NK>(p, grid, ds->sm_count, st);
+            return flat ? launch_gemm128<MODE_MX, BL_FLAT>(p, grid, st) : launch_gemm128<MODE_MX, BL_NK>(p, grid, st);
         default:
             if (BN == 256) return flat ? launch_gemm<256, MODE_ACC, BL_FLAT>(p, grid, st) : launch_gemm<256, MODE_ACC, BL_NK>(p, grid, st);
-            return flat ? launch_gemm128<MODE_ACC, BL_FLAT>(p, grid, ds->sm_count, st) : launch_gemm128<MODE_ACC, BL_NK>(p, grid, ds->sm_count, st);
+            return flat ? launch_gemm128<MODE_ACC, BL_FLAT>(p, grid, st) : launch_gemm128<MODE_ACC, BL_NK>(p, grid, st);
     }
 }
 
