@@ -260,8 +260,12 @@ int64_t mx_skinny_kblocks(int64_t m, int64_t panels, int sm_count) {
 // (At 1024 8-bit operands lose 1 us, block scales 0.5; MX 1705 x 256 x 1536 6.4 / 6.9, 8-bit 12 x 4232 x 3328 8.1 / 8.7.)
 constexpr int kMaxTileSplits = 8;
 constexpr int kSplitClusters[kMaxTileSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};     // resident at once on 148 SMs
-// *equal: the K blocks that a CTA would take as long for
-int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, int sm_count, int64_t* equal = nullptr) {
+// Tiles of up to 24 rows, the grid just too large for three CTAs a tile (46 to 50 tiles): two are slower than one where rows of A and B are
+// not whole 128-byte lines apart, and up to 47 K blocks where B comes out of L2; with more tiles a whole tile is the slow one.  Whole /
+// split, us, without scales: 4 x 6024 x 5872 15.6 / 19.7, x 8176 23.0 / 29.7, x 5376 with B from HBM 15.9 / 14.5, out of L2 12.0 / 13.9.  Mean
+// of split / whole over 3000 sizes: other pitches 0.98 (0.7 to 1.4), whole lines and 48 K blocks or more 0.84, with B out of L2 0.87.
+// *equal: the K blocks that a CTA would take as long for; lines: rows of A and B whole 128-byte lines apart
+int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, bool lines, int sm_count, int64_t* equal = nullptr) {
     const int64_t exchange = slow ? 9 + tiles / 32 : (m <= 32 ? 15 : 13) + tiles / 12;
     if (equal) *equal = kblocks;
     if (kblocks <= exchange) return 1;
@@ -270,6 +274,7 @@ int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, int sm_cou
     for (int s = 2; s <= kMaxTileSplits; ++s) {
         const int64_t per = (kblocks + s - 1) / s, cost = per + exchange + (s > 4 ? 2 : 0);
         if (per * (s - 1) >= kblocks || tiles > static_cast<int64_t>(kSplitClusters[s]) * sm_count / 148 || cost >= best_cost) continue;
+        if (s == 2 && m <= 24 && tiles <= 50 && !(lines && kblocks >= 48)) continue;
         best = s;
         best_cost = cost;
     }
@@ -412,7 +417,8 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
             // another matter: who names a tile gets it whole, with the bits that every kind of whole tile gives.
             if (!pair_only && !(a->flags & B200_GEMM_INPUTS_READY)) {
                 int64_t equal;
-                const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, sm_count, &equal);
+                const bool lines = a->stride_a % 128 == 0 && (a->b_layout == B200_B_FLAT_16x16 || a->stride_b % 128 == 0);
+                const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, lines, sm_count, &equal);
                 if (s > 1 && 10 * 128 * (ab16 ? 155 : a->scale_mode == B200_SCALE_BLOCK ? 125 : 130) * equal < best * kblocks) pl.splits = s;
             }
         }

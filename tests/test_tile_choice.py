@@ -63,6 +63,15 @@ def test_split_of_few_tiles(native, mode, m, n, k, parts):
     assert k_split(native, m, n, k, mode, hint=ONE) == 1                # a tile that is asked for stays whole
 
 
+# few rows and 46 to 50 tiles: two CTAs a tile only where rows are whole lines apart and K is long
+@pytest.mark.parametrize("m,n,k,parts", [
+    (4, 6024, 5872, 1), (11, 6152, 5376, 1), (24, 6264, 8176, 1), (24, 6264, 6144, 2), (24, 6264, 6016, 1), (25, 6264, 8176, 2),
+    (4, 6392, 6256, 1), (4, 6520, 6256, 2), (4, 5752, 6256, 3), (4, 6024, 8192, 2)])
+def test_split_of_few_rows(native, m, n, k, parts):
+    assert k_split(native, m, n, k) == parts
+    assert k_split(native, m, n // 16 * 16, k // 2, bf16=True) == parts
+
+
 def test_split_of_few_tiles_bf16(native):
     assert [k_split(native, *p, bf16=True) for p in ((100, 512, 4096), (256, 4608, 2048), (256, 4608, 4096), (4096, 4096, 4096))] == [8, 1, 2, 1]
 
