@@ -114,7 +114,7 @@ struct GemmCfg {
     static_assert(!SPLIT || (BN == 128 && BM * BN * 4 <= RING_BYTES), "the partial sums fit the ring");
 };
 
-// Block scales: a warp that reads every scale of a tile once, a few K groups before the TMA producer asks for the operands, so that the
+// Block scales: a warp that reads from every line of a tile's scales once, a few K groups before the TMA producer asks for the operands, so that the
 // epilogue finds it in L1.  An epilogue warp that runs behind has some 300 clocks between asking for a group's scales and using
 // them; a load that L1 misses takes 350 of a quiet L2 and 700 behind the operand tiles in flight, an L1 hit 110.  A hint: nothing waits
 // for it.  (prefetch.global.L1 comes as far as L2, a later load takes 280 clocks: a third of the gain.)
@@ -124,12 +124,15 @@ struct ScaleToucher {
     int q = 0;                                               // K groups behind this one
     // One tile: A's rows [row0, row0 + 128), B's columns from col0 on.  *requested: the K block the producer is at.  False: give up.
     __device__ __forceinline__ bool tile(const GemmParams& p, int b, int row0, int col0, int bn, int groups, int lane, volatile int* requested,
-                                         volatile int* abort_flag, int kb0 = 0) {
-        // a lane per 16 bytes of A's 128 rows, and per 128-column block of B that the tile may touch
-        const int row = row0 + lane * 4, blk = (col0 >> 7) + lane;
-        const float* pa = p.sfa + b * p.sfa_batch + static_cast<long long>(kb0) * p.sfa_stride + (row < p.m ? row : p.m - 1);
-        const bool col_ok = lane <= (bn + 127) / 128 && (blk << 7) < p.n;
-        const float* pb = p.sfb + b * p.sfb_batch + (col_ok ? static_cast<long long>(blk) * p.sfb_stride : 0) + kb0;
+                                         volatile int* abort_flag) {
+        // A: the lanes' rows are at most five apart and the first and the last of the 128 are among them, so that every 32-byte sector has
+        // one, wherever a group's scales begin.  B: two lanes for each 128-column block of the tile, the first and the last of the groups.
+        // (A lane per 16 bytes of A and per block of B missed a sector where a row of scales is not a whole number of them, us, best of 15:
+        // 16381 x 7168 x 8192 923.4 / 918.4; 16384 rows the same.)
+        const int row = row0 + lane * 127 / 31, blk = (col0 >> 7) + (lane >> 1);
+        const float* pa = p.sfa + b * p.sfa_batch + (row < p.m ? row : p.m - 1);
+        const bool col_ok = blk <= (col0 + bn - 1) >> 7 && (blk << 7) < p.n;
+        const float* pb = p.sfb + b * p.sfb_batch + (col_ok ? static_cast<long long>(blk) * p.sfb_stride : 0);
         bool go = true;
         for (int g = 0; g < groups && go; g += kBatch) {
             const int cnt = groups - g < kBatch ? groups - g : kBatch;
@@ -145,7 +148,7 @@ struct ScaleToucher {
 #pragma unroll
             for (int i = 0; i < kBatch; ++i)
                 if (i < cnt) x[i] = ld_nc_f32(pa + static_cast<long long>(g + i) * p.sfa_stride);
-            if (col_ok) x[kBatch] = ld_nc_f32(pb + g);
+            if (col_ok) x[kBatch] = ld_nc_f32(pb + g + (lane & 1 ? cnt - 1 : 0));
             q += cnt;
         }
         return go;
