@@ -59,26 +59,32 @@ def test_scale_rows_of_any_pitch(api, tile):
     check(api, 201, 256, 640, tile, pad=3)
 
 
-# Layers back to back, scales rewritten in the same memory each time: a pair kernel reads them into L1 ahead of their use, and must not
-# find there what they were in the layer before.  Against the same layers run one at a time.
-@pytest.mark.parametrize("m,n,k", [(600, 768, 640), (2309, 2048, 1152)])
-def test_scales_rewritten_between_layers(api, m, n, k):
+# Layers back to back, operand and scales written into the same memory each time, by the quantiser directly in front of the GEMM, whose CTAs may
+# be there while it writes: a warp or an epilogue that found a scale in L1 must not find what it was in the layer before.  Grids of many
+# rounds, of one, and so small that a layer's CTAs come while those of the one before are still at work; rows of scales that share
+# a sector with the next group's.  Against the same layers with a synchronisation after each launch.
+@pytest.mark.parametrize("tile", [4, 6, 7, 8, 2, 1, 0])
+@pytest.mark.parametrize("m,n,k", [(600, 768, 640), (2309, 2048, 1152), (129, 512, 512), (333, 7168, 2048)])
+def test_scales_rewritten_between_layers(api, m, n, k, tile):
     g = torch.Generator(device=DEV).manual_seed(m)
     w, sfb = api.quantize_128x128(torch.randn(n, k, generator=g, device=DEV))
     xs = [torch.randn(m, k, generator=g, device=DEV, dtype=torch.bfloat16) * 4.0 ** i for i in range(6)]
-    alone = []
-    for x in xs:
-        q, sfa = api.quantize_act_bf16_1x128(x)
-        alone.append(api.gemm_a8w8_blockscale(q, w, sfa, sfb, tile=4))
-        torch.cuda.synchronize()
     q, sfa = api.quantize_act_bf16_1x128(xs[0])
-    buf, where, chained = q.clone(), sfa.clone(), []
-    torch.cuda.synchronize()
-    for x in xs:
-        q, sfa = api.quantize_act_bf16_1x128(x)
-        buf.copy_(q)
-        where.copy_(sfa)
-        chained.append(api.gemm_a8w8_blockscale(buf, w, where, sfb, tile=4))
-    torch.cuda.synchronize()
+
+    def layers(sync):
+        outs = [torch.zeros(m, n, dtype=torch.bfloat16, device=DEV) for _ in xs]
+        torch.cuda.synchronize()
+        for x, out in zip(xs, outs):
+            api.quantize_act_bf16_1x128(x, q, sfa)
+            if sync:
+                torch.cuda.synchronize()
+            api.gemm_a8w8_blockscale(q, w, sfa, sfb, out=out, tile=tile)
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    alone, chained = layers(True), layers(False)
     assert api.last_status() == 0
     assert all(torch.equal(a, b) for a, b in zip(alone, chained))
+    assert not torch.equal(alone[0], alone[1])
