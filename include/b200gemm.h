@@ -155,7 +155,8 @@ int b200_gemm_a8w8_simple(const b200_gemm_args* args, void* cuda_stream);
  * device buffers owned by the library, runs the GEMM and copies C back; returns after the copy-back.
  * Device buffers are cached per device and grown on demand; b200_release() frees them.  Single-batch problems
  * with M >= 2048 (not MX) run as row slabs whose copy-back overlaps the next slab's upload and GEMM on a second,
- * library-owned stream; the call still returns only when all of C is on the host.
+ * library-owned stream; the call still returns only when all of C is on the host.  A slab is launched as a call of its own
+ * rows, which with TILE_AUTO decides the order of its K sums (see b200_gemm_check).
  * Pageable operands and results pass through a pinned ring of 24 MB per device, which up to eleven threads of the library
  * fill and empty (fewer where the process may use fewer CPUs); where there is no pinned memory the driver stages them.
  * Whatever the call returns, nothing of it is still running then: no copy touches the caller's memory any more.  A

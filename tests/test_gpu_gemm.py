@@ -278,8 +278,8 @@ def test_host_buffer_entry_point(api, O):
 
 @pytest.mark.parametrize("m", [2048, 2300, 4096])
 def test_host_buffer_entry_point_row_slabs(api, O, m):
-    """Large M: the host entry runs row slabs with the copy-back on a second stream.  Every row of C must arrive and
-    equal the device-resident result bit for bit (same kernels, same tiles within a slab boundary of 256 rows)."""
+    """Large M: the host entry runs row slabs with the copy-back on a second stream.  Every row of C must arrive.
+    (A slab is a call of its own with its own M, so the kind of tile, and for few tiles with a long K the order of its sums, are a slab's.)"""
     from gcnasm_b200 import _lib as L
 
     n, k = 640, 512
@@ -300,6 +300,21 @@ def test_host_buffer_entry_point_row_slabs(api, O, m):
     cu = np.zeros((m, n), np.float32)
     api.gemm_a8w8_host(a, b, cu)                                     # unscaled, fp32 out
     assert_close(O, cu[::53], O.gemm_ref_nt(a, b)[::53], "host slabs unscaled")
+
+
+def test_host_slabs_whose_tiles_are_split(api):
+    """Slabs of few tiles with a long K, each split over clusters, where the whole matrix has too many tiles for that.  Whole numbers of at
+    most 2: sums below 2^15, exact in any order, so the slabs' result is the exact one as the whole matrix's is."""
+    m, n, k = 2048, 640, 8192
+    g = torch.Generator(device=DEV).manual_seed(6)
+    x, y = (torch.randint(-2, 3, (rows, k), generator=g, device=DEV) for rows in (m, n))
+    a, b = api.cast_e4m3(x.float()), api.cast_e4m3(y.float())
+    want = (x.double() @ y.double().t()).float()
+    assert torch.equal(api.gemm_a8w8(a, b, out_dtype=torch.float32), want) and api.last_k_split() is None
+    c = np.full((m, n), np.nan, np.float32)
+    api.gemm_a8w8_host(a.cpu().numpy(), b.cpu().numpy(), c)
+    assert api.last_k_split() is not None
+    assert np.array_equal(c, want.cpu().numpy())
 
 
 def test_chained_launches_with_inputs_ready(api, O):
