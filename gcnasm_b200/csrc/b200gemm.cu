@@ -414,8 +414,12 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 }
             }
             // Few tiles with a long K: 128 x 128 tiles whose K is split may be the better ones (w as for a grid of one round).  A hint is
-            // another matter: who names a tile gets it whole, with the bits that every kind of whole tile gives.
-            if (!pair_only && !(a->flags & B200_GEMM_INPUTS_READY)) {
+            // another matter: who names a tile gets it whole, with the bits that every kind of whole tile gives.  Where inputs are ready a
+            // pair tile is kept, since it starts under its predecessor and a split one waits (in a chain, pair / split, us: 8-bit 256 x 512 x
+            // 8192 2.9 / 8.3, 256 x 4608 x 8192 10.6 / 14.1, block scales 3.0 / 9.1, 12.3 / 16.0); a whole single-CTA tile waits as well (whole /
+            // split: 8-bit 100 x 512 x 8192 15.1 / 7.4, MX 256 x 4608 x 8192 21.6 / 16.7, bf16 256 x 2048 x 4096 15.4 / 10.6).
+            const bool starts_early = (a->flags & B200_GEMM_INPUTS_READY) && hint != B200_TILE_128x128 && hint != B200_TILE_128x256;
+            if (!pair_only && !starts_early) {
                 int64_t equal;
                 const bool lines = a->stride_a % 128 == 0 && (a->b_layout == B200_B_FLAT_16x16 || a->stride_b % 128 == 0);
                 const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, lines, sm_count, &equal);

@@ -130,10 +130,10 @@ int b200_last_tail_split(int32_t* first_tile, int32_t* parts);
 /* Validates `args` exactly as b200_gemm_a8w8 would, without touching the GPU. Also reports the tile
  * configuration the launcher would pick (a b200_tile_hint value) when `chosen_tile` is not null.  That is the tile of a
  * launch in which a tile's K stays together, and as a hint it is computed just so: whole tiles, of whatever kind, sum K in one
- * order, so their results agree to the last bit.  With TILE_AUTO (inputs not ready) a grid of few tiles with a long K may be
- * computed on 128x128 tiles instead, each shared by the CTAs of a cluster that take a part of K: fp32 sums in another order, the
- * same from run to run.  Whether it is depends on the number of tiles, so with TILE_AUTO the last bits of a row can depend on how
- * many rows, columns and batches the call has.                                                                        */
+ * order, so their results agree to the last bit.  With TILE_AUTO a grid of few tiles with a long K may be computed on 128x128
+ * tiles instead, each shared by the CTAs of a cluster that take a part of K (if the inputs are ready, only where the whole tile
+ * would be a single CTA's: a pair's starts early): fp32 sums in another order, the same from run to run.  Whether it is depends
+ * on the number of tiles, so with TILE_AUTO the last bits of a row can depend on how many rows, columns and batches the call has. */
 int b200_gemm_check(const b200_gemm_args* args, int32_t* chosen_tile);
 /* The other half of that answer: how many CTAs share the K of a tile in this launch.  1: whole tiles of the kind that
  * b200_gemm_check reports (or the skinny-M kernel, which splits K by rules of its own).  2 to 8: 128x128 tiles, so many CTAs each.   */

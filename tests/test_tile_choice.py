@@ -51,15 +51,17 @@ def test_one_round(native, mode, m, n, k, tile):
     assert choice(native, m, n, k, mode) == tile
 
 
-# few tiles with a long K: the launch splits K, whatever kind of whole tile it would take; calls whose inputs are ready, slabs on their way, one
-# B for all batches and the skinny-M kernel do not
+# few tiles with a long K: the launch splits K, whatever kind of whole tile it would take; the skinny-M kernel has its own splits
 @pytest.mark.parametrize("mode,m,n,k,parts", [
     (L.SCALE_BLOCK, 256, 512, 4224, 7), (L.SCALE_BLOCK, 256, 512, 8192, 8), (L.SCALE_BLOCK, 1024, 1024, 8192, 2), (L.SCALE_BLOCK, 256, 512, 512, 1),
     (L.SCALE_NONE, 256, 512, 8192, 8), (L.SCALE_NONE, 256, 8192, 8192, 1), (L.SCALE_NONE, 256, 4608, 4096, 1), (L.SCALE_NONE, 256, 4608, 8192, 2),
+    (L.SCALE_NONE, 100, 512, 8192, 8), (L.SCALE_BLOCK, 100, 512, 8192, 8), (L.SCALE_MX, 256, 512, 8192, 8),
     (L.SCALE_BLOCK, 256, 4608, 4096, 2), (L.SCALE_MX, 256, 4608, 4096, 2), (L.SCALE_NONE, 16, 512, 8192, 1), (L.SCALE_NONE, 16, 520, 8192, 8)])
 def test_split_of_few_tiles(native, mode, m, n, k, parts):
     assert k_split(native, m, n, k, mode) == parts
-    assert k_split(native, m, n, k, mode, flags=L.GEMM_INPUTS_READY) == 1
+    # inputs that are ready: a pair tile starts early and stays, a whole tile of one CTA would wait as a split one does
+    early = choice(native, m, n, k, mode, flags=L.GEMM_INPUTS_READY) not in (ONE, ONE256)
+    assert k_split(native, m, n, k, mode, flags=L.GEMM_INPUTS_READY) == (1 if early else parts)
     assert k_split(native, m, n, k, mode, hint=ONE) == 1                # a tile that is asked for stays whole
 
 
