@@ -83,8 +83,9 @@ __device__ __forceinline__ bool mbar_probe(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 #define B200_EPI_WAIT(bar, ph, af, st, code) (mbar_probe(bar, ph) || mbar_wait<false, 0>(bar, ph, af, st, code))
-// The TMA producer thread sits on the scheduler that hosts no issuer (warp 1 issues, 1 and 2 did when this was measured; warp w runs on scheduler w % 4):
-// measured against warp 0, 1.5-2 % on the 4096 x 7168 x 2048 and 16384 x 7168 x 8192 problems, nothing on 8192^3.
+// The TMA producer thread: which of the free role warps it is (1 issues, one reads scales ahead; warp w runs on scheduler w % 4) does not
+// show any more.  Producer and reader on warps 3 and 0 / 2 and 0 / 0 and 3 / 2 and 3 / 0 and 2, us: block scales 16384 x 7168 x 8192 912 / 919 / 918 /
+// 920 / 918, 4096 x 7168 x 2048 60.8 / 60.7 / 60.6 / 60.8 / 60.7; unscaled 8192^3 456 each.  (With two polling issuers warp 3 had been worth 1.5-2 %.)
 static constexpr int kProducerWarp = 3;
 
 // Building with -DB200_TRACE records clock64() stamps of the hand-offs of the first CTA pair into g_trace

@@ -109,10 +109,8 @@ __device__ __forceinline__ uint32_t mbar_try_wait_cluster(uint32_t bar, uint32_t
 
 // Bounded wait.  `abort_flag` is a CTA-shared int; `status` the device status word.  The fast path is a
 // bare try_wait loop (each try_wait already suspends the thread for a hardware-defined interval); only a
-// wait that has failed many times starts reading the wall clock and checking the abort flag.
-// kBackoffNs > 0 makes a waiting thread sleep between polls: the single-thread producer and MMA-issuer
-// roles use it so that their polling does not take issue slots from the epilogue warps that share their
-// scheduler.
+// wait that has failed many times starts reading the wall clock and checking the abort flag.  The issuers and the epilogue
+// warps wait like this.  kBackoffNs > 0: sleep between the tries (nobody's choice at present).
 template <bool kClusterScope = false, int kBackoffNs = 0>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code, unsigned long long budget_ns = kWaitBudgetNs) {
@@ -135,9 +133,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
-// Polling wait (mbarrier.test_wait never suspends the thread): for the latency-critical hand-offs between
-// the MMA issuer and the epilogue warps.  A suspended try_wait was observed to wake late when another
-// thread on the same scheduler is itself waiting on a different barrier.
+// Polling wait (mbarrier.test_wait never suspends the thread), kBackoffNs of sleep between the polls: the TMA producers of the pair and
+// the skinny-M kernel, single threads that are stages ahead.  Not for an issuer, a whole warp, whose polling takes issue slots from the
+// epilogue warps of its scheduler (the pair kernel's waits have the figures).
 template <bool kClusterScope = false, int kBackoffNs = 0>
 __device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                int* status, int code, unsigned long long budget_ns = kWaitBudgetNs) {
