@@ -40,7 +40,7 @@ def k_split(native, *problem, bf16=False, **more):
 ONE, ONE256, PAIR256, PAIR128, PAIR224 = L.TILE_128x128, L.TILE_128x256, L.TILE_PAIR_256x256, L.TILE_PAIR_256x128, L.TILE_PAIR_256x224
 
 
-# a grid of one round: with block scales and few tiles a long K is the pair's, without scales never; 256 columns are for a short K
+# a grid of one round, whole tiles: with block scales and few tiles a long K is the pair's, without scales never; 256 columns are for a short K
 @pytest.mark.parametrize("mode,m,n,k,tile", [
     (L.SCALE_BLOCK, 256, 512, 512, ONE), (L.SCALE_BLOCK, 256, 512, 4096, ONE), (L.SCALE_BLOCK, 256, 512, 4224, PAIR128),
     (L.SCALE_BLOCK, 256, 512, 8192, PAIR128), (L.SCALE_BLOCK, 1024, 1024, 8192, PAIR128), (L.SCALE_BLOCK, 2048, 1024, 8192, ONE),
