@@ -74,14 +74,8 @@ struct PairCfg {
 // through the async proxy (TMA complete_tx, tcgen05.commit) or tcgen05.fence, not through generic memory.
 #define B200_PROD_WAIT mbar_wait_poll<false, 64>
 #define B200_MMA_WAIT mbar_wait<false, 0>
-// One non-suspending look at the barrier before the suspending wait: an epilogue warp that runs behind finds the phase
-// already complete (measured: 0.7 % on 256 x 256 tiles, 4 % on the 224- and 192-column tiles).
-__device__ __forceinline__ bool mbar_probe(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
+// One non-suspending look before the suspending wait: an epilogue warp that runs behind finds the phase already complete
+// (measured: 0.7 % on 256 x 256 tiles, 4 % on the 224- and 192-column tiles).
 #define B200_EPI_WAIT(bar, ph, af, st, code) (mbar_probe(bar, ph) || mbar_wait<false, 0>(bar, ph, af, st, code))
 // The TMA producer thread: which of the free role warps it is (1 issues, one reads scales ahead; warp w runs on scheduler w % 4) does not
 // show any more.  Producer and reader on warps 3 and 0 / 2 and 0 / 0 and 3 / 2 and 3 / 0 and 2, us: block scales 16384 x 7168 x 8192 912 / 919 / 918 /

@@ -7,7 +7,8 @@
 // One persistent CTA per SM, 12 warps:
 //   warp 0      TMA producer   (one elected lane)  global -> shared ring, mbarrier complete_tx
 //   warp 1      UMMA issuer    (one elected lane)  tcgen05.mma kind::f8f6f4 / kind::mxf8f6f4, TMEM alloc
-//   warp 2      block scales, 256 columns: reads the scales into L1 ahead of their use (ScaleToucher)
+//   warp 2      block scales: brings the scales into shared memory beside the operands (128 columns), or reads them into L1 ahead of
+//               their use (256 columns, ScaleToucher)
 //   warp 3      idle, as warp 2 otherwise (register re-allocation works on whole warpgroups)
 //   warps 4-11  epilogue: TMEM -> registers -> scale -> global
 // TMEM holds two accumulator buffers of BN columns (four with block scales and BN = 128).  Per-tensor / unscaled / MX modes accumulate a
@@ -80,6 +81,7 @@ template <int BN_, int MODE_, int BLAYOUT_, bool SPLIT_ = false>
 struct GemmCfg {
     static constexpr bool SPLIT = SPLIT_;                           // a tile's K is split over a cluster
     static constexpr bool TOUCH = MODE_ == MODE_BLOCK && BN_ == 256;   // a warp reads the scales ahead of their use
+    static constexpr bool FEED = MODE_ == MODE_BLOCK && BN_ == 128;    // a warp brings the scales into shared memory beside the operands
     static constexpr bool AB16 = MODE_ == MODE_ACC16;               // bf16 operands: same bytes, kind::f16 MMAs
     static constexpr int BM = 128, BN = BN_, BK = 128, MODE = AB16 ? MODE_ACC : MODE_, BLAYOUT = BLAYOUT_;
     static constexpr int A_BYTES = BM * BK;
@@ -89,16 +91,23 @@ struct GemmCfg {
     static constexpr int SFB_BYTES = (MODE == MODE_MX) ? SFB_ATOMS * 512 : 0;
     static constexpr int STAGE_BYTES = ((A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES + 1023) / 1024) * 1024;
     static constexpr int OUT_STAGE_BYTES = 8 * kOutStageBytesPerWarp;        // store staging of the eight epilogue warps
-    static constexpr int ROOM = 227 * 1024 - 1024 /*barriers*/ - 1024 /*alignment slack*/;
+    // FEED: scales of so many K blocks, each the tile's rows of A and its block of B.  Eight warps that load the scales themselves wait for them
+    // however early they ask: a load queues behind all the operand tiles in flight, 200 KB a CTA.  Six register sets, requested six groups
+    // ahead / a ring that fills with the operands (and so with a stage less of those), us: 333 x 5120 x 2048 9.0 / 7.9, 128 x 8192 x 8192 23.9 / 20.1 (no
+    // loads at all 19.7), 512 x 4096 x 4096 13.9 / 12.0, 1024 x 1024 x 512 4.26 / 4.11, 2500 x 5120 x 3072 53.8 / 48.7.  Also tried on 128 x 8192 x 8192: the
+    // reading-ahead warp of the 256 columns 22.8, register sets of 8 and 16 groups loaded together 23.7, 22.0.  On 256 columns the epilogue's
+    // registers do not take it (spills, 333 x 7168 x 2048 12.0 / 15.2).
+    static constexpr int SF_SLOTS = FEED ? 16 : 0, SF_SLOT_BYTES = (BM + 4) * 4;
+    static constexpr int ROOM = 227 * 1024 - 1024 /*barriers*/ - 1024 /*alignment slack*/ - SF_SLOTS * SF_SLOT_BYTES;
     static constexpr int STAGES = (ROOM - OUT_STAGE_BYTES) / STAGE_BYTES;           // ring with the staging behind it
-    // Ring of a CTA with one tile, whose staging lies in the ring: 128 columns without MX scales seven stages instead of six.  Behind six
+    // Ring of a CTA with one tile, whose staging lies in the ring: 128 columns without block or MX scales seven stages instead of six.  Behind six
     // of them a long K waits for its operands, us, six / seven: 8-bit 128 x 8192 x 8192 19.8 / 18.4, 512 x 4096 x 4096 11.6 / 11.0, bf16
     // 128 x 8192 x 8192 35.1 / 33.0.  CTAs with several tiles keep the staging of its own: the next tile's loads are under way while
     // a result leaves, and stores from registers instead cost more than the stage gives (2500 x 5120 x 3072 45.0 / 41.5).
     static constexpr int STAGES_ONE = ROOM / STAGE_BYTES;
     static constexpr int STAGING_END = STAGES * STAGE_BYTES + OUT_STAGE_BYTES;
     static constexpr int RING_BYTES = STAGES_ONE * STAGE_BYTES > STAGING_END ? STAGES_ONE * STAGE_BYTES : STAGING_END;
-    static constexpr int SMEM_BYTES = RING_BYTES + 1024 /*barriers*/ + 1024 /*alignment slack*/;
+    static constexpr int SMEM_BYTES = RING_BYTES + 1024 /*barriers*/ + SF_SLOTS * SF_SLOT_BYTES + 1024 /*alignment slack*/;
     // accumulator buffers; 128 columns with block scales, a hand-off per K block: as many as tensor memory holds
     static constexpr int BUFS = (MODE == MODE_BLOCK && BN == 128) ? 4 : 2;
     static constexpr int ACC_COLS = BUFS * BN;
@@ -110,6 +119,8 @@ struct GemmCfg {
     static_assert(ACC_COLS + SF_COLS <= 512, "TMEM overflow");
     static_assert(BN % 32 == 0 && BN <= 256, "BN must be a multiple of 32, at most 256");
     static_assert(STAGES >= 3 && STAGES_ONE <= 8, "ring depth");
+    // a stage that is free says that the group STAGES + BUFS before its next one has been drained
+    static_assert(!FEED || STAGES_ONE + BUFS <= SF_SLOTS, "scales stay until their group has been drained");
     static_assert(OUT_STAGE_BYTES <= STAGES * STAGE_BYTES, "the staging fits the ring");
     static_assert(!SPLIT || (BN == 128 && BM * BN * 4 <= RING_BYTES), "the partial sums fit the ring");
 };
@@ -345,6 +356,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * Cfg::STAGES_ONE + 2 * BUFS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* requested = reinterpret_cast<volatile int*>(tmem_slot + 2);    // TOUCH: the K block the TMA producer is at
+    const uint32_t sf0 = smem_base + Cfg::RING_BYTES + 1024;                     // FEED: the scales
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -356,7 +368,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < Cfg::STAGES_ONE; ++s) {
-            mbar_init(bar_full0 + s * 8, 1);
+            mbar_init(bar_full0 + s * 8, Cfg::FEED ? 33 : 1);    // FEED: and every lane of the feeding warp
             mbar_init(bar_empty0 + s * 8, 1);
         }
         for (int s = 0; s < BUFS; ++s) {
@@ -438,17 +450,19 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             // ------------------------------ UMMA issuer (the warp; an elected lane issues) ------------
             const bool elected = elect_one() != 0;
             uint32_t s = 0, ph = 0, phase = 0;
-            bool ok = true;
+            // Block scales, two waits a K block: both barriers of the next one are looked at ahead of this one's MMAs, so that a wait that is over costs
+            // nothing then.  Without / with, us: 333 x 5120 x 2048 9.0 / 8.6, 512 x 4096 x 4096 14.0 / 13.5, 256 x 2048 x 8192 12.1 / 11.6; unscaled 10.3 / 10.5,
+            // the pair kernel 21.3 / 26.5 (256 x 512 x 8192): there the next operands or buffer are seldom ready yet.
+            bool ok = true, full_seen = false, free_seen = false;
             constexpr uint32_t idesc = make_idesc_f8(BM, BN);
             for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
                 for (int g = 0; g < groups && ok; ++g, ++phase) {
                     const uint32_t as = phase % BUFS;
                     const uint32_t aph = (phase / BUFS) & 1;
-                    if (!role_all<true>(mbar_wait(bar_acce0 + as * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
+                    if (!role_all<true>(free_seen) && !role_all<true>(mbar_wait(bar_acce0 + as * 8, aph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_ACC_E))) {
                         ok = false;
                         break;
                     }
-                    tc_fence_after();
                     const uint32_t tacc = tmem_base + as * BN;
                     for (int kb = 0; kb < kb_per_group; ++kb, next_stage(s, ph)) {
                         // The descriptors are formed before the wait, so that the MMAs follow it at once.  Behind it / before it, us, 128 x 128
@@ -461,9 +475,15 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         uint64_t db0 = Cfg::BLAYOUT == BL_NK ? make_smem_desc(sb, 16, 1024, kSwizzle128B) : make_smem_desc(sb, LBO, 128, kSwizzleNone);
                         uint64_t dsf0 = make_smem_desc(sb + Cfg::B_BYTES, 0, 128, kSwizzleNone);                 // MX
                         asm volatile("" : "+l"(da0), "+l"(db0), "+l"(dsf0));
-                        if (!role_all<true>(mbar_wait(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
+                        if (!role_all<true>(full_seen) && !role_all<true>(mbar_wait(bar_full0 + s * 8, ph, abort_flag, p.status, KSTAT_TIMEOUT_FULL))) {
                             ok = false;
                             break;
+                        }
+                        if constexpr (MODE == MODE_BLOCK) {
+                            uint32_t s1 = s, ph1 = ph;
+                            next_stage(s1, ph1);
+                            full_seen = mbar_probe(bar_full0 + s1 * 8, ph1);
+                            free_seen = mbar_probe(bar_acce0 + (phase + 1) % BUFS * 8, (((phase + 1) / BUFS) & 1) ^ 1);
                         }
                         tc_fence_after();
                         if (!elected) continue;
@@ -503,6 +523,37 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     go = touch.tile(p, b, mi * BM, ni * BN, BN, groups, lane, requested, abort_flag);
                 }
                 touch.finish(requested);
+            }
+        }
+        if constexpr (Cfg::FEED) {
+            if (warp == 2) {
+                // ------------------------------ scales into shared memory (the warp) ------------------------------
+                // Four-byte copies, since a row of scales begins anywhere; they count towards the stage's full barrier, and whoever then sees the
+                // group's accumulator sees its scales.
+                uint32_t s = 0, ph = 0, it = 0;
+                bool ok = true;
+                for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
+                    int b, mi, ni;
+                    tile_coords(p, t, b, mi, ni);
+                    const float* pa = p.sfa + b * p.sfa_batch + static_cast<long long>(kb0) * p.sfa_stride;
+                    int row[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) row[j] = mi * BM + j * 32 + lane < p.m ? mi * BM + j * 32 + lane : p.m - 1;
+                    const float* pb = p.sfb + b * p.sfb_batch + static_cast<long long>(ni) * p.sfb_stride + kb0;
+                    for (int kb = 0; kb < kblocks; ++kb, ++it, next_stage(s, ph)) {
+                        if (!role_all<true>(mbar_wait(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY))) {
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t slot = sf0 + it % Cfg::SF_SLOTS * Cfg::SF_SLOT_BYTES;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) cp_async_4(slot + (j * 32 + lane) * 4, pa + row[j]);
+                        if (lane == 0) cp_async_4(slot + BM * 4, pb + kb);
+                        cp_async_arrive(bar_full0 + s * 8);
+                        pa += p.sfa_stride;
+                    }
+                }
+                cp_async_wait_all();
             }
         }
         if constexpr (Cfg::SPLIT) {
@@ -568,55 +619,30 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 // four buffers keep the tensor core busy meanwhile.  Two buffers, handed back after the FMAs, scalar FMAs and stores
                 // from registers / this loop and staged stores, us: 100 x 7168 x 2048 10.6 / 9.2, 200 x 7168 x 2048 11.3 / 9.6, 512 x 4096 x
                 // 4096 16.8 / 15.0, 2500 x 5120 x 3072 77 / 59.
-                // Scales are requested six groups ahead, into six register sets that take turns (a copy from one to the
-                // other would wait for the load): a load queues behind the operand tiles in flight, and with the tensor core four buffers
-                // ahead there are more of those than with two.  Two / four / six / eight ahead, us: 128 x 8192 x 8192 32.8 / 27.8 / 25.6 /
-                // 25.1 (scalar FMAs, two buffers, one ahead: 31.4), 256 x 512 x 8192 27.2 / 24.5 / 23.6 / 23.6, 1024 x 1024 x 512 4.80 /
-                // 4.85 / 4.89 / 4.90; the loop's code grows with the sets.
                 unsigned long long acc2[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc2[j] = 0ull;
-                const float* sfa_p = p.sfa + b * p.sfa_batch + static_cast<long long>(kb0) * p.sfa_stride + (row < p.m ? row : 0);
-                const float* sfb_p = p.sfb + b * p.sfb_batch + static_cast<long long>(col_base / 128) * p.sfb_stride + kb0;
-                const bool col_ok = col_base < p.n;
-                constexpr int SETS = 6;
-                float sa[SETS], sb[SETS];
-                auto request = [&](const int set) {
-                    sa[set] = __ldg(sfa_p);
-                    sb[set] = col_ok ? __ldg(sfb_p) : 0.0f;
-                    sfa_p += p.sfa_stride;
-                    ++sfb_p;
-                };
-#pragma unroll
-                for (int set = 0; set < SETS; ++set)
-                    if (set < groups) request(set);
-                for (int g0 = 0; g0 < groups && ok; g0 += SETS) {
-#pragma unroll
-                    for (int set = 0; set < SETS; ++set) {
-                        const int g = g0 + set;
-                        if (g >= groups) break;
-                        const uint32_t as = phase % BUFS;
-                        const uint32_t aph = (phase / BUFS) & 1;
-                        if (!mbar_wait(bar_accf0 + as * 8, aph, abort_flag, p.status, KSTAT_TIMEOUT_ACC_F)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
-                        float v[64];
-                        tmem_ld32(taddr, v);
-                        tmem_ld32(taddr + 32, v + 32);
-                        const float sc = sa[set] * sb[set];
-                        const unsigned long long sc2 = pack_f32x2(sc, sc);
-                        tmem_ld_wait();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
-                        if (g + SETS < groups) request(set);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) acc2[j] = ffma2(pack_f32x2(v[2 * j], v[2 * j + 1]), sc2, acc2[j]);
-                        ++phase;
+                for (int g = 0; g < groups; ++g, ++phase) {
+                    const uint32_t as = phase % BUFS;
+                    const uint32_t aph = (phase / BUFS) & 1;
+                    if (!mbar_wait(bar_accf0 + as * 8, aph, abort_flag, p.status, KSTAT_TIMEOUT_ACC_F)) {
+                        ok = false;
+                        break;
                     }
+                    tc_fence_after();
+                    const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
+                    float v[64];
+                    tmem_ld32(taddr, v);
+                    tmem_ld32(taddr + 32, v + 32);
+                    const uint32_t slot = sf0 + phase % Cfg::SF_SLOTS * Cfg::SF_SLOT_BYTES;
+                    const float sc = ld_shared_f32(slot + row_in_tile * 4) * ld_shared_f32(slot + BM * 4);
+                    const unsigned long long sc2 = pack_f32x2(sc, sc);
+                    tmem_ld_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) acc2[j] = ffma2(pack_f32x2(v[2 * j], v[2 * j + 1]), sc2, acc2[j]);
                 }
                 if (ok) {
 #pragma unroll

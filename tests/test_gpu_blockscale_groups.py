@@ -54,6 +54,24 @@ def test_groups_across_tiles(api, tile, m, n, groups):
     check(api, m, n, 128 * groups, tile)
 
 
+# 128 columns: the scales go through a ring of sixteen groups, which begins again within a tile, at a tile's end and in a shared tile's
+# parts.  Rows of scales that begin anywhere.  Every sum is a multiple of 2^-5; with magnitudes that add up to less than 2^19 it takes 24 bits.
+@pytest.mark.parametrize("m,n,groups", [(129, 256, 15), (129, 256, 16), (131, 256, 17), (130, 256, 37), (1, 128, 40), (1601, 1664, 18)])
+@pytest.mark.parametrize("tile", [1, 0])
+def test_ring_of_scales_begins_again(api, m, n, groups, tile):
+    a, b, sfa, sfb, ref = problem(m, n, 128 * groups, m + groups, pad=1)
+    decode = torch.zeros(256, device=DEV, dtype=torch.float64)
+    for v, byte in E4M3.items():
+        decode[byte] = abs(v)
+    size = sum((decode[a[:, i:i + 128].long()] * sfa[i // 128].double()[:, None]) @
+               (decode[b[:, i:i + 128].long()] * sfb[:, i // 128].double().repeat_interleave(128)[:, None]).t() for i in range(0, 128 * groups, 128))
+    assert size.max() < 2 ** 19
+    c = api.gemm_a8w8_blockscale(a, b, sfa, sfb, out_dtype=torch.float32, tile=tile)
+    torch.cuda.synchronize()
+    assert api.last_status() == 0
+    assert torch.equal(c.double(), ref)
+
+
 @pytest.mark.parametrize("tile", [4, 1])
 def test_scale_rows_of_any_pitch(api, tile):
     check(api, 201, 256, 640, tile, pad=3)
