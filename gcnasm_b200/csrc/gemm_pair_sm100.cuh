@@ -478,10 +478,10 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) unpack_f32x2(acc_t[c * 16 + j], o[2 * j], o[2 * j + 1]);
                 if (p.out_dtype == OUT_BF16) {
-                    store_chunk_coalesced<32>(p, cbatch, out_stage, row0, col_first + c * 32, o, lane, vec_ok);
+                    store_chunk_coalesced<32, false>(p, cbatch, out_stage, row0, col_first + c * 32, o, lane, vec_ok);
                 } else {
-                    store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col_first + c * 32, o, lane, vec_ok);
-                    store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col_first + c * 32 + 16, o + 16, lane, vec_ok);
+                    store_chunk_coalesced<16, false>(p, cbatch, out_stage, row0, col_first + c * 32, o, lane, vec_ok);
+                    store_chunk_coalesced<16, false>(p, cbatch, out_stage, row0, col_first + c * 32 + 16, o + 16, lane, vec_ok);
                 }
             }
             return true;
@@ -682,20 +682,21 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
 #endif
                 } else if (ok) {
                     // 64-byte row segments: 32 columns of bf16 or 16 columns of fp32 per pass
+                    constexpr bool kRagged = NCH % 32 != 0;      // N is a multiple of 128, a chunk begins at a multiple of its width otherwise
                     if (p.out_dtype == OUT_BF16) {
 #pragma unroll
                         for (int c = 0; c + 1 < NCH / 16; c += 2) {
                             float o[32];
 #pragma unroll
                             for (int j = 0; j < 16; ++j) unpack_f32x2(acc[c * 8 + j], o[2 * j], o[2 * j + 1]);
-                            store_chunk_coalesced<32>(p, cbatch, out_stage, row0, col_base + c * 16, o, lane, vec_ok);
+                            store_chunk_coalesced<32, kRagged>(p, cbatch, out_stage, row0, col_base + c * 16, o, lane, vec_ok);
                         }
                         if ((NCH / 16) & 1) {
                             constexpr int c = NCH / 16 - 1;
                             float o[16];
 #pragma unroll
                             for (int j = 0; j < 8; ++j) unpack_f32x2(acc[c * 8 + j], o[2 * j], o[2 * j + 1]);
-                            store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col_base + c * 16, o, lane, vec_ok);
+                            store_chunk_coalesced<16, kRagged>(p, cbatch, out_stage, row0, col_base + c * 16, o, lane, vec_ok);
                         }
                     } else {
 #pragma unroll
@@ -703,7 +704,7 @@ gemm_a8w8_pair_sm100_kernel(const __grid_constant__ GemmParams p) {
                             float o[16];
 #pragma unroll
                             for (int j = 0; j < 8; ++j) unpack_f32x2(acc[c * 8 + j], o[2 * j], o[2 * j + 1]);
-                            store_chunk_coalesced<16>(p, cbatch, out_stage, row0, col_base + c * 16, o, lane, vec_ok);
+                            store_chunk_coalesced<16, kRagged>(p, cbatch, out_stage, row0, col_base + c * 16, o, lane, vec_ok);
                         }
                     }
                 }

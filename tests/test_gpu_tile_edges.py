@@ -83,3 +83,16 @@ def test_k_blocks_against_the_ring(api, mode, tile, kblocks):
     check(api, mode, 200, 512, k, tile)
     if kblocks in (1, 5, 6, 7, 8, 13):
         check(api, mode, 1400, 3840, k, tile)              # 330 tiles of 128 x 128, 165 of 128 x 256
+
+
+# columns of the last chunk of 32 (or 16): 16-byte pieces that are whole, and single elements behind them
+@pytest.mark.parametrize("mode,tile", [("none", 1), ("none", 2), ("none", 4), ("none", 6), ("none", 7), ("none", 8), ("mx", 1), ("mx", 4), ("bf16", 1), ("bf16", 2), ("bf16", 4)])
+@pytest.mark.parametrize("n", [1, 3, 4, 7, 8, 9, 12, 16, 20, 23, 24, 31, 32, 33, 40, 63, 120, 250, 509])
+def test_columns_of_a_chunk(api, mode, tile, n):
+    check(api, mode, 140, n, 128, tile, around=True)
+
+
+# block scales on 224-column pair tiles, whose chunks begin at any multiple of 16
+@pytest.mark.parametrize("n", [128, 256, 384, 512, 640, 896, 1024])
+def test_columns_of_a_chunk_with_block_scales(api, n):
+    check(api, "block", 140, n, 256, 7, around=True)
