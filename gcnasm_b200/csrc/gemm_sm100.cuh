@@ -188,40 +188,49 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int t, int& b, 
     ni = in_grp / rows;
 }
 
-// Store CNT consecutive output columns of one row, 16 bytes at a time where the address allows (vec_ok) and the columns are there.  Element by
-// element wherever one of the CNT columns is missing / so, bf16, us: 4000 x 4088 x 512 18.7 / 13.7, 100 x 2040 x 1024 9.2 / 7.0, MX 2000 x 2040 x
-// 1024 11.0 / 8.6, bf16 operands 2000 x 4040 x 512 11.6 / 11.15; fp32, whose elements are 4 bytes, the same (20.1).
+// Store CNT consecutive output columns of one row, 16 bytes at a time where the address allows (vec_ok) and the columns are there.  bf16, element by
+// element wherever one of the CNT columns is missing / by whole pieces, us: 4000 x 4088 x 512 18.7 / 13.7, 100 x 2040 x 1024 9.2 / 7.0, MX 2000 x
+// 2040 x 1024 11.0 / 8.6, bf16 operands 2000 x 4040 x 512 11.6 / 11.15.  fp32 gains nothing by pieces (4000 x 4072 x 512 20.1), and a chunk that is all there
+// has its own branch: both cost few rows their code (3 x 3592 x 256, fp32, 3.0 / 3.25).
 template <int CNT>
 __device__ __forceinline__ void store_row_chunk(const GemmParams& p, void* crow, int col0, const float* v,
                                                 bool vec_ok) {
+    const bool whole = vec_ok && col0 + CNT <= p.n;
     if (p.out_dtype == OUT_BF16) {
         __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(crow) + col0;
+        auto piece = [&](const int j) {
+            uint4 w;
+            w.x = pack_bf16x2(v[j + 0], v[j + 1]);
+            w.y = pack_bf16x2(v[j + 2], v[j + 3]);
+            w.z = pack_bf16x2(v[j + 4], v[j + 5]);
+            w.w = pack_bf16x2(v[j + 6], v[j + 7]);
+            *reinterpret_cast<uint4*>(dst + j) = w;
+        };
+        if (whole) {
 #pragma unroll
-        for (int j = 0; j < CNT; j += 8) {
-            if (vec_ok && col0 + j + 8 <= p.n) {
-                uint4 w;
-                w.x = pack_bf16x2(v[j + 0], v[j + 1]);
-                w.y = pack_bf16x2(v[j + 2], v[j + 3]);
-                w.z = pack_bf16x2(v[j + 4], v[j + 5]);
-                w.w = pack_bf16x2(v[j + 6], v[j + 7]);
-                *reinterpret_cast<uint4*>(dst + j) = w;
-            } else {
+            for (int j = 0; j < CNT; j += 8) piece(j);
+        } else {
 #pragma unroll
-                for (int i = j; i < j + 8; ++i)
-                    if (col0 + i < p.n) dst[i] = __float2bfloat16_rn(v[i]);
+            for (int j = 0; j < CNT; j += 8) {
+                if (vec_ok && col0 + j + 8 <= p.n) {
+                    piece(j);
+                } else {
+#pragma unroll
+                    for (int i = j; i < j + 8; ++i)
+                        if (col0 + i < p.n) dst[i] = __float2bfloat16_rn(v[i]);
+                }
             }
         }
     } else {
         float* dst = reinterpret_cast<float*>(crow) + col0;
+        if (whole) {
 #pragma unroll
-        for (int j = 0; j < CNT; j += 4) {
-            if (vec_ok && col0 + j + 4 <= p.n) {
+            for (int j = 0; j < CNT; j += 4)
                 *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            } else {
+        } else {
 #pragma unroll
-                for (int i = j; i < j + 4; ++i)
-                    if (col0 + i < p.n) dst[i] = v[i];
-            }
+            for (int j = 0; j < CNT; ++j)
+                if (col0 + j < p.n) dst[j] = v[j];
         }
     }
 }
