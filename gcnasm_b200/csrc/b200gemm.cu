@@ -864,7 +864,7 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
     else
         rc = make_flat_tmap(&p.tmap_w, a->ptr_b, a->n, a->k, a->batch, a->stride_b_batch, 128);
     if (rc) return rc;
-    rc = make_rowmajor_tmap(&p.tmap_x, a->ptr_a, a->m, a->k, a->stride_a, a->batch, a->stride_a_batch, pl.mt);
+    rc = make_rowmajor_tmap(&p.tmap_x, a->ptr_a, a->m, a->k, a->stride_a, a->batch, a->stride_a_batch, static_cast<uint32_t>(a->m));
     if (rc) return rc;
     p.c = a->ptr_c;
     p.sfa = static_cast<const float*>(a->ptr_sfa);
@@ -909,6 +909,14 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
     return B200_OK;
 }
 
+// Up to so many rows, A's box is of the rows that there are (what lies behind them in a stage is anything, and so are the rows of the
+// accumulator that nobody stores).  A box that reaches beyond the matrix is filled with zeros, but each row that is not there still
+// costs a request, all of them in few places of L2: boxes of 128 rows in a ring of six on 144 CTAs take 918 clocks each with one row there,
+// 806 with 24, 522 with 32 and more; boxes of 16 rows with one there 522.  128 rows / the rows there are, us: bf16 1 x 5440 x 1792 11.7 / 8.8, 16 x 5440 x
+// 2048 10.6 / 8.2, 4 x 8192 x 4096 18.9 / 14.5, 8-bit 5 x 5448 x 4096 10.5 / 7.9; 40 x 5440 x 2048 the same, 1 x 1024 x 1024 (8 tiles) 5.4 / 5.55.  The few rows
+// of a last tile below others are not worth a second box: its CTAs are half of a grid at most (8-bit 140 x 8192 x 2048 6.4 / 6.45).
+constexpr int kBoxRows = 64;
+
 int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStream_t st, bool ab16 = false) {
     int BN = 128;
     bool pair = false;
@@ -933,7 +941,8 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     const int BROWS = pair ? BN / 2 : BN;             // B rows one CTA loads
     GemmParams p;
     std::memset(&p, 0, sizeof(p));
-    int rc = make_rowmajor_tmap(&p.tmap_a, a->ptr_a, a->m, a->k, a->stride_a, a->batch, a->stride_a_batch, 128);
+    p.a_rows = !pair && a->m <= kBoxRows ? static_cast<int>(a->m) : 128;
+    int rc = make_rowmajor_tmap(&p.tmap_a, a->ptr_a, a->m, a->k, a->stride_a, a->batch, a->stride_a_batch, static_cast<uint32_t>(p.a_rows));
     if (rc) return rc;
     const bool b_shared = a->batch > 1 && a->stride_b_batch == 0;      // one B for every batch (validate(): pair tiles)
     const int64_t b_batches = b_shared ? 1 : a->batch;

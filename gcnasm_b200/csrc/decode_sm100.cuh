@@ -28,7 +28,7 @@ namespace b200 {
 
 struct DecodeParams {
     CUtensorMap tmap_w;          // weights: 3-D [batch][N][K] swizzled, or the 4-D flat view
-    CUtensorMap tmap_x;          // tokens:  3-D [batch][M][K], box 128 x MT, 128-byte swizzle
+    CUtensorMap tmap_x;          // tokens:  3-D [batch][M][K], box 128 x M, 128-byte swizzle (what lies in a stage behind the M tokens is anything)
     void* c;
     float* partial;              // split-K workspace [splits][batch][M][N] fp32, or null: the splits of a panel are a cluster
     const float* sfa;            // MX: the atoms (bytes), as are sfb and, in atoms and bytes, the strides
@@ -55,8 +55,7 @@ struct DecodeCfg {
     static constexpr int W_BYTES = BNW * BK;
     static constexpr int X_BYTES = MT * BK;
     static constexpr int SF_BYTES = MODE == MODE_MX ? 1024 : 0;     // MX: the atom of the weight rows, then that of the tokens
-    static constexpr int LOAD_BYTES = W_BYTES + X_BYTES + SF_BYTES;
-    static constexpr int STAGE_BYTES = ((LOAD_BYTES + 1023) / 1024) * 1024;
+    static constexpr int STAGE_BYTES = ((W_BYTES + X_BYTES + SF_BYTES + 1023) / 1024) * 1024;
     // combined scales [K groups of this CTA][MT]; problems whose groups do not fit are split along K by the launcher
     static constexpr int SF_SMEM = MODE == MODE_MX ? 0 : decode_sf_bytes(MT_);
     static constexpr int STAGES_RAW = (225 * 1024 - 1024 - SF_SMEM) / STAGE_BYTES;
@@ -118,6 +117,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
     // long (18432 x 7168).
     pdl_launch_dependents();
     const int first = nkb < STAGES ? nkb : STAGES;
+    const uint32_t load_bytes = Cfg::W_BYTES + p.m * BK + Cfg::SF_BYTES;
     // MX: atom (kb, 128-row block) of an image [batch][K/128][rows/128][512 B]
     auto mx_atom = [&](const float* image, long long batch_bytes, long long blocks, int kb, int blk) {
         return reinterpret_cast<const uint8_t*>(image) + b * batch_bytes + (static_cast<long long>(kb) * blocks + blk) * 512;
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
     auto request_weights = [&](int i) {
         const uint32_t sw = smem_base + i * Cfg::STAGE_BYTES;
         const uint32_t full = bar_full0 + i * 8;
-        mbar_arrive_expect_tx(full, Cfg::LOAD_BYTES);
+        mbar_arrive_expect_tx(full, load_bytes);
         if constexpr (Cfg::BLAYOUT == BL_NK)
             tma_load_3d(sw, &p.tmap_w, full, (kb0 + i) * BK, ni * BNW, b);
         else
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) decode_a8w8_sm100_kernel(cons
                 const uint32_t sw = smem_base + s * Cfg::STAGE_BYTES;
                 const uint32_t sx = sw + Cfg::W_BYTES;
                 const uint32_t full = bar_full0 + s * 8;
-                mbar_arrive_expect_tx(full, Cfg::LOAD_BYTES);
+                mbar_arrive_expect_tx(full, load_bytes);
                 if constexpr (Cfg::BLAYOUT == BL_NK)
                     tma_load_3d(sw, &p.tmap_w, full, kb * BK, ni * BNW, b);
                 else

@@ -30,7 +30,7 @@ enum : int { BL_NK = 0, BL_FLAT = 1 };
 enum : int { OUT_F32 = 0, OUT_BF16 = 1 };
 
 struct GemmParams {
-    CUtensorMap tmap_a;          // u8 [batch][M][K], box 128 x 128, 128-byte swizzle
+    CUtensorMap tmap_a;          // u8 [batch][M][K], box 128 bytes x a_rows, 128-byte swizzle
     CUtensorMap tmap_b;          // u8 [batch][N][K] (same box) or the flat 4-D view
     CUtensorMap tmap_sfa;        // pair kernels, MX: scale atoms as u8 [atoms*2][256], box 256 x 2
     CUtensorMap tmap_sfb;        // pair kernels, MX: box 256 x 2*atoms
@@ -44,6 +44,7 @@ struct GemmParams {
     long long sfa_stride, sfb_stride, sfa_batch, sfb_batch;
     int m, n, k, batch;
     int tiles_m, tiles_n, tiles_total, kblocks;
+    int a_rows;                  // rows of A's box (single-CTA kernels): 128, or M where that is little
     int out_dtype;
     int c_tma;                   // block-scale pair kernels: finished tiles leave through TMA bulk stores
     int inputs_ready;            // pair kernels: operands do not depend on the previous kernel (see b200_gemm_flags)
@@ -433,6 +434,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
                 int b, mi, ni;
                 tile_coords(p, t, b, mi, ni);
+                const uint32_t bytes = p.a_rows * BK + Cfg::B_BYTES + Cfg::SFA_BYTES + Cfg::SFB_BYTES;
                 for (int kb = kb0; kb < kb0 + kblocks; ++kb, next_stage(s, ph)) {
                     if (!mbar_wait(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY)) {
                         ok = false;
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     const uint32_t sb = sa + Cfg::A_BYTES;
                     const uint32_t full = bar_full0 + s * 8;
                     if constexpr (Cfg::TOUCH) *requested = asked++;
-                    mbar_arrive_expect_tx(full, Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES + Cfg::SFB_BYTES);
+                    mbar_arrive_expect_tx(full, bytes);
                     tma_load_3d(sa, &p.tmap_a, full, kb * BK, mi * BM, b);
                     if constexpr (Cfg::BLAYOUT == BL_NK)
                         tma_load_3d(sb, &p.tmap_b, full, kb * BK, ni * BN, b);

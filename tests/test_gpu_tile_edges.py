@@ -96,3 +96,28 @@ def test_columns_of_a_chunk(api, mode, tile, n):
 @pytest.mark.parametrize("n", [128, 256, 384, 512, 640, 896, 1024])
 def test_columns_of_a_chunk_with_block_scales(api, n):
     check(api, "block", 140, n, 256, 7, around=True)
+
+
+# few rows: a stage holds what an earlier launch left behind them -- here NaNs, in every byte of every operand tile -- and nothing of it may show
+@pytest.mark.parametrize("mode,tile,nan", [("none", 1, 0x7F), ("none", 2, 0x7F), ("none", 3, 0x7F), ("mx", 1, 0x7F), ("mx", 3, 0x7F), ("bf16", 1, 0xFF), ("bf16", 2, 0xFF), ("block", 3, 0x7F)])
+@pytest.mark.parametrize("m", [1, 8, 17, 33, 63, 64, 65])
+def test_rows_that_are_not_there(api, mode, tile, nan, m):
+    if tile == 3 and m > 64:
+        return
+    k, n = 1792, 19200                                   # every ring goes round, every SM has a CTA
+    junk = torch.full((64 if tile == 3 else 128, k), nan, dtype=torch.uint8, device=DEV)
+    wide = torch.full((n, k), nan, dtype=torch.uint8, device=DEV)
+    run, ref = call(api, mode, whole(m, k // 2 if mode == "bf16" else k, 1), whole(n, k // 2 if mode == "bf16" else k, 2), tile)
+    if mode == "bf16":
+        api.gemm_a16w16(junk.view(torch.bfloat16), wide.view(torch.bfloat16), tile=tile)
+    elif mode == "mx":
+        ones = [torch.full((api.mx_sf_relayout(torch.full((r, k // 32), 127, dtype=torch.uint8, device=DEV), r, k).numel(),), 127, dtype=torch.uint8, device=DEV) for r in (junk.shape[0], n)]
+        api.gemm_a8w8_mx(junk, wide, *ones, tile=tile)
+    elif mode == "block":
+        api.gemm_a8w8_blockscale(junk, wide, torch.ones(k // 128, junk.shape[0], device=DEV), torch.ones(n // 128, k // 128, device=DEV), tile=tile)
+    else:
+        api.gemm_a8w8(junk, wide, tile=tile)
+    out = torch.full((m, n), 7.0, device=DEV)
+    run(out)
+    assert torch.equal(out, ref)
+    assert api.last_status() == 0
