@@ -35,6 +35,7 @@ EXPORTS = (
     "b200_flag_write", "b200_flag_wait", "b200_stream_copy", "b200_ipc_alloc", "b200_ipc_open", "b200_ipc_close", "b200_ipc_free",
     "b200_slab_bytes", "b200_slab_upload", "b200_last_status", "b200_peek_status", "b200_selftest_bounded_wait", "b200_last_cuda_error", "b200_strerror", "b200_sm_count", "b200_release",
     "b200_version", "b200_launch_count", "b200_last_tail_split", "b200_gemm_check_split", "b200_gemm_a16w16_check_split", "b200_last_k_split",
+    "b200_gemm_check_columns", "b200_last_columns",
 )
 
 
@@ -131,6 +132,8 @@ def lib() -> C.CDLL:
         "b200_gemm_check_split": (i32, [C.POINTER(GemmArgs), C.POINTER(i32)]),
         "b200_gemm_a16w16_check_split": (i32, [C.POINTER(GemmArgs), C.POINTER(i32)]),
         "b200_last_k_split": (i32, []),
+        "b200_gemm_check_columns": (i32, [C.POINTER(GemmArgs), i32, C.POINTER(i32)]),
+        "b200_last_columns": (i32, []),
     }
     for name, (res, args) in sig.items():
         fn = getattr(L, name)

@@ -354,3 +354,8 @@ def last_tail_split():
 def last_k_split():
     """CTAs per tile of this thread's last tile-kernel launch when the K of a tile was split over a cluster, otherwise None."""
     return lib().b200_last_k_split() or None
+
+
+def last_columns():
+    """Columns of a tile of this thread's last tile-kernel launch."""
+    return lib().b200_last_columns()

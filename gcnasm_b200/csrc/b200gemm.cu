@@ -228,6 +228,7 @@ struct Plan {
     int tile;        // b200_tile_hint value actually used
     int mt;          // decode token block
     int splits;      // decode K splits; otherwise, above 1: 128 x 128 tiles, each shared by so many CTAs, whatever `tile` says
+    int columns;     // above 0: one CTA's tiles of 128 rows and so many columns, whatever `tile` says
 };
 
 // MX with few tokens: the K blocks from which the skinny-M kernel beats the 128 x 128 tiles, which have the shorter fixed part.  Its own
@@ -282,6 +283,28 @@ int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, bool lines
     return best;
 }
 
+// One CTA's tiles in a grid of one round: the fewest columns that make one.  A K block takes what its operand tiles take out of L2, 128 rows of
+// A and the tile's of B at some 70 bytes a clock, and the way in and out of a tile is the shorter the narrower it is, so as long as SMs are
+// idle a narrower tile on more of them wins; and 160 to 224 columns make one round of what would be two of 128, or 256 with SMs idle.  us, kind of tile as
+// before / narrowest, mean over 1300 to 1500 sizes each (up to 3000 rows, 18432 columns, K 8192): unscaled 0.884, block scales 0.896, bf16 0.874.
+//   8-bit         256 x 512 x 1024    128 columns 4.5 / 32 3.6       333 x 7168 x 2048   256 columns 10.7 / 160 8.5    700 x 2048 x 7168  128 15.6 / 96 14.9
+//   block scales  129 x 1024 x 1024   128         5.0 / 32 4.1       333 x 7168 x 2048   256         11.9 / 160 9.7    100 x 7168 x 2048  128  7.8 / 64  7.1
+//   bf16          64 x 8192 x 2048    128        10.4 / 64 9.7       333 x 7168 x 1024   256 (pair)  10.9 / 160 8.5
+// Not 96 or 224 columns for a short K (96 for 128: 175 x 6272 x 384 3.72 / 3.86; 224 for 256: 269 x 10240 x 256 4.96 / 5.67), not 224 with block scales,
+// whose 256 columns take no longer, and nothing in the place of 256 (two rows of tiles and a long K are the pair's: 430 x 8448 x 7552 26.8 / 29.8).
+// apart: the tile would be a pair's and rows are not whole 128-byte lines apart.  Every row of a box then lies in two lines, what a K block takes out of L2
+// 1.6 times as much, and a pair, which takes less of it, is ahead of wide tiles from some K on; narrow over pair by K blocks, mean: 8-bit 160 columns 0.94 from 16
+// to 24 (950 x 2816 x 2672 12.4 / 13.5), 1.03 to 36 and 1.09 above; 192 0.87 up to 10, then 1.04, 1.24 above 36; bf16 224 1.0 from 24 on (658 x 4872 x 6000 24.0 / 30.0, x 6016 20.0 / 20.0).
+int one_round_columns(int64_t tm, int64_t n, int64_t batch, int64_t kblocks, bool block, bool apart, bool ab16, int sm_count) {
+    for (int w : {32, 64, 96, 128, 160, 192, 224}) {
+        if (tm * ((n + w - 1) / w) * batch > sm_count) continue;
+        if ((w == 96 || w == 224) && kblocks < 6) continue;
+        if (apart && kblocks >= (ab16 ? (w == 224 ? 24 : 1 << 30) : w >= 192 ? 10 : w == 160 ? 20 : 1 << 30)) return 0;
+        return w == 224 && block ? 0 : w;
+    }
+    return 0;
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ab16: `a` is the byte view of a bf16 problem (K and the A/B strides counted in bytes)
@@ -326,7 +349,7 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
     if (b_shared && a->scale_mode == B200_SCALE_BLOCK && a->stride_sfb_batch != 0) return B200_ERR_BAD_ARG;
     if (pair_only && a->m <= 128) return B200_ERR_UNSUPPORTED;
 
-    Plan pl{B200_TILE_128x128, 0, 1};
+    Plan pl{B200_TILE_128x128, 0, 1, 0};
     const int64_t kblocks = (a->k + 127) / 128;
     const bool decode_ok = !pair_only && !ab16 && a->m <= 64 && (a->n % 16 == 0);
     int hint = a->tile_hint;
@@ -424,6 +447,15 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 const bool lines = a->stride_a % 128 == 0 && (a->b_layout == B200_B_FLAT_16x16 || a->stride_b % 128 == 0);
                 const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, lines, sm_count, &equal);
                 if (s > 1 && 10 * 128 * (ab16 ? 155 : a->scale_mode == B200_SCALE_BLOCK ? 125 : 130) * equal < best * kblocks) pl.splits = s;
+                const bool block = a->scale_mode == B200_SCALE_BLOCK, single = hint == B200_TILE_128x128 || hint == B200_TILE_128x256;
+                const int columns = mx ? 0 : one_round_columns(tm1, a->n, a->batch, kblocks, block, !single && !lines, ab16, sm_count);
+                // A split takes as long as `equal` K blocks on 128 columns; narrow tiles are worth three more (block scales four, 32 columns one more).
+                // Narrow over split by kblocks - equal, mean of 640 / 870 sizes: 8-bit 0.956 at 0 and 1, 0.988 at 2 and 3, 1.033 at 4 and 5; block scales
+                // 0.892, 0.938, 1.004, 1.07 at 6 and 7; bf16 1.045, 1.07; 8-bit rows not whole lines apart 0.94, 0.995 (100 x 4480 x 3312 8.9 / 10.7).  Not for few rows, whose sums are quick (2 x 392 x 2816 4.4 / 6.1, block scales 68 x 384 x
+                // 2304, two batches, 6.1 / 6.6).
+                const int64_t worth = ab16 || a->m <= 80 ? 0 : !lines ? 1 : (block ? 4 : 3) + (columns == 32);
+                if (columns && kblocks - equal < worth) pl.splits = 1;
+                if (pl.splits == 1) pl.columns = columns;
             }
         }
     }
@@ -562,7 +594,7 @@ int split_clusters(const b200_gemm_args* a, bool ab16, int size, int sm_count) {
     }
 }
 
-thread_local int t_last_k_split = 0;           // the calling thread's last tile-kernel launch (b200_last_k_split)
+thread_local int t_last_k_split = 0, t_last_columns = 0;           // the calling thread's last tile-kernel launch (b200_last_k_split, b200_last_columns)
 // 128 x 128 tiles on one CTA each or, with p.splits > 1, on a cluster each
 template <int MODE, int BL>
 int launch_gemm128(const GemmParams& p, int grid, cudaStream_t st) {
@@ -573,6 +605,23 @@ int launch_gemm128(const GemmParams& p, int grid, cudaStream_t st) {
     if (rc) return rc;
     t_last_k_split = p.splits;
     return launch_pdl_cluster(p.splits, kernel, static_cast<unsigned>(p.tiles_total * p.splits), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
+}
+
+// ... and of any width that is built
+template <int MODE, int BL>
+int launch_columns(int columns, const GemmParams& p, int grid, cudaStream_t st) {
+    switch (columns) {
+        case 32: return launch_gemm<32, MODE, BL>(p, grid, st);
+        case 64: return launch_gemm<64, MODE, BL>(p, grid, st);
+        case 96: return launch_gemm<96, MODE, BL>(p, grid, st);
+        case 128: return launch_gemm128<MODE, BL>(p, grid, st);
+        case 160: return launch_gemm<160, MODE, BL>(p, grid, st);
+        case 192: return launch_gemm<192, MODE, BL>(p, grid, st);
+        case 224:
+            if constexpr (MODE != MODE_BLOCK) return launch_gemm<224, MODE, BL>(p, grid, st);
+            else return B200_ERR_UNSUPPORTED;
+        default: return launch_gemm<256, MODE, BL>(p, grid, st);
+    }
 }
 
 // K splits of the decode kernel that work as one cluster (above 8 the size is not portable and asked for explicitly)
@@ -915,7 +964,7 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
 // 806 with 24, 522 with 32 and more; boxes of 16 rows with one there 522.  128 rows / the rows there are, us: bf16 1 x 5440 x 1792 11.7 / 8.8, 16 x 5440 x
 // 2048 10.6 / 8.2, 4 x 8192 x 4096 18.9 / 14.5, 8-bit 5 x 5448 x 4096 10.5 / 7.9; 40 x 5440 x 2048 the same, 1 x 1024 x 1024 (8 tiles) 5.4 / 5.55.  The few rows
 // of a last tile below others are not worth a second box: its CTAs are half of a grid at most (8-bit 140 x 8192 x 2048 6.4 / 6.45).
-constexpr int kBoxRows = 64;
+constexpr int kBoxRows = 127;
 
 int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStream_t st, bool ab16 = false) {
     int BN = 128;
@@ -929,13 +978,13 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
                                                           : split_clusters<BL_NK>(a, ab16, splits, ds->sm_count);
         if (room < tiles) splits = 1;
     }
-    switch (splits > 1 ? B200_TILE_128x128 : pl.tile) {
+    switch (splits > 1 || pl.columns ? B200_TILE_128x128 : pl.tile) {
         case B200_TILE_128x256: BN = 256; break;
         case B200_TILE_PAIR_256x256: BN = 256; pair = true; break;
         case B200_TILE_PAIR_256x224: BN = 224; pair = true; break;
         case B200_TILE_PAIR_256x192: BN = 192; pair = true; break;
         case B200_TILE_PAIR_256x128: BN = 128; pair = true; break;
-        default: BN = 128; break;
+        default: BN = pl.columns ? pl.columns : 128; break;
     }
     const int BMT = pair ? 256 : 128;                 // output rows per tile
     const int BROWS = pair ? BN / 2 : BN;             // B rows one CTA loads
@@ -1011,6 +1060,7 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
         p.sfb_batch = a->stride_sfb_batch;
     }
     t_last_k_split = 0;
+    t_last_columns = BN;
     const bool flat = a->b_layout == B200_B_FLAT_16x16;
     if (pair && BN == 256 && !ab16 && a->scale_mode != B200_SCALE_MX) {
         const int sms = ds->sm_count;
@@ -1027,8 +1077,7 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     if (ab16) {
         if (pair) return flat ? launch_pair<256, MODE_ACC16, BL_FLAT>(p, ds->sm_count, st) : launch_pair<256, MODE_ACC16, BL_NK>(p, ds->sm_count, st);
         const int grid16 = p.tiles_total < ds->sm_count ? p.tiles_total : ds->sm_count;
-        if (BN == 256) return flat ? launch_gemm<256, MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm<256, MODE_ACC16, BL_NK>(p, grid16, st);
-        return flat ? launch_gemm128<MODE_ACC16, BL_FLAT>(p, grid16, st) : launch_gemm128<MODE_ACC16, BL_NK>(p, grid16, st);
+        return flat ? launch_columns<MODE_ACC16, BL_FLAT>(BN, p, grid16, st) : launch_columns<MODE_ACC16, BL_NK>(BN, p, grid16, st);
     }
     if (pair) {
         switch (BN) {
@@ -1041,13 +1090,11 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     const int grid = p.tiles_total < ds->sm_count ? p.tiles_total : ds->sm_count;
     switch (a->scale_mode) {
         case B200_SCALE_BLOCK:
-            if (BN == 256) return flat ? launch_gemm<256, MODE_BLOCK, BL_FLAT>(p, grid, st) : launch_gemm<256, MODE_BLOCK, BL_NK>(p, grid, st);
-            return flat ? launch_gemm128<MODE_BLOCK, BL_FLAT>(p, grid, st) : launch_gemm128<MODE_BLOCK, BL_NK>(p, grid, st);
+            return flat ? launch_columns<MODE_BLOCK, BL_FLAT>(BN, p, grid, st) : launch_columns<MODE_BLOCK, BL_NK>(BN, p, grid, st);
         case B200_SCALE_MX:
             return flat ? launch_gemm128<MODE_MX, BL_FLAT>(p, grid, st) : launch_gemm128<MODE_MX, BL_NK>(p, grid, st);
         default:
-            if (BN == 256) return flat ? launch_gemm<256, MODE_ACC, BL_FLAT>(p, grid, st) : launch_gemm<256, MODE_ACC, BL_NK>(p, grid, st);
-            return flat ? launch_gemm128<MODE_ACC, BL_FLAT>(p, grid, st) : launch_gemm128<MODE_ACC, BL_NK>(p, grid, st);
+            return flat ? launch_columns<MODE_ACC, BL_FLAT>(BN, p, grid, st) : launch_columns<MODE_ACC, BL_NK>(BN, p, grid, st);
     }
 }
 
@@ -1090,6 +1137,17 @@ int b200_gemm_check_split(const b200_gemm_args* args, int32_t* parts) {
     Plan pl;
     int rc = validate(args, 148, &pl);
     if (rc == B200_OK && parts) *parts = pl.tile == B200_TILE_DECODE ? 1 : pl.splits;
+    return rc;
+}
+
+static int byte_view16(const b200_gemm_args* a, b200_gemm_args* v);
+int b200_gemm_check_columns(const b200_gemm_args* args, int32_t bf16_operands, int32_t* columns) {
+    b200_gemm_args v;
+    int rc = bf16_operands ? byte_view16(args, &v) : B200_OK;
+    if (rc) return rc;
+    Plan pl;
+    rc = validate(bf16_operands ? &v : args, 148, &pl, bf16_operands != 0);
+    if (rc == B200_OK && columns) *columns = pl.columns;
     return rc;
 }
 
@@ -1775,5 +1833,6 @@ int b200_last_tail_split(int32_t* first_tile, int32_t* parts) {
     return t_last_tail[1] > 0 ? 1 : 0;
 }
 int b200_last_k_split(void) { return t_last_k_split; }
+int b200_last_columns(void) { return t_last_columns; }
 
 }  // extern "C"

@@ -7,18 +7,21 @@
 // One persistent CTA per SM, 12 warps:
 //   warp 0      TMA producer   (one elected lane)  global -> shared ring, mbarrier complete_tx
 //   warp 1      UMMA issuer    (one elected lane)  tcgen05.mma kind::f8f6f4 / kind::mxf8f6f4, TMEM alloc
-//   warp 2      block scales: brings the scales into shared memory beside the operands (128 columns), or reads them into L1 ahead of
+//   warp 2      block scales: brings the scales into shared memory beside the operands (up to 192 columns), or reads them into L1 ahead of
 //               their use (256 columns, ScaleToucher)
 //   warp 3      idle, as warp 2 otherwise (register re-allocation works on whole warpgroups)
 //   warps 4-11  epilogue: TMEM -> registers -> scale -> global
-// TMEM holds two accumulator buffers of BN columns (four with block scales and BN = 128).  Per-tensor / unscaled / MX modes accumulate a
+// TMEM holds two accumulator buffers of BN columns (three or four with block scales and fewer than 192).  Per-tensor / unscaled / MX modes accumulate a
 // whole tile in one buffer while the epilogue drains the other.  Block-scale mode gives every
 // 128-wide K group a FRESH buffer (the reference does the same with a fresh MFMA accumulator,
 // kernel_template.hpp:317,334) and the epilogue warps fold it into register accumulators with
 // acc += partial * (sfa[g][row] * sfb[nblk][g]) -- the analogue of scale_c_tile.
-// Few tiles with a long K: the CTAs of a cluster take a part of a 128 x 128 tile's K each (SPLIT) and sum their results in
+// Tiles are 128 rows by 128 or 256 columns, or in a grid of one round by as few as bring all SMs to work (32 to 224, one_round_columns() of
+// the launcher).  Few tiles with a long K: the CTAs of a cluster take a part of a 128 x 128 tile's K each (SPLIT) and sum their results in
 // distributed shared memory; tile_splits() of the launcher says when.
 #pragma once
+
+#include <type_traits>
 
 #include "sm100_ptx.cuh"
 
@@ -82,7 +85,7 @@ template <int BN_, int MODE_, int BLAYOUT_, bool SPLIT_ = false>
 struct GemmCfg {
     static constexpr bool SPLIT = SPLIT_;                           // a tile's K is split over a cluster
     static constexpr bool TOUCH = MODE_ == MODE_BLOCK && BN_ == 256;   // a warp reads the scales ahead of their use
-    static constexpr bool FEED = MODE_ == MODE_BLOCK && BN_ == 128;    // a warp brings the scales into shared memory beside the operands
+    static constexpr bool FEED = MODE_ == MODE_BLOCK && BN_ != 256;    // a warp brings the scales into shared memory beside the operands
     static constexpr bool AB16 = MODE_ == MODE_ACC16;               // bf16 operands: same bytes, kind::f16 MMAs
     static constexpr int BM = 128, BN = BN_, BK = 128, MODE = AB16 ? MODE_ACC : MODE_, BLAYOUT = BLAYOUT_;
     static constexpr int A_BYTES = BM * BK;
@@ -92,7 +95,7 @@ struct GemmCfg {
     static constexpr int SFB_BYTES = (MODE == MODE_MX) ? SFB_ATOMS * 512 : 0;
     static constexpr int STAGE_BYTES = ((A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES + 1023) / 1024) * 1024;
     static constexpr int OUT_STAGE_BYTES = 8 * kOutStageBytesPerWarp;        // store staging of the eight epilogue warps
-    // FEED: scales of so many K blocks, each the tile's rows of A and its block of B.  Eight warps that load the scales themselves wait for them
+    // FEED: scales of so many K blocks, each the tile's rows of A and its one or two blocks of B.  Eight warps that load the scales themselves wait for them
     // however early they ask: a load queues behind all the operand tiles in flight, 200 KB a CTA.  Six register sets, requested six groups
     // ahead / a ring that fills with the operands (and so with a stage less of those), us: 333 x 5120 x 2048 9.0 / 7.9, 128 x 8192 x 8192 23.9 / 20.1 (no
     // loads at all 19.7), 512 x 4096 x 4096 13.9 / 12.0, 1024 x 1024 x 512 4.26 / 4.11, 2500 x 5120 x 3072 53.8 / 48.7.  Also tried on 128 x 8192 x 8192: the
@@ -100,25 +103,27 @@ struct GemmCfg {
     // registers do not take it (spills, 333 x 7168 x 2048 12.0 / 15.2).
     static constexpr int SF_SLOTS = FEED ? 16 : 0, SF_SLOT_BYTES = (BM + 4) * 4;
     static constexpr int ROOM = 227 * 1024 - 1024 /*barriers*/ - 1024 /*alignment slack*/ - SF_SLOTS * SF_SLOT_BYTES;
-    static constexpr int STAGES = (ROOM - OUT_STAGE_BYTES) / STAGE_BYTES;           // ring with the staging behind it
+    static constexpr int STAGES = (ROOM - OUT_STAGE_BYTES) / STAGE_BYTES < 8 ? (ROOM - OUT_STAGE_BYTES) / STAGE_BYTES : 8;   // ring with the staging behind it
     // Ring of a CTA with one tile, whose staging lies in the ring: 128 columns without block or MX scales seven stages instead of six.  Behind six
     // of them a long K waits for its operands, us, six / seven: 8-bit 128 x 8192 x 8192 19.8 / 18.4, 512 x 4096 x 4096 11.6 / 11.0, bf16
     // 128 x 8192 x 8192 35.1 / 33.0.  CTAs with several tiles keep the staging of its own: the next tile's loads are under way while
     // a result leaves, and stores from registers instead cost more than the stage gives (2500 x 5120 x 3072 45.0 / 41.5).
-    static constexpr int STAGES_ONE = ROOM / STAGE_BYTES;
+    static constexpr int STAGES_ONE = ROOM / STAGE_BYTES < 8 ? ROOM / STAGE_BYTES : 8;
     static constexpr int STAGING_END = STAGES * STAGE_BYTES + OUT_STAGE_BYTES;
     static constexpr int RING_BYTES = STAGES_ONE * STAGE_BYTES > STAGING_END ? STAGES_ONE * STAGE_BYTES : STAGING_END;
     static constexpr int SMEM_BYTES = RING_BYTES + 1024 /*barriers*/ + SF_SLOTS * SF_SLOT_BYTES + 1024 /*alignment slack*/;
-    // accumulator buffers; 128 columns with block scales, a hand-off per K block: as many as tensor memory holds
-    static constexpr int BUFS = (MODE == MODE_BLOCK && BN == 128) ? 4 : 2;
+    // accumulator buffers; block scales, a hand-off per K block: up to four, as many as tensor memory holds
+    static constexpr int BUFS = !FEED ? 2 : BN <= 128 ? 4 : 512 / BN;
     static constexpr int ACC_COLS = BUFS * BN;
     static constexpr int SF_COLS = (MODE == MODE_MX) ? 4 + 4 * SFB_ATOMS : 0;
     static constexpr int TMEM_COLS = (ACC_COLS + SF_COLS) <= 32 ? 32 : (ACC_COLS + SF_COLS) <= 64 ? 64
                                    : (ACC_COLS + SF_COLS) <= 128 ? 128 : (ACC_COLS + SF_COLS) <= 256 ? 256 : 512;
     static constexpr int NCH = BN / 2;              // columns owned by one epilogue thread
+    static constexpr bool STRADDLE = BN % 128 != 0 && 128 % BN != 0;    // a tile lies in two of the 128-column scale blocks
     static constexpr int THREADS = 384;
     static_assert(ACC_COLS + SF_COLS <= 512, "TMEM overflow");
     static_assert(BN % 32 == 0 && BN <= 256, "BN must be a multiple of 32, at most 256");
+    static_assert(MODE != MODE_MX || BN % 128 == 0, "MX scale atoms cover 128 columns");
     static_assert(STAGES >= 3 && STAGES_ONE <= 8, "ring depth");
     // a stage that is free says that the group STAGES + BUFS before its next one has been drained
     static_assert(!FEED || STAGES_ONE + BUFS <= SF_SLOTS, "scales stay until their group has been drained");
@@ -554,7 +559,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     int row[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) row[j] = mi * BM + j * 32 + lane < p.m ? mi * BM + j * 32 + lane : p.m - 1;
-                    const float* pb = p.sfb + b * p.sfb_batch + static_cast<long long>(ni) * p.sfb_stride + kb0;
+                    // (a tile of a width between lies in two 128-column blocks of B; the second may be beyond the last)
+                    const int blk = ni * BN / 128 + lane;
+                    const float* pb = p.sfb + b * p.sfb_batch + static_cast<long long>(blk * 128 < p.n ? blk : p.n / 128 - 1) * p.sfb_stride + kb0;
                     for (int kb = 0; kb < kblocks; ++kb, ++it, next_stage(s, ph)) {
                         if (!role_all<true>(mbar_wait(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY))) {
                             ok = false;
@@ -563,7 +570,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         const uint32_t slot = sf0 + it % Cfg::SF_SLOTS * Cfg::SF_SLOT_BYTES;
 #pragma unroll
                         for (int j = 0; j < 4; ++j) cp_async_4(slot + (j * 32 + lane) * 4, pa + row[j]);
-                        if (lane == 0) cp_async_4(slot + BM * 4, pb + kb);
+                        if (lane <= (Cfg::STRADDLE ? 1 : 0)) cp_async_4(slot + (BM + lane) * 4, pb + kb);
                         cp_async_arrive(bar_full0 + s * 8);
                         pa += p.sfa_stride;
                     }
@@ -608,64 +615,104 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             // 48 x 2048 x 1024 5.28 / 5.32).  (Block scales have no such tiles but the last of many rows.)
             const int rows = p.m - mi * BM;
             const bool direct = MODE != MODE_BLOCK && (rows <= 32 || rows - quad * 32 < 32);
-            auto put32 = [&](const int c, const float* o) {              // this warp's 32 rows x columns [32 c, 32 c + 32) of its part
+            // this warp's 32 rows x CW columns of its part, from column `c` of it on
+            auto put = [&](auto width, const int c, const float* o) {
+                constexpr int CW = decltype(width)::value;
                 if constexpr (Cfg::SPLIT) {
                     // partial sums, row by row; the 16-byte pieces of eight neighbouring rows lie in different banks
                     uint8_t* mine = smem_gen + row_in_tile * (BN * 4);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        *reinterpret_cast<float4*>(mine + (((half * (NCH / 4) + c * 8 + j) ^ (lane & 7)) << 4)) =
+                    for (int j = 0; j < CW / 4; ++j)
+                        *reinterpret_cast<float4*>(mine + (((half * (NCH / 4) + c / 4 + j) ^ (lane & 7)) << 4)) =
                             make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
                     return;
                 }
-                const int row0 = mi * BM + quad * 32, col0 = col_base + c * 32;
-                if (direct || !vec_ok || col0 + 32 > p.n) {
-                    if (row < p.m) store_row_chunk<32>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, o, vec_ok);
+                const int row0 = mi * BM + quad * 32, col0 = col_base + c;
+                if (direct || !vec_ok || col0 + CW > p.n) {
+                    if (row < p.m) store_row_chunk<CW>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, o, vec_ok);
                 } else if (p.out_dtype == OUT_BF16) {
-                    store_chunk_staged<32, true>(p, cbatch, out_stage, row0, col0, o, lane);
+                    store_chunk_staged<CW, true>(p, cbatch, out_stage, row0, col0, o, lane);
                 } else {
-                    store_chunk_staged<16, false>(p, cbatch, out_stage, row0, col0, o, lane);
-                    store_chunk_staged<16, false>(p, cbatch, out_stage, row0, col0 + 16, o + 16, lane);
+#pragma unroll
+                    for (int j = 0; j < CW; j += 16) store_chunk_staged<16, false>(p, cbatch, out_stage, row0, col0 + j, o + j, lane);
                 }
             };
+            using W32 = std::integral_constant<int, 32>;
+            using W16 = std::integral_constant<int, 16>;
 
-            if constexpr (MODE == MODE_BLOCK && NCH == 64) {
+            if constexpr (Cfg::FEED) {
                 // 64 columns per thread leave room to have both loads of a group in flight, and the buffer goes back before the FMAs;
                 // four buffers keep the tensor core busy meanwhile.  Two buffers, handed back after the FMAs, scalar FMAs and stores
                 // from registers / this loop and staged stores, us: 100 x 7168 x 2048 10.6 / 9.2, 200 x 7168 x 2048 11.3 / 9.6, 512 x 4096 x
                 // 4096 16.8 / 15.0, 2500 x 5120 x 3072 77 / 59.
-                unsigned long long acc2[32];
+                constexpr int C32 = NCH / 32, TAIL = NCH % 32;       // loads of a group: 32 columns each, and one of 16
+                static_assert(TAIL == 0 || TAIL == 16, "a thread's columns are a multiple of 16");
+                unsigned long long acc2[NCH / 2];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) acc2[j] = 0ull;
-                for (int g = 0; g < groups; ++g, ++phase) {
-                    const uint32_t as = phase % BUFS;
-                    const uint32_t aph = (phase / BUFS) & 1;
-                    if (!mbar_wait(bar_accf0 + as * 8, aph, abort_flag, p.status, KSTAT_TIMEOUT_ACC_F)) {
-                        ok = false;
-                        break;
+                for (int j = 0; j < NCH / 2; ++j) acc2[j] = 0ull;
+                // Columns up to the next scale block, and which of the tile's two blocks they begin in.  A loop for each place where the
+                // blocks meet within a thread's columns (one loop that chooses: 512 x 4096 x 4096 on 160 columns 16.2 -> 15.7 us).
+                const int left = 128 - (col_base & 127);
+                const int blk = Cfg::STRADDLE ? (col_base >> 7) - (ni * BN >> 7) : 0;
+                const uint32_t sf_row = sf0 + row_in_tile * 4, sf_col = sf0 + (BM + blk) * 4;
+                auto k_loop = [&](auto left_tag) {
+                    constexpr int LEFT = decltype(left_tag)::value;
+                    for (int g = 0; g < groups; ++g, ++phase) {
+                        const uint32_t as = phase % BUFS;
+                        const uint32_t aph = (phase / BUFS) & 1;
+                        if (!mbar_wait(bar_accf0 + as * 8, aph, abort_flag, p.status, KSTAT_TIMEOUT_ACC_F)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
+                        float v[NCH];
+#pragma unroll
+                        for (int c = 0; c < C32; ++c) tmem_ld32(taddr + c * 32, v + c * 32);
+                        if constexpr (TAIL) tmem_ld16(taddr + C32 * 32, v + C32 * 32);
+                        const uint32_t slot = phase % Cfg::SF_SLOTS * Cfg::SF_SLOT_BYTES;
+                        const float sa = ld_shared_f32(sf_row + slot);
+                        const float sc = sa * ld_shared_f32(sf_col + slot);
+                        const unsigned long long sc2 = pack_f32x2(sc, sc);
+                        unsigned long long sd2 = sc2;
+                        if constexpr (LEFT < NCH) {
+                            const float sd = sa * ld_shared_f32(sf_col + 4 + slot);
+                            sd2 = pack_f32x2(sd, sd);
+                        }
+                        tmem_ld_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
+#pragma unroll
+                        for (int j = 0; j < NCH / 2; ++j) acc2[j] = ffma2(pack_f32x2(v[2 * j], v[2 * j + 1]), 2 * j < LEFT ? sc2 : sd2, acc2[j]);
                     }
-                    tc_fence_after();
-                    const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
-                    float v[64];
-                    tmem_ld32(taddr, v);
-                    tmem_ld32(taddr + 32, v + 32);
-                    const uint32_t slot = sf0 + phase % Cfg::SF_SLOTS * Cfg::SF_SLOT_BYTES;
-                    const float sc = ld_shared_f32(slot + row_in_tile * 4) * ld_shared_f32(slot + BM * 4);
-                    const unsigned long long sc2 = pack_f32x2(sc, sc);
-                    tmem_ld_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_acce0 + as * 8);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) acc2[j] = ffma2(pack_f32x2(v[2 * j], v[2 * j + 1]), sc2, acc2[j]);
+                };
+                if constexpr (!Cfg::STRADDLE) {
+                    k_loop(std::integral_constant<int, NCH>{});
+                } else {
+                    if (left >= NCH) k_loop(std::integral_constant<int, NCH>{});
+                    else if (NCH > 64 && left == 64) k_loop(std::integral_constant<int, 64>{});
+                    else if (TAIL && NCH > 48 && left == 48) k_loop(std::integral_constant<int, 48>{});
+                    else if (left == 32) k_loop(std::integral_constant<int, 32>{});
+                    else if constexpr (TAIL) k_loop(std::integral_constant<int, 16>{});
                 }
                 if (ok) {
+                    float o[32];
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        float o[32];
+                    for (int c = 0; c < C32; ++c) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j) unpack_f32x2(acc2[c * 16 + j], o[2 * j], o[2 * j + 1]);
-                        put32(c, o);
+                        // (N is a multiple of 128: 16 columns are all there or none of them)
+                        if (!TAIL || col_base + c * 32 + 32 <= p.n) {
+                            put(W32{}, c * 32, o);
+                        } else if (col_base + c * 32 + 16 <= p.n) {
+                            put(W16{}, c * 32, o);
+                        }
+                    }
+                    if constexpr (TAIL) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) unpack_f32x2(acc2[C32 * 16 + j], o[2 * j], o[2 * j + 1]);
+                        if (col_base + C32 * 32 + 16 <= p.n) put(W16{}, C32 * 32, o);
                     }
                 }
             } else if constexpr (MODE == MODE_BLOCK) {
@@ -720,7 +767,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         float o[32];
 #pragma unroll
                         for (int j = 0; j < 16; ++j) unpack_f32x2(acc2[c * 16 + j], o[2 * j], o[2 * j + 1]);
-                        put32(c, o);
+                        put(W32{}, c * 32, o);
                     }
                 }
             } else {
@@ -732,13 +779,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 }
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + tmem_lane + as * BN + half * NCH;
-                float v[2][32];
-                tmem_ld32(taddr, v[0]);
+                constexpr int CW = NCH % 32 == 0 ? 32 : 16, NC = NCH / CW;
+                float v[2][CW];
+                tmem_ld<CW>(taddr, v[0]);
 #pragma unroll
-                for (int c = 0; c < NCH / 32; ++c) {
+                for (int c = 0; c < NC; ++c) {
                     tmem_ld_wait();
-                    if (c + 1 < NCH / 32) tmem_ld32(taddr + (c + 1) * 32, v[(c + 1) & 1]);
-                    if (c + 1 == NCH / 32) {
+                    if (c + 1 < NC) tmem_ld<CW>(taddr + (c + 1) * CW, v[(c + 1) & 1]);
+                    if (c + 1 == NC) {
                         // every column of this warp is in registers: hand the buffer back early
                         tc_fence_before();
                         __syncwarp();
@@ -746,9 +794,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                     }
                     if (MODE == MODE_ACC && !Cfg::SPLIT) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[c & 1][j] *= tscale;
+                        for (int j = 0; j < CW; ++j) v[c & 1][j] *= tscale;
                     }
-                    put32(c, v[c & 1]);
+                    put(std::integral_constant<int, CW>{}, c * CW, v[c & 1]);
                 }
                 ++phase;
             }
