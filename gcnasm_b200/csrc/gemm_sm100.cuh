@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                             ok = false;
                             break;
                         }
-                        if constexpr (MODE == MODE_BLOCK) {
+                        if constexpr (Cfg::FEED) {
                             uint32_t s1 = s, ph1 = ph;
                             next_stage(s1, ph1);
                             full_seen = mbar_probe(bar_full0 + s1 * 8, ph1);
@@ -629,7 +629,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                 }
                 const int row0 = mi * BM + quad * 32, col0 = col_base + c;
                 if (direct || !vec_ok || col0 + CW > p.n) {
-                    if (row < p.m) store_row_chunk<CW>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, o, vec_ok);
+                    // (block scales: N is a multiple of 128, so that a chunk is all there or not at all, and these are the stores of an unaligned C)
+                    if (row < p.m) store_row_chunk<CW>(p, cbatch + static_cast<size_t>(row) * p.ldc * esz, col0, o, MODE != MODE_BLOCK && vec_ok);
                 } else if (p.out_dtype == OUT_BF16) {
                     store_chunk_staged<CW, true>(p, cbatch, out_stage, row0, col0, o, lane);
                 } else {
