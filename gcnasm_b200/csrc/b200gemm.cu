@@ -1038,6 +1038,7 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
     p.kblocks = static_cast<int>((a->k + 127) / 128);
     p.kb_per_split = (p.kblocks + splits - 1) / splits;
     p.splits = splits;
+    p.b_ahead = !pair && p.tiles_m > 1 && p.tiles_total <= ds->sm_count && a->n * a->k >= (int64_t{6} << 20) ? 1 : 0;
     p.out_dtype = a->out_dtype;
     p.inputs_ready = (a->flags & (B200_GEMM_INPUTS_READY | B200_GEMM_BATCH_READY)) ? 1 : 0;
     p.b_shared = b_shared ? 1 : 0;

@@ -62,6 +62,7 @@ struct GemmParams {
     int tail_first, tail_split;
     // single-CTA 128 x 128 tiles: the CTAs of a cluster take kb_per_split K blocks each of one tile (splits == 1: whole tiles)
     int splits, kb_per_split;
+    int b_ahead;                 // single-CTA kernels, block scales, one round: the first K blocks of B are asked for ahead
     int* status;
 };
 
@@ -385,6 +386,22 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
     // back to back: 8-bit 122 x 256 x 5120 12.3 / 11.4, quantiser and block-scale 100 x 7168 x 2048 12.1 / 11.0, MX 40 x 2048 x 2048
     // 10.0 / 8.8, bf16 1 x 4096 x 4096 16.6 / 16.0.
     pdl_launch_dependents();
+    // With block scales a quantiser runs in front, as a rule, which leaves HBM idle.  Where B is a microsecond of it and more and several CTAs share a
+    // tile of it, those of the first row of tiles ask for their first ring of B into L2 before the wait.  Quantiser and GEMM, weights
+    // from HBM, not / so, us: 333 x 7168 x 2048 12.7 / 12.3, 500 x 8192 x 1024 11.25 / 10.6, 250 x 6144 x 1024 8.5 / 8.1, 180 x 9600 x 3072 15.0 / 14.5, 1000 x
+    // 4096 x 2048 16.2 / 15.8; one row of tiles 120 x 4096 x 2048 9.0 / 9.1; MX 200 x 6144 x 4096 15.9 / 16.1.  Not without scales: behind another GEMM
+    // it takes from that one's tail, twice where rows are not whole lines apart (802 x 4232 x 1776 13.4 / 13.8).
+    if constexpr (MODE == MODE_BLOCK && !Cfg::SPLIT) {
+        if (threadIdx.x == 3 * 32 && p.b_ahead) {
+            int b, mi, ni;
+            tile_coords(p, blockIdx.x, b, mi, ni);
+            const int most = mi > 0 ? 0 : (p.kblocks < static_cast<int>(stages) ? p.kblocks : static_cast<int>(stages));
+            for (int kb = 0; kb < most; ++kb) {
+                if constexpr (Cfg::BLAYOUT == BL_NK) tma_prefetch_3d(&p.tmap_b, kb * BK, ni * BN, b);
+                else tma_prefetch_4d(&p.tmap_b, 0, ni * (BN / 16), kb * (BK / 16), b);
+            }
+        }
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < Cfg::STAGES_ONE; ++s) {
             mbar_init(bar_full0 + s * 8, Cfg::FEED ? 33 : 1);    // FEED: and every lane of the feeding warp
