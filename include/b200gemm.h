@@ -134,7 +134,7 @@ int b200_last_tail_split(int32_t* first_tile, int32_t* parts);
  * tiles instead, each shared by the CTAs of a cluster that take a part of K (if the inputs are ready, only where the whole tile
  * would be a single CTA's: a pair's starts early): fp32 sums in another order, the same from run to run.  Whether it is depends
  * on the number of tiles, so with TILE_AUTO the last bits of a row can depend on how many rows, columns and batches the call has.
- * A grid of one round may be computed on one CTA's tiles of another width (b200_gemm_check_columns): whole tiles, the same bits. */
+ * A grid of few rounds may be computed on one CTA's tiles of another width (b200_gemm_check_columns): whole tiles, the same bits. */
 int b200_gemm_check(const b200_gemm_args* args, int32_t* chosen_tile);
 /* The other half of that answer: how many CTAs share the K of a tile in this launch.  1: whole tiles of the kind that
  * b200_gemm_check reports (or of the width that b200_gemm_check_columns does, or the skinny-M kernel, which splits K by rules of its own).
@@ -142,7 +142,7 @@ int b200_gemm_check(const b200_gemm_args* args, int32_t* chosen_tile);
 int b200_gemm_check_split(const b200_gemm_args* args, int32_t* parts);
 /* What the calling thread's last launch of a tile kernel did: the CTAs per tile when K was split, otherwise 0.        */
 int b200_last_k_split(void);
-/* Columns of the 128-row tiles, one CTA each, on which a grid of one round is computed with TILE_AUTO, 32 to 224; 0: the tile that
+/* Columns of the 128-row tiles, one CTA each, on which a grid of few rounds is computed with TILE_AUTO, 32 to 224; 0: the tile that
  * b200_gemm_check reports, or a split one.  bf16_operands: the answer for b200_gemm_a16w16.                            */
 int b200_gemm_check_columns(const b200_gemm_args* args, int32_t bf16_operands, int32_t* columns);
 /* Columns of the tiles of the calling thread's last tile-kernel launch (a pair's too).                                 */

@@ -31,6 +31,10 @@ def test_choice(native):
     assert columns(native, 100, 148 * 32, 896) == 32 and columns(native, 100, 148 * 32 + 8, 896) == 64
     assert columns(native, 140, 4744, 640) == 128 and columns(native, 140, 14216, 640) == 0 and columns(native, 140, 74 * 224 + 8, 896) == 0
     assert columns(native, 140, 360, 896, batch=7) == 64
+    # several rounds without scales: 160 and 192 where they fill the last one better; a pair's tile stays where rows are not whole lines apart and K is long
+    assert columns(native, 2000, 3000, 1024, bf16=True) == 192 and columns(native, 1100, 5120, 512, bf16=True) == 160
+    assert columns(native, 4096, 4096, 4096, bf16=True) == 0 and columns(native, 2000, 3000, 1000, bf16=True) == 0 and columns(native, 2000, 3000, 504, bf16=True) == 192
+    assert columns(native, 1200, 5120, 2048, L.SCALE_BLOCK) == 0
     # not: a tile that is asked for, K that is split, MX, few tokens on the skinny-M kernel, inputs that are ready where the tile is a pair's
     assert columns(native, 140, 360, 896, hint=L.TILE_128x128) == 0 and columns(native, 256, 512, 8192) == 0
     assert columns(native, 140, 2432, 896, L.SCALE_MX) == 0 and columns(native, 64, 2432, 896) == 0
@@ -59,6 +63,21 @@ def test_widths(api, mode, w, n, nb, kblocks):
             assert torch.equal(big[1:m + 1, left:n + left], ref.to(dt))
             big[1:m + 1, left:n + left] = 7.0
             assert torch.all(big == 7.0)
+    assert api.last_status() == 0
+
+
+# several tiles per CTA: rings, accumulator buffers and the staging beside the ring run on from one to the next
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,w,m,n", [("bf16", 192, 2003, 3000), ("bf16", 160, 1101, 5112), ("none", 192, 574, 10180), ("none", 160, 300, 14776)])
+@pytest.mark.parametrize("kblocks", [1, 3, 5, 6, 9])
+def test_several_rounds(api, mode, w, m, n, kblocks):
+    k = kblocks * (64 if mode == "bf16" else 128)
+    run, ref = call(api, mode, whole(m, k, 1), whole(n, k, 2), 0)
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.full((m, n), 7.0, dtype=dt, device=DEV)
+        run(out)
+        assert api.last_columns() == w
+        assert torch.equal(out, ref.to(dt))
     assert api.last_status() == 0
 
 
