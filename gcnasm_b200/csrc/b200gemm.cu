@@ -261,13 +261,14 @@ int64_t mx_skinny_kblocks(int64_t m, int64_t panels, int sm_count) {
 }
 
 // CTAs that share a 128 x 128 tile, each with a part of K: as many as bring the K blocks of a CTA down furthest, if the clusters are all
-// resident and what is saved is worth more than the exchange of the partial sums.  In K blocks, that takes 9 (block and MX scales, 0.31
-// us a block) or 13 (0.21 us; 15 on tiles of few rows, whose blocks are shorter) on few tiles, more on many, and a cluster of more than
-// four two more.  Whole / split, us, weights from HBM, K = 2048, 4096, 8192:
-//   8-bit         100 x 512 (4 tiles)    6.5 / 6.2    9.9 / 6.6   16.7 / 7.5     256 x 4608 (72)   7.2 / 8.3   10.8 / 10.4   17.6 / 14.4
-//                 256 x 2048 (32)        6.9 / 7.6   10.4 / 8.8   17.3 / 10.9
-//   block scales  100 x 512              8.2 / 6.8   13.2 / 7.3   23.3 / 8.5     256 x 4608        9.1 / 9.2   14.2 / 12.0   24.3 / 17.1
-//                 256 x 2048             8.7 / 8.2   13.8 / 9.6   23.9 / 12.4
+// resident and what is saved is worth more than the exchange of the partial sums.  In K blocks, that takes 9 (block and MX scales, 0.25 and
+// 0.31 us a block) or 13 (0.2 us; 15 on tiles of few rows, whose blocks are shorter) on few tiles, more on many, and a cluster of more than
+// four two more.  Whole 128 x 128 tiles / split, us, weights from HBM, K = 2048, 4096, 8192 (narrow whole tiles where that is in brackets):
+//   8-bit         100 x 512 (4 tiles)    6.2 (5.6)    9.2 / 6.6   15.1 / 7.5     256 x 4608 (72)   6.9 (6.3)    9.9 (9.4)    16.4 / 14.2
+//                 256 x 2048 (32)        6.5 (5.8)    9.6 / 8.7   15.6 / 10.8
+//   block scales  100 x 512              6.9 (6.1)   10.6 / 6.9   18.8 / 7.8     256 x 4608        7.4 (6.9)   11.9 / 10.8   20.1 / 15.0
+//                 256 x 2048             7.2 (6.3)   11.4 / 9.0   19.5 / 11.3
+//   MX            100 x 512              7.4 / 6.4   11.8 / 6.8   20.8 / 8.1     256 x 4608        8.1 / 8.1   12.7 / 11.5   21.8 / 16.8
 // (At 1024 8-bit operands lose 1 us, block scales 0.5; MX 1705 x 256 x 1536 6.4 / 6.9, 8-bit 12 x 4232 x 3328 8.1 / 8.7.)
 constexpr int kMaxTileSplits = 8;
 constexpr int kSplitClusters[kMaxTileSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};     // resident at once on 148 SMs
@@ -275,6 +276,8 @@ constexpr int kSplitClusters[kMaxTileSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 
 // not whole 128-byte lines apart, and up to 47 K blocks where B comes out of L2; with more tiles a whole tile is the slow one.  Whole /
 // split, us, without scales: 4 x 6024 x 5872 15.6 / 19.7, x 8176 23.0 / 29.7, x 5376 with B from HBM 15.9 / 14.5, out of L2 12.0 / 13.9.  Mean
 // of split / whole over 3000 sizes: other pitches 0.98 (0.7 to 1.4), whole lines and 48 K blocks or more 0.84, with B out of L2 0.87.
+// (What had made them slower were the rows of A's box that are not there, see kBoxRows.  Since that box is of the rows that there are two CTAs are the
+// faster ones at these sizes too, 4 x 6024 x 5872 12.1 / 11.1, out of L2 11.3 / 9.4; the line still stands, with the test that holds it.)
 // *equal: the K blocks that a CTA would take as long for; lines: rows of A and B whole 128-byte lines apart
 int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, bool lines, int sm_count, int64_t* equal = nullptr) {
     const int64_t exchange = slow ? 9 + tiles / 32 : (m <= 32 ? 15 : 13) + tiles / 12;
