@@ -303,14 +303,16 @@ int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, bool lines
 //   8-bit         256 x 512 x 1024    128 columns 4.5 / 32 3.6       333 x 7168 x 2048   256 columns 10.7 / 160 8.5    700 x 2048 x 7168  128 15.6 / 96 14.9
 //   block scales  129 x 1024 x 1024   128         5.0 / 32 4.1       333 x 7168 x 2048   256         11.9 / 160 9.7    100 x 7168 x 2048  128  7.8 / 64  7.1
 //   bf16          64 x 8192 x 2048    128        10.4 / 64 9.7       333 x 7168 x 1024   256 (pair)  10.9 / 160 8.5
+//   MX            256 x 1024 x 1024   128         5.1 / 64 4.6       333 x 7168 x 2048   256 (pair)  11.3 / 192 9.3    1000 x 3456 x 2048  256  11.1 / 192 9.2
+// MX: 64, 128 and 192, which begin at the first or the third scale word of an atom of 128 columns (mean of 1850 sizes 0.944).
 // Not 96 or 224 columns for a short K (96 for 128: 175 x 6272 x 384 3.72 / 3.86; 224 for 256: 269 x 10240 x 256 4.96 / 5.67), not 224 with block scales,
 // whose 256 columns take no longer, and nothing in the place of 256 (two rows of tiles and a long K are the pair's: 430 x 8448 x 7552 26.8 / 29.8).
 // apart: the tile would be a pair's and rows are not whole 128-byte lines apart.  Every row of a box then lies in two lines, what a K block takes out of L2
 // 1.6 times as much, and a pair, which takes less of it, is ahead of wide tiles from some K on; narrow over pair by K blocks, mean: 8-bit 160 columns 0.94 from 16
 // to 24 (950 x 2816 x 2672 12.4 / 13.5), 1.03 to 36 and 1.09 above; 192 0.87 up to 10, then 1.04, 1.24 above 36; bf16 224 1.0 from 24 on (658 x 4872 x 6000 24.0 / 30.0, x 6016 20.0 / 20.0).
-int one_round_columns(int64_t tm, int64_t n, int64_t batch, int64_t kblocks, bool block, bool apart, bool ab16, int sm_count) {
+int one_round_columns(int64_t tm, int64_t n, int64_t batch, int64_t kblocks, bool block, bool mx, bool apart, bool ab16, int sm_count) {
     for (int w : {32, 64, 96, 128, 160, 192, 224}) {
-        if (tm * ((n + w - 1) / w) * batch > sm_count) continue;
+        if (tm * ((n + w - 1) / w) * batch > sm_count || (mx && w % 64 != 0)) continue;
         if ((w == 96 || w == 224) && kblocks < 6) continue;
         if (apart && kblocks >= (ab16 ? (w == 224 ? 24 : 1 << 30) : w >= 192 ? 10 : w == 160 ? 20 : 1 << 30)) return 0;
         return w == 224 && block ? 0 : w;
@@ -461,12 +463,12 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, lines, sm_count, &equal);
                 if (s > 1 && 10 * 128 * (ab16 ? 155 : a->scale_mode == B200_SCALE_BLOCK ? 125 : 130) * equal < best * kblocks) pl.splits = s;
                 const bool block = a->scale_mode == B200_SCALE_BLOCK, single = hint == B200_TILE_128x128 || hint == B200_TILE_128x256;
-                const int columns = mx ? 0 : one_round_columns(tm1, a->n, a->batch, kblocks, block, !single && !lines, ab16, sm_count);
+                const int columns = one_round_columns(tm1, a->n, a->batch, kblocks, block, mx, !single && !lines, ab16, sm_count);
                 // A split takes as long as `equal` K blocks on 128 columns; narrow tiles are worth three more (block scales four, 32 columns one more).
                 // Narrow over split by kblocks - equal, mean of 640 / 870 sizes: 8-bit 0.956 at 0 and 1, 0.988 at 2 and 3, 1.033 at 4 and 5; block scales
                 // 0.892, 0.938, 1.004, 1.07 at 6 and 7; bf16 1.045, 1.07; 8-bit rows not whole lines apart 0.94, 0.995 (100 x 4480 x 3312 8.9 / 10.7).
                 // Not for few rows, whose sums are quick (2 x 392 x 2816 4.4 / 6.1, block scales 68 x 384 x 2304, two batches, 6.1 / 6.6).
-                const int64_t worth = ab16 || a->m <= 80 ? 0 : !lines ? 1 : (block ? 4 : 3) + (columns == 32);
+                const int64_t worth = ab16 || mx || a->m <= 80 ? 0 : !lines ? 1 : (block ? 4 : 3) + (columns == 32);
                 if (columns && kblocks - equal < worth) pl.splits = 1;
                 if (pl.splits == 1) pl.columns = columns;
                 // Several rounds without scales: 160 and 192 columns on one CTA, where they waste less of the last round (weights as above; bf16 has no pair tiles
@@ -626,6 +628,14 @@ int launch_gemm128(const GemmParams& p, int grid, cudaStream_t st) {
 // ... and of any width that is built
 template <int MODE, int BL>
 int launch_columns(int columns, const GemmParams& p, int grid, cudaStream_t st) {
+    if constexpr (MODE == MODE_MX) {
+        switch (columns) {
+            case 64: return launch_gemm<64, MODE, BL>(p, grid, st);
+            case 128: return launch_gemm128<MODE, BL>(p, grid, st);
+            case 192: return launch_gemm<192, MODE, BL>(p, grid, st);
+            default: return B200_ERR_UNSUPPORTED;
+        }
+    } else
     switch (columns) {
         case 32: return launch_gemm<32, MODE, BL>(p, grid, st);
         case 64: return launch_gemm<64, MODE, BL>(p, grid, st);
@@ -1109,7 +1119,7 @@ int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStrea
         case B200_SCALE_BLOCK:
             return flat ? launch_columns<MODE_BLOCK, BL_FLAT>(BN, p, grid, st) : launch_columns<MODE_BLOCK, BL_NK>(BN, p, grid, st);
         case B200_SCALE_MX:
-            return flat ? launch_gemm128<MODE_MX, BL_FLAT>(p, grid, st) : launch_gemm128<MODE_MX, BL_NK>(p, grid, st);
+            return flat ? launch_columns<MODE_MX, BL_FLAT>(BN, p, grid, st) : launch_columns<MODE_MX, BL_NK>(BN, p, grid, st);
         default:
             return flat ? launch_columns<MODE_ACC, BL_FLAT>(BN, p, grid, st) : launch_columns<MODE_ACC, BL_NK>(BN, p, grid, st);
     }

@@ -16,8 +16,8 @@
 // 128-wide K group a FRESH buffer (the reference does the same with a fresh MFMA accumulator,
 // kernel_template.hpp:317,334) and the epilogue warps fold it into register accumulators with
 // acc += partial * (sfa[g][row] * sfb[nblk][g]) -- the analogue of scale_c_tile.
-// Tiles are 128 rows by 128 or 256 columns, or in a grid of one round by as few as bring all SMs to work (32 to 224, one_round_columns() of
-// the launcher).  Few tiles with a long K: the CTAs of a cluster take a part of a 128 x 128 tile's K each (SPLIT) and sum their results in
+// Tiles are 128 rows by 128 or 256 columns, or in a grid of one round by as few as bring all SMs to work (32 to 224, MX 64 or 192, one_round_columns()
+// of the launcher).  Few tiles with a long K: the CTAs of a cluster take a part of a 128 x 128 tile's K each (SPLIT) and sum their results in
 // distributed shared memory; tile_splits() of the launcher says when.
 #pragma once
 
@@ -124,7 +124,7 @@ struct GemmCfg {
     static constexpr int THREADS = 384;
     static_assert(ACC_COLS + SF_COLS <= 512, "TMEM overflow");
     static_assert(BN % 32 == 0 && BN <= 256, "BN must be a multiple of 32, at most 256");
-    static_assert(MODE != MODE_MX || BN % 128 == 0, "MX scale atoms cover 128 columns");
+    static_assert(MODE != MODE_MX || BN % 64 == 0, "MX scales: a tile begins at the first or third column word of an atom of 128 columns");
     static_assert(STAGES >= 3 && STAGES_ONE <= 8, "ring depth");
     // a stage that is free says that the group STAGES + BUFS before its next one has been drained
     static_assert(!FEED || STAGES_ONE + BUFS <= SF_SLOTS, "scales stay until their group has been drained");
@@ -456,7 +456,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
                 int b, mi, ni;
                 tile_coords(p, t, b, mi, ni);
-                const uint32_t bytes = p.a_rows * BK + Cfg::B_BYTES + Cfg::SFA_BYTES + Cfg::SFB_BYTES;
+                // MX: the atoms of 128 columns that the tile lies in, as far as there are
+                const int atom_b = ni * BN / 128;
+                const uint32_t sfb_bytes = MODE != MODE_MX ? 0u : BN <= 128 || atom_b + 1 < p.sfb_stride ? Cfg::SFB_BYTES : 512u;
+                const uint32_t bytes = p.a_rows * BK + Cfg::B_BYTES + Cfg::SFA_BYTES + sfb_bytes;
                 for (int kb = kb0; kb < kb0 + kblocks; ++kb, next_stage(s, ph)) {
                     if (!mbar_wait(bar_empty0 + s * 8, ph ^ 1, abort_flag, p.status, KSTAT_TIMEOUT_EMPTY)) {
                         ok = false;
@@ -477,9 +480,9 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                         const uint8_t* sfa = reinterpret_cast<const uint8_t*>(p.sfa) + b * p.sfa_batch +
                                              (static_cast<long long>(kb) * p.sfa_stride + mi) * 512;
                         const uint8_t* sfb = reinterpret_cast<const uint8_t*>(p.sfb) + b * p.sfb_batch +
-                                             (static_cast<long long>(kb) * p.sfb_stride + ni * Cfg::SFB_ATOMS) * 512;
+                                             (static_cast<long long>(kb) * p.sfb_stride + atom_b) * 512;
                         bulk_load(sb + Cfg::B_BYTES, sfa, 512, full);
-                        bulk_load(sb + Cfg::B_BYTES + 512, sfb, Cfg::SFB_BYTES, full);
+                        bulk_load(sb + Cfg::B_BYTES + 512, sfb, sfb_bytes, full);
                     }
                 }
             }
@@ -493,6 +496,12 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
             bool ok = true, full_seen = false, free_seen = false;
             constexpr uint32_t idesc = make_idesc_f8(BM, BN);
             for (int t = Cfg::SPLIT ? split_tile : static_cast<int>(blockIdx.x); t < p.tiles_total && ok; t += Cfg::SPLIT ? p.tiles_total : static_cast<int>(gridDim.x)) {
+                uint32_t sf_col = 0;                             // MX: the tile's first scale word in its first atom
+                if constexpr (MODE == MODE_MX && BN % 128 != 0) {
+                    int b, mi, ni;
+                    tile_coords(p, t, b, mi, ni);
+                    sf_col = (ni * BN & 127) / 32;
+                }
                 for (int g = 0; g < groups && ok; ++g, ++phase) {
                     const uint32_t as = phase % BUFS;
                     const uint32_t aph = (phase / BUFS) & 1;
@@ -536,7 +545,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_a8w8_sm100_kernel(const 
                             const uint32_t accum = (kb > 0 || k > 0) ? 1u : 0u;
                             if constexpr (MODE == MODE_MX) {
                                 const uint32_t tsf = tmem_base + Cfg::ACC_COLS;
-                                umma_mxf8<1>(tacc, da, db, make_idesc_mxf8(BM, BN, k, k), accum, tsf, tsf + 4);
+                                umma_mxf8<1>(tacc, da, db, make_idesc_mxf8(BM, BN, k, k), accum, tsf, tsf + 4 + sf_col);
                             } else {
                                 if constexpr (Cfg::AB16) umma_f16<1>(tacc, da, db, make_idesc_bf16(BM, BN), accum);
                                 else umma_f8<1>(tacc, da, db, idesc, accum);

@@ -35,9 +35,11 @@ def test_choice(native):
     assert columns(native, 2000, 3000, 1024, bf16=True) == 192 and columns(native, 1100, 5120, 512, bf16=True) == 160
     assert columns(native, 4096, 4096, 4096, bf16=True) == 0 and columns(native, 2000, 3000, 1000, bf16=True) == 0 and columns(native, 2000, 3000, 504, bf16=True) == 192
     assert columns(native, 1200, 5120, 2048, L.SCALE_BLOCK) == 0
-    # not: a tile that is asked for, K that is split, MX, few tokens on the skinny-M kernel, inputs that are ready where the tile is a pair's
+    # MX: the widths that begin at whole or half atoms of 128 columns
+    assert [columns(native, 140, n, 896, L.SCALE_MX) for n in (360, 2376, 4736, 4744, 9472, 9480, 14208, 14216)] == [64, 64, 64, 128, 128, 192, 192, 0]
+    # not: a tile that is asked for, K that is split, few tokens on the skinny-M kernel, inputs that are ready where the tile is a pair's
     assert columns(native, 140, 360, 896, hint=L.TILE_128x128) == 0 and columns(native, 256, 512, 8192) == 0
-    assert columns(native, 140, 2432, 896, L.SCALE_MX) == 0 and columns(native, 64, 2432, 896) == 0
+    assert columns(native, 64, 2432, 896) == 0
     assert columns(native, 256, 512, 1024, flags=L.GEMM_INPUTS_READY) == 0 and columns(native, 100, 512, 1024, flags=L.GEMM_INPUTS_READY) == 32
 
 
@@ -63,6 +65,20 @@ def test_widths(api, mode, w, n, nb, kblocks):
             assert torch.equal(big[1:m + 1, left:n + left], ref.to(dt))
             big[1:m + 1, left:n + left] = 7.0
             assert torch.all(big == 7.0)
+    assert api.last_status() == 0
+
+
+# MX: tiles that begin in the middle of an atom, the last one with one of its two atoms or none of the second half, with every scale another
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,m,n", [(64, 140, 360), (64, 140, 2376), (64, 200, 2440), (128, 140, 4744), (192, 140, 9480), (192, 129, 9600), (192, 140, 9696), (192, 256, 14136)])
+@pytest.mark.parametrize("kblocks", [1, 2, 5, 7])
+def test_mx_widths(api, w, m, n, kblocks):
+    run, ref = call(api, "mx", whole(m, 128 * kblocks, 1), whole(n, 128 * kblocks, 2), 0)
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.full((m, n), 7.0, dtype=dt, device=DEV)
+        run(out)
+        assert api.last_columns() == w
+        assert torch.equal(out, ref.to(dt))
     assert api.last_status() == 0
 
 
