@@ -474,12 +474,13 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 // Several rounds without scales: 160 and 192 columns on one CTA, where they waste less of the last round (weights as above; bf16 has no pair tiles
                 // of other widths to choose from).  Tile as before / so, mean of random sizes: bf16 0.865 (a third of 1690 sizes change), 8-bit 0.88 (one of 16);
                 // 2000 x 3000 x 1024 bf16 15.5 / 14.7, 1000 x 6000 x 512 10.7 / 9.5.  A pair stays where rows are not whole lines apart, from ten K blocks on (bf16 1.0
-                // at 16 to 24, 1.07 above 40), and with block scales, whose 160 and 192 columns take as long as 256 (700 x 8192 x 1024 12.6 / 13.4).
-                if (pl.splits == 1 && !columns && !mx && !block && (single || lines || kblocks < 10)) {
+                // at 16 to 24, 1.07 above 40), and with block scales, whose 160 and 192 columns take as long as 256 (700 x 8192 x 1024 12.6 / 13.4).  MX: 192 columns
+                // for the pair's 256, up to ten K blocks (0.81 up to three, 0.88 to nine, then 0.97 and above twenty 1.02).
+                if (pl.splits == 1 && !columns && !block && (mx ? !single && kblocks < 10 : single || lines || kblocks < 10)) {
                     constexpr int kWide[2][2] = {{160, 135}, {192, 125}};
                     for (const auto& c : kWide) {
                         const int64_t rounds = (tm1 * ((a->n + c[0] - 1) / c[0]) * a->batch + sm_count - 1) / sm_count, cost = rounds * 10 * c[0] * c[1];
-                        if (rounds > 1 && cost < best) {
+                        if (rounds > 1 && cost < best && !(mx && c[0] != 192)) {
                             best = cost;
                             pl.columns = c[0];
                         }

@@ -35,6 +35,7 @@ def test_choice(native):
     assert columns(native, 2000, 3000, 1024, bf16=True) == 192 and columns(native, 1100, 5120, 512, bf16=True) == 160
     assert columns(native, 4096, 4096, 4096, bf16=True) == 0 and columns(native, 2000, 3000, 1000, bf16=True) == 0 and columns(native, 2000, 3000, 504, bf16=True) == 192
     assert columns(native, 1200, 5120, 2048, L.SCALE_BLOCK) == 0
+    assert columns(native, 776, 5504, 1152, L.SCALE_MX, batch=2) == 192 and columns(native, 776, 5504, 1280, L.SCALE_MX, batch=2) == 0
     # MX: the widths that begin at whole or half atoms of 128 columns
     assert [columns(native, 140, n, 896, L.SCALE_MX) for n in (360, 2376, 4736, 4744, 9472, 9480, 14208, 14216)] == [64, 64, 64, 128, 128, 192, 192, 0]
     # not: a tile that is asked for, K that is split, few tokens on the skinny-M kernel, inputs that are ready where the tile is a pair's
@@ -84,7 +85,7 @@ def test_mx_widths(api, w, m, n, kblocks):
 
 # several tiles per CTA: rings, accumulator buffers and the staging beside the ring run on from one to the next
 @pytest.mark.gpu
-@pytest.mark.parametrize("mode,w,m,n", [("bf16", 192, 2003, 3000), ("bf16", 160, 1101, 5112), ("none", 192, 574, 10180), ("none", 160, 300, 14776)])
+@pytest.mark.parametrize("mode,w,m,n", [("bf16", 192, 2003, 3000), ("bf16", 160, 1101, 5112), ("none", 192, 574, 10180), ("none", 160, 300, 14776), ("mx", 192, 2171, 4352)])
 @pytest.mark.parametrize("kblocks", [1, 3, 5, 6, 9])
 def test_several_rounds(api, mode, w, m, n, kblocks):
     k = kblocks * (64 if mode == "bf16" else 128)
