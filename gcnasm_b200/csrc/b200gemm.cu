@@ -989,7 +989,7 @@ int run_decode(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStr
 // accumulator that nobody stores).  A box that reaches beyond the matrix is filled with zeros, but each row that is not there still
 // costs a request, all of them in few places of L2: boxes of 128 rows in a ring of six on 144 CTAs take 918 clocks each with one row there,
 // 806 with 24, 522 with 32 and more; boxes of 16 rows with one there 522.  128 rows / the rows there are, us: bf16 1 x 5440 x 1792 11.7 / 8.8, 16 x 5440 x
-// 2048 10.6 / 8.2, 4 x 8192 x 4096 18.9 / 14.5, 8-bit 5 x 5448 x 4096 10.5 / 7.9; 40 x 5440 x 2048 the same, 1 x 1024 x 1024 (8 tiles) 5.4 / 5.55.  The few rows
+// 2048 10.6 / 8.2, 4 x 8192 x 4096 18.9 / 14.5, 8-bit 5 x 5448 x 4096 10.5 / 7.9; 40 x 5440 x 2048 and 1 x 1024 x 1024 (8 tiles) the same.  The few rows
 // of a last tile below others are not worth a second box: its CTAs are half of a grid at most (8-bit 140 x 8192 x 2048 6.4 / 6.45).
 constexpr int kBoxRows = 127;
 
