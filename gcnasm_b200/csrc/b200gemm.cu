@@ -267,6 +267,52 @@ int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, bool lines
     return best;
 }
 
+// How the rows of an operand lie in memory, best first: each begins at a whole 128-byte line; at whole 32-byte sectors, some at a line; all of them within a line; every other
+// one within a sector; all of them within a sector (a view that begins at an odd multiple of 16 bytes).  A row of a box then is in two lines, with the last two also in five
+// sectors instead of four.
+enum : int { kLines = 0, kSectors = 1, kOffLines = 2, kHalfSectors = 3, kNoSectors = 4 };
+int row_starts(const void* base, int64_t pitch, int64_t batch_stride) {
+    if (pitch % 32 != 0) return kHalfSectors;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(base) | static_cast<uintptr_t>(batch_stride);
+    return (at & 31) != 0 ? kNoSectors : pitch % 128 != 0 ? kSectors : (at & 127) != 0 ? kOffLines : kLines;
+}
+
+// A grid of one round on `w` columns against a pair's tiles: the K blocks from which the pair is kept.  It takes less out of L2 for a K block, and of what the rows make
+// dear; one CTA has the shorter way in and out.  One CTA / pair, mean over K blocks (100,000 random sizes; * with two rows of tiles):
+//   whole sectors  8-bit  160   0.95 at 20;  192 0.92 at 9;  bf16 224 1.00 from 24 on, 160 and 192 0.75 to 0.96
+//   off lines      8-bit  160   0.95 to 24, 1.03 above, 1.09 from 40;  192 1.00 at 12, 1.03 at 20, 1.17 above 40, * 0.96 at 15, 1.05 at 20;  224 1.08 to 1.16 (1794 x 1888 x 7168 28.3 / 22.4)
+//                  bf16   192   0.99 at 35, 1.05 above 40;  224 0.98 at 20, 1.04 at 27, 1.12 above 30;  MX 192 0.97 at 27, 1.02 at 35, 1.06 above 40
+//   half sectors   8-bit  160   0.97 from 12 to 14, 1.01 to 17, then 1.03;  192 0.98 at 9
+//                  bf16   160   0.99 from 33 to 38, then 1.01 to 1.03, * 0.97 at 24, 1.02 at 27;  192 0.96 from 15, 1.00 from 18, 1.03 from 24, then to 1.13, * 1.00 at 15, 1.07 at
+//                               18 (142 x 13792 x 3480 37.2 / 30.9);  224 0.98 from 9, 1.00 from 12, 1.04 from 15 to 1.10, * 1.03 from 9
+//   no sectors     8-bit  160   0.97 from 9 to 14, then 1.04 to 1.19;  192 0.99 at 9, 1.10 from 12 on to 1.36;  224 1.25 to 1.46;  bf16 about as half sectors;  MX 192 0.96 from
+//                               12, 1.00 from 15, 1.04 from 21 to 1.20
+int64_t pair_from(int w, int64_t tm, int rows, bool block, bool mx, bool ab16) {
+    constexpr int64_t never = int64_t{1} << 62;
+    if (w < 160 || rows == kLines || (block && rows == kOffLines)) return never;
+    if (ab16) {
+        if (rows <= kOffLines) return w == 224 ? 24 : w == 192 && rows == kOffLines ? 40 : never;
+        return w == 160 ? (tm <= 2 ? 25 : 36) : w == 192 ? (tm <= 2 ? 15 : 18) : (tm <= 2 ? 10 : 13);
+    }
+    if (mx) return rows == kNoSectors ? 16 : rows == kOffLines ? 34 : 10;
+    if (w == 160) return rows == kSectors ? 20 : rows == kOffLines ? 25 : 15;
+    return rows == kOffLines ? (tm <= 2 ? 16 : 13) : 10;
+}
+
+// ... and in several rounds against a pair's 256 columns.  By K blocks, 192 columns: half sectors 8-bit 0.97 at 6, 0.99 at 7, 1.05 at 8, bf16 0.99 at 8, 1.00 at 9, MX 0.99 at 9;
+// no sectors 8-bit 0.97 at 5, 1.03 at 6, bf16 0.98 at 6, 1.00 at 7, MX 0.98 at 7, 1.00 at 8; off lines 8-bit 1.00 at 11, 1.04 at 14, bf16 0.97 at 14, 1.00 at 17.  160 columns: off
+// lines 1.00 at 35, 1.02 above; no sectors 8-bit 1.04 at 9, bf16 0.95 at 11.
+int64_t pair_from_rounds(int w, int rows, bool mx, bool ab16) {
+    if (mx) return rows == kNoSectors ? 8 : 10;
+    switch (rows) {
+        case kLines: return int64_t{1} << 62;
+        case kOffLines: return w == 160 ? 40 : ab16 ? 17 : 12;
+        case kHalfSectors: return w == 160 ? 10 : ab16 ? 9 : 7;
+        case kNoSectors: return w == 160 ? (ab16 ? 14 : 9) : ab16 ? 7 : 6;
+        default: return 10;
+    }
+}
+
 // One CTA's tiles in a grid of one round: the fewest columns that make one.  A K block takes what its operand tiles take out of L2, 128 rows of
 // A and the tile's of B at some 70 bytes a clock, and the way in and out of a tile is the shorter the narrower it is, so as long as SMs are
 // idle a narrower tile on more of them wins; and 160 to 224 columns make one round of what would be two of 128, or 256 with SMs idle.  us, kind of tile as
@@ -278,14 +324,12 @@ int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, bool lines
 // MX: 64, 128 and 192, which begin at the first or the third scale word of an atom of 128 columns (mean of 1850 sizes 0.944).
 // Not 96 or 224 columns for a short K (96 for 128: 175 x 6272 x 384 3.72 / 3.86; 224 for 256: 269 x 10240 x 256 4.96 / 5.67), not 224 with block scales,
 // whose 256 columns take no longer, and nothing in the place of 256 (two rows of tiles and a long K are the pair's: 430 x 8448 x 7552 26.8 / 29.8).
-// apart: the tile would be a pair's and rows are not whole 128-byte lines apart.  Every row of a box then lies in two lines, what a K block takes out of L2
-// 1.6 times as much, and a pair, which takes less of it, is ahead of wide tiles from some K on; narrow over pair by K blocks, mean: 8-bit 160 columns 0.94 from 16
-// to 24 (950 x 2816 x 2672 12.4 / 13.5), 1.03 to 36 and 1.09 above; 192 0.87 up to 10, then 1.04, 1.24 above 36; bf16 224 1.0 from 24 on (658 x 4872 x 6000 24.0 / 30.0, x 6016 20.0 / 20.0).
-int one_round_columns(int64_t tm, int64_t n, int64_t batch, int64_t kblocks, bool block, bool mx, bool apart, bool ab16, int sm_count) {
+// pair: the tile would be a pair's, rows: how they lie in memory (see row_starts).
+int one_round_columns(int64_t tm, int64_t n, int64_t batch, int64_t kblocks, bool block, bool mx, bool pair, int rows, bool ab16, int sm_count) {
     for (int w : {32, 64, 96, 128, 160, 192, 224}) {
         if (tm * ((n + w - 1) / w) * batch > sm_count || (mx && w % 64 != 0)) continue;
         if ((w == 96 || w == 224) && kblocks < 6) continue;
-        if (apart && kblocks >= (ab16 ? (w == 224 ? 24 : 1 << 30) : w >= 192 ? 10 : w == 160 ? 20 : 1 << 30)) return 0;
+        if (pair && kblocks >= pair_from(w, tm, rows, block, mx, ab16)) return 0;
         return w == 224 && block ? 0 : w;
     }
     return 0;
@@ -430,16 +474,21 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
             const bool starts_early = (a->flags & B200_GEMM_INPUTS_READY) && hint != B200_TILE_128x128 && hint != B200_TILE_128x256;
             if (!pair_only && !starts_early) {
                 int64_t equal;
-                const bool lines = a->stride_a % 128 == 0 && (a->b_layout == B200_B_FLAT_16x16 || a->stride_b % 128 == 0);
+                const int rows_a = row_starts(a->ptr_a, a->stride_a, a->batch > 1 ? a->stride_a_batch : 0);
+                const int rows_b = a->b_layout == B200_B_FLAT_16x16 ? kLines : row_starts(a->ptr_b, a->stride_b, a->batch > 1 ? a->stride_b_batch : 0);
+                const int rows = rows_a > rows_b ? rows_a : rows_b;
+                const bool lines = rows == kLines || rows == kOffLines;
                 const int s = tile_splits(a->m, tm1 * ((a->n + 127) / 128) * a->batch, kblocks, slow, lines, sm_count, &equal);
                 if (s > 1 && 10 * 128 * (ab16 ? 155 : a->scale_mode == B200_SCALE_BLOCK ? 125 : 130) * equal < best * kblocks) pl.splits = s;
                 const bool block = a->scale_mode == B200_SCALE_BLOCK, single = hint == B200_TILE_128x128 || hint == B200_TILE_128x256;
-                const int columns = one_round_columns(tm1, a->n, a->batch, kblocks, block, mx, !single && !lines, ab16, sm_count);
-                // A split takes as long as `equal` K blocks on 128 columns; narrow tiles are worth three more (block scales four, 32 columns one more).
-                // Narrow over split by kblocks - equal, mean of 640 / 870 sizes: 8-bit 0.956 at 0 and 1, 0.988 at 2 and 3, 1.033 at 4 and 5; block scales
-                // 0.892, 0.938, 1.004, 1.07 at 6 and 7; bf16 1.045, 1.07; 8-bit rows not whole lines apart 0.94, 0.995 (100 x 4480 x 3312 8.9 / 10.7).
+                const int columns = one_round_columns(tm1, a->n, a->batch, kblocks, block, mx, !single, rows, ab16, sm_count);
+                // A split takes as long as `equal` K blocks on 128 columns; narrow tiles are worth two more (block scales three), 32 columns one more.
+                // Narrow over split by kblocks - equal, mean of 430 / 990 sizes: 8-bit 0.93 at 1, 0.95 at 2, 0.97 at 3; block scales 0.86, 0.89, 0.92, 0.95 at 4.
+                // Rows that begin within sectors: 8-bit 32 columns 0.99 at 1, 1.02 at 2, otherwise to 1.14; block scales 64 columns 0.97, 1.01, 1.01, 32 as above.
                 // Not for few rows, whose sums are quick (2 x 392 x 2816 4.4 / 6.1, block scales 68 x 384 x 2304, two batches, 6.1 / 6.6).
-                const int64_t worth = ab16 || mx || a->m <= 80 ? 0 : !lines ? 1 : (block ? 4 : 3) + (columns == 32);
+                int64_t worth = (block ? 4 : 3) + (columns == 32);
+                if (ab16 || mx || a->m <= 80) worth = 0;
+                else if (!lines) worth = rows != kNoSectors ? 1 : columns != 32 ? (block ? 2 : 1) : block ? worth : 2;
                 if (columns && kblocks - equal < worth) pl.splits = 1;
                 if (pl.splits == 1) pl.columns = columns;
                 // Several rounds without scales: 160 and 192 columns on one CTA, where they waste less of the last round (weights as above; bf16 has no pair tiles
@@ -447,11 +496,16 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 // 2000 x 3000 x 1024 bf16 15.5 / 14.7, 1000 x 6000 x 512 10.7 / 9.5.  A pair stays where rows are not whole lines apart, from ten K blocks on (bf16 1.0
                 // at 16 to 24, 1.07 above 40), and with block scales, whose 160 and 192 columns take as long as 256 (700 x 8192 x 1024 12.6 / 13.4).  MX: 192 columns
                 // for the pair's 256, up to ten K blocks (0.81 up to three, 0.88 to nine, then 0.97 and above twenty 1.02).
-                if (pl.splits == 1 && !columns && !block && (mx ? !single && kblocks < 10 : single || lines || kblocks < 10)) {
+                // Not for a pair's 224 or 192 where rows begin within sectors (1.00 to 1.06; 2546 x 1304 x 912 10.0 / 9.3, 1352 x 2480 x 1040, two batches, 17.2 / 15.1),
+                // nor for 224 of whole sectors (1.00).
+                if (pl.splits == 1 && !columns && !block) {
                     constexpr int kWide[2][2] = {{160, 135}, {192, 125}};
+                    const bool pair224 = hint == B200_TILE_PAIR_256x224, narrow_pair = pair224 || hint == B200_TILE_PAIR_256x192;
                     for (const auto& c : kWide) {
                         const int64_t rounds = (tm1 * ((a->n + c[0] - 1) / c[0]) * a->batch + sm_count - 1) / sm_count, cost = rounds * 10 * c[0] * c[1];
-                        if (rounds > 1 && cost < best && !(mx && c[0] != 192)) {
+                        if ((mx && (single || c[0] != 192)) || (!single && kblocks >= pair_from_rounds(c[0], rows, mx, ab16))) continue;
+                        if (c[0] == 192 && ((narrow_pair && rows >= kHalfSectors) || (pair224 && rows == kSectors))) continue;
+                        if (rounds > 1 && cost < best) {
                             best = cost;
                             pl.columns = c[0];
                         }

@@ -133,7 +133,8 @@ int b200_last_tail_split(int32_t* first_tile, int32_t* parts);
  * order, so their results agree to the last bit.  With TILE_AUTO a grid of few tiles with a long K may be computed on 128x128
  * tiles instead, each shared by the CTAs of a cluster that take a part of K (if the inputs are ready, only where the whole tile
  * would be a single CTA's: a pair's starts early): fp32 sums in another order, the same from run to run.  Whether it is depends
- * on the number of tiles, so with TILE_AUTO the last bits of a row can depend on how many rows, columns and batches the call has.
+ * on the number of tiles and on how the operands' rows lie in memory (their pitch and where they begin, modulo 128 bytes), so with
+ * TILE_AUTO the last bits of a row can depend on how many rows, columns and batches the call has, and on views of other operands.
  * A grid of few rounds may be computed on one CTA's tiles of another width (b200_gemm_check_columns): whole tiles, the same bits. */
 int b200_gemm_check(const b200_gemm_args* args, int32_t* chosen_tile);
 /* The other half of that answer: how many CTAs share the K of a tile in this launch.  1: whole tiles of the kind that
