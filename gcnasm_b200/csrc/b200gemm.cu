@@ -279,6 +279,7 @@ int row_starts(const void* base, int64_t pitch, int64_t batch_stride) {
 
 // A grid of one round on `w` columns against a pair's tiles: the K blocks from which the pair is kept.  It takes less out of L2 for a K block, and of what the rows make
 // dear; one CTA has the shorter way in and out.  One CTA / pair, mean over K blocks (100,000 random sizes; * with two rows of tiles):
+//   whole lines    8-bit  192*  0.96 from 16 on, 1.00 at 24 to 31, 1.04 above (245 x 11920 x 6272 21.9 / 20.1), more rows 0.85 to 0.98; 224* 1.00 to 31, 1.02 above, four rows 1.01 from 40
 //   whole sectors  8-bit  160   0.95 at 20;  192 0.92 at 9;  bf16 224 1.00 from 24 on, 160 and 192 0.75 to 0.96
 //   off lines      8-bit  160   0.95 to 24, 1.03 above, 1.09 from 40;  192 1.00 at 12, 1.03 at 20, 1.17 above 40, * 0.96 at 15, 1.05 at 20;  224 1.08 to 1.16 (1794 x 1888 x 7168 28.3 / 22.4)
 //                  bf16   192   0.99 at 35, 1.05 above 40;  224 0.98 at 20, 1.04 at 27, 1.12 above 30;  MX 192 0.97 at 27, 1.02 at 35, 1.06 above 40
@@ -289,7 +290,8 @@ int row_starts(const void* base, int64_t pitch, int64_t batch_stride) {
 //                               12, 1.00 from 15, 1.04 from 21 to 1.20
 int64_t pair_from(int w, int64_t tm, int rows, bool block, bool mx, bool ab16) {
     constexpr int64_t never = int64_t{1} << 62;
-    if (w < 160 || rows == kLines || (block && rows == kOffLines)) return never;
+    if (w < 160 || (block && rows == kOffLines)) return never;
+    if (rows == kLines) return ab16 || mx || block ? never : w == 192 && tm <= 2 ? 28 : w == 224 && tm <= 4 ? (tm <= 2 ? 32 : 40) : never;
     if (ab16) {
         if (rows <= kOffLines) return w == 224 ? 24 : w == 192 && rows == kOffLines ? 40 : never;
         return w == 160 ? (tm <= 2 ? 25 : 36) : w == 192 ? (tm <= 2 ? 15 : 18) : (tm <= 2 ? 10 : 13);
@@ -497,14 +499,14 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 // at 16 to 24, 1.07 above 40), and with block scales, whose 160 and 192 columns take as long as 256 (700 x 8192 x 1024 12.6 / 13.4).  MX: 192 columns
                 // for the pair's 256, up to ten K blocks (0.81 up to three, 0.88 to nine, then 0.97 and above twenty 1.02).
                 // Not for a pair's 224 or 192 where rows begin within sectors (1.00 to 1.06; 2546 x 1304 x 912 10.0 / 9.3, 1352 x 2480 x 1040, two batches, 17.2 / 15.1),
-                // nor for 224 of whole sectors (1.00).
+                // nor for 224 of whole sectors (1.00) or of whole lines in three rounds (1.00).
                 if (pl.splits == 1 && !columns && !block) {
                     constexpr int kWide[2][2] = {{160, 135}, {192, 125}};
                     const bool pair224 = hint == B200_TILE_PAIR_256x224, narrow_pair = pair224 || hint == B200_TILE_PAIR_256x192;
                     for (const auto& c : kWide) {
                         const int64_t rounds = (tm1 * ((a->n + c[0] - 1) / c[0]) * a->batch + sm_count - 1) / sm_count, cost = rounds * 10 * c[0] * c[1];
                         if ((mx && (single || c[0] != 192)) || (!single && kblocks >= pair_from_rounds(c[0], rows, mx, ab16))) continue;
-                        if (c[0] == 192 && ((narrow_pair && rows >= kHalfSectors) || (pair224 && rows == kSectors))) continue;
+                        if (c[0] == 192 && ((narrow_pair && rows >= kHalfSectors) || (pair224 && (rows == kSectors || (rounds > 2 && kblocks >= 10))))) continue;
                         if (rounds > 1 && cost < best) {
                             best = cost;
                             pl.columns = c[0];

@@ -72,6 +72,12 @@ def test_one_operand_or_batch_is_enough(native):
         assert columns(native, "bf16", a) == w
 
 
+# rows at whole lines, 8-bit: 192 and 224 columns of two or four rows of tiles until K is long; 192 in three rounds for a pair's 224 until then, too
+@pytest.mark.parametrize("m,n,w,first", [(250, 14144, 192, 28), (250, 16512, 224, 32), (500, 8224, 224, 40), (600, 5504, 192, None), (2888, 3624, 192, 10), (250, 11712, 160, None)])
+def test_whole_lines_and_a_long_k(native, m, n, w, first):
+    assert [columns(native, "none", laid_out("none", m, n, kb, "lines")) for kb in range(6, 65)] == [w if first is None or kb < first else 0 for kb in range(6, 65)]
+
+
 def placed(x, extra, begin):
     """x's bytes with rows `extra` bytes further apart, in a buffer of NaNs, from `begin` bytes behind a line on"""
     rows, width = x.shape[0], x.shape[1] * x.element_size()
