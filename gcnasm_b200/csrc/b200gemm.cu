@@ -485,12 +485,14 @@ int validate(const b200_gemm_args* a, int sm_count, Plan* plan, bool ab16 = fals
                 const bool block = a->scale_mode == B200_SCALE_BLOCK, single = hint == B200_TILE_128x128 || hint == B200_TILE_128x256;
                 const int columns = one_round_columns(tm1, a->n, a->batch, kblocks, block, mx, !single, rows, ab16, sm_count);
                 // A split takes as long as `equal` K blocks on 128 columns; narrow tiles are worth two more (block scales three), 32 columns one more.
-                // Narrow over split by kblocks - equal, mean of 430 / 990 sizes: 8-bit 0.93 at 1, 0.95 at 2, 0.97 at 3; block scales 0.86, 0.89, 0.92, 0.95 at 4.
+                // Narrow over split by kblocks - equal, mean of 430 / 990 sizes: 8-bit 32 columns 0.92 at 1, 0.94 at 2, 0.96 at 3, from five parts on with up to 112 rows 1.06 at 3
+                // (92 x 448 x 2688 6.2 / 5.8), 64 columns of several rows of tiles for two parts 1.02 at 1 and 2 (2106 x 312 x 4608 11.4 / 9.8); block scales 0.86, 0.89, 0.92, 0.95 at 4.
                 // Rows that begin within sectors: 8-bit 32 columns 0.99 at 1, 1.02 at 2, otherwise to 1.14; block scales 64 columns 0.97, 1.01, 1.01, 32 as above.
                 // Not for few rows, whose sums are quick (2 x 392 x 2816 4.4 / 6.1, block scales 68 x 384 x 2304, two batches, 6.1 / 6.6).
-                int64_t worth = (block ? 4 : 3) + (columns == 32);
+                int64_t worth = (block ? 4 : 3) + (columns == 32 && !(!block && s > 4 && a->m <= 112));
                 if (ab16 || mx || a->m <= 80) worth = 0;
                 else if (!lines) worth = rows != kNoSectors ? 1 : columns != 32 ? (block ? 2 : 1) : block ? worth : 2;
+                else if (!block && columns == 64 && tm1 > 1 && s == 2) worth = 1;
                 if (columns && kblocks - equal < worth) pl.splits = 1;
                 if (pl.splits == 1) pl.columns = columns;
                 // Several rounds without scales: 160 and 192 columns on one CTA, where they waste less of the last round (weights as above; bf16 has no pair tiles

@@ -78,6 +78,14 @@ def test_whole_lines_and_a_long_k(native, m, n, w, first):
     assert [columns(native, "none", laid_out("none", m, n, kb, "lines")) for kb in range(6, 65)] == [w if first is None or kb < first else 0 for kb in range(6, 65)]
 
 
+# K split over CTAs against narrow whole tiles, unscaled: 64 columns of several rows of tiles for two CTAs a tile, 32 of few rows for more than four
+@pytest.mark.parametrize("m,n,k,parts,w", [(2106, 312, 4608, 2, 0), (2106, 312, 4736, 2, 0), (614, 1136, 3584, 1, 64), (92, 448, 2688, 7, 0), (112, 448, 2688, 7, 0), (113, 448, 2688, 1, 32)])
+def test_split_or_narrow(native, m, n, k, parts, w):
+    a, v = laid_out("none", m, n, k // 128, "lines"), C.c_int32(-1)
+    assert native.b200_gemm_check_split(C.byref(a), C.byref(v)) == L.OK and v.value == parts
+    assert columns(native, "none", a) == w
+
+
 def placed(x, extra, begin):
     """x's bytes with rows `extra` bytes further apart, in a buffer of NaNs, from `begin` bytes behind a line on"""
     rows, width = x.shape[0], x.shape[1] * x.element_size()
