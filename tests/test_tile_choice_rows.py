@@ -86,6 +86,14 @@ def test_split_or_narrow(native, m, n, k, parts, w):
     assert columns(native, "none", a) == w
 
 
+# one row of tiles, every other row of the operands within a sector: 96 columns give way to 128 where those have two SMs a tile and K is long
+@pytest.mark.parametrize("m,n,kblocks,w", [(100, 9568, 16, 96), (100, 9568, 17, 128), (100, 9728, 17, 128), (100, 9736, 17, 96)])
+def test_two_sms_a_tile(native, m, n, kblocks, w):
+    assert columns(native, "none", laid_out("none", m, n, kblocks, "half sectors")) == w
+    assert columns(native, "none", laid_out("none", m, n, kblocks, "sectors")) == 96
+    assert columns(native, "none", laid_out("none", m, n, kblocks, "no sectors")) == 96
+
+
 def placed(x, extra, begin):
     """x's bytes with rows `extra` bytes further apart, in a buffer of NaNs, from `begin` bytes behind a line on"""
     rows, width = x.shape[0], x.shape[1] * x.element_size()
