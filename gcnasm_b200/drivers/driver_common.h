@@ -41,6 +41,20 @@ namespace drv {
         }                                                                                         \
     } while (0)
 
+// What a call launches, for the printed line: the --tile value of its tiles, 0 with their columns where none names them (widths that only the
+// automatic choice takes), and the CTAs that share the K of one.
+inline std::string launch_text(const b200_gemm_args& args, bool bf16_operands = false) {
+    int32_t tile = 0, k_split = 0, columns = 0;
+    DRV_B200(bf16_operands ? b200_gemm_a16w16_check(&args, &tile) : b200_gemm_check(&args, &tile));
+    DRV_B200(bf16_operands ? b200_gemm_a16w16_check_split(&args, &k_split) : b200_gemm_check_split(&args, &k_split));
+    DRV_B200(b200_gemm_check_columns(&args, bf16_operands, &columns));
+    if (k_split > 1 || columns == 128) tile = B200_TILE_128x128;
+    else if (columns) tile = B200_TILE_AUTO;
+    std::string text = "tile_config=" + std::to_string(tile) + ", k_split=" + std::to_string(k_split);
+    if (columns && tile == B200_TILE_AUTO) text += ", columns=" + std::to_string(columns);
+    return text;
+}
+
 struct Options {
     int m = 256, n = 512, k = 256, batch = 8;      // the reference defaults (gemm_a8w8_8wave.cc:666-669)
     int verify = 1;

@@ -185,11 +185,8 @@ int main(int argc, char** argv) {
     args.out_dtype = bf16 ? B200_OUT_BF16 : B200_OUT_F32;
     args.tile_hint = o.tile;
 
-    int32_t tile = 0, k_split = 0;
-    DRV_B200(b200_gemm_check(&args, &tile));
-    DRV_B200(b200_gemm_check_split(&args, &k_split));
-    std::printf("Launching GEMM kernel: M=%d, N=%d, K=%d, batch=%d, tile_config=%d, k_split=%d, sms=%d\n", o.m, o.n, o.k, o.batch,
-                k_split > 1 ? B200_TILE_128x128 : tile, k_split, b200_sm_count());
+    std::printf("Launching GEMM kernel: M=%d, N=%d, K=%d, batch=%d, %s, sms=%d\n", o.m, o.n, o.k, o.batch,
+                launch_text(args).c_str(), b200_sm_count());
     DRV_B200(b200_gemm_a8w8(&args, nullptr));
     DRV_CUDA(cudaDeviceSynchronize());
     if (int st = b200_last_status()) {
