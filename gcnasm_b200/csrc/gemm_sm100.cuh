@@ -198,7 +198,8 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int t, int& b, 
 // Store CNT consecutive output columns of one row, 16 bytes at a time where the address allows (vec_ok) and the columns are there.  bf16, element by
 // element wherever one of the CNT columns is missing / by whole pieces, us: 4000 x 4088 x 512 18.7 / 13.7, 100 x 2040 x 1024 9.2 / 7.0, MX 2000 x
 // 2040 x 1024 11.0 / 8.6, bf16 operands 2000 x 4040 x 512 11.6 / 11.15.  fp32 gains nothing by pieces (4000 x 4072 x 512 20.1), and a chunk that is all there
-// has its own branch: both cost few rows their code (3 x 3592 x 256, fp32, 3.0 / 3.25).
+// has its own branch: both cost few rows their code (3 x 3592 x 256, fp32, 3.0 / 3.25).  A chunk that lies behind the last column is left out as a whole: its
+// pieces, all looked at one by one, cost a last tile of few rows 0.6 (bf16 18 x 8512 x 64, four batches, 128 x 256 tiles 4.91 / 4.29; 40 rows 5.06 / 4.63).
 template <int CNT>
 __device__ __forceinline__ void store_row_chunk(const GemmParams& p, void* crow, int col0, const float* v,
                                                 bool vec_ok) {
@@ -216,7 +217,7 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, void* crow,
         if (whole) {
 #pragma unroll
             for (int j = 0; j < CNT; j += 8) piece(j);
-        } else {
+        } else if (!vec_ok || col0 < p.n) {
 #pragma unroll
             for (int j = 0; j < CNT; j += 8) {
                 if (vec_ok && col0 + j + 8 <= p.n) {
