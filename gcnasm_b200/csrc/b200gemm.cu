@@ -247,8 +247,9 @@ constexpr int kSplitClusters[kMaxTileSplits + 1] = {0, 148, 74, 45, 33, 26, 22, 
 // not whole 128-byte lines apart, and up to 47 K blocks where B comes out of L2; with more tiles a whole tile is the slow one.  Whole /
 // split, us, without scales: 4 x 6024 x 5872 15.6 / 19.7, x 8176 23.0 / 29.7, x 5376 with B from HBM 15.9 / 14.5, out of L2 12.0 / 13.9.  Mean
 // of split / whole over 3000 sizes: other pitches 0.98 (0.7 to 1.4), whole lines and 48 K blocks or more 0.84, with B out of L2 0.87.
-// (What had made them slower were the rows of A's box that are not there, see kBoxRows.  Since that box is of the rows that there are two CTAs are the
-// faster ones at these sizes too, 4 x 6024 x 5872 12.1 / 11.1, out of L2 11.3 / 9.4; the line still stands, with the test that holds it.)
+// (What had made them slower were the rows of A's box that are not there, see kBoxRows.  Since that box is of the rows that there are, these calls run on whole tiles of 64
+// columns, and two CTAs a tile would be the faster ones at these sizes too: 4 x 6024 x 5872 11.7 / 10.7, out of L2 11.0 / 9.0, bf16 24 x 6256 x 4088 16.1 / 14.4, 14.6 / 12.9; 146
+// random sizes 0.86 to 0.94, 0.78 to 0.87.  The line is older and test_split_of_few_rows holds it.)
 // *equal: the K blocks that a CTA would take as long for; lines: rows of A and B whole 128-byte lines apart
 int tile_splits(int64_t m, int64_t tiles, int64_t kblocks, bool slow, bool lines, int sm_count, int64_t* equal = nullptr) {
     const int64_t exchange = slow ? 9 + tiles / 32 : (m <= 32 ? 15 : 13) + tiles / 12;
@@ -1028,8 +1029,8 @@ constexpr int kBoxRows = 127;
 int run_gemm(const b200_gemm_args* a, const Plan& pl, DeviceState* ds, cudaStream_t st, bool ab16 = false) {
     int BN = 128;
     bool pair = false;
-    // The plan took the clusters that are resident at once from a table; where this device holds fewer, the tile that the split was
-    // compared with is the better one.
+    // The plan took the clusters that are resident at once from a table; where this device holds fewer, the tile that b200_gemm_check reports is launched whole.
+    // (On 148 SMs, and on any part of them, as many are resident as the table says.)
     int splits = pl.splits;
     if (splits > 1) {
         const int64_t tiles = (a->m + 127) / 128 * ((a->n + 127) / 128) * a->batch;

@@ -3,8 +3,8 @@
 // The reference runs its one 256x256x128 tile for every M (opus_fmm/flatmm_a8w8_gfx950.cc:684-687,
 // out-of-range rows clamped at :268, stores predicated at :537-541); for M <= 64 that wastes the
 // machine, and the job is purely a weight stream.  Here the operands are swapped: a 128(N) x 128(K)
-// weight tile is the UMMA M-side operand and the (zero-padded) token block is the UMMA N-side
-// operand, so D[n][token] lands in TMEM with one weight row per lane.  One CTA owns one 128-row
+// weight tile is the UMMA M-side operand and the block of 16, 32 or 64 tokens (what lies behind the last one
+// is anything) is the UMMA N-side operand, so D[n][token] lands in TMEM with one weight row per lane.  One CTA owns one 128-row
 // weight panel (optionally one K slice of it) and streams it through a deep TMA ring; HBM is the bound.
 //
 // Weights are accepted row-major [N,K] (128-byte swizzled tiles) or in the reference's pre-shuffled

@@ -9,7 +9,8 @@
 //   warp 1      UMMA issuer    (one elected lane)  tcgen05.mma kind::f8f6f4 / kind::mxf8f6f4, TMEM alloc
 //   warp 2      block scales: brings the scales into shared memory beside the operands (up to 192 columns), or reads them into L1 ahead of
 //               their use (256 columns, ScaleToucher)
-//   warp 3      idle, as warp 2 otherwise (register re-allocation works on whole warpgroups)
+//   warp 3      block scales in a grid of one round: asks for the first ring of B ahead of the wait for the predecessor; idle otherwise, as warp 2 is
+//               without block scales (register re-allocation works on whole warpgroups)
 //   warps 4-11  epilogue: TMEM -> registers -> scale -> global
 // TMEM holds two accumulator buffers of BN columns (three or four with block scales and fewer than 192).  Per-tensor / unscaled / MX modes accumulate a
 // whole tile in one buffer while the epilogue drains the other.  Block-scale mode gives every
@@ -17,7 +18,7 @@
 // kernel_template.hpp:317,334) and the epilogue warps fold it into register accumulators with
 // acc += partial * (sfa[g][row] * sfb[nblk][g]) -- the analogue of scale_c_tile.
 // Tiles are 128 rows by 128 or 256 columns, or in a grid of one round by as few as bring all SMs to work (32 to 224, MX 64 or 192, one_round_columns()
-// of the launcher).  Few tiles with a long K: the CTAs of a cluster take a part of a 128 x 128 tile's K each (SPLIT) and sum their results in
+// of the launcher), or without block scales in several rounds by 160 or 192 (MX 192) where those waste less of the last one.  Few tiles with a long K: the CTAs of a cluster take a part of a 128 x 128 tile's K each (SPLIT) and sum their results in
 // distributed shared memory; tile_splits() of the launcher says when.
 #pragma once
 
